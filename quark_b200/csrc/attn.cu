@@ -78,7 +78,10 @@ constexpr int kVRows = 80;  // 64 channels + 16 rows of ones (row sum of P)
 template <bool kFp8>
 struct AttnSmem {
   static constexpr int kEs = kFp8 ? 1 : 2;
-  static constexpr int kStages = kFp8 ? 4 : 3;
+  // Even: tile j sits in stage j % kStages, so a stage then belongs to one group's tiles.  With three stages a group waited
+  // for a phase of a stage whose previous phase the other group watches: where that earlier copy was still on its way, the
+  // parity wait returned at once and the scores came from the stale tile (6 of 100 bf16 calls with key splits at 360p).
+  static constexpr int kStages = 4;
   static constexpr int kQBytes = kQTile * 64 * kEs;          // 16 KB | 8 KB
   static constexpr int kKBytes = kKeyTile * 64 * kEs;        // 16 KB | 8 KB
   static constexpr int kVTile = kVRows * 128;                // one 128-byte-wide V^T tile incl. ones rows: 10 KB
@@ -92,6 +95,7 @@ struct AttnSmem {
   static constexpr int kBarOff = kStageOff + kStages * kStageBytes;
   static constexpr int kTotal = kBarOff + 512 + 1024;
   static_assert(kStages * kStageBytes >= 66 * 128 * 4, "merge buffer aliases the stage area");
+  static_assert(kStages % 2 == 0 && kTotal <= 227 * 1024, "see kStages; shared memory of one CTA");
 };
 
 // 2^x on the FMA and integer pipes, for the share of the exponentials that the special-function unit
