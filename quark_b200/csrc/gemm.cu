@@ -1,29 +1,24 @@
-// C[M,N] = epilogue(A[M,K] . B[N,K]^T) on the sm_100a tensor cores.
+// C[M,N] = epilogue(A[M,K] . B[N,K]^T) on the sm_100a tensor cores: tiles of one CTA (gemm_pair.cu has the tiles of a pair of
+// CTAs that large products use), and the host side of both.
 //
 // One CTA computes one 128 x BN output tile over one K slice.  Warp 0 feeds a ring of
 // shared-memory stages with TMA (128-byte swizzle), one thread of warp 1 issues
 // tcgen05.mma into a TMEM accumulator, warps 2-9 read the accumulator back (one row per thread, two
-// warps per TMEM lane quarter sharing each row's columns) and run the epilogue: 320 threads per CTA.  bf16 operands use kind::f16 (K = 16 per instruction), e4m3
-// operands kind::f8f6f4 (K = 32); both move 128 bytes of K per stage row, so the two paths share
-// every address computation.
+// warps per TMEM lane quarter sharing each row's columns) and run the epilogue: 320 threads per CTA.  bf16 operands use
+// kind::f16 (K = 16 per instruction), e4m3 operands kind::f8f6f4 (K = 32); both move 128 bytes of K per stage row, so the two
+// paths share every address computation.
 //
-// K can be split over `splits` CTAs per tile: each writes its f32 partial tile to the
-// workspace, takes a ticket on the tile's counter, and the CTA that draws the last ticket adds
-// the partials in slice order (so the sum does not depend on which CTA came last), applies the
-// epilogue and stores.  No CTA ever waits for another.
+// K can be split over `splits` CTAs per tile.  As the CTAs of one thread-block cluster they push the rows that other CTAs will
+// finish into those CTAs' shared memory; after one cluster barrier each CTA sums its 128 / splits rows in slice order and runs
+// the epilogue on them.  Through the workspace (any number of slices) each CTA writes its partial tile and takes a ticket, and
+// the CTA that draws the last ticket adds the partials in slice order.  Either way the sum does not depend on which CTA came
+// last, and no CTA waits for another outside its cluster.
 #include <atomic>
 
-#include <cuda.h>
-
-#include "common.cuh"
-#include "rope.cuh"
-#include "sm100.cuh"
+#include "gemm_common.cuh"
 
 namespace qb {
 
-constexpr int kBM = 128;          // rows of A per tile = TMEM lanes
-constexpr int kRowBytes = 128;    // bytes of K per stage row = one swizzle atom
-constexpr int kGemmThreads = 320; // 10 warps: TMA, MMA, 2 x 4 epilogue (two warps per TMEM lane quarter)
 constexpr int kSmemBudget = 200 * 1024;
 
 #ifdef QB_GEMM_TRACE
@@ -34,374 +29,21 @@ __device__ __forceinline__ long long gtime() { long long t; asm volatile("mov.u6
 #define QB_GT(pt) do { } while (0)
 #endif
 
-// What the QKV projection's fused epilogue needs beyond the GEMM: per-head RMS norm of Q and K, value
-// residual on V, RoPE(K) and the KV-cache append happen on the accumulator tile, before anything is
-// written (the stand-alone kernels are in qkv_post.cu and kv.cu; results are bit-identical to them).
-struct QkvTail {
-  const uint16_t* qkv_first;  // may be null: no value residual
-  const float* lamb;
-  const int32_t* frame_t;
-  const int32_t* frozen;
-  void* K_cache;
-  void* Vt_cache;
-  int32_t* segments;
-  int32_t* n_segments;
-  const float* rope_xy;
-  const float* k_scale;  // optional per-KV-head cache scales (see qb_kv_params)
-  const float* v_scale;
-  int n_q_heads, n_kv_heads, tpf, nb, pd, max_segments, kv_fp8;
-  // Quilt: the cache keeps tokens qoff, qoff + quilt, ... of the frame (tpf / quilt of them); slots, capacity and the
-  // segment table are those of a frame of tpf / quilt tokens (src/quark/kernels/kv_cache_update/reference.py:201-207)
-  int quilt, qoff;
-  float eps;
-};
-
-struct GemmArgs {
-  int M, N, K;
-  int kb_total, kb_per_split, splits;
-  int cluster;  // K slices are the CTAs of one thread-block cluster and are summed through distributed shared memory
-  int b_const;  // no kernel still in flight writes B (weights): its first tiles are fetched ahead of the grid dependency
-  int c_dtype, activation, rows_per_gate;
-  const float* a_scale;
-  const float* w_scale;
-  const uint16_t* bias;
-  const uint16_t* gate;
-  const uint16_t* residual;
-  void* C;
-  float* partials;
-  int* counters;
-  unsigned int* status;
-  int qkv_mode;  // the fused QKV epilogue below replaces the plain one (128-column tiles only)
-  QkvTail qkv;
-  // Row-parallel GEMM of a tensor-parallel rank: row m of the bf16 partial goes to the rank that owns that row in the
-  // cross-GPU reduction (m / tp_rpo), into that rank's staging area for partials from this rank (peer-mapped memory,
-  // plain stores over NVLink): tp_dst[owner] + (m % tp_rpo) * N.  tp_world == 0: the ordinary output C.
-  int tp_world, tp_rpo;
-  uint16_t* tp_dst[8];
-  // Grouped GEMM (mixture of experts): the 128-row tile i of A belongs to expert tile_expert[i] and is multiplied with
-  // rows [expert * N, expert * N + N) of B; a tile with expert -1 is skipped.  NULL: the ordinary GEMM.
-  const int* tile_expert;
-};
-
 template <int BN>
 struct GemmSmem {
   static constexpr int kStageBytes = kBM * kRowBytes + BN * kRowBytes;
   static constexpr int kStages = (kSmemBudget / kStageBytes) > 8 ? 8 : (kSmemBudget / kStageBytes);
-  static constexpr int kBarOffset = kStages * kStageBytes;
+  // partial sums that the other K slices of the cluster push, and this CTA's own: 128 / splits rows of f32 from each.  They need
+  // memory of their own, since a slower CTA's stages are in use while its peers push: 64-column tiles only.
+  static constexpr int kSliceBytes = BN == 64 ? kBM * BN * 4 : 0;
+  static constexpr int kSliceOffset = kStages * kStageBytes;
+  static constexpr int kBarOffset = kSliceOffset + kSliceBytes;
   static constexpr int kColOffset = kBarOffset + 256;            // per-column scale, bias, gate of this tile as f32
   static constexpr int kTotal = kColOffset + 3 * BN * 4 + 1024;  // + alignment slack
+  static_assert(kTotal <= 227 * 1024, "shared memory of one CTA");
 };
 
-// Applies the epilogue to 8 consecutive columns of one row and stores them.
-__device__ __forceinline__ void epilogue_store8(const GemmArgs& g, float (&v)[8], int m, int n) {
-  if (g.a_scale != nullptr || g.w_scale != nullptr) {
-    const float sa = g.a_scale ? *g.a_scale : 1.0f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] *= g.w_scale ? sa * __ldg(g.w_scale + n + j) : sa;
-  }
-  if (g.bias != nullptr) {
-    const uint4 b = *reinterpret_cast<const uint4*>(g.bias + n);  // may be the output of the kernel before (MLPFusion)
-    const uint32_t w[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      v[2 * j] += bf16lo(w[j]);
-      v[2 * j + 1] += bf16hi(w[j]);
-    }
-  }
-  if (g.activation == 1) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = silu_fast(v[j]);
-  }
-  if (g.gate != nullptr) {
-    const size_t grow = static_cast<size_t>(m / g.rows_per_gate) * g.N;
-    const uint4 gt = *reinterpret_cast<const uint4*>(g.gate + grow + n);
-    const uint4 rs = *reinterpret_cast<const uint4*>(g.residual + static_cast<size_t>(m) * g.N + n);
-    const uint32_t gw[4] = {gt.x, gt.y, gt.z, gt.w};
-    const uint32_t rw[4] = {rs.x, rs.y, rs.z, rs.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      v[2 * j] = __fadd_rn(bf16lo(rw[j]), __fmul_rn(bf16lo(gw[j]), v[2 * j]));
-      v[2 * j + 1] = __fadd_rn(bf16hi(rw[j]), __fmul_rn(bf16hi(gw[j]), v[2 * j + 1]));
-    }
-  }
-  const size_t off = static_cast<size_t>(m) * g.N + n;
-  if (g.c_dtype == QB_BF16) {
-    uint4 o;
-    o.x = pack_bf16x2(v[0], v[1]);
-    o.y = pack_bf16x2(v[2], v[3]);
-    o.z = pack_bf16x2(v[4], v[5]);
-    o.w = pack_bf16x2(v[6], v[7]);
-    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(g.C) + off) = o;
-  } else if (g.c_dtype == QB_E4M3) {
-    uint2 o;
-    o.x = pack_e4m3x4(v[0], v[1], v[2], v[3]);
-    o.y = pack_e4m3x4(v[4], v[5], v[6], v[7]);
-    *reinterpret_cast<uint2*>(static_cast<uint8_t*>(g.C) + off) = o;
-  } else {
-    float4* dst = reinterpret_cast<float4*>(static_cast<float*>(g.C) + off);
-    dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-    dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-  }
-}
-
-// Thread-block cluster helpers: hardware barrier over all threads of the cluster, and loads from
-// the shared memory of another CTA of the cluster.
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, int cta_rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(cta_rank));
-  return r;
-}
-__device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-
-// ---------------------------------------------------------------- fused epilogue of the QKV projection
-// Tile = 128 tokens x 2 heads (128 columns).  Epilogue warp w owns the 32 tokens of TMEM lane quarter
-// w % 4 and head (w - 2) / 4 of the tile, so every thread holds one whole head of one token: the head's
-// RMS norm, the value residual and the K rotation need no exchange between threads.  Arithmetic, rounding
-// points and summation order are those of qkv_post.cu (and through it of head_rmsnorm, value_residual_packed
-// and kv_cache_update), so the bytes written are the same.  V is transposed through the idle stage memory.
-constexpr int kQkvVPitch = 72;  // 16-bit words per token row of the V staging tile
-
-template <bool kCacheFp8>
-__device__ __forceinline__ void qkv_tail_epilogue(const GemmArgs& g, uint8_t* smem, float* tm, uint64_t* acc_bar, volatile int* abort_flag,
-                                                  uint32_t tmem_base, int warp, int lane, int m0, int n0) {
-  constexpr int kEs = kCacheFp8 ? 1 : 2;
-  const QkvTail& q = g.qkv;
-  const int half = (warp - 2) >> 2, lane_grp = warp & 3;
-  const int row = lane_grp * 32 + lane;
-  const int t = m0 + row;  // token
-  const bool valid = t < g.M;
-  const int et = threadIdx.x - 64;  // 0 .. 255
-  const int col0 = n0 + half * 64;  // first column of this thread's head
-  const int k_off = q.n_q_heads * 64, v_off = (q.n_q_heads + q.n_kv_heads) * 64;
-  const int kind = col0 < k_off ? 0 : col0 < v_off ? 1 : 2;  // Q, K or V head (uniform over the warp)
-  const bool in_n = col0 < g.N;
-  const int ft = *after_wait(q.frame_t);  // written on the device: ordinary loads, after the grid dependency
-  const int frozen = *after_wait(q.frozen);
-  const int tpf_c = q.tpf / q.quilt;  // tokens of a frame that the cache keeps
-  const int L = q.nb * tpf_c;
-  const int cap = L + tpf_c;
-  // this thread's token in the cache: kept iff it is one of the quilt's residue class
-  const bool kept = (t - q.qoff) >= 0 && (t - q.qoff) % q.quilt == 0;
-  const int tc = (t - q.qoff) / q.quilt;
-  const int bucket = (ft + q.pd - 1) / q.pd;
-  const int slot = bucket % q.nb;
-  const bool is_write = (ft % q.pd) == 0;
-  const bool ring = is_write && frozen == 0;
-
-  if (et < 8) temporal_cos_sin(ft, et, tm);
-  if (blockIdx.x == 0 && blockIdx.y == 0 && et == 32) {  // segment table: one thread of the grid
-    int sg[6] = {0, 0, 0, 0, 0, 0};
-    int n;
-    if (is_write && bucket >= q.nb) {
-      sg[1] = slot * tpf_c;
-      sg[2] = (slot + 1) * tpf_c;
-      sg[3] = (q.nb - slot - 1) * tpf_c;
-      sg[4] = L;
-      sg[5] = tpf_c;
-      n = 3;
-    } else {
-      sg[1] = min(bucket, q.nb) * tpf_c;
-      sg[2] = L;
-      sg[3] = tpf_c;
-      n = 2;
-    }
-#pragma unroll
-    for (int i = 0; i < 6; ++i)
-      if (i < 2 * q.max_segments) q.segments[i] = sg[i];
-    for (int i = 6; i < 2 * q.max_segments; ++i) q.segments[i] = 0;
-    q.n_segments[0] = n;
-  }
-  // while the main loop runs: what this thread's head needs from global memory
-  float xy[16];
-  uint32_t vf[32];
-  const bool mix = kind == 2 && q.qkv_first != nullptr;
-  const float lam = mix ? *q.lamb : 0.f;
-  if (kind == 1 && valid && in_n) {
-    const float4* rp = reinterpret_cast<const float4*>(q.rope_xy + static_cast<size_t>(t) * 16);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float4 v = __ldg(rp + i);
-      xy[4 * i] = v.x; xy[4 * i + 1] = v.y; xy[4 * i + 2] = v.z; xy[4 * i + 3] = v.w;
-    }
-  }
-  if (mix && valid && in_n) {
-    const uint4* fp = reinterpret_cast<const uint4*>(q.qkv_first + static_cast<size_t>(t) * g.N + col0);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const uint4 v = fp[i];  // the first block's QKV, written earlier in this pass
-      vf[4 * i] = v.x; vf[4 * i + 1] = v.y; vf[4 * i + 2] = v.z; vf[4 * i + 3] = v.w;
-    }
-  }
-  asm volatile("bar.sync 2, 256;" ::: "memory");  // temporal cos / sin visible
-
-  const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc_bar), 0, abort_flag, g.status, QB_DEV_WAIT_TIMEOUT_GEMM));
-  tc_fence_after();
-  uint16_t* vt = reinterpret_cast<uint16_t*>(smem);  // [2 heads][128 tokens][kQkvVPitch], over the stage memory (idle now)
-  if (ok) {
-    const uint32_t taddr = tmem_base + (static_cast<uint32_t>(lane_grp * 32) << 16) + half * 64;
-    uint32_t r0[32], r1[32];
-    tmem_ld32(taddr, r0);
-    tmem_ld32(taddr + 32, r1);
-    tmem_wait_ld_into(r0);
-    tmem_loaded(r1);
-    // the projection's output as the unfused path would store and re-read it: scaled (acc * (a_scale * w_scale[n]),
-    // as the plain epilogue does) and rounded to bf16
-    float f[64];
-    if (g.a_scale != nullptr || g.w_scale != nullptr) {
-      const float sa = g.a_scale ? *g.a_scale : 1.0f;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float c0 = (g.w_scale && in_n) ? sa * __ldg(g.w_scale + col0 + j) : sa;
-        const float c1 = (g.w_scale && in_n) ? sa * __ldg(g.w_scale + col0 + 32 + j) : sa;
-        r0[j] = __float_as_uint(__uint_as_float(r0[j]) * c0);
-        r1[j] = __float_as_uint(__uint_as_float(r1[j]) * c1);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      f[j] = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r0[j])));
-      f[32 + j] = __bfloat162float(__float2bfloat16_rn(__uint_as_float(r1[j])));
-    }
-    uint32_t o[32];  // the head as it goes to qkv_out: 64 bf16
-    if (kind < 2) {
-      // sum of squares in the order of the 4-lanes-per-head kernel: per 16 elements 8 + 8, then pairs of sixteenths
-      float sq[4];
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        float sa = 0.f, sb = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) sa += f[16 * l + j] * f[16 * l + j];
-#pragma unroll
-        for (int j = 8; j < 16; ++j) sb += f[16 * l + j] * f[16 * l + j];
-        sq[l] = sa + sb;
-      }
-      const float ss = (sq[0] + sq[1]) + (sq[2] + sq[3]);
-      const float inv = 1.0f / sqrtf(ss * (1.0f / 64.0f) + q.eps);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) o[j] = pack_bf16x2(__fmul_rn(f[2 * j], inv), __fmul_rn(f[2 * j + 1], inv));
-    } else if (mix) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float c0 = f[2 * j], c1 = f[2 * j + 1];
-        o[j] = pack_bf16x2(__fadd_rn(c0, __fmul_rn(lam, __fsub_rn(bf16lo(vf[j]), c0))),
-                           __fadd_rn(c1, __fmul_rn(lam, __fsub_rn(bf16hi(vf[j]), c1))));
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) o[j] = pack_bf16x2(f[2 * j], f[2 * j + 1]);
-    }
-    if (valid && in_n) {
-      uint16_t* dst = static_cast<uint16_t*>(g.C) + static_cast<size_t>(t) * g.N + col0;
-#pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const uint32_t w[8] = {o[8 * h], o[8 * h + 1], o[8 * h + 2], o[8 * h + 3], o[8 * h + 4], o[8 * h + 5], o[8 * h + 6], o[8 * h + 7]};
-        st_global_v8(dst + 16 * h, w);
-      }
-    }
-    if (kind == 1 && valid && in_n && kept) {
-      // rotate what the stand-alone append would read back (the bf16-rounded normalised K): y0 = pairs' first
-      // outputs, y1 = their second outputs; a cache row is y0[0..31] followed by y1[0..31]
-      const int head = (col0 - k_off) >> 6;
-      const float inv_k = q.k_scale != nullptr ? __fdiv_rn(1.0f, __ldg(q.k_scale + head)) : 1.0f;  // * 1 changes no bit
-      float y0[32], y1[32];
-#pragma unroll
-      for (int pr = 0; pr < 32; ++pr) {
-        float c, sn;
-        pair_cos_sin(pr, xy, tm, c, sn);
-        const float x0 = bf16lo(o[pr]), x1 = bf16hi(o[pr]);
-        y0[pr] = __fmul_rn(__fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, sn)), inv_k);
-        y1[pr] = __fmul_rn(__fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, sn)), inv_k);
-      }
-      uint8_t* kc = static_cast<uint8_t*>(q.K_cache);
-      const size_t row_bytes = 64 * kEs;
-      uint8_t* tail = kc + (static_cast<size_t>(head) * cap + L + tc) * row_bytes;
-      uint8_t* rr = kc + (static_cast<size_t>(head) * cap + static_cast<size_t>(slot) * tpf_c + tc) * row_bytes;
-      if (kCacheFp8) {
-        uint32_t w0[8], w1[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          w0[j] = pack_e4m3x4(y0[4 * j], y0[4 * j + 1], y0[4 * j + 2], y0[4 * j + 3]);
-          w1[j] = pack_e4m3x4(y1[4 * j], y1[4 * j + 1], y1[4 * j + 2], y1[4 * j + 3]);
-        }
-        st_global_v8(tail, w0);
-        st_global_v8(tail + 32, w1);
-        if (ring) {
-          st_global_v8(rr, w0);
-          st_global_v8(rr + 32, w1);
-        }
-      } else {
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          uint32_t w[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int e = 16 * (h & 1) + 2 * j;  // 16 values per 32-byte store; h < 2: y0, h >= 2: y1
-            w[j] = h < 2 ? pack_bf16x2(y0[e], y0[e + 1]) : pack_bf16x2(y1[e], y1[e + 1]);
-          }
-          st_global_v8(tail + 32 * h, w);
-          if (ring) st_global_v8(rr + 32 * h, w);
-        }
-      }
-    }
-    if (kind == 2) {  // the mixed V head of this token into the staging tile, 16-byte rows of 8 channels
-      uint16_t* vrow = vt + (half * 128 + row) * kQkvVPitch;
-#pragma unroll
-      for (int c8 = 0; c8 < 8; ++c8)
-        *reinterpret_cast<uint4*>(vrow + c8 * 8) = make_uint4(o[4 * c8], o[4 * c8 + 1], o[4 * c8 + 2], o[4 * c8 + 3]);
-    }
-  }
-  asm volatile("bar.sync 2, 256;" ::: "memory");  // V staging complete
-  if (ok) {
-    // transposed 16-byte stores: one channel x (8 | 16) consecutive cached tokens each, for the V heads of this tile.
-    // The tile's cached tokens are its rows qoff, qoff + quilt, ... (m0 is a multiple of the quilt factor).
-    constexpr int kTokPerVec = 16 / kEs;
-    const int cached_rows = 128 / q.quilt;
-    const int vec_per_ch = cached_rows / kTokPerVec;
-    uint8_t* vc = static_cast<uint8_t*>(q.Vt_cache);
-#pragma unroll 1
-    for (int hh = 0; hh < 2; ++hh) {
-      const int hcol = n0 + hh * 64;
-      if (hcol < v_off || hcol >= g.N) continue;
-      const int head = (hcol - v_off) >> 6;
-      const float inv_v = q.v_scale != nullptr ? __fdiv_rn(1.0f, __ldg(q.v_scale + head)) : 1.0f;
-      const uint16_t* src = vt + hh * 128 * kQkvVPitch;
-      for (int v = et; v < 64 * vec_per_ch; v += 256) {
-        const int d = v / vec_per_ch, j = v % vec_per_ch;
-        const int c1 = j * kTokPerVec;                  // first cached token of the vector, inside the tile
-        const int c_abs = m0 / q.quilt + c1;            // ... and inside the frame's cached tokens
-        if (c_abs + kTokPerVec > tpf_c) continue;
-        auto sv = [&](int i) { return src[(q.qoff + (c1 + i) * q.quilt) * kQkvVPitch + d]; };
-        uint32_t w[4];
-        if (kCacheFp8) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            w[i] = pack_e4m3x4(__fmul_rn(bf16_bits_to_f32(sv(4 * i)), inv_v), __fmul_rn(bf16_bits_to_f32(sv(4 * i + 1)), inv_v),
-                               __fmul_rn(bf16_bits_to_f32(sv(4 * i + 2)), inv_v), __fmul_rn(bf16_bits_to_f32(sv(4 * i + 3)), inv_v));
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint16_t lo = sv(2 * i), hi = sv(2 * i + 1);
-            w[i] = q.v_scale != nullptr ? pack_bf16x2(__fmul_rn(bf16_bits_to_f32(lo), inv_v), __fmul_rn(bf16_bits_to_f32(hi), inv_v))
-                                        : static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
-          }
-        }
-        const uint4 ov = make_uint4(w[0], w[1], w[2], w[3]);
-        const size_t ch = (static_cast<size_t>(head) * 64 + d) * cap;
-        *reinterpret_cast<uint4*>(vc + (ch + L + c_abs) * kEs) = ov;
-        if (ring) *reinterpret_cast<uint4*>(vc + (ch + static_cast<size_t>(slot) * tpf_c + c_abs) * kEs) = ov;
-      }
-    }
-  }
-}
-
-template <int BN, bool FP8>
+template <int BN, bool FP8, bool QKV>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs g) {
   using L = GemmSmem<BN>;
@@ -409,8 +51,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   constexpr int kKElems = FP8 ? 128 : 64;  // elements of K per stage
   constexpr uint32_t kTmemCols = BN < 32 ? 32 : BN;
   constexpr uint32_t kIdesc = FP8 ? umma_idesc(0, 0, kBM, BN) : umma_idesc(1, 1, kBM, BN);
-  constexpr int kStgPitch = BN + 4;  // f32 words per staged row: the pad spreads a column of rows over the banks
-  static_assert(kBM * kStgPitch * 4 <= L::kStages * L::kStageBytes, "staging tile must fit in the stage memory");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -439,8 +79,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   const int kb0 = split * g.kb_per_split;
   const int kb1 = min(kb0 + g.kb_per_split, g.kb_total);
   const int n_iter = kb1 - kb0;
-  const bool clustered = g.cluster != 0 && g.splits > 1;
-  const bool use_staging = clustered;  // a single slice goes straight from TMEM to global memory (measured faster)
+  const uint32_t stage_tx = g.a_rows * kRowBytes + BN * kRowBytes;
+  const bool clustered = L::kSliceBytes > 0 && g.cluster != 0;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
@@ -460,7 +100,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  if (clustered) cluster_sync();  // every CTA of the cluster is there before anyone pushes to it
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   grid_dep_launch();  // set-up is done: the next kernel in the stream may begin its own
@@ -474,7 +115,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const int ahead = g.b_const ? min(kStages, n_iter) : 0;
       for (int it = 0; it < ahead; ++it) {
         const uint32_t fb = smem_u32(&full_bar[it]);
-        mbar_arrive_expect_tx(fb, L::kStageBytes);
+        mbar_arrive_expect_tx(fb, stage_tx);
         tma_load_2d(smem_u32(smem + it * L::kStageBytes + kBM * kRowBytes), &tmB, fb, (kb0 + it) * kKElems, b_row0 + n0);
       }
       grid_dep_wait();
@@ -487,7 +128,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const uint32_t ph = (it / kStages) & 1;
         if (!mbar_wait(smem_u32(&empty_bar[s]), ph ^ 1, abort_flag, g.status, QB_DEV_WAIT_TIMEOUT_GEMM)) break;
         const uint32_t fb = smem_u32(&full_bar[s]);
-        mbar_arrive_expect_tx(fb, L::kStageBytes);
+        mbar_arrive_expect_tx(fb, stage_tx);
         uint8_t* a_s = smem + s * L::kStageBytes;
         tma_load_2d(smem_u32(a_s), &tmA, fb, (kb0 + it) * kKElems, m0);
         tma_load_2d(smem_u32(a_s + kBM * kRowBytes), &tmB, fb, (kb0 + it) * kKElems, b_row0 + n0);
@@ -537,21 +178,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const int row = lane_grp * 32 + lane;
     const int m = m0 + row;
     grid_dep_wait();  // bias / gate / residual are read and C is written only after the earlier kernels are done
-    bool qkv_done = false;
-    if constexpr (BN == 128) {
-      if (g.qkv_mode) {
-        float* tm = reinterpret_cast<float*>(smem + L::kColOffset);
-        if (g.qkv.kv_fp8)
-          qkv_tail_epilogue<true>(g, smem, tm, acc_bar, abort_flag, tmem_base, warp, lane, m0, n0);
-        else
-          qkv_tail_epilogue<false>(g, smem, tm, acc_bar, abort_flag, tmem_base, warp, lane, m0, n0);
-        qkv_done = true;
-      }
-    }
     // The fast epilogue needs whole 32-column chunks inside N, 32-byte aligned rows of C, and one gate row
     // for the whole tile; anything else takes the general path below.
     const int m_last = min(m0 + kBM, g.M) - 1;
-    const bool fast = !qkv_done && g.splits == 1 && g.N % 32 == 0 && (reinterpret_cast<uintptr_t>(g.C) & 31u) == 0 &&
+    const bool fast = !QKV && g.splits == 1 && g.N % 32 == 0 && (reinterpret_cast<uintptr_t>(g.C) & 31u) == 0 &&
                       (g.gate == nullptr || m0 / g.rows_per_gate == m_last / g.rows_per_gate);
     // Two warps share each TMEM lane quarter (w and w + 4 see the same 32 rows): in the fast epilogue the
     // first takes the even 32-column chunks of the row, the second the odd ones.  The other epilogue paths
@@ -560,6 +190,40 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     constexpr int kMyChunks = BN / 64;  // 32-column chunks per warp
     constexpr int kResInRegs = BN <= 128 ? 1 : 0;
     uint32_t res[kResInRegs ? kMyChunks * 16 : 1];
+    const int slice_rows = kBM / (clustered ? g.splits : 1), slice_row0 = clustered ? split * slice_rows : 0;  // rows this CTA finishes
+    const bool one_gate = g.gate == nullptr || m0 / g.rows_per_gate == m_last / g.rows_per_gate;
+    uint4 pre[QKV || BN == 64 ? BN / 32 : 1][2];  // QKV: see qkv_prefetch; slices: the residuals of the 8-column groups this thread finishes
+    if (QKV || (clustered && one_gate)) {
+      float* col = reinterpret_cast<float*>(smem + L::kColOffset);
+      const int et = threadIdx.x - 64;
+      const float sa = g.a_scale ? *g.a_scale : 1.0f;
+      const size_t grow = g.gate ? static_cast<size_t>(m0 / g.rows_per_gate) * g.N : 0;
+      for (int j = et; j < BN; j += 256) {
+        const int n = n0 + j;
+        const bool in = n < g.N;
+        col[j] = (in && g.w_scale) ? sa * __ldg(g.w_scale + n) : sa;
+        if (!QKV) {
+          col[BN + j] = (in && g.bias) ? bf16_bits_to_f32(g.bias[n]) : 0.f;
+          col[2 * BN + j] = (in && g.gate) ? bf16_bits_to_f32(g.gate[grow + n]) : 0.f;
+        }
+      }
+      if constexpr (QKV) {
+        const QkvFrame fr = qkv_frame(g.qkv);
+        if (et < 8) temporal_cos_sin(fr.ft, et, col + BN);
+        if (blockIdx.x == 0 && blockIdx.y == 0 && split == 0 && et == 32) qkv_segments(g.qkv, fr);
+        qkv_prefetch<BN>(g, et, slice_row0, slice_rows, m0, n0, pre);
+      } else if constexpr (BN == 64) {
+        if (g.gate != nullptr) {
+#pragma unroll
+          for (int k = 0; k < BN / 32; ++k) {
+            const int r = et / (BN / 8) + 256 / (BN / 8) * k, mm = m0 + slice_row0 + r, n = n0 + et % (BN / 8) * 8;
+            pre[k][0] = make_uint4(0u, 0u, 0u, 0u);
+            if (r < slice_rows && mm < g.M && n < g.N) pre[k][0] = *reinterpret_cast<const uint4*>(g.residual + static_cast<size_t>(mm) * g.N + n);
+          }
+        }
+      }
+      asm volatile("bar.sync 2, 256;" ::: "memory");
+    }
     if (fast) {
       // while the main loop runs: per-column vectors of this tile to shared memory, this row's residual to registers
       float* col = reinterpret_cast<float*>(smem + L::kColOffset);
@@ -587,7 +251,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       }
       asm volatile("bar.sync 2, 256;" ::: "memory");
     }
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc_bar), 0, abort_flag, g.status, QB_DEV_WAIT_TIMEOUT_GEMM));
+    bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc_bar), 0, abort_flag, g.status, QB_DEV_WAIT_TIMEOUT_GEMM));
+    if (!fast) ok = all_of_epilogue(ok);  // the paths below meet at barriers: the 256 threads take the same one
     if (threadIdx.x == 64) QB_GT(5);
     tc_fence_after();
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(lane_grp * 32) << 16);
@@ -673,7 +338,50 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
       }
-    } else if (half == 1 || qkv_done) {
+    } else if (QKV) {
+      if constexpr (QKV) {
+        float* col = reinterpret_cast<float*>(smem + L::kColOffset);
+        uint16_t* vt = reinterpret_cast<uint16_t*>(smem);  // over the stage memory (this CTA's MMAs are done)
+        if (clustered) {
+          if (ok) push_slices<1, BN>(smem + L::kSliceOffset, taddr, split, 0, row, half, g.splits);
+          cluster_sync();  // warps 0 and 1 join it below
+        } else if (ok) {  // scaled (acc * (a_scale * w_scale[n])) and rounded to bf16, as the plain epilogue would store it
+          const bool has_scale = g.a_scale != nullptr || g.w_scale != nullptr;
+#pragma unroll 1
+          for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
+            uint32_t r[32];
+            tmem_ld32(taddr + c * 32, r);
+            tmem_wait_ld_into(r);
+            uint32_t w[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              float a = __uint_as_float(r[2 * j]), b = __uint_as_float(r[2 * j + 1]);
+              if (has_scale) {
+                a *= col[c * 32 + 2 * j];
+                b *= col[c * 32 + 2 * j + 1];
+              }
+              w[j] = pack_bf16x2(a, b);
+            }
+            uint4* dst = reinterpret_cast<uint4*>(vt + row * (BN + 8) + c * 32);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) dst[v] = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+          }
+          asm volatile("bar.sync 2, 256;" ::: "memory");
+        }
+        if (ok) {
+          const float4* parts = reinterpret_cast<const float4*>(smem + L::kSliceOffset);
+          if (g.qkv.kv_fp8) qkv_finish<BN, true>(g, parts, vt, col, col + BN, clustered ? g.splits : 1, slice_row0, slice_rows, m0, n0, pre);
+          else qkv_finish<BN, false>(g, parts, vt, col, col + BN, clustered ? g.splits : 1, slice_row0, slice_rows, m0, n0, pre);
+        }
+      }
+    } else if (clustered) {
+      if constexpr (BN == 64 && !QKV) {
+        if (ok) push_slices<1, BN>(smem + L::kSliceOffset, taddr, split, 0, row, half, g.splits);
+        cluster_sync();  // every slice's share of this CTA's rows has arrived after this barrier (warps 0 and 1 join it below)
+        if (ok) finish_slices<BN>(g, reinterpret_cast<const float4*>(smem + L::kSliceOffset), reinterpret_cast<const float*>(smem + L::kColOffset), m0, n0,
+                                  slice_row0, slice_rows, one_gate, pre);
+      }
+    } else if (half == 1) {
       // the general paths below are written for the first four epilogue warps
     } else if (ok && g.splits == 1) {
 #pragma unroll 1
@@ -693,19 +401,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             }
           }
         }
-      }
-    } else if (ok && use_staging) {
-      // accumulator row -> staging tile in the (now idle) stage memory, f32, padded pitch: one row per thread
-      float* dst = reinterpret_cast<float*>(smem) + static_cast<size_t>(row) * kStgPitch;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld32(taddr + c * 32, r);
-        tmem_wait_ld_into(r);
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          *reinterpret_cast<float4*>(dst + c * 32 + q * 4) = make_float4(__uint_as_float(r[q * 4]), __uint_as_float(r[q * 4 + 1]),
-                                                                        __uint_as_float(r[q * 4 + 2]), __uint_as_float(r[q * 4 + 3]));
       }
     } else if (ok) {
       // K slices through the global workspace: partial tile out, ticket, last CTA adds the slices in order
@@ -756,48 +451,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
   }
 
-  // ---------------- epilogue, part 2: every staged tile of the cluster is complete after this barrier
   tc_fence_before();
-  if (clustered) {
-    cluster_sync();
-  } else {
-    __syncthreads();
+  if (clustered && warp < 2) {
+    __syncwarp();
+    cluster_sync();  // the barrier after which the epilogue warps read what was pushed to them
   }
-  if (use_staging && warp >= 2 && warp < 6 && *abort_flag == 0) {
-    // Rows are dealt out to the CTAs of the cluster; each sums its rows over all slices, in slice order,
-    // reading the peers' staging tiles through distributed shared memory.  Consecutive threads take
-    // consecutive groups of 8 columns, so global loads and stores are coalesced.
-    const int n_slices = clustered ? g.splits : 1;
-    const int rows_per_cta = kBM / n_slices;
-    const int row_begin = clustered ? split * rows_per_cta : 0;
-    const uint32_t stg_base = smem_u32(smem);
-    const int et = threadIdx.x - 64;  // 0..127
-#pragma unroll 1
-    for (int i8 = et; i8 < rows_per_cta * (BN / 8); i8 += 128) {
-      const int rr = row_begin + i8 / (BN / 8);
-      const int c8 = (i8 % (BN / 8)) * 8;
-      const int mm = m0 + rr, n = n0 + c8;
-      if (mm >= g.M || n >= g.N) continue;
-      const uint32_t local = stg_base + (static_cast<uint32_t>(rr) * kStgPitch + c8) * 4u;
-      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      if (clustered) {
-        for (int s = 0; s < n_slices; ++s) {
-          const uint32_t remote = map_to_cta(local, s);
-          const float4 x = ld_dsmem_f4(remote), y = ld_dsmem_f4(remote + 16);
-          v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-          v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
-        }
-      } else {
-        const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem) + static_cast<size_t>(rr) * kStgPitch + c8);
-        const float4 x = src[0], y = src[1];
-        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-        v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
-      }
-      epilogue_store8(g, v, mm, n);
-    }
-  }
-  if (clustered) cluster_sync();  // nobody leaves while a peer may still read its staging tile
-
   __syncthreads();
   if (threadIdx.x == 0) QB_GT(6);
   if (warp == 1) {
@@ -854,26 +512,26 @@ static int32_t make_tmap_2d(CUtensorMap* tm, const void* base, int elem_bytes, u
 // call with more tiles expects to find zero).
 constexpr size_t kCounterBytes = 64u << 10;  // 16384 tiles
 
-struct GemmPlan {
-  int bn, splits, kb_total, kb_per_split;
-  int cluster;  // slices summed inside a thread-block cluster (2, 4 or 8 slices) instead of through the workspace
-  size_t counters_bytes, aq_bytes, partial_bytes;
-};
-
-static int num_sms() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-      n = 148;
-  }
+int num_sms() {
+  static const int n = [] {
+    int v = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+    return v;
+  }();
   return n;
 }
 
-// Picks the tile width and the number of K slices from a small cost model (cycles per CTA:
-// the slower of tensor-core issue and operand delivery per 128 bytes of K, plus fixed costs),
-// so that every call with the same shape makes the same choice.
-static GemmPlan plan_gemm(const qb_gemm_params& p) {
+#ifdef QB_GEMM_TUNE
+static int g_tune[3] = {0, 0, 0};  // cg, bn, splits; 0 = choose
+extern "C" void qb_debug_gemm_tune(int cg, int bn, int s) { g_tune[0] = cg; g_tune[1] = bn; g_tune[2] = s; }
+#endif
+
+// Whether `s` K slices of a tile can be summed inside a cluster (of at most 8 CTAs): the widths whose partial sums have room.
+static bool cluster_slices(int cg, int bn, int s) { return cg == 1 ? bn == 64 && (s == 2 || s == 4 || s == 8) : bn == 128 && s == 2; }
+
+// Picks the CTAs per tile, the tile width and the number of K slices from a small cost model in ns, so that every call with the
+// same shape makes the same choice.  `grouped`: 128-row tiles belong to different experts, so no pairs and no slices.
+static GemmPlan plan_gemm(const qb_gemm_params& p, bool grouped = false, int max_cg = 2, double* cost_out = nullptr) {
   const bool fp8 = p.compute_dtype == QB_E4M3;
   const int k_elems = fp8 ? 128 : 64;
   GemmPlan best{};
@@ -882,50 +540,57 @@ static GemmPlan plan_gemm(const qb_gemm_params& p) {
   const int kb_total = (p.K + k_elems - 1) / k_elems;
   const int bns[3] = {256, 128, 64};
   const int ss[10] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16};
-  for (int bn : bns) {
-    if (p.tile_n != 0 && p.tile_n != bn) continue;
-    if (p.tile_n == 0 && bn > 64 && bn / 2 >= p.N) continue;  // tile mostly empty
-    const int tiles = ((p.M + kBM - 1) / kBM) * ((p.N + bn - 1) / bn);
-    for (int s : ss) {
-      if (p.split_k != 0 && p.split_k != s) continue;
-      if (s > kb_total) continue;
-      const int kbps = (kb_total + s - 1) / s;
-      const int s_eff = (kb_total + kbps - 1) / kbps;
-      if (s_eff != s) continue;
-      const long ctas = static_cast<long>(tiles) * s;
-      const long waves = (ctas + sms - 1) / sms;
-      // Cycles per 128 bytes of K: the slower of what one SM can take in (150 + 2.3 BN, fitted at M = 128 where
-      // few CTAs run) and its share of the L2's aggregate delivery when a whole wave pulls at once (about
-      // 9000 bytes per clock over the chip: 19 TB/s measured at M = 512).  Fixed cost: launch, set-up, first
-      // tile, epilogue (2.8 us at BN = 64).  K slices add the staging, the cluster barrier and the reduction
-      // through distributed shared memory (3.5 - 5.7 us measured for 2 - 4 slices), or the far slower trip
-      // through the workspace (12 - 14 us), so slices pay only when they multiply the number of busy SMs or
-      // K is long.  Measured at M = 128, bf16, 2048 x 8192: 22 us in one slice, 12 us in 4 cluster slices.
-      const long in_wave = ctas < sms ? ctas : sms;
-      const double stage_bytes = 128.0 * (kBM + bn);
-      const double per_sm = 150.0 + 2.3 * bn, shared = in_wave * stage_bytes / 9000.0;
-      const double per_kb = per_sm > shared ? per_sm : shared;
-      double cta = kbps * per_kb + 5000.0 + bn * 12.0;
-      const bool cl = (p.reserved & 1) == 0 && (s == 2 || s == 4 || s == 8);
-      if (s > 1 && !cl && static_cast<size_t>(tiles) * sizeof(int) > kCounterBytes) continue;  // more tiles than counters
-      if (s > 1) cta += cl ? 7500.0 + bn * 20.0 + s * bn * 4.0 : 26000.0;
-      const double cost = waves * cta;
-      if (cost < best_cost) {
-        best_cost = cost;
-        best.bn = bn;
-        best.splits = s;
-        best.kb_total = kb_total;
-        best.kb_per_split = kbps;
-        best.cluster = (s > 1 && cl) ? 1 : 0;
+  for (int cg = 1; cg <= max_cg; ++cg) {
+    if (cg == 2 && (grouped || p.M <= kBM || (p.reserved & 1) != 0)) continue;
+    for (int bn : bns) {
+      if (p.tile_n != 0 && p.tile_n != bn) continue;
+      if (cg == 2 && bn == 64) continue;
+      if (p.tile_n == 0 && bn > 64 && bn / 2 >= p.N) continue;  // tile mostly empty
+      const int tiles = ((p.M + cg * kBM - 1) / (cg * kBM)) * ((p.N + bn - 1) / bn);
+      for (int s : ss) {
+        if (p.split_k != 0 && p.split_k != s) continue;
+        if (s > kb_total || (grouped && s > 1)) continue;
+#ifdef QB_GEMM_TUNE
+        if ((g_tune[0] && g_tune[0] != cg) || (g_tune[1] && g_tune[1] != bn) || (g_tune[2] && g_tune[2] != s)) continue;
+#endif
+        const int kbps = (kb_total + s - 1) / s;
+        if ((kb_total + kbps - 1) / kbps != s) continue;
+        const bool cl = s > 1 && (p.reserved & 1) == 0 && cluster_slices(cg, bn, s);
+        if (s > 1 && p.split_k == 0 && kbps < 4) continue;  // too little K to share
+        if (s > 1 && !cl && (cg == 2 || static_cast<size_t>(tiles) * sizeof(int) > kCounterBytes)) continue;  // more tiles than counters
+        // Measured with 128 CTAs, e4m3 and bf16 alike: ns per 128 bytes of K, and the rest of a launch that waits for the one
+        // before it.  Tiles run in rounds over the SMs; a pair's CTAs stay for all rounds and hide all epilogues but the last.
+        // Slices add their exchange: through the cluster it grows with the CTAs that push at once (16 CTAs 0.4 us, 128 CTAs
+        // 1.3 - 2.5 us), the trip through the workspace is far slower.
+        const double per_kb = cg == 1 ? (bn == 64 ? 143.0 : bn == 128 ? 190.0 : 390.0) : (bn == 128 ? 155.0 : 290.0);
+        const double fixed = cg == 1 ? (bn == 64 ? 3150.0 : bn == 128 ? 3600.0 : 3400.0) : (bn == 128 ? 5200.0 : 5500.0);
+        const double tail = cg == 1 ? 2200.0 + 7.0 * bn : bn == 128 ? 3200.0 : 4500.0;
+        const long units = static_cast<long>(tiles) * (cl ? 1 : s);
+        const long slots = cl && s == 4 ? 33 : cl && s == 8 ? 15 : sms / (cg * (cl ? s : 1));  // clusters that run at once
+        const long rounds = (units + slots - 1) / slots;
+        const double body = kbps * per_kb;
+        double cost = fixed + body + (rounds - 1) * (cg == 1 ? body + tail : body > tail ? body : tail);
+        if (s > 1) cost += cg == 2 ? 4000.0 : cl ? 300.0 + 12.0 * tiles * s : 9000.0;
+        if (cost < best_cost) {
+          best_cost = cost;
+          best.cg = cg;
+          best.bn = bn;
+          best.splits = s;
+          best.kb_total = kb_total;
+          best.kb_per_split = kbps;
+          best.cluster = cl ? 1 : 0;
+        }
       }
     }
   }
   if (best.bn == 0) {  // forced values that fit nothing: fall back to the plain configuration
+    best.cg = 1;
     best.bn = p.tile_n ? p.tile_n : 128;
     best.splits = 1;
     best.kb_total = kb_total;
     best.kb_per_split = kb_total;
   }
+  if (cost_out != nullptr) *cost_out = best_cost;
   best.counters_bytes = kCounterBytes;
   best.aq_bytes = (fp8 && p.a_dtype == QB_BF16) ? round_up(static_cast<size_t>(p.M) * p.K, 1024) : 0;
   best.partial_bytes = (best.splits > 1 && !best.cluster) ? static_cast<size_t>(best.splits) * p.M * p.N * sizeof(float) : 0;
@@ -952,11 +617,17 @@ static int32_t validate_gemm(const qb_gemm_params* p) {
   return QB_OK;
 }
 
-template <int BN, bool FP8>
+template <int BN, bool FP8, bool QKV>
 static int32_t launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& args, dim3 grid, cudaStream_t st) {
   using L = GemmSmem<BN>;
-  QB_CUDA_OK(cudaFuncSetAttribute(gemm_kernel<BN, FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-  if (args.cluster && args.splits > 1) {
+  static std::atomic<unsigned long long> configured{0};  // one bit per device
+  int dev = 0;
+  QB_CUDA_OK(cudaGetDevice(&dev));
+  if (dev >= 64 || (configured.load(std::memory_order_relaxed) >> dev & 1) == 0) {
+    QB_CUDA_OK(cudaFuncSetAttribute(gemm_kernel<BN, FP8, QKV>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
+    if (dev < 64) configured.fetch_or(1ull << dev, std::memory_order_relaxed);
+  }
+  if (args.cluster) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kGemmThreads);
@@ -971,12 +642,20 @@ static int32_t launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_dependent_launch ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_kernel<BN, FP8>, tmA, tmB, args);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_kernel<BN, FP8, QKV>, tmA, tmB, args);
     ++g_launch_count;
     if (e != cudaSuccess) return fail(QB_ERR_LAUNCH, "gemm kernel (cluster of %d): %s", args.splits, cudaGetErrorString(e));
     return QB_OK;
   }
-  return launch_dep("gemm kernel", gemm_kernel<BN, FP8>, grid, dim3(kGemmThreads), L::kTotal, st, tmA, tmB, args);
+  return launch_dep("gemm kernel", gemm_kernel<BN, FP8, QKV>, grid, dim3(kGemmThreads), L::kTotal, st, tmA, tmB, args);
+}
+
+template <bool FP8>
+static int32_t launch_gemm(int bn, bool qkv, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& g, dim3 grid, cudaStream_t st) {
+  if (qkv) return bn == 128 ? launch_gemm<128, FP8, true>(tmA, tmB, g, grid, st) : launch_gemm<64, FP8, true>(tmA, tmB, g, grid, st);
+  if (bn == 256) return launch_gemm<256, FP8, false>(tmA, tmB, g, grid, st);
+  if (bn == 128) return launch_gemm<128, FP8, false>(tmA, tmB, g, grid, st);
+  return launch_gemm<64, FP8, false>(tmA, tmB, g, grid, st);
 }
 
 int32_t quantize_e4m3_launch(const void* X, void* out, size_t n, int32_t src_dtype, cudaStream_t st);
@@ -988,6 +667,13 @@ using namespace qb;
 #ifdef QB_GEMM_TRACE
 extern "C" int32_t qb_debug_gemm_trace(void* host_out) {
   return cudaMemcpyFromSymbol(host_out, qb::g_gemm_trace, sizeof(qb::g_gemm_trace)) == cudaSuccess ? 0 : -1;
+}
+#endif
+
+#ifdef QB_GEMM_TUNE
+extern "C" int32_t qb_debug_gemm_plan(const qb_gemm_params* p) {
+  const GemmPlan pl = plan_gemm(*p);
+  return pl.cg * 1000000 + pl.bn * 1000 + pl.splits * 10 + pl.cluster;
 }
 #endif
 
@@ -1005,6 +691,28 @@ struct TpDest {
   uint16_t* dst[8];
 };
 
+// The QKV projection with its fused epilogue: tiles of one or two heads of one CTA, and the K slices that the plain projection
+// would have with 64-column tiles, as long as whole 16-byte vectors of cached V tokens lie in the 128 / S rows that a CTA finishes.
+static GemmPlan plan_qkv(const qb_gemm_params& p, const QkvTail& t) {
+  qb_gemm_params q = p;
+  GemmPlan best{};
+  double best_cost = 1e30;
+  for (int bn = 64; bn <= 128; bn += 64) {
+    for (int s = 1; s <= (bn == 64 ? 4 : 1); s *= 2) {
+      if (s > 1 && (kBM / s % t.quilt != 0 || kBM / s / t.quilt < (t.kv_fp8 ? 16 : 8))) continue;
+      q.tile_n = bn;
+      q.split_k = s;
+      double cost = 0;
+      const GemmPlan pl = plan_gemm(q, false, 1, &cost);
+      if (pl.splits == s && pl.cluster == (s > 1) && cost < best_cost) {
+        best_cost = cost;
+        best = pl;
+      }
+    }
+  }
+  return best;
+}
+
 static int32_t gemm_run(const void* A, const void* B, void* C, const void* bias, const void* gate, const void* residual,
                         const qb_gemm_params* p, void* workspace, size_t workspace_bytes, void* stream, const QkvTail* tail,
                         bool clear_counters = false, const TpDest* tp = nullptr, const int* tile_expert = nullptr, int n_experts = 1) {
@@ -1020,7 +728,8 @@ static int32_t gemm_run(const void* A, const void* B, void* C, const void* bias,
                p->gate_groups, p->M);
     rows_per_gate = p->M / p->gate_groups;
   }
-  const GemmPlan pl = plan_gemm(*p);
+  GemmPlan pl = plan_gemm(*p, tile_expert != nullptr, tp != nullptr ? 1 : 2);
+  if (tail != nullptr) pl = plan_qkv(*p, *tail);
   const size_t need = pl.counters_bytes + pl.aq_bytes + pl.partial_bytes;
   const bool uses_ws = pl.aq_bytes > 0 || pl.partial_bytes > 0;
   if (uses_ws) {
@@ -1033,7 +742,6 @@ static int32_t gemm_run(const void* A, const void* B, void* C, const void* bias,
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   unsigned int* status = status_word();
   QB_REQUIRE(status != nullptr, QB_ERR_CUDA, "gemm: device status word unavailable");
-  if (tail != nullptr) QB_REQUIRE(pl.bn == 128 && pl.splits == 1, QB_ERR_INVALID_ARG, "gemm_qkv_post: needs 128-column tiles and one K slice");
   if (clear_counters && pl.partial_bytes > 0) QB_CUDA_OK(cudaMemsetAsync(ws, 0, pl.counters_bytes, st));
   const void* a_ptr = A;
   if (pl.aq_bytes > 0) {
@@ -1042,15 +750,9 @@ static int32_t gemm_run(const void* A, const void* B, void* C, const void* bias,
     if (rc != QB_OK) return rc;
     a_ptr = aq;
   }
-  CUtensorMap tmA, tmB;
-  const int es = fp8 ? 1 : 2;
-  rc = make_tmap_2d(&tmA, a_ptr, es, p->M, p->K, kBM);
-  if (rc != QB_OK) return rc;
-  rc = make_tmap_2d(&tmB, B, es, static_cast<uint64_t>(p->N) * n_experts, p->K, pl.bn);
-  if (rc != QB_OK) return rc;
-
   GemmArgs g{};
   g.M = p->M; g.N = p->N; g.K = p->K;
+  g.a_rows = p->M < kBM ? (p->M + 7) / 8 * 8 : kBM;
   g.kb_total = pl.kb_total; g.kb_per_split = pl.kb_per_split; g.splits = pl.splits;
   g.cluster = pl.cluster;
   g.b_const = (p->reserved & 2) != 0;
@@ -1072,7 +774,6 @@ static int32_t gemm_run(const void* A, const void* B, void* C, const void* bias,
     for (int r = 0; r < tp->world; ++r) g.tp_dst[r] = tp->dst[r];
   }
   if (tail != nullptr) {
-    g.qkv_mode = 1;
     g.qkv = *tail;
   }
   if (tile_expert != nullptr) {
@@ -1084,15 +785,16 @@ static int32_t gemm_run(const void* A, const void* B, void* C, const void* bias,
     g.tile_expert = tile_expert;
   }
 
+  if (pl.cg == 2) return launch_gemm_pair(pl, a_ptr, B, g, fp8, st);
+  CUtensorMap tmA, tmB;
+  const int es = fp8 ? 1 : 2;
+  rc = make_tmap_2d(&tmA, a_ptr, es, p->M, p->K, g.a_rows);
+  if (rc != QB_OK) return rc;
+  rc = make_tmap_2d(&tmB, B, es, static_cast<uint64_t>(p->N) * n_experts, p->K, pl.bn);
+  if (rc != QB_OK) return rc;
+
   dim3 grid((p->N + pl.bn - 1) / pl.bn, (p->M + kBM - 1) / kBM, pl.splits);
-  if (fp8) {
-    if (pl.bn == 256) return launch_gemm<256, true>(tmA, tmB, g, grid, st);
-    if (pl.bn == 128) return launch_gemm<128, true>(tmA, tmB, g, grid, st);
-    return launch_gemm<64, true>(tmA, tmB, g, grid, st);
-  }
-  if (pl.bn == 256) return launch_gemm<256, false>(tmA, tmB, g, grid, st);
-  if (pl.bn == 128) return launch_gemm<128, false>(tmA, tmB, g, grid, st);
-  return launch_gemm<64, false>(tmA, tmB, g, grid, st);
+  return fp8 ? launch_gemm<true>(pl.bn, tail != nullptr, tmA, tmB, g, grid, st) : launch_gemm<false>(pl.bn, tail != nullptr, tmA, tmB, g, grid, st);
 }
 
 extern "C" int32_t qb_gemm(const void* A, const void* B, void* C, const void* bias, const void* gate, const void* residual,
@@ -1132,8 +834,7 @@ extern "C" int32_t qb_gemm_qkv_post(const void* A, const void* B, void* qkv_out,
                  aligned16(qkv_first) && aligned16(rope_xy),
              QB_ERR_ALIGN, "gemm_qkv_post: qkv_out and K_cache must be 32-byte aligned, the other pointers 16-byte aligned");
   qb_gemm_params p = *gp;
-  p.tile_n = 128;
-  p.split_k = 1;
+  p.tile_n = p.split_k = 0;
   QkvTail t{};
   t.qkv_first = static_cast<const uint16_t*>(qkv_first);
   t.lamb = lamb; t.frame_t = frame_t; t.frozen = frozen;

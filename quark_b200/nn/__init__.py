@@ -233,9 +233,10 @@ class MoE(Module):
         h = _cached(self, "h", (M, H), "bf16")
         partials = _cached(self, "partials", (E * M, D), "f32")
         for e in range(E):
-            qf.gemm(xq, self.expert_in.data.rows(e * H, (e + 1) * H), compute_dtype=cd, activation="silu", out=h, b_constant=True)
+            # one K slice, as the grouped GEMMs have: both schedules give the same bits
+            qf.gemm(xq, self.expert_in.data.rows(e * H, (e + 1) * H), compute_dtype=cd, activation="silu", out=h, split_k=1, b_constant=True)
             qf.gemm(h, self.expert_out.data.rows(e * D, (e + 1) * D), out_dtype="f32", compute_dtype=cd, out=partials.rows(e * M, (e + 1) * M),
-                    b_constant=True)  # fmt: skip
+                    split_k=1, b_constant=True)  # fmt: skip
         return qf.moe_combine(partials, weights, out=_cached(self, "out", (M, D), "bf16"))
 
 
