@@ -24,26 +24,53 @@ __all__ = [
 ]  # fmt: skip
 
 
-def _p(t) -> C.c_void_p:
-    return C.c_void_p(t.data_ptr() if t is not None else None)
+def _p(t) -> int | None:
+    return t.data_ptr() if t is not None else None
 
 
-def _s() -> C.c_void_p:
-    return C.c_void_p(_stream.active_stream())
+_s = _stream.active_stream
 
 
 def _dt(t) -> str:
     d = getattr(t, "dtype", None)
-    if not isinstance(d, str):
+    if d.__class__ is not str and not isinstance(d, str):
         raise TypeError(f"expected a QuarkTensor, got {type(t).__name__}")
     return d
 
 
-def _code(name: str | None, default: str) -> int:
-    name = default if name is None else (name.value if hasattr(name, "value") else name)
+def _code(name: str) -> int:
     if name not in _lib.DTYPE_CODE:
         raise TypeError(f"unsupported dtype {name!r}")
     return _lib.DTYPE_CODE[name]
+
+
+def _name(dtype) -> str | None:
+    """A dtype given as a string, as an enum member of a caller, or not at all."""
+    return dtype if dtype is None or dtype.__class__ is str else dtype.value if hasattr(dtype, "value") else dtype
+
+
+# The parameter structs of calls already made, by their field values: filling one through ctypes takes longer than the rest of a
+# call.  Bounded; a struct is never written after it is made, so calls from several threads may share it.
+_PARAMS: dict = {}
+
+
+def _params(cls, *values):
+    """``(struct, byref(struct), [])``; the list is for what a caller derives from the struct alone (a workspace size)."""
+    key = (cls, values)
+    got = _PARAMS.get(key)
+    if got is None:
+        if len(_PARAMS) >= 4096:
+            _PARAMS.clear()
+        p = cls(*values)
+        got = _PARAMS[key] = (p, C.byref(p), [])
+    return got
+
+
+def _need(params, entry) -> int:
+    """Workspace bytes that ``entry`` wants for the struct, asked once."""
+    if not params[2]:
+        params[2].append(int(entry(params[1])))
+    return params[2][0]
 
 
 # ---------------------------------------------------------------------------
@@ -154,13 +181,13 @@ def gemm(A, B, out_dtype=None, compute_dtype=None, b_shuffled=False, activation=
         raise NotImplementedError("qf.gemm: b_shuffled=True is not supported (disabled upstream as well)")
     if A.ndim < 2 or B.ndim != 2:
         raise ValueError(f"qf.gemm: A must be at least rank-2 and B rank-2, got {A.shape} and {B.shape}")
-    K = int(A.shape[-1])
+    K = A.shape[-1]
     M = A.numel // K
-    N = int(B.shape[0])
-    if int(B.shape[1]) != K:
+    N = B.shape[0]
+    if B.shape[1] != K:
         raise ValueError(f"qf.gemm: A is [..., {K}] but B is {B.shape} (expected [N, {K}])")
     a_dt, b_dt = _dt(A), _dt(B)
-    cd = compute_dtype.value if hasattr(compute_dtype, "value") else compute_dtype
+    cd = _name(compute_dtype)
     if cd is None:
         cd = b_dt if b_dt == "e4m3" else a_dt
     if cd not in ("bf16", "e4m3"):
@@ -169,7 +196,7 @@ def gemm(A, B, out_dtype=None, compute_dtype=None, b_shuffled=False, activation=
         raise ValueError(f"qf.gemm: unsupported activation {activation!r}")
     if (gate is None) != (residual is None):
         raise ValueError("qf.gemm: gate and residual must be given together")
-    od = out_dtype.value if hasattr(out_dtype, "value") else out_dtype
+    od = _name(out_dtype)
     if od is None:
         od = out.dtype if out is not None else "bf16"
     if out is None:
@@ -183,19 +210,13 @@ def gemm(A, B, out_dtype=None, compute_dtype=None, b_shuffled=False, activation=
             raise ValueError(f"qf.gemm: gate must be [{gate_groups}, {N}] and residual [{M}, {N}]")
         if M % gate_groups:
             raise ValueError(f"qf.gemm: gate_groups={gate_groups} does not divide M={M}")
-    p = _lib.GemmParams(
-        M=M, N=N, K=K, a_dtype=_code(a_dt, "bf16"), b_dtype=_code(b_dt, "bf16"), c_dtype=_code(od, "bf16"),
-        compute_dtype=_code(cd, "bf16"), activation=1 if activation == "silu" else 0, gate_groups=int(gate_groups),
-        split_k=int(split_k), tile_n=int(tile_n), reserved=int(slice_mode) | (2 if b_constant else 0),
-        a_scale=a_scale.data_ptr() if a_scale is not None else None,
-        w_scale=w_scale.data_ptr() if w_scale is not None else None,
-    )  # fmt: skip
+    p = _params(_lib.GemmParams, M, N, K, _code(a_dt), _code(b_dt), _code(od), _code(cd), 1 if activation == "silu" else 0, int(gate_groups), int(split_k),
+                int(tile_n), int(slice_mode) | (2 if b_constant else 0), _p(a_scale), _p(w_scale))  # fmt: skip
     lib = _lib.load()
-    need = int(lib.qb_gemm_workspace_bytes(C.byref(p)))
-    ws = _workspace(need)
-    _lib.check(
-        lib.qb_gemm(_p(A), _p(B), _p(out), _p(bias), _p(gate), _p(residual), C.byref(p), _p(ws), ws.nbytes if ws is not None else 0, _s())
-    )
+    ws = _workspace(_need(p, lib.qb_gemm_workspace_bytes))
+    rc = lib.qb_gemm(A.data_ptr(), B.data_ptr(), out.data_ptr(), _p(bias), _p(gate), _p(residual), p[1], _p(ws), ws.nbytes if ws is not None else 0, _s())
+    if rc:
+        _lib.check(rc)
     return out
 
 
@@ -210,14 +231,11 @@ def gemm_tp(A, B, arena, *, compute_dtype=None, b_constant=False):
         raise ValueError(f"qf.gemm_tp: A {tuple(A.shape)} x B {tuple(B.shape)} is not the [{arena.rows}, {arena.D}] partial of the arena")
     a_dt, b_dt = _dt(A), _dt(B)
     cd = compute_dtype or (b_dt if b_dt == "e4m3" else a_dt)
-    gp = _lib.GemmParams(
-        M=M, N=N, K=K, a_dtype=_code(a_dt, "bf16"), b_dtype=_code(b_dt, "bf16"), c_dtype=_code("bf16", "bf16"), compute_dtype=_code(cd, "bf16"),
-        activation=0, gate_groups=1, split_k=1, tile_n=0, reserved=2 if b_constant else 0, a_scale=None, w_scale=None,
-    )  # fmt: skip
+    gp = _params(_lib.GemmParams, M, N, K, _code(a_dt), _code(b_dt), _code("bf16"), _code(cd), 0, 1, 1, 0, 2 if b_constant else 0, None, None)
     tp = arena.params()
     lib = _lib.load()
-    ws = _workspace(int(lib.qb_gemm_workspace_bytes(C.byref(gp))))
-    _lib.check(lib.qb_gemm_tp(_p(A), _p(B), C.byref(gp), C.byref(tp), _p(ws), ws.nbytes if ws is not None else 0, _s()))
+    ws = _workspace(_need(gp, lib.qb_gemm_workspace_bytes))
+    _lib.check(lib.qb_gemm_tp(_p(A), _p(B), gp[1], C.byref(tp), _p(ws), ws.nbytes if ws is not None else 0, _s()))
 
 
 def quantize_e4m3(X, *, out=None):
@@ -253,6 +271,8 @@ def quantize_e4m3_rows(X, *, out=None, scale_out=None):
 
 
 def _head_scales(who, n_kv_heads, k_scale, v_scale):
+    if k_scale is None and v_scale is None:
+        return None, None
     for name, t in (("k_scale", k_scale), ("v_scale", v_scale)):
         if t is not None and (_dt(t) != "f32" or t.numel != n_kv_heads):
             raise ValueError(f"{who}: {name} must be an f32 tensor of {n_kv_heads} per-head scales")
@@ -325,19 +345,16 @@ def kv_cache_update(K, V, frame_t, frozen, Vt_cache, segments, n_segments, K_cac
     if int(n_segments.shape[0]) != B:
         raise ValueError(f"qf.kv_cache_update: n_segments shape {tuple(n_segments.shape)} != ({B},)")
     kvd = _dt(K_cache)
-    want = kv_dtype.value if hasattr(kv_dtype, "value") else kv_dtype
+    want = _name(kv_dtype)
     if want is not None and want != kvd:
         raise TypeError(f"qf.kv_cache_update: kv_dtype={want!r} but the caches are {kvd!r}")
     if _dt(Vt_cache) != kvd or kvd not in ("bf16", "e4m3"):
         raise TypeError(f"qf.kv_cache_update: cache dtypes {kvd!r} / {_dt(Vt_cache)!r}")
     ks, vs = _head_scales("qf.kv_cache_update", n_kv_heads, k_scale, v_scale)
-    p = _lib.KvParams(
-        n_q_heads=n_q_heads, n_kv_heads=n_kv_heads, H_spatial=H_spatial, W_spatial=W_spatial, num_buckets=num_buckets,
-        pinned_dilation=pinned_dilation, kv_dtype=_lib.DTYPE_CODE[kvd], max_segments=max_segments, quilt_factor=quilt_factor,
-        packed_qkv=1 if packed_qkv else 0, quilt_offset=quilt_offset, k_scale=ks, v_scale=vs,
-    )  # fmt: skip
-    tail = (_p(frame_t), _p(frozen), _p(K_cache), _p(Vt_cache), _p(segments), _p(n_segments), _p(rope_table(H_spatial, W_spatial)),
-            C.byref(p), _s())  # fmt: skip
+    p = _params(_lib.KvParams, n_q_heads, n_kv_heads, H_spatial, W_spatial, num_buckets, pinned_dilation, _lib.DTYPE_CODE[kvd], max_segments,
+                quilt_factor, 1 if packed_qkv else 0, quilt_offset, ks, vs)  # fmt: skip
+    tail = (frame_t.data_ptr(), frozen.data_ptr(), K_cache.data_ptr(), Vt_cache.data_ptr(), segments.data_ptr(), n_segments.data_ptr(),
+            rope_table(H_spatial, W_spatial).data_ptr(), p[1], _s())  # fmt: skip
     lib = _lib.load()
     _lib.check(lib.qb_kv_cache_update(_p(K), *tail) if packed_qkv else lib.qb_kv_cache_update_kv(_p(K), _p(V), *tail))
     return K_cache, Vt_cache, segments, n_segments
@@ -368,15 +385,11 @@ def qkv_post(QKV, QKV_first, lamb, frame_t, frozen, Vt_cache, segments, n_segmen
         raise TypeError(f"qf.qkv_post: cache dtypes {kvd!r} / {_dt(Vt_cache)!r}")
     out = _like(QKV, out, "qf.qkv_post")
     ks, vs = _head_scales("qf.qkv_post", n_kv_heads, k_scale, v_scale)
-    p = _lib.KvParams(
-        n_q_heads=n_q_heads, n_kv_heads=n_kv_heads, H_spatial=H_spatial, W_spatial=W_spatial, num_buckets=num_buckets,
-        pinned_dilation=pinned_dilation, kv_dtype=_lib.DTYPE_CODE[kvd], max_segments=max_segments, quilt_factor=1, packed_qkv=1,
-        k_scale=ks, v_scale=vs,
-    )  # fmt: skip
+    p = _params(_lib.KvParams, n_q_heads, n_kv_heads, H_spatial, W_spatial, num_buckets, pinned_dilation, _lib.DTYPE_CODE[kvd], max_segments, 1, 1, 0, ks, vs)
     _lib.check(
         _lib.load().qb_qkv_post(
             _p(QKV), _p(QKV_first), _p(lamb), _p(out), _p(frame_t), _p(frozen), _p(K_cache), _p(Vt_cache), _p(segments),
-            _p(n_segments), _p(rope_table(H_spatial, W_spatial)), C.byref(p), float(eps), _s(),
+            _p(n_segments), _p(rope_table(H_spatial, W_spatial)), p[1], float(eps), _s(),
         )
     )  # fmt: skip
     return out
@@ -388,9 +401,9 @@ def gemm_qkv_post(A, B, QKV_first, lamb, frame_t, frozen, Vt_cache, segments, n_
     """``qkv_post(gemm(A, B))`` in one launch: the QKV projection whose epilogue normalises the Q and K heads,
     mixes V with the first block's, rotates K and appends K / V to the caches (same bytes as the two calls;
     no reference counterpart as a single call).  Returns the packed QKV that ``owl_attn`` reads."""
-    K = int(A.shape[-1])
+    K = A.shape[-1]
     M = A.numel // K
-    N = int(B.shape[0])
+    N = B.shape[0]
     tpf = int(H_spatial) * int(W_spatial)
     if M != tpf or N != (n_q_heads + 2 * n_kv_heads) * 64 or int(B.shape[1]) != K:
         raise ValueError(f"qf.gemm_qkv_post: A {tuple(A.shape)} x B {tuple(B.shape)} is not the [{tpf}, {(n_q_heads + 2 * n_kv_heads) * 64}] projection")
@@ -413,25 +426,18 @@ def gemm_qkv_post(A, B, QKV_first, lamb, frame_t, frozen, Vt_cache, segments, n_
         out = QuarkTensor.empty(M, N, dtype="bf16")
     elif out.numel != M * N or out.dtype != "bf16":
         raise ValueError(f"qf.gemm_qkv_post: out is {out.shape} {out.dtype}, expected ({M}, {N}) bf16")
-    gp = _lib.GemmParams(
-        M=M, N=N, K=K, a_dtype=_code(a_dt, "bf16"), b_dtype=_code(b_dt, "bf16"), c_dtype=_code("bf16", "bf16"),
-        compute_dtype=_code(cd, "bf16"), activation=0, gate_groups=1, split_k=1, tile_n=128, reserved=2,
-        a_scale=a_scale.data_ptr() if a_scale is not None else None, w_scale=w_scale.data_ptr() if w_scale is not None else None,
-    )  # fmt: skip
+    gp = _params(_lib.GemmParams, M, N, K, _code(a_dt), _code(b_dt), _code("bf16"), _code(cd), 0, 1, 1, 0, 2, _p(a_scale), _p(w_scale))
     if w_scale is not None and (_dt(w_scale) != "f32" or w_scale.numel != N):
         raise ValueError(f"qf.gemm_qkv_post: w_scale must be f32 [{N}]")
     ks, vs = _head_scales("qf.gemm_qkv_post", n_kv_heads, k_scale, v_scale)
-    kp = _lib.KvParams(
-        n_q_heads=n_q_heads, n_kv_heads=n_kv_heads, H_spatial=H_spatial, W_spatial=W_spatial, num_buckets=num_buckets,
-        pinned_dilation=pinned_dilation, kv_dtype=_lib.DTYPE_CODE[kvd], max_segments=max_segments, quilt_factor=quilt_factor, packed_qkv=1,
-        quilt_offset=quilt_offset, k_scale=ks, v_scale=vs,
-    )  # fmt: skip
+    kp = _params(_lib.KvParams, n_q_heads, n_kv_heads, H_spatial, W_spatial, num_buckets, pinned_dilation, _lib.DTYPE_CODE[kvd], max_segments,
+                 quilt_factor, 1, quilt_offset, ks, vs)  # fmt: skip
     lib = _lib.load()
-    ws = _workspace(int(lib.qb_gemm_workspace_bytes(C.byref(gp))))
+    ws = _workspace(_need(gp, lib.qb_gemm_workspace_bytes))
     _lib.check(
         lib.qb_gemm_qkv_post(
             _p(A), _p(B), _p(out), _p(QKV_first), _p(lamb), _p(frame_t), _p(frozen), _p(K_cache), _p(Vt_cache), _p(segments), _p(n_segments),
-            _p(rope_table(H_spatial, W_spatial)), C.byref(gp), C.byref(kp), float(eps), _p(ws), ws.nbytes if ws is not None else 0, _s(),
+            _p(rope_table(H_spatial, W_spatial)), gp[1], kp[1], float(eps), _p(ws), ws.nbytes if ws is not None else 0, _s(),
         )
     )  # fmt: skip
     return out
@@ -481,7 +487,7 @@ def owl_attn(Q, K_cache, Vt_cache, segments, n_segments, B, n_kv_heads, gqa_rati
     if _dt(Q) != "bf16":
         raise TypeError(f"qf.owl_attn: Q dtype {_dt(Q)!r} (expected bf16)")
     kvd = _dt(K_cache)
-    cd = compute_dtype.value if hasattr(compute_dtype, "value") else compute_dtype
+    cd = _name(compute_dtype)
     if cd is None:
         cd = "bf16"
     if cd not in ("bf16", "e4m3") or kvd not in ("bf16", "e4m3"):
@@ -496,7 +502,7 @@ def owl_attn(Q, K_cache, Vt_cache, segments, n_segments, B, n_kv_heads, gqa_rati
         conv(K_cache, out=Ks)
         conv(Vt_cache, out=Vs)
         K_cache, Vt_cache, kvd = Ks, Vs, cd
-    od = out_dtype.value if hasattr(out_dtype, "value") else out_dtype
+    od = _name(out_dtype)
     if od not in (None, "bf16"):
         raise NotImplementedError(f"qf.owl_attn: out_dtype {od!r} (only bf16)")
     if out is None:
@@ -509,19 +515,14 @@ def owl_attn(Q, K_cache, Vt_cache, segments, n_segments, B, n_kv_heads, gqa_rati
         if _DUMMY_FRAME_T is None:
             _DUMMY_FRAME_T = QuarkTensor.zeros(1, dtype="s32")
         frame_t = _DUMMY_FRAME_T
-    p = _lib.AttnParams(
-        n_kv_heads=n_kv_heads, gqa_ratio=gqa_ratio, H_spatial=H_spatial, W_spatial=W_spatial, num_buckets=num_buckets,
-        pinned_dilation=pinned_dilation, kv_dtype=_lib.DTYPE_CODE[kvd], compute_dtype=_lib.DTYPE_CODE[cd],
-        max_segments=max_segments, packed_qkv=1 if packed_qkv else 0, quilt_factor=quilt_factor, kv_splits=int(kv_splits),
-        k_scale=k_scale.data_ptr() if k_scale is not None else None,
-        v_scale=v_scale.data_ptr() if v_scale is not None else None,
-    )  # fmt: skip
+    p = _params(_lib.AttnParams, n_kv_heads, gqa_ratio, H_spatial, W_spatial, num_buckets, pinned_dilation, _lib.DTYPE_CODE[kvd], _lib.DTYPE_CODE[cd],
+                max_segments, 1 if packed_qkv else 0, quilt_factor, int(kv_splits), _p(k_scale), _p(v_scale))  # fmt: skip
     lib = _lib.load()
-    ws = _attn_workspace(int(lib.qb_owl_attn_workspace_bytes(C.byref(p))))
+    ws = _attn_workspace(_need(p, lib.qb_owl_attn_workspace_bytes))
     _lib.check(
         lib.qb_owl_attn(
-            _p(Q), _p(K_cache), _p(Vt_cache), _p(segments), _p(n_segments), _p(frame_t), _p(out), _p(out_q),
-            _p(rope_table(H_spatial, W_spatial)), C.byref(p), _p(ws), ws.nbytes if ws is not None else 0, _s(),
+            Q.data_ptr(), K_cache.data_ptr(), Vt_cache.data_ptr(), segments.data_ptr(), n_segments.data_ptr(), frame_t.data_ptr(), out.data_ptr(), _p(out_q),
+            rope_table(H_spatial, W_spatial).data_ptr(), p[1], _p(ws), ws.nbytes if ws is not None else 0, _s(),
         )
     )  # fmt: skip
     return out
@@ -720,11 +721,8 @@ def kv_cast_appended(K_cache, Vt_cache, K_shadow, Vt_shadow, frame_t, frozen, *,
         raise TypeError("qf.kv_cast_appended: the shadow pair must have the other of the two cache dtypes")
     if K_shadow.numel != K_cache.numel or Vt_shadow.numel != Vt_cache.numel:
         raise ValueError("qf.kv_cast_appended: the shadow pair must have the caches' shapes")
-    p = _lib.KvParams(
-        n_q_heads=0, n_kv_heads=n_kv_heads, H_spatial=H_spatial, W_spatial=W_spatial, num_buckets=num_buckets, pinned_dilation=pinned_dilation,
-        kv_dtype=_lib.DTYPE_CODE[kvd], max_segments=3, quilt_factor=quilt_factor, packed_qkv=1, quilt_offset=0, k_scale=None, v_scale=None,
-    )  # fmt: skip
-    _lib.check(_lib.load().qb_kv_cast_appended(_p(K_cache), _p(Vt_cache), _p(K_shadow), _p(Vt_shadow), _p(frame_t), _p(frozen), C.byref(p), _s()))
+    p = _params(_lib.KvParams, 0, n_kv_heads, H_spatial, W_spatial, num_buckets, pinned_dilation, _lib.DTYPE_CODE[kvd], 3, quilt_factor, 1, 0, None, None)
+    _lib.check(_lib.load().qb_kv_cast_appended(_p(K_cache), _p(Vt_cache), _p(K_shadow), _p(Vt_shadow), _p(frame_t), _p(frozen), p[1], _s()))
 
 
 def moe_slots(M: int, E: int, top_k: int) -> int:
@@ -781,13 +779,11 @@ def gemm_grouped(A, B, tile_expert, *, n_experts: int, out_dtype="bf16", compute
         out = QuarkTensor.empty(M, N, dtype=out_dtype)
     elif out.numel != M * N or _dt(out) != out_dtype:
         raise ValueError(f"qf.gemm_grouped: out must be {out_dtype} [{M}, {N}]")
-    p = _lib.GemmParams(
-        M=M, N=N, K=K, a_dtype=_code(a_dt, "bf16"), b_dtype=_code(b_dt, "bf16"), c_dtype=_code(out_dtype, "bf16"), compute_dtype=_code(cd, "bf16"),
-        activation=1 if activation == "silu" else 0, gate_groups=1, split_k=1, tile_n=0, reserved=2 if b_constant else 0, a_scale=None, w_scale=None,
-    )  # fmt: skip
+    p = _params(_lib.GemmParams, M, N, K, _code(a_dt), _code(b_dt), _code(_name(out_dtype)), _code(cd), 1 if activation == "silu" else 0, 1, 1, 0,
+                2 if b_constant else 0, None, None)  # fmt: skip
     lib = _lib.load()
-    ws = _workspace(int(lib.qb_gemm_grouped_workspace_bytes(C.byref(p))))
-    _lib.check(lib.qb_gemm_grouped(_p(A), _p(B), _p(out), _p(tile_expert), int(n_experts), C.byref(p), _p(ws), ws.nbytes if ws is not None else 0, _s()))
+    ws = _workspace(_need(p, lib.qb_gemm_grouped_workspace_bytes))
+    _lib.check(lib.qb_gemm_grouped(_p(A), _p(B), _p(out), _p(tile_expert), int(n_experts), p[1], _p(ws), ws.nbytes if ws is not None else 0, _s()))
     return out
 
 

@@ -60,15 +60,20 @@ def _numel(shape) -> int:
 
 
 class QuarkTensor:
-    __slots__ = ("_storage", "_offset", "shape", "dtype")
+    # numel, nbytes and the address are read several times by every call that takes the tensor: worked out once
+    __slots__ = ("_storage", "_offset", "_ptr", "shape", "dtype", "ndim", "numel", "nbytes")
 
     def __init__(self, storage, shape, dtype: str, offset: int = 0):
         if dtype not in _ITEMSIZE:
             raise TypeError(f"QuarkTensor: unsupported dtype {dtype!r}")
         self._storage = storage
         self._offset = int(offset)
+        self._ptr = storage.ptr + self._offset
         self.shape = tuple(int(s) for s in shape)
         self.dtype = dtype
+        self.ndim = len(self.shape)
+        self.numel = _numel(self.shape)
+        self.nbytes = self.numel * _ITEMSIZE[dtype]
 
     # ---- construction
     @staticmethod
@@ -109,19 +114,7 @@ class QuarkTensor:
 
     # ---- introspection
     def data_ptr(self) -> int:
-        return self._storage.ptr + self._offset
-
-    @property
-    def ndim(self) -> int:
-        return len(self.shape)
-
-    @property
-    def numel(self) -> int:
-        return _numel(self.shape)
-
-    @property
-    def nbytes(self) -> int:
-        return self.numel * _ITEMSIZE[self.dtype]
+        return self._ptr
 
     @property
     def quark_dtype(self) -> str:
