@@ -208,14 +208,22 @@ def kernel_launch_count() -> int:
     return int(load().qb_kernel_launch_count())
 
 
+# Counts the changes made through the two switches below: a captured graph keeps the setting it was captured with.
+settings_version = 0
+
+
 def set_dependent_launch(enabled: bool) -> bool:
     """Turns the overlap of a kernel's set-up with its predecessor's tail on or off; returns the old setting."""
+    global settings_version
+    settings_version += 1
     return bool(load().qb_set_dependent_launch(1 if enabled else 0))
 
 
 def set_attn_exact_exp(enabled: bool) -> bool:
     """e4m3 attention: ``True`` computes every probability with ``ex2.approx``; ``False`` (the default) builds every second one
     on the FMA pipe from a centred chord of ``2^x`` (see ``qb_set_attn_exact_exp``).  Returns the old setting."""
+    global settings_version
+    settings_version += 1
     return bool(load().qb_set_attn_exact_exp(1 if enabled else 0))
 
 

@@ -47,6 +47,34 @@ class CtrlInput:
     scroll_wheel: int = 0
 
 
+class _AppendGraph:
+    """The commit pass of ``Engine.append_frame`` as a CUDA graph: issued call by call the pass is bound by the host.  It holds the
+    addresses it was captured with, so ``current()`` says whether the model still has the tensors it had then."""
+
+    def __init__(self, engine: "Engine", ctrl_dev):
+        self._settings = _lib.settings_version
+        self._blocks = list(engine.model.blocks)
+        self._params = [(p, p.data) for _, p in engine.model.named_parameters()]
+        self._caches = [(kc, kc.K_cache, kc.Vt_cache, kc.k_scale, kc.v_scale) for kc in (b.kv_cache for b in self._blocks)]
+        si = engine.gen.n_denoise
+        self._luts = [(b, si, b._cond_lut[si]) for b in self._blocks]
+        self._out_lut = (engine.model, si, engine.model._out_norm_luts[si])
+        with _stream.capture_graph() as cap:
+            engine._append_pass(ctrl_dev)
+        self._graph = cap.graph
+
+    def current(self) -> bool:
+        model, si, rows = self._out_lut
+        return (self._settings == _lib.settings_version and model._out_norm_luts[si] is rows and all(p.data is d for p, d in self._params)
+                and all(b._cond_lut[i] is r for b, i, r in self._luts)
+                and all(kc.K_cache is K and kc.Vt_cache is V and kc.k_scale is ks and kc.v_scale is vs for kc, K, V, ks, vs in self._caches))  # fmt: skip
+
+    def launch(self) -> None:
+        for b in self._blocks:
+            b.kv_cache.sync_shadow()
+        self._graph.launch()
+
+
 class Engine:
     def __init__(self, model_uri=None, *, cfg: Waypoint15Config | None = None, quant="fp8", load_weights=True, seed: int = 0,
                  params: dict | None = None, device: int = 0, use_graph: bool = True, comm=None, device_noise: bool = False,
@@ -76,6 +104,7 @@ class Engine:
             self.model.prepare()
         self.gen = GenerateFrame(self.model)
         self._use_graph = use_graph
+        self._append_graph = None  # the commit pass of append_frame, captured once it has run eagerly
         # A sharded session (comm.world > 1) waits for its peers inside every frame.  With `watchdog_s` set, a frame that
         # takes longer aborts the communicator from a timer thread, so that a rank whose peer died returns with an error
         # instead of waiting inside a collective (runtime.nccl.Watchdog).  The reference is single-GPU: no counterpart.
@@ -156,6 +185,7 @@ class Engine:
         """Drops the captured frame graph (a communicator whose collectives it holds cannot be destroyed
         before); the engine runs eagerly afterwards unless a new graph is captured."""
         self.gen._graph = None
+        self._append_graph = None
         self._use_graph = False
         import gc
 
@@ -202,14 +232,24 @@ class Engine:
         advance the frame counter (``src/quark/engine/cuda.py:177-195`` without the VAE)."""
         self._noise_host.array[:] = self._to_bf16(latent)
         self._h2d(self._append_dev, self._noise_host.ptr, self.cfg.latent_numel * 2)
-        ctrl_emb = self.model.encode_ctrl(self._encode_ctrl(ctrl))
-        self.model(self._append_dev, sigma_idx=self.gen.n_denoise, frame_t=self.gen.frame_t, ctrl_emb=ctrl_emb, frozen=False)
-        from . import functional as qf
-
-        qf.increment(self.gen.frame_t)
+        ctrl_dev = self._encode_ctrl(ctrl)
+        if self._append_graph is not None and self._append_graph.current():
+            self._append_graph.launch()
+        else:
+            self._append_graph = None
+            self._append_pass(ctrl_dev)
+            if self._use_graph and self.model.comm is None:  # every buffer of the pass exists now
+                self._append_graph = _AppendGraph(self, ctrl_dev)
         _stream.synchronize()
         self._frame += 1
         return np.asarray(latent)
+
+    def _append_pass(self, ctrl_dev) -> None:
+        from . import functional as qf
+
+        ctrl_emb = self.model.encode_ctrl(ctrl_dev)
+        self.model(self._append_dev, sigma_idx=self.gen.n_denoise, frame_t=self.gen.frame_t, ctrl_emb=ctrl_emb, frozen=False)
+        qf.increment(self.gen.frame_t)
 
     def gen_frame(self, ctrl=None, return_img: bool = True, *, noise=None):
         """Generate the next latent frame: 4 denoise NFEs + 1 commit NFE (``engine/cuda.py:197-255``).
@@ -252,11 +292,11 @@ class Engine:
         saved = []
         for blk in self.model.blocks:
             kc = blk.kv_cache
-            saved.append([(t, t.to_numpy()) for t in (kc.K_cache, kc.Vt_cache, kc.segments, kc.n_segments)])
+            for t in (kc.K_cache, kc.Vt_cache, kc.segments, kc.n_segments):
+                saved.append((t, QuarkTensor.empty(*t.shape, dtype=t.dtype).copy_from(t)))
         self.gen.prepare_graph(self._noise_dev, self._ctrl_dev, start_frame_t=self._frame)
-        for items in saved:
-            for t, host in items:
-                t.copy_from_numpy(host)
+        for t, copy in saved:
+            t.copy_from(copy)
         for blk in self.model.blocks:
             blk.kv_cache.refresh_shadow()
         _stream.synchronize()

@@ -100,7 +100,9 @@ class ModuleList(Module):
 
 def _cached(module, key: str, shape, dtype) -> QuarkTensor:
     """Per-module output buffers keyed by (name, shape, dtype) (``src/quark/nn/layers.py:236-258``)."""
-    cache = module.__dict__.setdefault("_bufs", {})
+    cache = module.__dict__.get("_bufs")
+    if cache is None:
+        cache = module.__dict__["_bufs"] = {}
     k = (key, tuple(shape), dtype)
     buf = cache.get(k)
     if buf is None:
@@ -427,6 +429,13 @@ class KVCacheUpdate(Module):
             qf.kv_cast_appended(self.K_cache, self.Vt_cache, self._shadow[0], self._shadow[1], frame_t if frame_t is not None else self.frame_t,
                                 self._frozen[1 if frozen else 0], **self._kw)  # fmt: skip
         return self._shadow
+
+    def sync_shadow(self) -> None:
+        """Converts both caches whole if they were written from the host since they were last (a captured pass only converts the
+        rows its own append writes)."""
+        if getattr(self, "_shadow", None) is not None:
+            if self._shadow_seen != (self.K_cache._storage.host_writes, self.Vt_cache._storage.host_writes):
+                self.refresh_shadow()
 
     def refresh_shadow(self) -> None:
         """Converts both caches whole (after the caches were written by anything but the append)."""
