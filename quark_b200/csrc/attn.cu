@@ -41,12 +41,15 @@
 // writing P(i) never waits for PV(i - 1).  exp2 is ex2.approx.f32 in both paths: measured on B200,
 // ex2.approx.f16x2 issues at half the rate of the f32 form (no gain per element) and the f16x2 -> e4m3x2
 // conversion is four times slower than f32 -> e4m3x2.
+#include <atomic>
+
 #include <cuda.h>
 
 #include "attn_common.cuh"
 
 namespace qb {
 
+int num_sms();
 int32_t make_tmap_2d_sw(CUtensorMap* tm, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint32_t box_rows,
                         uint32_t box_cols, int swizzle_bytes);
 
@@ -94,6 +97,7 @@ struct AttnSmem {
   static constexpr int kStageOff = kPOff + 2 * kPBufs * kPBytes;
   static constexpr int kBarOff = kStageOff + kStages * kStageBytes;
   static constexpr int kTotal = kBarOff + 512 + 1024;
+  static_assert(kStages * kStageBytes >= 266 * 68 * 4, "merge area of the cluster splits (7 CTAs need most) aliases the stage area");
   static_assert(kStages * kStageBytes >= 66 * 128 * 4, "merge buffer aliases the stage area");
   static_assert(kStages % 2 == 0 && kTotal <= 227 * 1024, "see kStages; shared memory of one CTA");
 };
@@ -172,9 +176,17 @@ __device__ __forceinline__ void p_chunk(const uint32_t (&sc)[32], int c, float s
   }
 }
 
-// kSplit: the keys of a (query tile, head) are shared by gridDim.z CTAs (see AttnArgs::partials).  The
-// unsplit kernel is an instantiation of its own so that none of this reaches its instruction stream.
-template <bool kFp8, bool kSplit, bool kLin>
+// Whether the keys of a (query tile, head) are shared by gridDim.z CTAs, and how their results are brought together: through the
+// workspace (see AttnArgs::partials), or, the CTAs being one thread-block cluster, in shared memory.  The unsplit kernel is an
+// instantiation of its own so that none of this reaches its instruction stream.
+enum { kUnsplit = 0, kSplitWorkspace = 1, kSplitCluster = 2 };
+
+// Cluster splits: 2 groups x S CTAs leave 64 outputs, m and the row sum of each query row with the CTA that writes the row
+// (128 / S rows each), [2 S][rows][kMergePitch] f32.
+constexpr int kMergePitch = 68;
+__host__ __device__ constexpr int merge_rows(int splits) { return (kQTile + splits - 1) / splits; }
+
+template <bool kFp8, int kSplit, bool kLin>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const AttnArgs a) {
   using L = AttnSmem<kFp8>;
@@ -289,9 +301,9 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     if (threadIdx.x == 0) atomicOr(a.status, QB_DEV_BAD_SEGMENT);
   }
   // this CTA's share of the key tiles: tiles tile0 .. tile0 + n_tiles - 1 of the list
-  const int n_splits = kSplit ? static_cast<int>(gridDim.z) : 1;
+  const int n_splits = kSplit != kUnsplit ? static_cast<int>(gridDim.z) : 1;
   int tile0 = 0;
-  if (kSplit) {
+  if (kSplit != kUnsplit) {
     tile0 = static_cast<int>(blockIdx.z) * n_tiles / n_splits;
     n_tiles = static_cast<int>(blockIdx.z + 1) * n_tiles / n_splits - tile0;
   }
@@ -626,6 +638,48 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     }
 
     if (warp == 4) QB_TR(4, 0, 4);
+    if constexpr (kSplit == kSplitCluster) {
+      // Both groups of every CTA of the cluster hand their rows to the CTA that writes them (against the merge of the groups and
+      // the trip through the workspace, 360p, 4 CTAs: e4m3 13.4 -> 12.1 us, bf16 16.0 -> 13.9 us).
+      const int S = static_cast<int>(gridDim.z), rows = merge_rows(S);
+      float* area = reinterpret_cast<float*>(smem + L::kStageOff);
+      cluster_sync();  // the stages of every CTA are free (its tensor work and TMA traffic are finished)
+      {
+        const uint32_t base = map_to_cta(smem_u32(area), r / rows);
+        const int part = 2 * static_cast<int>(blockIdx.z) + g, rl = r % rows;
+        const uint32_t row_at = base + static_cast<uint32_t>((part * rows + rl) * kMergePitch) * 4u;
+#pragma unroll
+        for (int d = 0; d < 64; d += 4)
+          st_dsmem_v4(row_at + d * 4u, __float_as_uint(o[d]), __float_as_uint(o[d + 1]), __float_as_uint(o[d + 2]), __float_as_uint(o[d + 3]));
+        st_dsmem_v4(row_at + 256u, __float_as_uint(m_run), __float_as_uint(l_run), 0u, 0u);
+      }
+      cluster_sync();
+      const float vs = a.v_scale ? __ldg(a.v_scale + kvh) : 1.0f;
+      for (int i = threadIdx.x - 128; i < rows * 8; i += 256) {  // 8 outputs of a row per thread
+        const int rl = i >> 3, d0 = (i & 7) * 8, rr = static_cast<int>(blockIdx.z) * rows + rl;
+        if (rr >= kQTile || q0 + rr >= a.tpf) continue;
+        float m = -1.0e30f;
+        for (int q = 0; q < 2 * S; ++q) m = fmaxf(m, area[(q * rows + rl) * kMergePitch + 64]);
+        float l = 0.f, e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int q = 0; q < 2 * S; ++q) {
+          const float* part = area + (q * rows + rl) * kMergePitch;
+          const float w = ex2_approx(part[64] - m);
+          l = fmaf(w, part[65], l);
+          const float4 x = *reinterpret_cast<const float4*>(part + d0), y = *reinterpret_cast<const float4*>(part + d0 + 4);
+          e[0] = fmaf(w, x.x, e[0]); e[1] = fmaf(w, x.y, e[1]); e[2] = fmaf(w, x.z, e[2]); e[3] = fmaf(w, x.w, e[3]);
+          e[4] = fmaf(w, y.x, e[4]); e[5] = fmaf(w, y.y, e[5]); e[6] = fmaf(w, y.z, e[6]); e[7] = fmaf(w, y.w, e[7]);
+        }
+        const float inv = l > 0.f ? vs / l : 0.f;
+        const size_t at = static_cast<size_t>(q0 + rr) * a.o_row + static_cast<size_t>(qh) * a.o_head + d0;
+        uint32_t w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(e[2 * q] * inv, e[2 * q + 1] * inv);
+        *reinterpret_cast<uint4*>(a.out + at) = make_uint4(w[0], w[1], w[2], w[3]);
+        if (a.out_q != nullptr)  // narrowed from the bf16-rounded values: equals a separate bf16 -> e4m3 cast
+          *reinterpret_cast<uint2*>(a.out_q + at) = make_uint2(pack_e4m3x4(bf16lo(w[0]), bf16hi(w[0]), bf16lo(w[1]), bf16hi(w[1])),
+                                                               pack_e4m3x4(bf16lo(w[2]), bf16hi(w[2]), bf16lo(w[3]), bf16hi(w[3])));
+      }
+    } else {
     // ---------------- merge the two groups (tensor work and TMA traffic are finished for both after the barrier)
     asm volatile("bar.sync 2, 256;" ::: "memory");
     if (warp == 4) QB_TR(4, 0, 5);
@@ -637,7 +691,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       for (int d = 0; d < 64; ++d) comb[(2 + d) * 128 + r] = o[d];
     }
     asm volatile("bar.sync 2, 256;" ::: "memory");
-    if (g == 0 && !kSplit) {
+    if (g == 0 && kSplit == kUnsplit) {
       if (ok && row_ok && *abort_flag == 0) {
         const float m1 = comb[r], l1 = comb[128 + r];
         const float m = fmaxf(m_run, m1);
@@ -665,7 +719,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
           }
         }
       }
-    } else if (kSplit && g == 0) {
+    } else if (kSplit == kSplitWorkspace && g == 0) {
       // keys shared with other CTAs.  This CTA's result for the row: both groups brought to a common maximum,
       // not yet divided by the row sum
       const bool good = ok && *abort_flag == 0;
@@ -727,9 +781,15 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         }
       }
     }
+    }
   }
 
   if (warp == 4) QB_TR(4, 0, 6);
+  if (kSplit == kSplitCluster && warp < 4) {  // the softmax warps' two barriers
+    __syncwarp();
+    cluster_sync();
+    cluster_sync();
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 4) QB_TR(4, 0, 7);
@@ -781,12 +841,85 @@ static int attn_key_splits(const qb_attn_params* p) {
   const int tpf = p->H_spatial * p->W_spatial;
   const int items = ((tpf + kQTile - 1) / kQTile) * p->n_kv_heads * p->gqa_ratio;
   const int tiles = ((p->num_buckets + 1) * (tpf / (p->quilt_factor > 0 ? p->quilt_factor : 1)) + kKeyTile - 1) / kKeyTile;  // at most
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-  int n = sms / (items > 0 ? items : 1);
+  int n = num_sms() / (items > 0 ? items : 1);
   if (n > tiles / 3) n = tiles / 3;
   if (n > 8) n = 8;
   return n < 2 ? 1 : n;
+}
+
+template <typename K>
+static int32_t configure(K kernel, int smem_bytes, std::atomic<unsigned long long>& done) {  // once per device
+  int dev = 0;
+  QB_CUDA_OK(cudaGetDevice(&dev));
+  if (dev < 64 && (done.load(std::memory_order_relaxed) >> dev & 1) != 0) return QB_OK;
+  QB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+  if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_relaxed);
+  return QB_OK;
+}
+
+static cudaLaunchConfig_t attn_config(dim3 grid, int smem_bytes, cudaStream_t st, cudaLaunchAttribute (&attr)[2]) {  // grid.z = CTAs of a cluster
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kAttnThreads);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = grid.z;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g_dependent_launch ? 2 : 1;
+  return cfg;
+}
+
+// `splits` CTAs share the keys of each (query tile, head), as a cluster of up to 8 CTAs where the chip holds that many clusters at
+// once (B200: 15 of 8 CTAs, 33 of 4, 74 of 2); a wish for more is cut down to what it holds, a number that the caller forced goes
+// through the workspace instead.
+template <bool kFp8, bool kLin>
+static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnArgs& a, int Hq, int splits, bool forced, cudaStream_t st) {
+  constexpr int kSmem = AttnSmem<kFp8>::kTotal;
+  const unsigned q_tiles = (a.tpf + kQTile - 1) / kQTile;
+  const int items = static_cast<int>(q_tiles) * Hq;
+  int cluster = splits > 8 ? (forced ? 1 : 8) : splits;
+  if (cluster > 1) {
+    static std::atomic<unsigned long long> done{0};
+    static std::atomic<int> held[9];  // clusters of this many CTAs that run at once (0 = not asked yet)
+    const int32_t rc = configure(owl_attn_kernel<kFp8, kSplitCluster, kLin>, kSmem, done);
+    if (rc != QB_OK) return rc;
+    cudaLaunchAttribute attr[2];
+    while (cluster > 1) {
+      int n = held[cluster].load(std::memory_order_relaxed);
+      if (n == 0) {
+        const cudaLaunchConfig_t cfg = attn_config(dim3(q_tiles, Hq, cluster), kSmem, st, attr);
+        if (cudaOccupancyMaxActiveClusters(&n, owl_attn_kernel<kFp8, kSplitCluster, kLin>, &cfg) != cudaSuccess || n <= 0) {
+          cudaGetLastError();
+          n = 1;
+        }
+        held[cluster].store(n, std::memory_order_relaxed);
+      }
+      if (items <= n) break;
+      cluster = forced ? 1 : cluster - 1;
+    }
+    if (cluster > 1) {
+      const cudaLaunchConfig_t cfg = attn_config(dim3(q_tiles, Hq, cluster), kSmem, st, attr);
+      const cudaError_t e = cudaLaunchKernelEx(&cfg, owl_attn_kernel<kFp8, kSplitCluster, kLin>, tmK, tmV, a);
+      ++g_launch_count;
+      if (e != cudaSuccess) return fail(QB_ERR_LAUNCH, "owl_attn kernel (cluster of %d): %s", cluster, cudaGetErrorString(e));
+      return QB_OK;
+    }
+  }
+  if (splits > 1 && forced) {
+    static std::atomic<unsigned long long> done{0};
+    const int32_t rc = configure(owl_attn_kernel<kFp8, kSplitWorkspace, kLin>, kSmem, done);
+    if (rc != QB_OK) return rc;
+    return launch_dep("owl_attn kernel", owl_attn_kernel<kFp8, kSplitWorkspace, kLin>, dim3(q_tiles, Hq, splits), dim3(kAttnThreads), kSmem, st, tmK, tmV, a);
+  }
+  static std::atomic<unsigned long long> done{0};
+  const int32_t rc = configure(owl_attn_kernel<kFp8, kUnsplit, kLin>, kSmem, done);
+  if (rc != QB_OK) return rc;
+  return launch_dep("owl_attn kernel", owl_attn_kernel<kFp8, kUnsplit, kLin>, dim3(q_tiles, Hq), dim3(kAttnThreads), kSmem, st, tmK, tmV, a);
 }
 
 // The tickets take a fixed area at the start of the workspace (4096 (query tile, head) items; more only for a
@@ -865,17 +998,11 @@ extern "C" int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void*
     a.tickets = static_cast<int*>(workspace);
     a.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + attn_ticket_bytes(p));
   }
-  dim3 grid((tpf + kQTile - 1) / kQTile, Hq, splits);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // bf16, one CTA per (query tile, head): the three-group kernel of attn4.cu (66.7 against 70.3 us at 720p).  In the
   // e4m3 path it is the slower one (57.7 against 52.2 us): its per-chunk fixed work outweighs the extra warps.
   if (splits == 1 && !fp8 && attn4_enabled()) return launch_attn4(K_cache, Vt_cache, a, p->n_kv_heads, fp8, st);
-  auto launch = [&](auto kernel, int smem_bytes) -> int32_t {
-    QB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-    return launch_dep("owl_attn kernel", kernel, grid, dim3(kAttnThreads), smem_bytes, st, tmK, tmV, a);
-  };
-  if (fp8 && !g_attn_exact_exp)
-    return splits > 1 ? launch(owl_attn_kernel<true, true, true>, AttnSmem<true>::kTotal) : launch(owl_attn_kernel<true, false, true>, AttnSmem<true>::kTotal);
-  if (fp8) return splits > 1 ? launch(owl_attn_kernel<true, true, false>, AttnSmem<true>::kTotal) : launch(owl_attn_kernel<true, false, false>, AttnSmem<true>::kTotal);
-  return splits > 1 ? launch(owl_attn_kernel<false, true, false>, AttnSmem<false>::kTotal) : launch(owl_attn_kernel<false, false, false>, AttnSmem<false>::kTotal);
+  const bool forced = p->kv_splits > 0;
+  if (!fp8) return launch_attn<false, false>(tmK, tmV, a, Hq, splits, forced, st);
+  return g_attn_exact_exp ? launch_attn<true, false>(tmK, tmV, a, Hq, splits, forced, st) : launch_attn<true, true>(tmK, tmV, a, Hq, splits, forced, st);
 }
