@@ -514,12 +514,14 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     const uint32_t tmem_o = tmem_s + kOCol;                          // ... and of its O accumulator
     float m_run = -1.0e30f;
     bool ok = true;
+    // every segment a multiple of the tile (720p: 512 keys a bucket): no tile needs a mask, so none is looked up
+    const bool whole = ((seg[1] | seg[3] | seg[5]) & (kKeyTile - 1)) == 0;
     const int my_tiles = n_tiles > g ? (n_tiles - g + 1) / 2 : 0;
 
     for (int i = 0; i < my_tiles && ok; ++i) {
       if (lane_grp == 0) QB_TR(g, i, 0);
-      int row, valid;
-      locate_tile(seg, tile0 + 2 * i + g, row, valid);
+      int row, valid = kKeyTile;
+      if (!whole) locate_tile(seg, tile0 + 2 * i + g, row, valid);
       if (lane_grp == 0) QB_TR(g, i, 1);
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[g]), i & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
       if (!ok) break;
@@ -999,7 +1001,7 @@ extern "C" int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void*
     a.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + attn_ticket_bytes(p));
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // bf16, one CTA per (query tile, head): the three-group kernel of attn4.cu (66.7 against 70.3 us at 720p).  In the
+  // bf16, one CTA per (query tile, head): the three-group kernel of attn4.cu (60.0 against 70.3 us at 720p).  In the
   // e4m3 path it is the slower one (57.7 against 52.2 us): its per-chunk fixed work outweighs the extra warps.
   if (splits == 1 && !fp8 && attn4_enabled()) return launch_attn4(K_cache, Vt_cache, a, p->n_kv_heads, fp8, st);
   const bool forced = p->kv_splits > 0;

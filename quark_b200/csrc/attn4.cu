@@ -8,10 +8,10 @@
 // TMEM: per group one S chunk (64 columns) and the output accumulator O (80 columns: 64 outputs and, from the rows of
 // ones under every V^T chunk, the row sum of exactly the rounded P that is multiplied with V).
 // As in attn.cu: P = 2^(score - m) with m the maximum the row was last rescaled to (O is rescaled only when a chunk's
-// maximum exceeds m by more than kSlack), e4m3 P scaled by 2^5, two P buffers per group in the fp8 path, every wait
+// maximum exceeds m by more than kSlack), e4m3 P scaled by 2^5, two P buffers per group, every wait
 // bounded, a malformed segment table reported and treated as empty.  The three partial results are merged at the end.
 //
-// Measured on B200 at 720p (512 queries x 32 heads x 8320 keys, us per launch; attn.cu in brackets): bf16 66.7 (70.3),
+// Measured on B200 at 720p (512 queries x 32 heads x 8320 keys, us per launch; attn.cu in brackets): bf16 60.0 (70.3),
 // e4m3 57.7 (52.2).  The extra warp per scheduler pays in the bf16 path, where attn.cu has one P tile per group and three
 // stages; in the e4m3 path the fixed work per chunk (barrier waits, TMEM loads, maxima: the same per 64 keys as attn.cu
 // spends per 128) outweighs it, so e4m3 calls stay with attn.cu.  A variant with four groups (16 softmax warps, 96
@@ -47,7 +47,9 @@ struct A4Smem {
   static constexpr int kKBytes = kA4Chunk * kRowBytes;       // 4 KB | 8 KB: K chunk
   static constexpr int kVBytes = kA4VRows * kRowBytes;       // 5 KB | 10 KB: V^T chunk and the rows of ones
   static constexpr int kPBytes = 128 * kRowBytes;            // 8 KB | 16 KB
-  static constexpr int kPBufs = kFp8 ? 2 : 1;
+  // Two P buffers per group: with one, P(i) waited for PV(i - 1), i.e. for the MMA warp to wake up and the tensor core to finish,
+  // in every chunk (bf16, 720p: 67.5 -> 60.0 us; 128 buckets 466 -> 428 us).
+  static constexpr int kPBufs = 2;
   static constexpr int kStageBytes = kKBytes + kVBytes;      // 9 KB | 18 KB (a multiple of the swizzle atom: 512 | 1024)
   static constexpr int kQOff = 0;
   static constexpr int kPOff = kQOff + kQBytes;
@@ -347,11 +349,13 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     const uint32_t tmem_o = tmem_base + kOCol + g * kOStride + lane_addr;
     float m_run = -1.0e30f;
     bool ok = true;
+    // every segment a multiple of the chunk (the usual case): no chunk needs a mask, so none is looked up
+    const bool whole = ((seg[1] | seg[3] | seg[5]) & (kA4Chunk - 1)) == 0;
     const int my_chunks = n_chunks > g ? (n_chunks - g + G - 1) / G : 0;
 
     for (int i = 0; i < my_chunks && ok; ++i) {
-      int row, valid;
-      locate_chunk(seg, g + G * i, row, valid);
+      int row, valid = kA4Chunk;
+      if (!whole) locate_chunk(seg, g + G * i, row, valid);
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[g]), i & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
       if (!ok) break;
       tc_fence_after();
