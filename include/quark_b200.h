@@ -118,7 +118,9 @@ typedef struct {
   int32_t reserved;                  /* flags.  bit 0, slice mode: 0 = sum K slices inside a thread-block cluster when there
                                         are 2, 4 or 8 of them (no workspace traffic); 1 = always through the workspace.
                                         bit 1: B is constant (weights; no kernel in flight writes it), so its first tiles
-                                        may be fetched before the kernels ahead of this one in the stream have finished */
+                                        may be fetched before the kernels ahead of this one in the stream have finished.
+                                        bit 2 (qb_gemm_grouped, e4m3 C): the result is rounded to bf16 before it is
+                                        narrowed, as if it had been stored in bf16 and quantised by the next GEMM */
   const float* a_scale; /* [1]  optional */
   const float* w_scale; /* [N]  optional */
 } qb_gemm_params;
@@ -342,6 +344,8 @@ int32_t qb_moe_route_slots(const void* logits, int32_t* slot_token, float* slot_
  * activations in slot order, the A operand of the grouped in-projection (the reference's moe_inproj gathers while it
  * loads, src/quark/functional/moe_inproj.py). */
 int32_t qb_moe_gather(const void* X, const int32_t* slot_token, void* out, int32_t n_slots, int32_t row_bytes, void* stream);
+/* The same from bf16 rows of D elements (a multiple of 16) to e4m3 (as qb_quantize_e4m3): the narrowing and the gather in one pass. */
+int32_t qb_moe_gather_e4m3(const void* X, const int32_t* slot_token, void* out, int32_t n_slots, int32_t D, void* stream);
 /* Grouped GEMM: C[128 i .. 128 i + 127, :] = epilogue(A[same rows] . B[e N .. e N + N - 1, :]^T) with e = tile_expert[i];
  * tiles with e < 0 are skipped (their rows of C are left as they are).  A [p->M, K] with p->M a multiple of 128,
  * B [n_experts * p->N, K], C [p->M, p->N]; plain or SiLU epilogue, no bias / gate / scales.  Replaces qf.moe_inproj and

@@ -149,6 +149,7 @@ SIGNATURES = {
     "qb_moe_slots": (_Z, [_I, _I, _I]),
     "qb_moe_route_slots": (_I, [_P, _P, _P, _P, _P, _P, _I, _I, _I, _P]),
     "qb_moe_gather": (_I, [_P, _P, _P, _I, _I, _P]),
+    "qb_moe_gather_e4m3": (_I, [_P, _P, _P, _I, _I, _P]),
     "qb_gemm_grouped_workspace_bytes": (_Z, [C.POINTER(GemmParams)]),
     "qb_gemm_grouped": (_I, [_P, _P, _P, _P, _I, C.POINTER(GemmParams), _P, _Z, _P]),
     "qb_moe_reduce": (_I, [_P, _P, _P, _P, _I, _I, _I, _P]),

@@ -323,6 +323,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               st_global_v8(dst + 16 * h, w);
             }
           } else if (g.c_dtype == QB_E4M3) {
+            if (g.through_bf16) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
+            }
             uint32_t w[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) w[j] = pack_e4m3x4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
@@ -613,7 +617,7 @@ static int32_t validate_gemm(const qb_gemm_params* p) {
   QB_REQUIRE(p->activation == 0 || p->activation == 1, QB_ERR_INVALID_ARG, "gemm: activation %d", p->activation);
   QB_REQUIRE(p->tile_n == 0 || p->tile_n == 64 || p->tile_n == 128 || p->tile_n == 256, QB_ERR_INVALID_ARG, "gemm: tile_n %d", p->tile_n);
   QB_REQUIRE(p->split_k >= 0 && p->split_k <= 16, QB_ERR_INVALID_ARG, "gemm: split_k %d", p->split_k);
-  QB_REQUIRE(p->reserved >= 0 && p->reserved <= 3, QB_ERR_INVALID_ARG, "gemm: flags %d", p->reserved);
+  QB_REQUIRE(p->reserved >= 0 && p->reserved <= 7, QB_ERR_INVALID_ARG, "gemm: flags %d", p->reserved);
   return QB_OK;
 }
 
@@ -756,6 +760,8 @@ static int32_t gemm_run(const void* A, const void* B, void* C, const void* bias,
   g.kb_total = pl.kb_total; g.kb_per_split = pl.kb_per_split; g.splits = pl.splits;
   g.cluster = pl.cluster;
   g.b_const = (p->reserved & 2) != 0;
+  g.through_bf16 = (p->reserved & 4) != 0;
+  QB_REQUIRE(!g.through_bf16 || tile_expert != nullptr, QB_ERR_UNSUPPORTED, "gemm: flag bit 2 belongs to the grouped GEMM");
   g.c_dtype = p->c_dtype; g.activation = p->activation; g.rows_per_gate = rows_per_gate;
   g.a_scale = p->a_scale; g.w_scale = p->w_scale;
   g.bias = static_cast<const uint16_t*>(bias);

@@ -41,6 +41,7 @@ struct GemmArgs {
   int a_rows;  // rows of A in a box: 128, or M rounded up to 8 below that (rows past it hold what was there: never stored)
   int kb_total, kb_per_split, splits;
   int cluster;  // K slices are the CTAs of one thread-block cluster and are summed through distributed shared memory
+  int through_bf16;  // an e4m3 C is rounded to bf16 first (grouped GEMM)
   int b_const;  // no kernel still in flight writes B (weights): its first tiles are fetched ahead of the grid dependency
   int c_dtype, activation, rows_per_gate;
   const float* a_scale;
@@ -106,6 +107,10 @@ __device__ __forceinline__ void epilogue_store8(const GemmArgs& g, float (&v)[8]
     o.w = pack_bf16x2(v[6], v[7]);
     *reinterpret_cast<uint4*>(static_cast<uint16_t*>(g.C) + off) = o;
   } else if (g.c_dtype == QB_E4M3) {
+    if (g.through_bf16) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
+    }
     uint2 o;
     o.x = pack_e4m3x4(v[0], v[1], v[2], v[3]);
     o.y = pack_e4m3x4(v[4], v[5], v[6], v[7]);

@@ -413,96 +413,148 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* partials,
 constexpr int kMoeTile = 128;
 constexpr int kMoeRouteThreads = 1024;
 
-__device__ __forceinline__ void moe_topk(const uint16_t* row, int E, int top_k, int (&ex)[kMoeMaxExperts], float (&wt)[kMoeMaxExperts]) {
-  float l[kMoeMaxExperts];
-  for (int e = 0; e < E; ++e) l[e] = bf16_bits_to_f32(row[e]);
-  unsigned taken = 0;
-  float top = 0.f, sum = 0.f;
-  for (int k = 0; k < top_k; ++k) {
-    int best = -1;
-    for (int e = 0; e < E; ++e)
-      if (!((taken >> e) & 1u) && (best < 0 || l[e] > l[best])) best = e;
-    taken |= 1u << best;
-    if (k == 0) top = l[best];
-    ex[k] = best;
-    wt[k] = expf(l[best] - top);
-    sum += wt[k];
+// The logits of one token in registers (-inf past E, which no choice reaches: an equal logit never replaces a lower index).
+template <int kE>
+__device__ __forceinline__ void moe_logits(const uint16_t* row, int E, bool vec, float (&l)[kE]) {
+#pragma unroll
+  for (int v = 0; v < kE / 8; ++v) {
+    if (vec && v * 8 < E) {
+      const uint4 x = *reinterpret_cast<const uint4*>(row + v * 8);
+      float f[8];
+      unpack8(x, f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) l[v * 8 + j] = f[j];
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) l[v * 8 + j] = v * 8 + j < E ? bf16_bits_to_f32(row[v * 8 + j]) : __uint_as_float(0xff800000u);
+    }
   }
-  for (int k = 0; k < top_k; ++k) wt[k] = wt[k] / sum;
+}
+// The largest logit whose expert is not in `taken` (the lowest index of equal ones).
+template <int kE>
+__device__ __forceinline__ int moe_best(const float (&l)[kE], unsigned taken, float& value) {
+  int best = -1;
+#pragma unroll
+  for (int e = 0; e < kE; ++e) {
+    if (!((taken >> e) & 1u) && (best < 0 || l[e] > value)) {
+      best = e;
+      value = l[e];
+    }
+  }
+  return best;
 }
 
+// One thread per token, 1024 tokens at a time.  A choice's rank among its expert's is made of the choices of earlier chunks, of
+// earlier warps (a scan over the warps' counts, one warp per expert) and of earlier lanes (the warp's ballot).  Logits and choices
+// stay in registers: with arrays indexed by the choice, counts through shared atomics and a loop over the warps per choice 512
+// tokens of 8 experts took 10 us.
+template <int kE>
 __global__ void __launch_bounds__(kMoeRouteThreads) moe_route_slots_kernel(const uint16_t* logits, int* slot_token,
                                                                             float* slot_weight, int* tile_expert,
                                                                             int* token_slot, int* counts_out, int M, int E,
                                                                             int top_k, int n_slots) {
   grid_dep_wait();
   grid_dep_launch();
-  __shared__ int count[kMoeMaxExperts], offset[kMoeMaxExperts + 1], base[kMoeMaxExperts];
-  __shared__ int warp_tot[kMoeMaxExperts][kMoeRouteThreads / 32];
+  constexpr int kWarps = kMoeRouteThreads / 32;
+  __shared__ int count[32], offset[33], base[32];
+  __shared__ unsigned mask[kWarps][32];  // [warp][expert]: lanes that chose it
+  __shared__ int before[kWarps][33];     // [warp][expert]: choices of earlier warps of the chunk
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid < kMoeMaxExperts) count[tid] = 0;
-  __syncthreads();
-  int ex[kMoeMaxExperts];
-  float wt[kMoeMaxExperts];
-  // pass 1: how many tokens each expert receives
-  for (int t = tid; t < M; t += kMoeRouteThreads) {
-    moe_topk(logits + static_cast<size_t>(t) * E, E, top_k, ex, wt);
-    for (int k = 0; k < top_k; ++k) atomicAdd(&count[ex[k]], 1);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    int cum = 0;
-    for (int e = 0; e < E; ++e) {
-      offset[e] = cum;
-      base[e] = 0;
-      cum += (count[e] + kMoeTile - 1) / kMoeTile * kMoeTile;
-      if (counts_out != nullptr) counts_out[e] = count[e];
-    }
-    offset[E] = cum;
-  }
-  __syncthreads();
-  // pass 2: tokens in chunks of one per thread, in order; a choice's rank among its expert's = choices of earlier chunks
-  // + of earlier warps of this chunk + of earlier lanes of this warp
-  for (int t0 = 0; t0 < M; t0 += kMoeRouteThreads) {
-    const int t = t0 + tid;
-    const bool live = t < M;
-    if (live) moe_topk(logits + static_cast<size_t>(t) * E, E, top_k, ex, wt);
+  const bool vec = E % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15u) == 0;
+  const int n_chunks = (M + kMoeRouteThreads - 1) / kMoeRouteThreads;
+  float l[kE];
+  float top = 0.f, sum = 0.f;
+  bool live = false;
+  // a chunk's choices, its masks and the scan over its warps; returns expert `warp`'s choices in the chunk (in warps below E)
+  auto chunk = [&](int c) {
+    const int t = c * kMoeRouteThreads + tid;
+    live = t < M;
     unsigned mine = 0;
-    if (live)
-      for (int k = 0; k < top_k; ++k) mine |= 1u << ex[k];
-    unsigned before[kMoeMaxExperts];  // lanes of this warp that chose expert e, below this lane
-    for (int e = 0; e < E; ++e) {
-      const unsigned b = __ballot_sync(0xffffffffu, (mine >> e) & 1u);
-      before[e] = __popc(b & ((1u << lane) - 1u));
-      if (lane == 0) warp_tot[e][warp] = __popc(b);
-    }
-    __syncthreads();
+    sum = 0.f;
     if (live) {
+      moe_logits<kE>(logits + static_cast<size_t>(t) * E, E, vec, l);
       for (int k = 0; k < top_k; ++k) {
-        const int e = ex[k];
-        int rank = base[e] + static_cast<int>(before[e]);
-        for (int w = 0; w < warp; ++w) rank += warp_tot[e][w];
-        const int slot = offset[e] + rank;
+        float v = 0.f;
+        mine |= 1u << moe_best<kE>(l, mine, v);
+        if (k == 0) top = v;
+        sum += expf(v - top);
+      }
+    }
+    unsigned own = 0;
+#pragma unroll
+    for (int e = 0; e < kE; ++e) {
+      const unsigned b = __ballot_sync(0xffffffffu, (mine >> e) & 1u);
+      if (lane == e) own = b;
+    }
+    mask[warp][lane] = own;
+    __syncthreads();
+    int total = 0;
+    if (warp < E) {
+      const int n = __popc(mask[lane][warp]);
+      int inc = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += x;
+      }
+      before[lane][warp] = inc - n;
+      total = __shfl_sync(0xffffffffu, inc, 31);
+    }
+    return total;
+  };
+  if (tid < 32) {
+    count[tid] = 0;
+    base[tid] = 0;
+  }
+  for (int c = 0; c < n_chunks; ++c) {  // how many tokens each expert receives
+    __syncthreads();
+    const int total = chunk(c);
+    if (warp < E && lane == 0) count[warp] += total;
+  }
+  __syncthreads();
+  if (warp == 0) {  // first slot of each expert's run
+    const int n = lane < E ? count[lane] : 0;
+    if (lane < E && counts_out != nullptr) counts_out[lane] = n;
+    const int padded = (n + kMoeTile - 1) / kMoeTile * kMoeTile;
+    int inc = padded;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += x;
+    }
+    offset[lane] = inc - padded;
+    if (lane == 31) offset[32] = inc;
+  }
+  __syncthreads();
+  for (int c = 0; c < n_chunks; ++c) {
+    int total = 0;
+    if (n_chunks > 1) {  // a single chunk's state is still there
+      total = chunk(c);
+      __syncthreads();
+    }
+    if (live) {
+      const int t = c * kMoeRouteThreads + tid;
+      unsigned taken = 0;
+      for (int k = 0; k < top_k; ++k) {
+        float v = 0.f;
+        const int e = moe_best<kE>(l, taken, v);
+        taken |= 1u << e;
+        const int slot = offset[e] + base[e] + before[warp][e] + __popc(mask[warp][e] & ((1u << lane) - 1u));
         slot_token[slot] = t;
-        slot_weight[slot] = wt[k];
+        slot_weight[slot] = expf(v - top) / sum;
         token_slot[static_cast<size_t>(t) * top_k + k] = slot;
       }
     }
     __syncthreads();
-    if (tid < E) {
-      int tot = 0;
-      for (int w = 0; w < kMoeRouteThreads / 32; ++w) tot += warp_tot[tid][w];
-      base[tid] += tot;
-    }
-    __syncthreads();
+    if (n_chunks > 1 && warp < E && lane == 0) base[warp] += total;
   }
   // padding slots and the tile table
-  for (int e = 0; e < E; ++e)
-    for (int s = offset[e] + count[e] + tid; s < offset[e + 1]; s += kMoeRouteThreads) {
+  for (int e = warp; e < E; e += kWarps)
+    for (int s = offset[e] + count[e] + lane; s < (e + 1 < E ? offset[e + 1] : offset[32]); s += 32) {
       slot_token[s] = -1;
       slot_weight[s] = 0.f;
     }
-  for (int s = offset[E] + tid; s < n_slots; s += kMoeRouteThreads) {
+  for (int s = offset[32] + tid; s < n_slots; s += kMoeRouteThreads) {
     slot_token[s] = -1;
     slot_weight[s] = 0.f;
   }
@@ -510,7 +562,7 @@ __global__ void __launch_bounds__(kMoeRouteThreads) moe_route_slots_kernel(const
     const int s = i * kMoeTile;
     int e = -1;
     for (int q = 0; q < E; ++q)
-      if (s >= offset[q] && s < offset[q + 1]) e = q;
+      if (s >= offset[q] && s < offset[q] + count[q]) e = q;
     tile_expert[i] = e;
   }
 }
@@ -526,6 +578,27 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const uint8_t* X, const
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (t >= 0) v = *reinterpret_cast<const uint4*>(X + static_cast<size_t>(t) * row_bytes + b);
     *reinterpret_cast<uint4*>(out + static_cast<size_t>(s) * row_bytes + b) = v;
+  }
+}
+
+// The same with the narrowing to e4m3 of what it gathers (16 elements per thread): the e4m3 experts' operand in one pass.
+__global__ void __launch_bounds__(128) moe_gather_e4m3_kernel(const uint16_t* X, const int* slot_token, uint8_t* out, int D) {
+  grid_dep_wait();
+  grid_dep_launch();
+  const int s = blockIdx.x;
+  const int t = slot_token[s];
+  for (int d = threadIdx.x * 16; d < D; d += 128 * 16) {
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (t >= 0) {
+      const uint4* x = reinterpret_cast<const uint4*>(X + static_cast<size_t>(t) * D + d);
+      float f[8];
+      unpack8(x[0], f);
+      const uint2 lo = pack8_e4m3(f);
+      unpack8(x[1], f);
+      const uint2 hi = pack8_e4m3(f);
+      v = make_uint4(lo.x, lo.y, hi.x, hi.y);
+    }
+    *reinterpret_cast<uint4*>(out + static_cast<size_t>(s) * D + d) = v;
   }
 }
 
@@ -892,7 +965,8 @@ int32_t qb_moe_route_slots(const void* logits, int32_t* slot_token, float* slot_
   QB_REQUIRE(M > 0 && E > 0 && E <= kMoeMaxExperts && top_k > 0 && top_k <= E, QB_ERR_INVALID_ARG, "moe_route_slots: M %d, E %d (at most %d), top_k %d", M, E,
              kMoeMaxExperts, top_k);
   const int n_slots = static_cast<int>(qb_moe_slots(M, E, top_k));
-  return launch_dep("moe_route_slots", moe_route_slots_kernel, dim3(1), dim3(kMoeRouteThreads), 0, static_cast<cudaStream_t>(stream),
+  auto kernel = E <= 8 ? moe_route_slots_kernel<8> : E <= 16 ? moe_route_slots_kernel<16> : moe_route_slots_kernel<32>;
+  return launch_dep("moe_route_slots", kernel, dim3(1), dim3(kMoeRouteThreads), 0, static_cast<cudaStream_t>(stream),
                     static_cast<const uint16_t*>(logits), slot_token, slot_weight, tile_expert, token_slot, counts, M, E, top_k, n_slots);
 }
 
@@ -902,6 +976,14 @@ int32_t qb_moe_gather(const void* X, const int32_t* slot_token, void* out, int32
   QB_REQUIRE(aligned16(X) && aligned16(out), QB_ERR_ALIGN, "moe_gather: pointers must be 16-byte aligned");
   return launch_dep("moe_gather", moe_gather_kernel, dim3(n_slots), dim3(256), 0, static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(X),
                     slot_token, static_cast<uint8_t*>(out), row_bytes);
+}
+
+int32_t qb_moe_gather_e4m3(const void* X, const int32_t* slot_token, void* out, int32_t n_slots, int32_t D, void* stream) {
+  QB_REQUIRE(X && slot_token && out, QB_ERR_INVALID_ARG, "moe_gather_e4m3: NULL pointer");
+  QB_REQUIRE(n_slots > 0 && D > 0 && D % 16 == 0, QB_ERR_INVALID_ARG, "moe_gather_e4m3: %d slots of %d elements (a multiple of 16)", n_slots, D);
+  QB_REQUIRE(aligned16(X) && aligned16(out), QB_ERR_ALIGN, "moe_gather_e4m3: pointers must be 16-byte aligned");
+  return launch_dep("moe_gather_e4m3", moe_gather_e4m3_kernel, dim3(n_slots), dim3(128), 0, static_cast<cudaStream_t>(stream),
+                    static_cast<const uint16_t*>(X), slot_token, static_cast<uint8_t*>(out), D);
 }
 
 int32_t qb_moe_reduce(const float* partials, const float* slot_weight, const int32_t* token_slot, void* out, int32_t M, int32_t D, int32_t top_k,

@@ -749,9 +749,15 @@ def moe_route_slots(logits, *, top_k: int, slot_token=None, slot_weight=None, ti
 
 
 def moe_gather(x, slot_token, *, out=None):
-    """``out[s] = x[slot_token[s]]`` (zeros for padding slots): the activations in slot order."""
+    """``out[s] = x[slot_token[s]]`` (zeros for padding slots): the activations in slot order.  An e4m3 ``out`` of a bf16 ``x``
+    receives them narrowed as ``quantize_e4m3`` does."""
     D = int(x.shape[-1])
     n = slot_token.numel
+    if out is not None and _dt(out) == "e4m3" and _dt(x) == "bf16":
+        if out.numel != n * D:
+            raise ValueError(f"qf.moe_gather: out must be [{n}, {D}]")
+        _lib.check(_lib.load().qb_moe_gather_e4m3(_p(x), _p(slot_token), _p(out), n, D, _s()))
+        return out
     es = {"bf16": 2, "e4m3": 1, "f32": 4}[_dt(x)]
     if out is None:
         out = QuarkTensor.empty(n, D, dtype=_dt(x))
@@ -761,9 +767,11 @@ def moe_gather(x, slot_token, *, out=None):
     return out
 
 
-def gemm_grouped(A, B, tile_expert, *, n_experts: int, out_dtype="bf16", compute_dtype=None, activation=None, out=None, b_constant=False):
+def gemm_grouped(A, B, tile_expert, *, n_experts: int, out_dtype="bf16", compute_dtype=None, activation=None, out=None, b_constant=False,
+                 through_bf16=False):  # fmt: skip
     """``C[tile i] = A[tile i] @ B[expert(i)].T`` over 128-row tiles of slot-sorted rows; tiles whose expert is -1 are skipped.
-    ``B`` is ``[n_experts * N, K]``.  Replaces ``qf.moe_inproj`` / ``qf.moe_outproj`` (``src/quark/nn/moe.py:307-338``)."""
+    ``B`` is ``[n_experts * N, K]``.  ``through_bf16``: an e4m3 result is rounded to bf16 first, as if it had been stored in bf16 and
+    narrowed by the next GEMM.  Replaces ``qf.moe_inproj`` / ``qf.moe_outproj`` (``src/quark/nn/moe.py:307-338``)."""
     K = int(A.shape[-1])
     M = A.numel // K
     if int(B.shape[0]) % int(n_experts) or int(B.shape[1]) != K:
@@ -780,7 +788,7 @@ def gemm_grouped(A, B, tile_expert, *, n_experts: int, out_dtype="bf16", compute
     elif out.numel != M * N or _dt(out) != out_dtype:
         raise ValueError(f"qf.gemm_grouped: out must be {out_dtype} [{M}, {N}]")
     p = _params(_lib.GemmParams, M, N, K, _code(a_dt), _code(b_dt), _code(_name(out_dtype)), _code(cd), 1 if activation == "silu" else 0, 1, 1, 0,
-                2 if b_constant else 0, None, None)  # fmt: skip
+                (2 if b_constant else 0) | (4 if through_bf16 else 0), None, None)  # fmt: skip
     lib = _lib.load()
     ws = _workspace(_need(p, lib.qb_gemm_grouped_workspace_bytes))
     _lib.check(lib.qb_gemm_grouped(_p(A), _p(B), _p(out), _p(tile_expert), int(n_experts), p[1], _p(ws), ws.nbytes if ws is not None else 0, _s()))

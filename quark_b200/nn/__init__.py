@@ -213,24 +213,26 @@ class MoE(Module):
         M, D, H, E = x.numel // int(x.shape[-1]), self._D, self._H, self._E
         cd = "e4m3" if self._fp8 else None
         logits = self.router(x)
-        xq = qf.quantize_e4m3(x, out=_cached(self, "xq", (M, D), "e4m3")) if self._fp8 else x  # once, not per expert
         if self._schedule == "sorted":
             n = qf.moe_slots(M, E, self._K)
             slot_token, slot_weight, tile_expert, token_slot = qf.moe_route_slots(
                 logits, top_k=self._K, slot_token=_cached(self, "slot_token", (n,), "s32"), slot_weight=_cached(self, "slot_weight", (n,), "f32"),
                 tile_expert=_cached(self, "tile_expert", (n // 128,), "s32"), token_slot=_cached(self, "token_slot", (M, self._K), "s32"),
             )  # fmt: skip
-            xs = qf.moe_gather(xq, slot_token, out=_cached(self, "xs", (n, D), xq.dtype))
+            # e4m3 experts: the tokens are narrowed as they are gathered, the hidden activations (bf16 values) as they are stored
+            od = "e4m3" if self._fp8 else "bf16"
+            xs = qf.moe_gather(x, slot_token, out=_cached(self, "xs", (n, D), od))
             if not getattr(self, "_partials_cleared", False):
                 # rows of padding tiles are never written nor read; start them from zero once so the buffer holds no junk
                 self._partials_cleared = True
-                _cached(self, "h_s", (n, H), "bf16").zero_()
+                _cached(self, "h_s", (n, H), od).zero_()
                 _cached(self, "partials_s", (n, D), "f32").zero_()
-            h = qf.gemm_grouped(xs, self.expert_in.data, tile_expert, n_experts=E, compute_dtype=cd, activation="silu",
-                                out=_cached(self, "h_s", (n, H), "bf16"), b_constant=True)  # fmt: skip
+            h = qf.gemm_grouped(xs, self.expert_in.data, tile_expert, n_experts=E, out_dtype=od, compute_dtype=cd, activation="silu",
+                                out=_cached(self, "h_s", (n, H), od), b_constant=True, through_bf16=self._fp8)  # fmt: skip
             partials = qf.gemm_grouped(h, self.expert_out.data, tile_expert, n_experts=E, out_dtype="f32", compute_dtype=cd,
                                        out=_cached(self, "partials_s", (n, D), "f32"), b_constant=True)  # fmt: skip
             return qf.moe_reduce(partials, slot_weight, token_slot, out=_cached(self, "out", (M, D), "bf16"))
+        xq = qf.quantize_e4m3(x, out=_cached(self, "xq", (M, D), "e4m3")) if self._fp8 else x  # once, not per expert
         weights = qf.moe_route(logits, top_k=self._K, out=_cached(self, "weights", (E, M), "f32"))
         h = _cached(self, "h", (M, H), "bf16")
         partials = _cached(self, "partials", (E * M, D), "f32")
