@@ -66,13 +66,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) QB_GT(0);
-  int b_row0 = 0;  // first row of this tile's expert in B
-  if (g.tile_expert != nullptr) {
-    grid_dep_wait();  // the table is written by the routing kernel just before
-    const int expert = g.tile_expert[blockIdx.y];
-    if (expert < 0) return;  // a padding tile: nothing allocated yet, the whole CTA leaves
-    b_row0 = expert * g.N;
-  }
   const int n0 = blockIdx.x * BN;
   const int m0 = blockIdx.y * kBM;
   const int split = blockIdx.z;
@@ -116,7 +109,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       for (int it = 0; it < ahead; ++it) {
         const uint32_t fb = smem_u32(&full_bar[it]);
         mbar_arrive_expect_tx(fb, stage_tx);
-        tma_load_2d(smem_u32(smem + it * L::kStageBytes + kBM * kRowBytes), &tmB, fb, (kb0 + it) * kKElems, b_row0 + n0);
+        tma_load_2d(smem_u32(smem + it * L::kStageBytes + kBM * kRowBytes), &tmB, fb, (kb0 + it) * kKElems, n0);
       }
       grid_dep_wait();
       QB_GT(2);
@@ -131,7 +124,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         mbar_arrive_expect_tx(fb, stage_tx);
         uint8_t* a_s = smem + s * L::kStageBytes;
         tma_load_2d(smem_u32(a_s), &tmA, fb, (kb0 + it) * kKElems, m0);
-        tma_load_2d(smem_u32(a_s + kBM * kRowBytes), &tmB, fb, (kb0 + it) * kKElems, b_row0 + n0);
+        tma_load_2d(smem_u32(a_s + kBM * kRowBytes), &tmB, fb, (kb0 + it) * kKElems, n0);
         issued = it + 1;
       }
       if (*abort_flag) {
@@ -323,10 +316,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               st_global_v8(dst + 16 * h, w);
             }
           } else if (g.c_dtype == QB_E4M3) {
-            if (g.through_bf16) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
-            }
             uint32_t w[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) w[j] = pack_e4m3x4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
@@ -534,8 +523,8 @@ extern "C" void qb_debug_gemm_tune(int cg, int bn, int s) { g_tune[0] = cg; g_tu
 static bool cluster_slices(int cg, int bn, int s) { return cg == 1 ? bn == 64 && (s == 2 || s == 4 || s == 8) : bn == 128 && s == 2; }
 
 // Picks the CTAs per tile, the tile width and the number of K slices from a small cost model in ns, so that every call with the
-// same shape makes the same choice.  `grouped`: 128-row tiles belong to different experts, so no pairs and no slices.
-static GemmPlan plan_gemm(const qb_gemm_params& p, bool grouped = false, int max_cg = 2, double* cost_out = nullptr) {
+// same shape makes the same choice.
+static GemmPlan plan_gemm(const qb_gemm_params& p, int max_cg = 2, double* cost_out = nullptr) {
   const bool fp8 = p.compute_dtype == QB_E4M3;
   const int k_elems = fp8 ? 128 : 64;
   GemmPlan best{};
@@ -545,7 +534,7 @@ static GemmPlan plan_gemm(const qb_gemm_params& p, bool grouped = false, int max
   const int bns[3] = {256, 128, 64};
   const int ss[10] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16};
   for (int cg = 1; cg <= max_cg; ++cg) {
-    if (cg == 2 && (grouped || p.M <= kBM || (p.reserved & 1) != 0)) continue;
+    if (cg == 2 && (p.M <= kBM || (p.reserved & 1) != 0)) continue;
     for (int bn : bns) {
       if (p.tile_n != 0 && p.tile_n != bn) continue;
       if (cg == 2 && bn == 64) continue;
@@ -553,7 +542,7 @@ static GemmPlan plan_gemm(const qb_gemm_params& p, bool grouped = false, int max
       const int tiles = ((p.M + cg * kBM - 1) / (cg * kBM)) * ((p.N + bn - 1) / bn);
       for (int s : ss) {
         if (p.split_k != 0 && p.split_k != s) continue;
-        if (s > kb_total || (grouped && s > 1)) continue;
+        if (s > kb_total) continue;
 #ifdef QB_GEMM_TUNE
         if ((g_tune[0] && g_tune[0] != cg) || (g_tune[1] && g_tune[1] != bn) || (g_tune[2] && g_tune[2] != s)) continue;
 #endif
@@ -707,11 +696,35 @@ static GemmPlan plan_qkv(const qb_gemm_params& p, const QkvTail& t) {
       q.tile_n = bn;
       q.split_k = s;
       double cost = 0;
-      const GemmPlan pl = plan_gemm(q, false, 1, &cost);
+      const GemmPlan pl = plan_gemm(q, 1, &cost);
       if (pl.splits == s && pl.cluster == (s > 1) && cost < best_cost) {
         best_cost = cost;
         best = pl;
       }
+    }
+  }
+  return best;
+}
+
+// Column width of the grouped GEMM's tiles: the one whose CTAs (256 rows of an expert each) take the fewest rounds over the SMs, by
+// the rows that its slots leave once every expert's run is padded to 128.
+static int plan_grouped(const qb_gemm_params& p, int n_experts) {
+  if (p.tile_n != 0) return p.tile_n;
+  const int kb = (p.K + (p.compute_dtype == QB_E4M3 ? 127 : 63)) / (p.compute_dtype == QB_E4M3 ? 128 : 64);
+  int rows = p.M - kBM * n_experts;
+  if (rows < p.M / 2) rows = p.M / 2;
+  const int per_expert = rows / n_experts + 1;
+  const bool two = per_expert > 96;  // about every second run then spills into a second tile of 128 rows
+  int best = 64;
+  double best_cost = 1e30;
+  for (int bn = 64; bn <= 256; bn *= 2) {
+    if (bn > 64 && bn / 2 >= p.N) continue;
+    const int ctas = n_experts * ((per_expert + 255) / 256) * ((p.N + bn - 1) / bn);
+    const double per_kb = two ? (bn == 64 ? 240.0 : bn == 128 ? 300.0 : 540.0) : (bn == 64 ? 150.0 : bn == 128 ? 220.0 : 420.0);
+    const double cost = ((ctas + num_sms() - 1) / num_sms()) * (kb * per_kb + 3500.0 + bn * 6.0);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = bn;
     }
   }
   return best;
@@ -732,7 +745,7 @@ static int32_t gemm_run(const void* A, const void* B, void* C, const void* bias,
                p->gate_groups, p->M);
     rows_per_gate = p->M / p->gate_groups;
   }
-  GemmPlan pl = plan_gemm(*p, tile_expert != nullptr, tp != nullptr ? 1 : 2);
+  GemmPlan pl = plan_gemm(*p, tp != nullptr ? 1 : 2);
   if (tail != nullptr) pl = plan_qkv(*p, *tail);
   const size_t need = pl.counters_bytes + pl.aq_bytes + pl.partial_bytes;
   const bool uses_ws = pl.aq_bytes > 0 || pl.partial_bytes > 0;
@@ -783,20 +796,20 @@ static int32_t gemm_run(const void* A, const void* B, void* C, const void* bias,
     g.qkv = *tail;
   }
   if (tile_expert != nullptr) {
+    QB_REQUIRE(p->M % kBM == 0, QB_ERR_UNSUPPORTED, "gemm_grouped: M = %d must be a multiple of 128", p->M);
     // per-column vectors would have to be per expert
-    // (a B tile that runs past the expert's last row only feeds columns >= N, which no epilogue stores)
-    QB_REQUIRE(pl.splits == 1 && p->M % kBM == 0, QB_ERR_UNSUPPORTED, "gemm_grouped: needs one K slice and M = %d a multiple of 128", p->M);
     QB_REQUIRE(tail == nullptr && tp == nullptr && bias == nullptr && gate == nullptr && p->w_scale == nullptr,
                QB_ERR_UNSUPPORTED, "gemm_grouped: takes the plain or the SiLU epilogue only");
     g.tile_expert = tile_expert;
   }
 
+  if (tile_expert != nullptr) return launch_gemm_grouped(plan_grouped(*p, n_experts), a_ptr, B, n_experts, g, fp8, st);
   if (pl.cg == 2) return launch_gemm_pair(pl, a_ptr, B, g, fp8, st);
   CUtensorMap tmA, tmB;
   const int es = fp8 ? 1 : 2;
   rc = make_tmap_2d(&tmA, a_ptr, es, p->M, p->K, g.a_rows);
   if (rc != QB_OK) return rc;
-  rc = make_tmap_2d(&tmB, B, es, static_cast<uint64_t>(p->N) * n_experts, p->K, pl.bn);
+  rc = make_tmap_2d(&tmB, B, es, p->N, p->K, pl.bn);
   if (rc != QB_OK) return rc;
 
   dim3 grid((p->N + pl.bn - 1) / pl.bn, (p->M + kBM - 1) / kBM, pl.splits);

@@ -59,8 +59,8 @@ struct GemmArgs {
   // plain stores over NVLink): tp_dst[owner] + (m % tp_rpo) * N.  tp_world == 0: the ordinary output C.
   int tp_world, tp_rpo;
   uint16_t* tp_dst[8];
-  // Grouped GEMM (mixture of experts): the 128-row tile i of A belongs to expert tile_expert[i] and is multiplied with
-  // rows [expert * N, expert * N + N) of B; a tile with expert -1 is skipped.  NULL: the ordinary GEMM.
+  // Grouped GEMM (mixture of experts, gemm_grouped.cu): the 128-row tile i of A belongs to expert tile_expert[i] and is multiplied
+  // with rows [expert * N, expert * N + N) of B; a tile with expert -1 is skipped.
   const int* tile_expert;
   // Pairs of CTAs only: the walk over the tiles (see tile_at in gemm_pair.cu) and the shared memory's layout
   int tiles_m, n_tiles, group_m, stages, scratch;
@@ -107,10 +107,6 @@ __device__ __forceinline__ void epilogue_store8(const GemmArgs& g, float (&v)[8]
     o.w = pack_bf16x2(v[6], v[7]);
     *reinterpret_cast<uint4*>(static_cast<uint16_t*>(g.C) + off) = o;
   } else if (g.c_dtype == QB_E4M3) {
-    if (g.through_bf16) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
-    }
     uint2 o;
     o.x = pack_e4m3x4(v[0], v[1], v[2], v[3]);
     o.y = pack_e4m3x4(v[4], v[5], v[6], v[7]);
@@ -216,6 +212,95 @@ __device__ __forceinline__ void finish_slices(const GemmArgs& g, const float4* p
     }
     if (one_gate) epilogue_store8_staged<BN>(g, v, m, n, col + c8 * 8, pre[k][0]);
     else epilogue_store8(g, v, m, n);
+  }
+}
+
+// Row m of the output in bytes.
+__device__ __forceinline__ uint8_t* row_of_c(const GemmArgs& g, int m) {
+  if (g.tp_world != 0) {
+    const int owner = m / g.tp_rpo;
+    return reinterpret_cast<uint8_t*>(g.tp_dst[owner] + static_cast<size_t>(m - owner * g.tp_rpo) * g.N);
+  }
+  const int es = g.c_dtype == QB_BF16 ? 2 : g.c_dtype == QB_E4M3 ? 1 : 4;
+  return static_cast<uint8_t*>(g.C) + static_cast<size_t>(m) * g.N * es;
+}
+
+// The plain epilogue on 16 columns of one row: r the accumulator, `col` at the first column's scale (bias BN, gate 2 BN words
+// further), `res` the residual.  Kept small and called in a loop: unrolled over the half row, with every branch in it, the
+// epilogue's instructions cost more to fetch (0.5 us a launch) than they took to run.
+template <int BN>
+__device__ __forceinline__ void epilogue16(const GemmArgs& g, const uint32_t (&r)[16], int m, int n, const float* col, const uint4* res, bool one_gate,
+                                           uint8_t* c_row, bool wide, bool store) {
+  float v[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+  if (g.a_scale != nullptr || g.w_scale != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] *= col[j];
+  }
+  if (g.bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] += col[BN + j];
+  }
+  if (g.activation == 1) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = silu_fast(v[j]);
+  }
+  const bool second = n + 8 < g.N;
+  if (g.gate != nullptr) {
+    const uint4 x = res[0], y = second ? res[1] : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t rw[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    if (one_gate) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[2 * j] = __fadd_rn(bf16lo(rw[j]), __fmul_rn(col[2 * BN + 2 * j], v[2 * j]));
+        v[2 * j + 1] = __fadd_rn(bf16hi(rw[j]), __fmul_rn(col[2 * BN + 2 * j + 1], v[2 * j + 1]));
+      }
+    } else {  // the tile spans several gate rows
+      const uint32_t* gt = reinterpret_cast<const uint32_t*>(g.gate + static_cast<size_t>(m / g.rows_per_gate) * g.N + n);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t w = j < 4 || second ? gt[j] : 0u;
+        v[2 * j] = __fadd_rn(bf16lo(rw[j]), __fmul_rn(bf16lo(w), v[2 * j]));
+        v[2 * j + 1] = __fadd_rn(bf16hi(rw[j]), __fmul_rn(bf16hi(w), v[2 * j + 1]));
+      }
+    }
+  }
+  if (!store) {  // (the values still have to be worked out: see the caller)
+#pragma unroll
+    for (int j = 0; j < 16; ++j) asm volatile("" ::"f"(v[j]));
+    return;
+  }
+  if (g.c_dtype == QB_BF16) {
+    uint32_t w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+    uint4* d = reinterpret_cast<uint4*>(c_row + 2 * n);
+    if (wide) {
+      st_global_v8(d, w);
+    } else {
+      d[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      if (second) d[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+  } else if (g.c_dtype == QB_E4M3) {
+    if (g.through_bf16) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(v[j]));
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = pack_e4m3x4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    if (wide) {
+      *reinterpret_cast<uint4*>(c_row + n) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else {
+      *reinterpret_cast<uint2*>(c_row + n) = make_uint2(w[0], w[1]);
+      if (second) *reinterpret_cast<uint2*>(c_row + n + 8) = make_uint2(w[2], w[3]);
+    }
+  } else {
+    float4* d = reinterpret_cast<float4*>(c_row + 4 * n);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < 2 || second) d[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
   }
 }
 
@@ -479,7 +564,8 @@ struct GemmPlan {
 };
 
 int num_sms();
-// Tensor maps and launch of the pair kernel for a plan with cg == 2.
+// Tensor maps and launch of the grouped kernel, and of the pair kernel for a plan with cg == 2.
+int32_t launch_gemm_grouped(int bn, const void* A, const void* B, int n_experts, const GemmArgs& g, bool fp8, cudaStream_t st);
 int32_t launch_gemm_pair(const GemmPlan& pl, const void* A, const void* B, const GemmArgs& g, bool fp8, cudaStream_t st);
 int32_t make_tmap_2d_sw(CUtensorMap* tm, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols,
                         int swizzle_bytes);
