@@ -95,6 +95,8 @@ __global__ void __launch_bounds__(kThreads, kMaxVec == 1 ? 4 : 2) ada_rmsnorm_ke
 // 8 threads per (row, head): 8 x 8 = 64 elements; heads >= n_norm_heads (the V heads) are copied.
 __global__ void __launch_bounds__(256) head_rmsnorm_kernel(const uint16_t* X, uint16_t* out, int rows,
                                                             int heads_total, int n_norm_heads, float eps) {
+  grid_dep_wait();
+  grid_dep_launch();
   const size_t gid = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   const size_t item = gid >> 3;  // (row, head)
   const int sub = gid & 7;
@@ -125,6 +127,8 @@ __global__ void __launch_bounds__(256) head_rmsnorm_kernel(const uint16_t* X, ui
 __global__ void __launch_bounds__(256) value_residual_kernel(const uint16_t* cur, const uint16_t* first,
                                                               const float* lamb, uint16_t* out, int rows,
                                                               int D_full, int v_off, int v_width) {
+  grid_dep_wait();
+  grid_dep_launch();
   const size_t i8 = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 8;
   if (i8 >= static_cast<size_t>(rows) * D_full) return;
   const int col = static_cast<int>(i8 % D_full);
@@ -145,6 +149,8 @@ __global__ void __launch_bounds__(256) value_residual_kernel(const uint16_t* cur
 __global__ void __launch_bounds__(256) gate_residual_kernel(const uint16_t* X, const uint16_t* Y,
                                                              const uint16_t* gate, uint16_t* out, int rows,
                                                              int D, int rows_per_group) {
+  grid_dep_wait();
+  grid_dep_launch();
   const size_t i8 = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 8;
   if (i8 >= static_cast<size_t>(rows) * D) return;
   const int row = static_cast<int>(i8 / D), col = static_cast<int>(i8 % D);
@@ -160,6 +166,8 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(const uint16_t* X, c
 // ---------------------------------------------------------------- SiLU / Euler / quantise
 __global__ void __launch_bounds__(256) silu_kernel(const uint16_t* X, uint16_t* out, uint8_t* out_q,
                                                     size_t n) {
+  grid_dep_wait();
+  grid_dep_launch();
   const size_t i8 = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 8;
   if (i8 + 8 <= n) {
     float f[8];
@@ -268,6 +276,7 @@ __global__ void __launch_bounds__(256) euler_kernel(const uint16_t* X, const uin
 
 template <bool kFromF32>
 __global__ void __launch_bounds__(256) quantize_kernel(const void* X, uint8_t* out, size_t n) {
+  grid_dep_wait();  // (no early release: what follows may be a GEMM that fetches these weights before its own wait)
   const size_t i8 = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 8;
   if (i8 + 8 <= n) {
     float f[8];
@@ -809,11 +818,8 @@ __global__ void __launch_bounds__(256) patch_move_kernel(const uint16_t* src, ui
 int32_t quantize_e4m3_launch(const void* X, void* out, size_t n, int32_t src_dtype, cudaStream_t st) {
   if (n == 0) return QB_OK;
   const unsigned blocks = static_cast<unsigned>((n + 2047) / 2048);
-  if (src_dtype == QB_F32)
-    quantize_kernel<true><<<blocks, 256, 0, st>>>(X, static_cast<uint8_t*>(out), n);
-  else
-    quantize_kernel<false><<<blocks, 256, 0, st>>>(X, static_cast<uint8_t*>(out), n);
-  return check_launch("quantize_e4m3");
+  return launch_dep("quantize_e4m3", src_dtype == QB_F32 ? quantize_kernel<true> : quantize_kernel<false>, dim3(blocks), dim3(256), 0, st, X,
+                    static_cast<uint8_t*>(out), n);
 }
 
 }  // namespace qb
@@ -862,9 +868,8 @@ int32_t qb_head_rmsnorm(const void* X, void* out, int32_t rows, int32_t n_q_head
   QB_REQUIRE(aligned16(X) && aligned16(out), QB_ERR_ALIGN, "head_rmsnorm: pointers must be 16-byte aligned");
   const int heads_total = n_q_heads + 2 * n_kv_heads;
   const size_t threads = static_cast<size_t>(rows) * heads_total * 8;
-  head_rmsnorm_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint16_t*>(X), static_cast<uint16_t*>(out), rows, heads_total, n_q_heads + n_kv_heads, eps);
-  return check_launch("head_rmsnorm");
+  return launch_dep("head_rmsnorm", head_rmsnorm_kernel, dim3(static_cast<unsigned>((threads + 255) / 256)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                    static_cast<const uint16_t*>(X), static_cast<uint16_t*>(out), rows, heads_total, n_q_heads + n_kv_heads, eps);
 }
 
 int32_t qb_value_residual_packed(const void* cur, const void* first, const float* lamb, void* out, int32_t rows, int32_t D_full,
@@ -874,10 +879,8 @@ int32_t qb_value_residual_packed(const void* cur, const void* first, const float
              "value_residual_packed: bad sizes");
   QB_REQUIRE(D_full % 8 == 0 && v_col_offset % 8 == 0 && v_width % 8 == 0, QB_ERR_ALIGN, "value_residual_packed: columns must be multiples of 8");
   QB_REQUIRE(aligned16(cur) && aligned16(first) && aligned16(out), QB_ERR_ALIGN, "value_residual_packed: pointers must be 16-byte aligned");
-  value_residual_kernel<<<blocks_for(static_cast<size_t>(rows) * D_full), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint16_t*>(cur), static_cast<const uint16_t*>(first), lamb, static_cast<uint16_t*>(out), rows, D_full,
-      v_col_offset, v_width);
-  return check_launch("value_residual_packed");
+  return launch_dep("value_residual_packed", value_residual_kernel, dim3(blocks_for(static_cast<size_t>(rows) * D_full)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                    static_cast<const uint16_t*>(cur), static_cast<const uint16_t*>(first), lamb, static_cast<uint16_t*>(out), rows, D_full, v_col_offset, v_width);
 }
 
 int32_t qb_ada_gate_residual(const void* X, const void* Y, const void* gate, void* out, int32_t rows, int32_t D, int32_t groups,
@@ -886,19 +889,16 @@ int32_t qb_ada_gate_residual(const void* X, const void* Y, const void* gate, voi
   QB_REQUIRE(rows > 0 && D > 0 && groups > 0 && rows % groups == 0, QB_ERR_INVALID_ARG, "ada_gate_residual: bad sizes");
   QB_REQUIRE(D % 8 == 0, QB_ERR_ALIGN, "ada_gate_residual: D must be a multiple of 8");
   QB_REQUIRE(aligned16(X) && aligned16(Y) && aligned16(gate) && aligned16(out), QB_ERR_ALIGN, "ada_gate_residual: pointers must be 16-byte aligned");
-  gate_residual_kernel<<<blocks_for(static_cast<size_t>(rows) * D), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint16_t*>(X), static_cast<const uint16_t*>(Y), static_cast<const uint16_t*>(gate), static_cast<uint16_t*>(out),
-      rows, D, rows / groups);
-  return check_launch("ada_gate_residual");
+  return launch_dep("ada_gate_residual", gate_residual_kernel, dim3(blocks_for(static_cast<size_t>(rows) * D)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                    static_cast<const uint16_t*>(X), static_cast<const uint16_t*>(Y), static_cast<const uint16_t*>(gate), static_cast<uint16_t*>(out), rows, D, rows / groups);
 }
 
 int32_t qb_silu(const void* X, void* out, void* out_q, size_t n, void* stream) {
   QB_REQUIRE(X && (out || out_q), QB_ERR_INVALID_ARG, "silu: NULL pointer");
   QB_REQUIRE(aligned16(X) && aligned16(out) && aligned16(out_q), QB_ERR_ALIGN, "silu: pointers must be 16-byte aligned");
   if (n == 0) return QB_OK;
-  silu_kernel<<<blocks_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint16_t*>(X), static_cast<uint16_t*>(out),
-                                                                            static_cast<uint8_t*>(out_q), n);
-  return check_launch("silu");
+  return launch_dep("silu", silu_kernel, dim3(blocks_for(n)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                    static_cast<const uint16_t*>(X), static_cast<uint16_t*>(out), static_cast<uint8_t*>(out_q), n);
 }
 
 int32_t qb_rmsnorm(const void* X, void* out, int32_t rows, int32_t D, float eps, void* stream) {

@@ -44,10 +44,12 @@ __global__ void __launch_bounds__(kKvThreads) kv_append_kernel(const KvArgs a) {
   __shared__ float tm[16];
   __shared__ __align__(16) uint16_t vt[kKvTile * kVPitch];
 
+  grid_dep_wait();
+  grid_dep_launch();
   const int head = blockIdx.y;
   const int t0 = blockIdx.x * kKvTile;
-  const int ft = *a.frame_t;
-  const int frozen = *a.frozen;
+  const int ft = *after_wait(a.frame_t);
+  const int frozen = *after_wait(a.frozen);
   const int L = a.nb * a.tpf;
   const int cap = L + a.tpf;
   const int bucket = (ft + a.pd - 1) / a.pd;
@@ -316,11 +318,8 @@ static int32_t kv_append(const void* k_src, const void* v_src, size_t row_stride
   a.quilt = p->quilt_factor; a.qoff = p->quilt_offset;
   a.tpf = tpf; a.nb = p->num_buckets; a.pd = p->pinned_dilation; a.max_segments = p->max_segments;
   dim3 grid((tpf + kKvTile - 1) / kKvTile, p->n_kv_heads);
-  if (p->kv_dtype == QB_E4M3)
-    kv_append_kernel<true><<<grid, kKvThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
-  else
-    kv_append_kernel<false><<<grid, kKvThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
-  return check_launch("kv_cache_update");
+  return launch_dep("kv_cache_update", p->kv_dtype == QB_E4M3 ? kv_append_kernel<true> : kv_append_kernel<false>, grid, dim3(kKvThreads), 0,
+                    static_cast<cudaStream_t>(stream), a);
 }
 
 extern "C" int32_t qb_kv_cache_update(const void* qkv, const int32_t* frame_t, const int32_t* frozen, void* K_cache, void* Vt_cache,
