@@ -187,7 +187,35 @@ def load():
         fn.restype = res
         fn.argtypes = args
     _lib = lib
+    _bind_fastcall(lib)
     return lib
+
+
+# The entry points that csrc/fastcall.c calls by address.
+FASTCALL = ("qb_gemm", "qb_gemm_workspace_bytes", "qb_ada_rmsnorm", "qb_rmsnorm", "qb_head_rmsnorm", "qb_ada_gate_residual", "qb_silu", "qb_add",
+            "qb_euler_step", "qb_quantize_e4m3", "qb_dequantize_e4m3")  # fmt: skip
+
+
+class _NoFastcall:
+    """Stands in where the extension was not built (it needs the interpreter's headers): takes no call."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+def fastcall():
+    """The C side of the smallest ``qf`` calls; it takes none of them before ``load()`` has told it the library's addresses."""
+    try:
+        from . import _fastcall
+    except ImportError:
+        return _NoFastcall()
+    return _fastcall
+
+
+def _bind_fastcall(lib) -> None:
+    from .runtime.tensor import QuarkTensor
+
+    fastcall().bind(QuarkTensor, {name: C.cast(getattr(lib, name), C.c_void_p).value for name in FASTCALL})
 
 
 def check(rc: int) -> None:

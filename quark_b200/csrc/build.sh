@@ -14,4 +14,12 @@ for f in runtime gemm gemm_pair gemm_grouped attn attn4 kv glue qkv_post tp; do
 done
 for p in "${pids[@]}"; do wait $p; done
 $NVCC -shared -o "$OUT" "$HERE"/build/{runtime,gemm,gemm_pair,gemm_grouped,attn,attn4,kv,glue,qkv_post,tp}.o -cudart static
+# The C side of the smallest calls (a CPython extension); without the interpreter's headers they stay in Python.
+PYTHON="${PYTHON:-python3}"
+PYINC="$($PYTHON -c 'import sysconfig; print(sysconfig.get_paths()["include"])')"
+if [ -f "$PYINC/Python.h" ]; then
+  ${CC:-gcc} -O2 -Wall -std=gnu11 -fPIC -shared -I"$PYINC" "$HERE/fastcall.c" -o "$HERE/../_fastcall.so"
+else
+  echo "no Python.h under $PYINC: _fastcall.so not built"
+fi
 echo "built $OUT"

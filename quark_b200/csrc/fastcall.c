@@ -158,6 +158,7 @@ static PyObject* fast_ada_rmsnorm(PyObject* self, PyObject* const* a, Py_ssize_t
       !tensor_or_none(a[6], &oq) || !stream_of(a[8], &st))
     Py_RETURN_NONE;
   const int act = activation_of(a[4]), only_q = a[7] == Py_True;
+  if (a[7] != Py_True && a[7] != Py_False) Py_RETURN_NONE;
   if (only_q) out.ptr = NULL;
   if (act < 0 || (only_q ? oq.ptr == NULL : out.ptr == NULL) || X.dtype != QB_BF16 || sc.dtype != QB_BF16 || bi.dtype != QB_BF16) Py_RETURN_NONE;
   const long long D = dim(&X, -1);

@@ -475,8 +475,27 @@ static EncodeTiledFn encode_tiled_fn() {
 // Tensor map of a contiguous row-major tensor [rows, cols] of 1- or 2-byte elements with a box of
 // [box_rows, box_cols] elements; box_cols * elem_bytes must equal the swizzle span (64 or 128).
 // Out-of-range parts of a box are filled with zeros.
+//
+// A map depends on its arguments alone, so each thread keeps the last few it made: a program calls with the same tensors again
+// and again, and the driver's encoder takes longer than the rest of a small call's host side.
 int32_t make_tmap_2d_sw(CUtensorMap* tm, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint32_t box_rows,
                         uint32_t box_cols, int swizzle_bytes) {
+  struct Made {
+    CUtensorMap map;
+    const void* base;  // NULL: empty
+    uint64_t rows, cols;
+    uint32_t box_rows, box_cols;
+    int elem_bytes, swizzle_bytes;
+  };
+  constexpr int kMade = 16;
+  static thread_local Made made[kMade];
+  const uint64_t h = (reinterpret_cast<uintptr_t>(base) >> 8) * 0x9E3779B97F4A7C15ull + box_rows;
+  Made& m = made[(h ^ (h >> 32)) % kMade];
+  if (m.base == base && base != nullptr && m.rows == rows && m.cols == cols && m.box_rows == box_rows && m.box_cols == box_cols && m.elem_bytes == elem_bytes &&
+      m.swizzle_bytes == swizzle_bytes) {
+    *tm = m.map;
+    return QB_OK;
+  }
   EncodeTiledFn enc = encode_tiled_fn();
   QB_REQUIRE(enc != nullptr, QB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   QB_REQUIRE((cols * elem_bytes) % 16 == 0, QB_ERR_ALIGN, "tensor map: row pitch of %llu bytes is not a multiple of 16",
@@ -490,6 +509,7 @@ int32_t make_tmap_2d_sw(CUtensorMap* tm, const void* base, int elem_bytes, uint6
   CUresult r = enc(tm, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   QB_REQUIRE(r == CUDA_SUCCESS, QB_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", static_cast<int>(r));
+  m = Made{*tm, base, rows, cols, box_rows, box_cols, elem_bytes, swizzle_bytes};
   return QB_OK;
 }
 
@@ -512,17 +532,12 @@ int num_sms() {
   return n;
 }
 
-#ifdef QB_GEMM_TUNE
-static int g_tune[3] = {0, 0, 0};  // cg, bn, splits; 0 = choose
-extern "C" void qb_debug_gemm_tune(int cg, int bn, int s) { g_tune[0] = cg; g_tune[1] = bn; g_tune[2] = s; }
-#endif
-
 // Whether `s` K slices of a tile can be summed inside a cluster (of at most 8 CTAs): the widths whose partial sums have room.
 static bool cluster_slices(int cg, int bn, int s) { return cg == 1 ? bn == 64 && (s == 2 || s == 4 || s == 8) : bn == 128 && s == 2; }
 
 // Picks the CTAs per tile, the tile width and the number of K slices from a small cost model in ns, so that every call with the
 // same shape makes the same choice.
-static GemmPlan plan_gemm(const qb_gemm_params& p, int max_cg = 2, double* cost_out = nullptr) {
+static GemmPlan make_plan(const qb_gemm_params& p, int max_cg, double* cost_out) {
   const bool fp8 = p.compute_dtype == QB_E4M3;
   const int k_elems = fp8 ? 128 : 64;
   GemmPlan best{};
@@ -541,9 +556,6 @@ static GemmPlan plan_gemm(const qb_gemm_params& p, int max_cg = 2, double* cost_
       for (int s : ss) {
         if (p.split_k != 0 && p.split_k != s) continue;
         if (s > kb_total) continue;
-#ifdef QB_GEMM_TUNE
-        if ((g_tune[0] && g_tune[0] != cg) || (g_tune[1] && g_tune[1] != bn) || (g_tune[2] && g_tune[2] != s)) continue;
-#endif
         const int kbps = (kb_total + s - 1) / s;
         if ((kb_total + kbps - 1) / kbps != s) continue;
         const bool cl = s > 1 && (p.reserved & 1) == 0 && cluster_slices(cg, bn, s);
@@ -581,11 +593,40 @@ static GemmPlan plan_gemm(const qb_gemm_params& p, int max_cg = 2, double* cost_
     best.kb_total = kb_total;
     best.kb_per_split = kb_total;
   }
-  if (cost_out != nullptr) *cost_out = best_cost;
+  *cost_out = best_cost;
   best.counters_bytes = kCounterBytes;
   best.aq_bytes = (fp8 && p.a_dtype == QB_BF16) ? round_up(static_cast<size_t>(p.M) * p.K, 1024) : 0;
   best.partial_bytes = (best.splits > 1 && !best.cluster) ? static_cast<size_t>(best.splits) * p.M * p.N * sizeof(float) : 0;
   return best;
+}
+
+// The plan of a shape that this thread planned a moment ago is read back: a call plans twice (its workspace, then its launch), and
+// the model above takes about as long as a launch.
+static GemmPlan plan_gemm(const qb_gemm_params& p, int max_cg = 2, double* cost_out = nullptr) {
+  struct Key {
+    int32_t M, N, K, a_dtype, compute_dtype, split_k, tile_n, no_cluster, max_cg;
+    bool operator==(const Key& o) const {
+      return M == o.M && N == o.N && K == o.K && a_dtype == o.a_dtype && compute_dtype == o.compute_dtype && split_k == o.split_k && tile_n == o.tile_n &&
+             no_cluster == o.no_cluster && max_cg == o.max_cg;
+    }
+  };
+  struct Made {
+    Key key;  // M 0: empty
+    GemmPlan plan;
+    double cost;
+  };
+  constexpr int kMade = 16;
+  static thread_local Made made[kMade];
+  const Key key{p.M, p.N, p.K, p.a_dtype, p.compute_dtype, p.split_k, p.tile_n, p.reserved & 1, max_cg};
+  const uint32_t h = (static_cast<uint32_t>(p.M) * 31u + static_cast<uint32_t>(p.N)) * 31u + static_cast<uint32_t>(p.K) + static_cast<uint32_t>(p.split_k) * 5u +
+                     static_cast<uint32_t>(p.tile_n >> 6);
+  Made& m = made[(h * 0x9E3779B1u >> 16) % kMade];
+  if (!(m.key == key)) {
+    m.plan = make_plan(p, max_cg, &m.cost);
+    m.key = key;
+  }
+  if (cost_out != nullptr) *cost_out = m.cost;
+  return m.plan;
 }
 
 static int32_t validate_gemm(const qb_gemm_params* p) {
@@ -658,13 +699,6 @@ using namespace qb;
 #ifdef QB_GEMM_TRACE
 extern "C" int32_t qb_debug_gemm_trace(void* host_out) {
   return cudaMemcpyFromSymbol(host_out, qb::g_gemm_trace, sizeof(qb::g_gemm_trace)) == cudaSuccess ? 0 : -1;
-}
-#endif
-
-#ifdef QB_GEMM_TUNE
-extern "C" int32_t qb_debug_gemm_plan(const qb_gemm_params* p) {
-  const GemmPlan pl = plan_gemm(*p);
-  return pl.cg * 1000000 + pl.bn * 1000 + pl.splits * 10 + pl.cluster;
 }
 #endif
 

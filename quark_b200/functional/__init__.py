@@ -24,6 +24,12 @@ __all__ = [
 ]  # fmt: skip
 
 
+# The calls below that only check their tensors and launch have a counterpart in C (csrc/fastcall.c) that takes the call when every
+# output is given and every check passes, and returns None otherwise.  The Python function then goes on: it allocates what is missing
+# and words the error.
+_fast = _lib.fastcall()
+
+
 def _p(t) -> int | None:
     return t.data_ptr() if t is not None else None
 
@@ -177,6 +183,13 @@ def gemm(A, B, out_dtype=None, compute_dtype=None, b_shuffled=False, activation=
     flight writes ``B`` (a weight matrix): the kernel then fetches its first ``B`` tiles while the kernels
     before it in the stream are still finishing.
     """
+    if out is not None and not b_shuffled:
+        rc = _fast.gemm(A, B, out_dtype, compute_dtype, activation, bias, gate, residual, gate_groups, out, a_scale, w_scale, split_k, tile_n,
+                        int(slice_mode) | (2 if b_constant else 0), _WS, _s())  # fmt: skip
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     if b_shuffled:
         raise NotImplementedError("qf.gemm: b_shuffled=True is not supported (disabled upstream as well)")
     if A.ndim < 2 or B.ndim != 2:
@@ -240,6 +253,12 @@ def gemm_tp(A, B, arena, *, compute_dtype=None, b_constant=False):
 
 def quantize_e4m3(X, *, out=None):
     """bf16 / f32 -> e4m3, unscaled, RN-even, saturating (``src/quark/functional/quantize_e4m3.py:25-69``)."""
+    if out is not None:
+        rc = _fast.quantize(X, out, _s())
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     dt = _dt(X)
     if dt not in ("bf16", "f32"):
         raise TypeError(f"qf.quantize_e4m3: source dtype {dt!r} is not supported")
@@ -281,6 +300,12 @@ def _head_scales(who, n_kv_heads, k_scale, v_scale):
 
 def dequantize_e4m3(X, *, out=None):
     """e4m3 -> bf16, exact (every e4m3 value is a bf16 value)."""
+    if out is not None:
+        rc = _fast.dequantize(X, out, _s())
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     if _dt(X) != "e4m3":
         raise TypeError(f"qf.dequantize_e4m3: source dtype {_dt(X)!r} (expected e4m3)")
     if out is None:
@@ -553,6 +578,12 @@ def ada_rmsnorm(X, scale, bias, eps: float = 1e-6, activation: str | None = None
     ``out_q`` (extension): an e4m3 tensor that also receives the result, for a following fp8 GEMM; with ``only_q`` the
     bf16 result is not written at all (``out_q`` is returned).
     """
+    if out is not None or only_q:
+        rc = _fast.ada_rmsnorm(X, scale, bias, eps, activation, out, out_q, only_q, _s())
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out_q if only_q else out
     _bf16_only("qf.ada_rmsnorm", X, scale, bias)
     D = int(X.shape[-1])
     rows = X.numel // D
@@ -574,6 +605,12 @@ def ada_rmsnorm(X, scale, bias, eps: float = 1e-6, activation: str | None = None
 
 def head_rmsnorm(X, n_q_heads: int, n_kv_heads: int, Dh: int, eps: float = 1e-6, *, out=None):
     """Per-head RMS norm of the Q and K heads of packed QKV (``src/quark/functional/head_rmsnorm.py:33``)."""
+    if out is not None:
+        rc = _fast.head_rmsnorm(X, n_q_heads, n_kv_heads, Dh, eps, out, _s())
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     _bf16_only("qf.head_rmsnorm", X)
     if X.ndim != 2 or int(X.shape[1]) != (n_q_heads + 2 * n_kv_heads) * Dh:
         raise ValueError(f"qf.head_rmsnorm: X shape {X.shape} is not [M, (n_q + 2 n_kv) * Dh]")
@@ -600,6 +637,12 @@ def value_residual_packed(QKV_curr, QKV_first, lamb, *, v_col_offset, v_width, o
 
 def ada_gate_residual(X, Y, gate, *, out=None):
     """``x + gate * y`` with the gate broadcast over groups of rows."""
+    if out is not None:
+        rc = _fast.gate_residual(X, Y, gate, out, _s())
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     _bf16_only("qf.ada_gate_residual", X, Y, gate)
     D = int(X.shape[-1])
     rows = X.numel // D
@@ -612,6 +655,12 @@ def ada_gate_residual(X, Y, gate, *, out=None):
 
 
 def silu(X, *, out=None, out_q=None):
+    if out is not None:
+        rc = _fast.silu(X, out, out_q, _s())
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     _bf16_only("qf.silu", X)
     out = _like(X, out, "qf.silu")
     if out_q is not None and (out_q.dtype != "e4m3" or out_q.numel != X.numel):
@@ -622,6 +671,12 @@ def silu(X, *, out=None, out_q=None):
 
 def rmsnorm(X, eps: float = 1e-6, *, out=None):
     """``x * rsqrt(mean(x^2, last dim) + eps)``, no gain (``src/quark/functional/rmsnorm.py:29-45``)."""
+    if out is not None:
+        rc = _fast.rmsnorm(X, eps, out, _s())
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     _bf16_only("qf.rmsnorm", X)
     D = int(X.shape[-1])
     out = _like(X, out, "qf.rmsnorm")
@@ -631,6 +686,12 @@ def rmsnorm(X, eps: float = 1e-6, *, out=None):
 
 def add(X, Y, *, out=None):
     """``x + y`` on same-shape bf16 tensors (the reference's ``elemwise_binary("add")``, ``src/quark/nn/layers.py:655-669``)."""
+    if out is not None:
+        rc = _fast.add(X, Y, out, _s())
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     _bf16_only("qf.add", X, Y)
     if Y.numel != X.numel:
         raise ValueError(f"qf.add: X {X.shape} and Y {Y.shape}")
@@ -641,6 +702,12 @@ def add(X, Y, *, out=None):
 
 def euler_step(X, V, Dsig, *, out=None):
     """``cast(f32(X) + f32(Dsig[0]) * f32(V), X.dtype)`` (``src/quark/functional/euler_step.py:36-41``)."""
+    if out is not None:
+        rc = _fast.euler_step(X, V, Dsig, out, _s())
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     _bf16_only("qf.euler_step", X, V)
     if V.numel != X.numel:
         raise ValueError(f"qf.euler_step: X {X.shape} and V {V.shape}")

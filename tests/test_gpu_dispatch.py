@@ -1,0 +1,187 @@
+"""The branches that a call's sizes choose: key shares of the attention, expert runs of the routing and of the grouped GEMM, column
+remainders of the GEMM epilogues, the captured append pass, and the calls that are checked and made in C."""
+
+import numpy as np
+import pytest
+
+from oracle import codec, ops
+from tests import util
+from tests.test_gpu_kernels import T, _attn_check, _check_gemm, _gemm_case
+from tests.util import bf16_randn, e4m3_randn, f32
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def qb():
+    import quark_b200 as q
+
+    q._lib.require_device(0)
+    yield q
+    q.runtime.synchronize()
+    assert q._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
+@pytest.mark.parametrize("H,W,Hk,gqa,nb,ft", [
+    (4, 16, 1, 1, 40, 60),  # one query tile, half of it empty: the widest sharing
+    (16, 8, 2, 1, 6, 3),  # fewer buckets than a cluster has CTAs
+    (12, 20, 3, 2, 5, 30),  # a second query tile of 112 rows, key tiles that end inside a share
+    (16, 16, 5, 2, 9, 100),
+    (16, 8, 8, 4, 16, 100),
+    (8, 18, 16, 2, 3, 9),  # more items than clusters fit at once
+])  # fmt: skip
+def test_attention_key_shares_by_size(qb, kv_dt, H, W, Hk, gqa, nb, ft):
+    r = util.rng([81, H, Hk])
+    tpf, cap, Hq = H * W, (nb + 1) * H * W, Hk * gqa
+    qkv = ops.head_rmsnorm(bf16_randn(r, (tpf, (Hq + 2 * Hk) * 64)), n_q_heads=Hq, n_kv_heads=Hk)
+    make = bf16_randn if kv_dt == "bf16" else e4m3_randn
+    Kc, Vc = make(r, (Hk * cap, 64)), make(r, (Hk * 64, cap))
+    segs, n = ops.compute_segments(ft, nb, tpf, 1)
+    args = (T(qb, qkv, "bf16"), T(qb, Kc, kv_dt), T(qb, Vc, kv_dt), T(qb, np.asarray(segs, np.int32)), T(qb, np.array([n], np.int32)), 1, Hk, gqa, H, W, nb, 1)
+    kw = dict(compute_dtype="e4m3" if kv_dt == "e4m3" else None, packed_qkv=True, frame_t=T(qb, np.array([ft], np.int32)))
+    want = ops.owl_attn(qkv, Kc, Vc, segs, [n], ft, n_kv_heads=Hk, gqa_ratio=gqa, H_spatial=H, W_spatial=W, kv_dtype=kv_dt,
+                        q_quant="e4m3" if kv_dt == "e4m3" else None)  # fmt: skip
+    for splits in (0, 1, 3, 8):
+        got = qb.qf.owl_attn(*args, kv_splits=splits, **kw).to_numpy()
+        _attn_check(got, want, f"attn {H}x{W} Hk={Hk} splits={splits} {kv_dt}", kv_dt == "e4m3")
+        np.testing.assert_array_equal(got, qb.qf.owl_attn(*args, kv_splits=splits, **kw).to_numpy())
+
+
+@pytest.mark.parametrize("M,E,K", [(1, 8, 2), (1025, 8, 4), (2500, 32, 3), (4096, 24, 2)])
+def test_routing_by_size(qb, M, E, K):
+    r = util.rng([82, M])
+    logits = bf16_randn(r, (M, E))
+    n = qb.qf.moe_slots(M, E, K)
+    got = [t.to_numpy().reshape(-1) for t in qb.qf.moe_route_slots(T(qb, logits, "bf16"), top_k=K)]
+    want = ops.moe_route_slots(logits, K, tile=128, total_slots=n)
+    for g, key in zip(got, ("slot_token", "slot_weight", "tile_expert", "token_slot")):
+        if key == "slot_weight":
+            np.testing.assert_allclose(g, want[key], atol=1e-6)
+        else:
+            np.testing.assert_array_equal(g, want[key].reshape(-1))
+
+
+@pytest.mark.parametrize("D", [16, 72 * 16])
+def test_gather_narrows_as_quantize_does(qb, D):
+    r = util.rng(83)
+    x = T(qb, bf16_randn(r, (100, D)), "bf16")
+    st = np.full(256, -1, np.int32)
+    st[:90] = r.permutation(100)[:90]
+    out = qb.qf.moe_gather(x, T(qb, st), out=T(qb, np.full((256, D), 0x7F, np.uint8), "e4m3")).to_numpy()
+    np.testing.assert_array_equal(out[:90], qb.qf.quantize_e4m3(x).to_numpy()[st[:90]])
+    assert not out[90:].any()
+
+
+@pytest.mark.parametrize("runs,N,K", [
+    ([1, 0, 0], 64, 64),  # one tile of one expert
+    ([3, 1, 2], 328, 192),  # odd numbers of tiles, columns that end inside a tile
+    ([2, 5, 0, 4], 1032, 2064),  # a K remainder
+])  # fmt: skip
+@pytest.mark.parametrize("fp8", [False, True])
+def test_grouped_gemm_by_expert_runs(qb, fp8, runs, N, K):
+    r = util.rng([84, N])
+    tiles = np.concatenate([np.full(c, e) for e, c in enumerate(runs)] + [[-1, -1]]).astype(np.int32)
+    E, M, dt = len(runs), 128 * len(tiles), "e4m3" if fp8 else "bf16"
+    A = e4m3_randn(r, (M, K)) if fp8 else bf16_randn(r, (M, K))
+    B = e4m3_randn(r, (E * N, K), 0.05) if fp8 else bf16_randn(r, (E * N, K), 0.05)
+    a, b, t = T(qb, A, dt), T(qb, B, dt), T(qb, tiles)
+    got = qb.qf.gemm_grouped(a, b, t, n_experts=E, activation="silu", compute_dtype=dt, out=T(qb, np.zeros((M, N), np.uint16), "bf16"))
+    g = got.to_numpy()
+    for i, e in enumerate(tiles[tiles >= 0]):
+        rows = slice(128 * i, 128 * i + 128)
+        want = ops.gemm(A[rows], B[e * N : (e + 1) * N], a_dtype=dt, b_dtype=dt, activation="silu", return_f32=True)
+        _check_gemm(T(qb, g[rows], "bf16"), want, f"tile {i} expert {e} fp8={fp8}", fp8)
+    # an e4m3 result through bf16 is the bf16 result narrowed
+    q = qb.qf.gemm_grouped(a, b, t, n_experts=E, activation="silu", compute_dtype=dt, out_dtype="e4m3", through_bf16=True,
+                           out=T(qb, np.zeros((M, N), np.uint8), "e4m3"))  # fmt: skip
+    np.testing.assert_array_equal(q.to_numpy(), qb.qf.quantize_e4m3(got).to_numpy())
+
+
+@pytest.mark.parametrize("M,N,kw", [
+    (1, 8, dict()),
+    (5, 72, dict(gate_groups=5)),
+    (130, 88, dict(gate_groups=2)),
+    (130, 152, dict(out_dtype="f32", bias=True)),
+    (200, 200, dict(out_dtype="e4m3", act="silu", bias=True)),
+    (260, 1000, dict(gate_groups=4)),
+])  # fmt: skip
+@pytest.mark.parametrize("fp8", [False, True])
+def test_epilogue_of_column_remainders(qb, M, N, kw, fp8):
+    got, want = _gemm_case(qb, M, N, 272, fp8=fp8, seed=M + N, split_k=1, **kw)
+    _check_gemm(got, want, f"{M}x{N} {kw} fp8={fp8}", fp8)
+
+
+@pytest.mark.parametrize("quant", ["bf16", "fp8"])
+def test_append_pass_captured_equals_call_by_call(qb, quant):
+    from quark_b200.models import QuantConfig, Waypoint15Config, make_params
+
+    q = QuantConfig.all_fp8() if quant == "fp8" else QuantConfig.all_bf16()
+    cfg = Waypoint15Config(d_model=128, n_layers=4, n_heads=2, n_kv_heads=1, height=8, width=8, channels=4, local_window=2, global_window=4,
+                           global_pinned_dilation=2, quant=q)  # fmt: skip
+    params = make_params(cfg, seed=5, weight_std=0.08)
+    r = util.rng(85)
+    engines = [qb.Engine(cfg=cfg, quant=q, params=params, use_graph=g) for g in (True, False)]
+    for i in range(6):
+        lat = codec.f32_to_bf16(r.standard_normal((1, cfg.latent_numel)).astype(np.float32))
+        for e in engines:
+            if i == 4:  # a parameter replaced after the capture has to be seen by the next append
+                p = dict(e.model.named_parameters())
+                name = next(k for k, v in p.items() if v.data.dtype == "bf16" and v.data.ndim == 2 and "weight" in k)
+                p[name].data = T(qb, np.zeros_like(p[name].data.to_numpy()), "bf16")
+            e.append_frame(lat)
+        for a, b in zip(engines[0].model.blocks, engines[1].model.blocks):
+            for x in ("K_cache", "Vt_cache", "segments", "n_segments"):
+                np.testing.assert_array_equal(getattr(a.kv_cache, x).to_numpy(), getattr(b.kv_cache, x).to_numpy())
+
+
+def test_calls_made_in_c_equal_the_python_path(qb, monkeypatch):
+    """Same bytes with and without the extension, and the Python path's errors for what it does not take."""
+    qf, r = qb.qf, util.rng(86)
+    assert not isinstance(qf._fast, qb._lib._NoFastcall)
+    x, y, lat = (T(qb, bf16_randn(r, (24, 256)), "bf16") for _ in range(3))
+    row = T(qb, bf16_randn(r, (3, 256)), "bf16")
+    w, wq = T(qb, bf16_randn(r, (72, 256)), "bf16"), T(qb, e4m3_randn(r, (72, 256)), "e4m3")
+    g72, r72, dsig = T(qb, bf16_randn(r, (3, 72)), "bf16"), T(qb, bf16_randn(r, (24, 72)), "bf16"), T(qb, np.array([0.3], np.float32))
+    e = lambda *s, dt="bf16": T(qb, np.zeros(s, {"bf16": np.uint16, "e4m3": np.uint8, "f32": np.float32}[dt]), dt)  # noqa: E731
+    calls = [
+        lambda: qf.gemm(x, w, out=e(24, 72)),
+        lambda: qf.gemm(x, wq, out=e(24, 72, dt="f32"), activation="silu", split_k=2, slice_mode=1),
+        lambda: qf.gemm(x, w, gate=g72, residual=r72, gate_groups=3, out=e(24, 72), b_constant=True),
+        lambda: qf.ada_rmsnorm(x, row, row, out=e(24, 256)),
+        lambda: qf.ada_rmsnorm(x, row, row, 1e-5, "silu", out_q=e(24, 256, dt="e4m3"), only_q=True),
+        lambda: qf.rmsnorm(x, out=e(24, 256)),
+        lambda: qf.head_rmsnorm(x, 2, 1, 64, out=e(24, 256)),
+        lambda: qf.ada_gate_residual(x, y, row, out=e(24, 256)),
+        lambda: qf.silu(x, out=e(24, 256), out_q=e(24, 256, dt="e4m3")),
+        lambda: qf.add(x, y, out=e(24, 256)),
+        lambda: qf.euler_step(x, y, dsig, out=e(24, 256)),
+        lambda: qf.quantize_e4m3(x, out=e(24, 256, dt="e4m3")),
+        lambda: qf.dequantize_e4m3(wq, out=e(72, 256)),
+    ]
+    wrong = [
+        (ValueError, lambda: qf.gemm(x, w, out=e(24, 64))),
+        (ValueError, lambda: qf.gemm(x, w, out=e(24, 72), out_dtype="f32")),
+        (ValueError, lambda: qf.gemm(x, w, out=e(24, 72), gate=g72)),
+        (ValueError, lambda: qf.gemm(x, w, out=e(24, 72), gate=g72, residual=r72, gate_groups=5)),
+        (TypeError, lambda: qf.gemm(x, w, out=e(24, 72), compute_dtype="f32")),
+        (qb._lib.QbError, lambda: qf.gemm(x, wq, out=e(24, 72), compute_dtype="bf16")),
+        (ValueError, lambda: qf.ada_rmsnorm(x, row, w, out=e(24, 256))),
+        (TypeError, lambda: qf.rmsnorm(wq, out=e(72, 256))),
+        (ValueError, lambda: qf.silu(x, out=e(24, 248))),
+        (ValueError, lambda: qf.add(x, w, out=e(24, 256))),
+        (TypeError, lambda: qf.euler_step(x, y, row, out=e(24, 256))),
+        (ValueError, lambda: qf.quantize_e4m3(x, out=e(24, 256))),
+        (TypeError, lambda: qf.dequantize_e4m3(x, out=e(24, 256))),
+    ]
+    first = [c().to_numpy() for c in calls]
+    for kind, c in wrong:
+        with pytest.raises(kind):
+            c()
+    monkeypatch.setattr(qf, "_fast", qb._lib._NoFastcall())
+    for a, c in zip(first, calls):
+        np.testing.assert_array_equal(a, c().to_numpy())
+    for kind, c in wrong:
+        with pytest.raises(kind):
+            c()
+    assert f32(first[0], "bf16").any()
