@@ -283,6 +283,10 @@ int32_t qb_set_attn_exact_exp(int32_t on);
  * head) in a fixed 16 KiB area (so calls of different geometries may share a workspace), which must be zero
  * before the first use (the kernel leaves it zero), followed by the CTAs' partial results; it must not be the workspace of qb_gemm.  Shares are summed in a fixed order. */
 size_t qb_owl_attn_workspace_bytes(const qb_attn_params* p);
+/* Bytes of workspace with which qb_owl_attn can use every SM for `p` (not less than the above, which it cannot do without): where
+ * the (query tile, head) items leave SMs idle and the history is long, CTAs on those SMs take a part of the items' keys and the partial
+ * results meet in the workspace (tickets as above). */
+size_t qb_owl_attn_scratch_bytes(const qb_attn_params* p);
 int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void* Vt_cache, const int32_t* segments,
                     const int32_t* n_segments, const int32_t* frame_t, void* out, void* out_q, const float* rope_xy,
                     const qb_attn_params* p, void* workspace, size_t workspace_bytes, void* stream);

@@ -126,6 +126,7 @@ SIGNATURES = {
     "qb_gemm_qkv_post": (_I, [_P] * 12 + [C.POINTER(GemmParams), C.POINTER(KvParams), _F, _P, _Z, _P]),
     "qb_rope_table_build": (_I, [_P, _I, _I, _P]),
     "qb_owl_attn_workspace_bytes": (_Z, [C.POINTER(AttnParams)]),
+    "qb_owl_attn_scratch_bytes": (_Z, [C.POINTER(AttnParams)]),
     "qb_owl_attn": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, C.POINTER(AttnParams), _P, _Z, _P]),
     "qb_ada_rmsnorm": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P]),
     "qb_rmsnorm": (_I, [_P, _P, _I, _I, _F, _P]),

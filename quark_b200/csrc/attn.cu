@@ -178,17 +178,159 @@ __device__ __forceinline__ void p_chunk(const uint32_t (&sc)[32], int c, float s
 
 // Whether the keys of a (query tile, head) are shared by gridDim.z CTAs, and how their results are brought together: through the
 // workspace (see AttnArgs::partials), or, the CTAs being one thread-block cluster, in shared memory.  The unsplit kernel is an
-// instantiation of its own so that none of this reaches its instruction stream.
-enum { kUnsplit = 0, kSplitWorkspace = 1, kSplitCluster = 2 };
+// instantiation of its own so that none of this reaches its instruction stream.  kHelped: the CTAs that
+// the items leave over take a part of the keys of several items each (KeyShares).
+enum { kUnsplit = 0, kSplitWorkspace = 1, kSplitCluster = 2, kHelped = 3 };
 
 // Cluster splits: 2 groups x S CTAs leave 64 outputs, m and the row sum of each query row with the CTA that writes the row
 // (128 / S rows each), [2 S][rows][kMergePitch] f32.
 constexpr int kMergePitch = 68;
+// Tiles j = 2 i + g, i = 0, 1, ..., below `end`: those of softmax group g.
+__device__ __forceinline__ int group_tiles(int end, int g) { return (end - g + 1) >> 1; }
 __host__ __device__ constexpr int merge_rows(int splits) { return (kQTile + splits - 1) / splits; }
+
+// The softmax threads' half of query row t of head qh and (group 0) its row of the RoPE table, on their way while something else
+// is done.
+__device__ __forceinline__ void load_q(const AttnArgs& a, int t, int qh, int g, uint4 (&q_pre)[4], float4 (&xy_pre)[4]) {
+  if (t >= a.tpf) return;
+  const uint4* src = reinterpret_cast<const uint4*>(after_wait(a.qkv) + static_cast<size_t>(t) * a.q_row + static_cast<size_t>(qh) * a.q_head + g * 32);
+#pragma unroll
+  for (int v = 0; v < 4; ++v) q_pre[v] = src[v];
+  if (g == 0) {
+    const float4* rp = reinterpret_cast<const float4*>(a.rope_xy + static_cast<size_t>(t) * 16);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xy_pre[i] = __ldg(rp + i);
+  }
+}
+
+// Q row -> RoPE -> shared memory (K-major, swizzled like a TMA tile).  Group 0 rotates pairs 0..15 (spatial angles), group 1 pairs
+// 16..31 (temporal angles, which follow the abort flags behind q_ready).
+template <bool kFp8>
+__device__ __forceinline__ void stage_q(uint8_t* smem, uint64_t* q_ready, int r, int g, bool row_ok, const uint4 (&q_pre)[4], const float4 (&xy_pre)[4], int lane) {
+  uint8_t* q_s = smem + AttnSmem<kFp8>::kQOff;
+  const float* tm = reinterpret_cast<const float*>(q_ready + 1) + 3;
+  float y0[16], y1[16];
+  if (row_ok) {
+    float xy[16];
+    if (g == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 v = xy_pre[i];
+        xy[4 * i] = v.x; xy[4 * i + 1] = v.y; xy[4 * i + 2] = v.z; xy[4 * i + 3] = v.w;
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const uint4 x = q_pre[v];
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int pl = v * 4 + j;
+        const int i = pl >> 1;
+        const float c = g == 0 ? xy[i] : tm[i];
+        const float s = g == 0 ? xy[8 + i] : tm[8 + i];
+        const float x0 = bf16lo(w[j]), x1 = bf16hi(w[j]);
+        y0[pl] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
+        y1[pl] = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int p = 0; p < 16; ++p) y0[p] = y1[p] = 0.f;
+  }
+  if (kFp8) {
+    // 64-byte rows; 16-byte chunk index XOR ((row >> 1) & 3); y0 of this group is chunk g, y1 chunk 2 + g
+    uint8_t* rowp = q_s + r * 64;
+    const int sw = (r >> 1) & 3;
+    *reinterpret_cast<uint4*>(rowp + ((g ^ sw) << 4)) =
+        make_uint4(pack_e4m3x4(y0[0], y0[1], y0[2], y0[3]), pack_e4m3x4(y0[4], y0[5], y0[6], y0[7]),
+                   pack_e4m3x4(y0[8], y0[9], y0[10], y0[11]), pack_e4m3x4(y0[12], y0[13], y0[14], y0[15]));
+    *reinterpret_cast<uint4*>(rowp + (((2 + g) ^ sw) << 4)) =
+        make_uint4(pack_e4m3x4(y1[0], y1[1], y1[2], y1[3]), pack_e4m3x4(y1[4], y1[5], y1[6], y1[7]),
+                   pack_e4m3x4(y1[8], y1[9], y1[10], y1[11]), pack_e4m3x4(y1[12], y1[13], y1[14], y1[15]));
+  } else {
+    // 128-byte rows; chunk XOR (row & 7); y0 of this group is chunks 2g, 2g+1, y1 chunks 4+2g, 5+2g
+    uint8_t* rowp = q_s + r * 128;
+    const int sw = r & 7;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      *reinterpret_cast<uint4*>(rowp + (((2 * g + c) ^ sw) << 4)) =
+          make_uint4(pack_bf16x2(y0[8 * c], y0[8 * c + 1]), pack_bf16x2(y0[8 * c + 2], y0[8 * c + 3]),
+                     pack_bf16x2(y0[8 * c + 4], y0[8 * c + 5]), pack_bf16x2(y0[8 * c + 6], y0[8 * c + 7]));
+      *reinterpret_cast<uint4*>(rowp + (((4 + 2 * g + c) ^ sw) << 4)) =
+          make_uint4(pack_bf16x2(y1[8 * c], y1[8 * c + 1]), pack_bf16x2(y1[8 * c + 2], y1[8 * c + 3]),
+                     pack_bf16x2(y1[8 * c + 4], y1[8 * c + 5]), pack_bf16x2(y1[8 * c + 6], y1[8 * c + 7]));
+    }
+  }
+  fence_proxy_async_smem();
+  warp_arrive(smem_u32(q_ready), lane);
+}
+
+// kHelped: the end of a piece, for the softmax warps.  Reads O, brings the groups' results together, asks for the next piece's
+// query rows and hands the finished rows on.  A function of its own, because what it works with (addresses, the places of pieces)
+// would otherwise be kept in registers, or spilled, through the loop over the tiles (46 -> 64 us at 720p).
+template <bool kFp8>
+__device__ __noinline__ NextPiece end_piece(const AttnArgs& a, uint8_t* smem, uint64_t* q_ready, uint32_t tmem_o, uint32_t o_final, int tiles, int item, int piece,
+                                            bool any, bool ok, float m_run) {
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(reinterpret_cast<uint32_t*>(q_ready + 1) + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = (warp - 4) >> 2, r = (warp & 3) * 32 + lane;
+  const KeyShares kr(a, tiles, kHelperCost);
+  const Piece done = kr.at(item), next = kr.at(item + 1);
+  int q0 = 0, qh = 0, kvh = 0;
+  uint4 q_pre[4];
+  float4 xy_pre[4];
+  if (next.n > 0) {
+    next.place(a, q0, qh, kvh);
+    load_q(a, q0 + r, qh, g, q_pre, xy_pre);
+  }
+  float o[64];
+  float l = 0.f;
+#pragma unroll
+  for (int d = 0; d < 64; ++d) o[d] = 0.f;
+  if (ok) {
+    ok = __all_sync(0xffffffffu, mbar_wait(o_final, piece & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
+    if (ok && any) {
+      tc_fence_after();
+      uint32_t oo[2][32];
+      tmem_ld32(tmem_o, oo[0]);
+      tmem_ld32(tmem_o + 32, oo[1]);
+      uint32_t lsum = tmem_ld1(tmem_o + 64);
+      tmem_wait_ld_into(oo[0]);
+      tmem_loaded(oo[1]);
+      tmem_loaded(lsum);
+#pragma unroll
+      for (int d = 0; d < 64; ++d) o[d] = __uint_as_float(oo[d >> 5][d & 31]);
+      l = __uint_as_float(lsum);
+    }
+  }
+  // The groups' results meet in the P area (every PV of the piece is finished; the next P is written after q_ready, for which
+  // group 0 arrives when it has read the other's rows).
+  float* comb = reinterpret_cast<float*>(smem + AttnSmem<kFp8>::kPOff);  // [66][128]
+  asm volatile("bar.sync 2, 256;" ::: "memory");
+  if (g == 1) {
+    comb[r] = m_run;
+    comb[128 + r] = l;
+#pragma unroll
+    for (int d = 0; d < 64; ++d) comb[(2 + d) * 128 + r] = o[d];
+  }
+  asm volatile("bar.sync 2, 256;" ::: "memory");
+  if (g == 0) {
+    const float m1 = comb[r], m = fmaxf(m_run, m1);
+    const float a0 = ex2_approx(m_run - m), a1 = ex2_approx(m1 - m);
+    l = l * a0 + comb[128 + r] * a1;
+    m_run = m;
+#pragma unroll
+    for (int d = 0; d < 64; ++d) o[d] = o[d] * a0 + comb[(2 + d) * 128 + r] * a1;
+  }
+  const bool good = ok && *abort_flag == 0;
+  if (next.n > 0) stage_q<kFp8>(smem, q_ready, r, g, q0 + r < a.tpf, q_pre, xy_pre, lane);
+  if (g == 0) kr.finish(a, done, r, good, m_run, l, o, reinterpret_cast<int*>(q_ready + 1) + 19);
+  return NextPiece{next.item, next.n, next.tile0, (next.item - kr.first_item) * done.n + next.n, kvh};
+}
 
 template <bool kFp8, int kSplit, bool kLin>
 __global__ void __launch_bounds__(kAttnThreads, 1)
-owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const AttnArgs a) {
+owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnArgs a) {
   using L = AttnSmem<kFp8>;
   constexpr int kStages = L::kStages;
   constexpr uint32_t kTmemCols = 512;
@@ -227,9 +369,9 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   if (warp == 4) QB_TR(4, 0, 0);
-  const int q0 = blockIdx.x * kQTile;
-  const int qh = blockIdx.y;
-  const int kvh = qh / a.gqa;
+  int q0 = blockIdx.x * kQTile;
+  int qh = blockIdx.y;
+  int kvh = qh / a.gqa;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmK);
@@ -301,9 +443,16 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     if (threadIdx.x == 0) atomicOr(a.status, QB_DEV_BAD_SEGMENT);
   }
   // this CTA's share of the key tiles: tiles tile0 .. tile0 + n_tiles - 1 of the list
-  const int n_splits = kSplit != kUnsplit ? static_cast<int>(gridDim.z) : 1;
+  const int n_splits = kSplit == kSplitWorkspace || kSplit == kSplitCluster ? static_cast<int>(gridDim.z) : 1;
   int tile0 = 0;
-  if (kSplit != kUnsplit) {
+  KeyShares kr;
+  Piece pc;
+  if (kSplit == kHelped) {
+    kr = KeyShares(a, n_tiles, kHelperCost);
+    pc = kr.first();
+    pc.place(a, q0, qh, kvh);
+  }
+  if (kSplit == kSplitWorkspace || kSplit == kSplitCluster) {
     tile0 = static_cast<int>(blockIdx.z) * n_tiles / n_splits;
     n_tiles = static_cast<int>(blockIdx.z + 1) * n_tiles / n_splits - tile0;
   }
@@ -313,20 +462,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   // (46.5 -> 46.3 us at 720p).
   uint4 q_pre[4];
   float4 xy_pre[4];
-  if (warp >= 4) {
-    const int g_ = (warp - 4) >> 2;
-    const int t_ = q0 + (warp & 3) * 32 + lane;
-    if (t_ < a.tpf) {
-      const uint4* src = reinterpret_cast<const uint4*>(after_wait(a.qkv) + static_cast<size_t>(t_) * a.q_row + static_cast<size_t>(qh) * a.q_head + g_ * 32);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) q_pre[v] = src[v];
-      if (g_ == 0) {
-        const float4* rp = reinterpret_cast<const float4*>(a.rope_xy + static_cast<size_t>(t_) * 16);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) xy_pre[i] = __ldg(rp + i);
-      }
-    }
-  }
+  if (warp >= 4) load_q(a, q0 + (warp & 3) * 32 + lane, qh, (warp - 4) >> 2, q_pre, xy_pre);
   if (threadIdx.x >= 96 && threadIdx.x < 104) temporal_cos_sin(*after_wait(a.frame_t), threadIdx.x - 96, tm);
   __syncthreads();
 
@@ -338,12 +474,22 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     // ---------------- TMA producer
     if (elect_one()) {
       int issued = 0;
-      for (int j = 0; j < n_tiles; ++j) {
+      int tile = tile0;  // within the item
+      if (kSplit == kHelped) {
+        n_tiles = kr.all_tiles();
+        tile = pc.tile0;
+      }
+      for (int j = 0; j < n_tiles; ++j, ++tile) {
+        if (kSplit == kHelped && tile == pc.tile0 + pc.n) {  // on to the next item
+          kr.next(pc);
+          tile = pc.tile0;
+          pc.place(a, q0, qh, kvh);
+        }
         const int s = j % kStages;
         const uint32_t ph = (j / kStages) & 1;
         if (!mbar_wait(smem_u32(&kv_empty[s]), ph ^ 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN)) break;
         int row, valid;
-        locate_tile(seg, tile0 + j, row, valid);
+        locate_tile(seg, tile, row, valid);
         const uint32_t fb = smem_u32(&kv_full[s]);
         mbar_arrive_expect_tx(fb, L::kKBytes + (kFp8 ? 1 : 2) * 64 * 128);
         uint8_t* st = smem + L::kStageOff + s * L::kStageBytes;
@@ -368,8 +514,11 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     // registers; once the group has written P(i) (and rescaled O if a row maximum jumped), O += P(i) V(i)
     // accumulates in the group's O columns.  S(i + 1) is issued ahead of PV(i).
     const int g = warp - 1;
-    const int n_g = n_tiles > g ? (n_tiles - g + 1) / 2 : 0;
-    if (elect_one() && n_g > 0) {
+    // A piece of work is a run of tiles of one item: all that this CTA has, or (kHelped) one after the other.  Tiles are counted
+    // over the pieces, so stages, barrier phases and the turns of the two groups run on; only O starts anew.
+    int i0 = 0, i1 = n_tiles > g ? (n_tiles - g + 1) / 2 : 0;  // the group's tiles of the piece
+    if (kSplit == kHelped) i1 = group_tiles(pc.n, g);
+    if (elect_one()) {
       const uint32_t q_addr = smem_u32(q_s);
       const uint32_t p_base = smem_u32(smem + L::kPOff + g * L::kPBufs * L::kPBytes);
       const uint32_t tmem_sg = tmem_base + g * kGroupCols;
@@ -391,15 +540,20 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       auto wait_tile = [&](int j) {
         return mbar_wait(smem_u32(&kv_full[j % kStages]), (j / kStages) & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
       };
-      bool ok = mbar_wait(smem_u32(q_ready), 0, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
-      ok = ok && wait_tile(g);
-      if (ok) {
-        tc_fence_after();
-        issue_s(0);
+      bool ok = true;
+      int end = pc.n;  // tiles of the CTA up to the end of the piece
+      for (int piece = 0; ok && (kSplit == kHelped ? pc.n > 0 : piece == 0); ++piece) {
+      if (kSplit == kHelped || i0 < i1) ok = mbar_wait(smem_u32(q_ready), piece & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
+      if (i0 < i1) {
+        ok = ok && wait_tile(2 * i0 + g);
+        if (ok) {
+          tc_fence_after();
+          issue_s(i0);
+        }
       }
-      for (int i = 0; i < n_g && ok; ++i) {
+      for (int i = i0; i < i1 && ok; ++i) {
         QB_TR(2 + g, i, 0);
-        if (i + 1 < n_g) {
+        if (i + 1 < i1) {
           ok = wait_tile(2 * (i + 1) + g);
           QB_TR(2 + g, i, 1);
           ok = ok && mbar_wait(smem_u32(&s_free[g]), i & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
@@ -418,13 +572,13 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         if (kFp8) {
           const uint64_t pd = umma_desc_k_sw128(p_addr), vd = umma_desc_k_sw128(v_addr);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f8(tmem_og, pd + 2 * k, vd + 2 * k, kIdescPV, (i | k) > 0);
+          for (int k = 0; k < 4; ++k) umma_f8(tmem_og, pd + 2 * k, vd + 2 * k, kIdescPV, i > i0 || k > 0);
         } else {
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             const uint64_t pd = umma_desc_k_sw128(p_addr + (k >> 2) * (L::kPBytes / 2));
             const uint64_t vd = umma_desc_k_sw128(v_addr + (k >> 2) * L::kVTile);
-            umma_f16(tmem_og, pd + 2 * (k & 3), vd + 2 * (k & 3), kIdescPV, (i | k) > 0);
+            umma_f16(tmem_og, pd + 2 * (k & 3), vd + 2 * (k & 3), kIdescPV, i > i0 || k > 0);
           }
         }
         umma_commit(smem_u32(&pv_done[g]));
@@ -433,7 +587,14 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       }
       // pv_done flips once per tile and the fp8 softmax warps rarely look at it, so its parity cannot tell
       // "all finished" from "two still in flight"; the end of the accumulation has a barrier of its own
-      if (ok) umma_commit(smem_u32(&o_final[g]));
+      if (ok && (kSplit == kHelped || i0 < i1)) umma_commit(smem_u32(&o_final[g]));
+      if (kSplit == kHelped) {
+        kr.next(pc);
+        i0 = i1;
+        end += pc.n;
+        i1 = group_tiles(end, g);
+      }
+      }
     }
   }
   } else {
@@ -447,78 +608,25 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     const uint32_t lane_addr = static_cast<uint32_t>(lane_grp * 32) << 16;
     uint8_t* p_g = smem + L::kPOff + g * L::kPBufs * L::kPBytes;
 
-    // Q row -> RoPE -> shared memory (K-major, swizzled like a TMA tile).  Group 0 rotates pairs
-    // 0..15 (spatial angles), group 1 pairs 16..31 (temporal angles).
-    {
-      float y0[16], y1[16];
-      if (row_ok) {
-        float xy[16];
-        if (g == 0) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float4 v = xy_pre[i];
-            xy[4 * i] = v.x; xy[4 * i + 1] = v.y; xy[4 * i + 2] = v.z; xy[4 * i + 3] = v.w;
-          }
-        }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const uint4 x = q_pre[v];
-          const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int pl = v * 4 + j;
-            const int i = pl >> 1;
-            const float c = g == 0 ? xy[i] : tm[i];
-            const float s = g == 0 ? xy[8 + i] : tm[8 + i];
-            const float x0 = bf16lo(w[j]), x1 = bf16hi(w[j]);
-            y0[pl] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
-            y1[pl] = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s));
-          }
-        }
-      } else {
-#pragma unroll
-        for (int p = 0; p < 16; ++p) y0[p] = y1[p] = 0.f;
-      }
-      if (kFp8) {
-        // 64-byte rows; 16-byte chunk index XOR ((row >> 1) & 3); y0 of this group is chunk g, y1 chunk 2 + g
-        uint8_t* rowp = q_s + r * 64;
-        const int sw = (r >> 1) & 3;
-        *reinterpret_cast<uint4*>(rowp + ((g ^ sw) << 4)) =
-            make_uint4(pack_e4m3x4(y0[0], y0[1], y0[2], y0[3]), pack_e4m3x4(y0[4], y0[5], y0[6], y0[7]),
-                       pack_e4m3x4(y0[8], y0[9], y0[10], y0[11]), pack_e4m3x4(y0[12], y0[13], y0[14], y0[15]));
-        *reinterpret_cast<uint4*>(rowp + (((2 + g) ^ sw) << 4)) =
-            make_uint4(pack_e4m3x4(y1[0], y1[1], y1[2], y1[3]), pack_e4m3x4(y1[4], y1[5], y1[6], y1[7]),
-                       pack_e4m3x4(y1[8], y1[9], y1[10], y1[11]), pack_e4m3x4(y1[12], y1[13], y1[14], y1[15]));
-      } else {
-        // 128-byte rows; chunk XOR (row & 7); y0 of this group is chunks 2g, 2g+1, y1 chunks 4+2g, 5+2g
-        uint8_t* rowp = q_s + r * 128;
-        const int sw = r & 7;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          *reinterpret_cast<uint4*>(rowp + (((2 * g + c) ^ sw) << 4)) =
-              make_uint4(pack_bf16x2(y0[8 * c], y0[8 * c + 1]), pack_bf16x2(y0[8 * c + 2], y0[8 * c + 3]),
-                         pack_bf16x2(y0[8 * c + 4], y0[8 * c + 5]), pack_bf16x2(y0[8 * c + 6], y0[8 * c + 7]));
-          *reinterpret_cast<uint4*>(rowp + (((4 + 2 * g + c) ^ sw) << 4)) =
-              make_uint4(pack_bf16x2(y1[8 * c], y1[8 * c + 1]), pack_bf16x2(y1[8 * c + 2], y1[8 * c + 3]),
-                         pack_bf16x2(y1[8 * c + 4], y1[8 * c + 5]), pack_bf16x2(y1[8 * c + 6], y1[8 * c + 7]));
-        }
-      }
-      fence_proxy_async_smem();
-      warp_arrive(smem_u32(q_ready), lane);
-      if (warp == 4) QB_TR(4, 0, 2);
-    }
-
-    const float ks = a.k_scale ? __ldg(a.k_scale + kvh) : 1.0f;
-    const float sl2 = ks * 0.125f * 1.4426950408889634f;  // scores -> log2 domain, 1/sqrt(64) folded in
+    stage_q<kFp8>(smem, q_ready, r, g, row_ok, q_pre, xy_pre, lane);
+    if (warp == 4) QB_TR(4, 0, 2);
     const uint32_t tmem_s = tmem_base + g * kGroupCols + lane_addr;  // this thread's row of the group's S
     const uint32_t tmem_o = tmem_s + kOCol;                          // ... and of its O accumulator
-    float m_run = -1.0e30f;
     bool ok = true;
     // every segment a multiple of the tile (720p: 512 keys a bucket): no tile needs a mask, so none is looked up
     const bool whole = ((seg[1] | seg[3] | seg[5]) & (kKeyTile - 1)) == 0;
-    const int my_tiles = n_tiles > g ? (n_tiles - g + 1) / 2 : 0;
+    int i0 = 0, i1 = n_tiles > g ? (n_tiles - g + 1) / 2 : 0;  // the group's tiles of the piece, as the MMA warp counts them
+    if (kSplit == kHelped) i1 = group_tiles(pc.n, g);
+    // What the end of a piece needs is worked out there from its item's number, so that it takes no registers in the loop.
+    int item = pc.item;
+    if (kSplit == kHelped) tile0 = pc.tile0;
+    bool more = kSplit != kHelped || pc.n > 0;
 
-    for (int i = 0; i < my_tiles && ok; ++i) {
+    for (int piece = 0; more; ++piece) {
+    const float ks = a.k_scale ? __ldg(a.k_scale + kvh) : 1.0f;
+    const float sl2 = ks * 0.125f * 1.4426950408889634f;  // scores -> log2 domain, 1/sqrt(64) folded in
+    float m_run = -1.0e30f;
+    for (int i = i0; i < i1 && ok; ++i) {
       if (lane_grp == 0) QB_TR(g, i, 0);
       int row, valid = kKeyTile;
       if (!whole) locate_tile(seg, tile0 + 2 * i + g, row, valid);
@@ -560,7 +668,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       }
       const float m_tile = max3f(max3f(mx[0], mx[1], mx[2]), mx[3], -1.0e30f) * sl2;
       if (lane_grp == 0) QB_TR(g, i, 4);
-      if (i == 0) {
+      if (i == i0) {
         m_run = m_tile;
       } else {
         const bool jump = m_tile > m_run + kSlack;
@@ -617,12 +725,23 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       if (lane_grp == 0) QB_TR(g, i, 7);
     }
     if (warp == 4) QB_TR(4, 0, 3);
+    if constexpr (kSplit == kHelped) {
+      const NextPiece next = end_piece<kFp8>(a, smem, q_ready, tmem_o, smem_u32(&o_final[g]), kr.tiles, item, piece, i0 < i1, ok, m_run);
+      item = next.item;
+      kvh = next.kvh;
+      tile0 = next.tile0 + next.n - next.done;
+      i0 = i1;
+      i1 = group_tiles(next.done, g);
+      more = next.n > 0;
+      continue;
+    }
+    more = kSplit == kHelped;
     // the group's result: 64 outputs and the row sum, still scaled by 2^(kPShift - m_run)
     float o[64];
     float l_run = 0.f;
 #pragma unroll
     for (int d = 0; d < 64; ++d) o[d] = 0.f;
-    if (ok && my_tiles > 0) {
+    if (ok && i0 < i1) {
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&o_final[g]), 0, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
       if (ok) {
         tc_fence_after();
@@ -784,6 +903,8 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       }
     }
     }
+    }
+    if (kSplit == kHelped && kr.tiles == 0) KeyShares::write_zeros(a, r, g, 2);
   }
 
   if (warp == 4) QB_TR(4, 0, 6);
@@ -859,6 +980,17 @@ static int32_t configure(K kernel, int smem_bytes, std::atomic<unsigned long lon
   return QB_OK;
 }
 
+// Whether the CTAs that the items leave over help with their keys (owned_tiles, at the longest history; the kernel decides again for
+// the keys that are valid).
+static bool attn_helped(const qb_attn_params* p, int splits) {
+  if (p->kv_dtype != QB_E4M3 && !attn4_enabled()) return false;
+  if (p->kv_splits != 0 || splits != 1) return false;
+  const int tpf = p->H_spatial * p->W_spatial, sms = num_sms();
+  const long long items = static_cast<long long>((tpf + kQTile - 1) / kQTile) * p->n_kv_heads * p->gqa_ratio;
+  const long long tiles = (static_cast<long long>(p->num_buckets + 1) * (tpf / (p->quilt_factor > 0 ? p->quilt_factor : 1)) + kKeyTile - 1) / kKeyTile;  // at most
+  return 2 * items > sms && items < sms && tiles < (1 << 24) && owned_tiles(static_cast<int>(items), sms, static_cast<int>(tiles), p->kv_dtype == QB_E4M3 ? kHelperCost : kHelperCost4 / 2) < tiles;
+}
+
 static cudaLaunchConfig_t attn_config(dim3 grid, int smem_bytes, cudaStream_t st, cudaLaunchAttribute (&attr)[2]) {  // grid.z = CTAs of a cluster
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
@@ -880,8 +1012,15 @@ static cudaLaunchConfig_t attn_config(dim3 grid, int smem_bytes, cudaStream_t st
 // once (B200: 15 of 8 CTAs, 33 of 4, 74 of 2); a wish for more is cut down to what it holds, a number that the caller forced goes
 // through the workspace instead.
 template <bool kFp8, bool kLin>
-static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnArgs& a, int Hq, int splits, bool forced, cudaStream_t st) {
+static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnArgs& a, int Hq, int splits, bool forced, bool helped,
+                           cudaStream_t st) {
   constexpr int kSmem = AttnSmem<kFp8>::kTotal;
+  if constexpr (kFp8) if (helped) {
+    static std::atomic<unsigned long long> done{0};
+    const int32_t rc = configure(owl_attn_kernel<kFp8, kHelped, kLin>, kSmem, done);
+    if (rc != QB_OK) return rc;
+    return launch_dep("owl_attn kernel", owl_attn_kernel<kFp8, kHelped, kLin>, dim3(num_sms()), dim3(kAttnThreads), kSmem, st, tmK, tmV, a);
+  }
   const unsigned q_tiles = (a.tpf + kQTile - 1) / kQTile;
   const int items = static_cast<int>(q_tiles) * Hq;
   int cluster = splits > 8 ? (forced ? 1 : 8) : splits;
@@ -942,6 +1081,13 @@ extern "C" size_t qb_owl_attn_workspace_bytes(const qb_attn_params* p) {
   return attn_ticket_bytes(p) + items * n * (66 * 128) * sizeof(float);
 }
 
+extern "C" size_t qb_owl_attn_scratch_bytes(const qb_attn_params* p) {
+  const size_t need = qb_owl_attn_workspace_bytes(p);
+  if (p == nullptr || p->H_spatial <= 0 || p->W_spatial <= 0 || p->n_kv_heads <= 0 || p->gqa_ratio <= 0 || p->num_buckets <= 0) return 0;
+  if (!attn_helped(p, attn_key_splits(p))) return need;
+  return attn_ticket_bytes(p) + static_cast<size_t>(2 * num_sms()) * kPartial * sizeof(float);
+}
+
 extern "C" int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void* Vt_cache, const int32_t* segments,
                                const int32_t* n_segments, const int32_t* frame_t, void* out, void* out_q, const float* rope_xy,
                                const qb_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {
@@ -1000,11 +1146,17 @@ extern "C" int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void*
     a.tickets = static_cast<int*>(workspace);
     a.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + attn_ticket_bytes(p));
   }
+  // the helpers want a workspace; a caller that gives none has one CTA per item
+  const bool helped = attn_helped(p, splits) && workspace != nullptr && aligned16(workspace) && workspace_bytes >= qb_owl_attn_scratch_bytes(p);
+  if (helped) {
+    a.tickets = static_cast<int*>(workspace);
+    a.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + attn_ticket_bytes(p));
+  }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // bf16, one CTA per (query tile, head): the three-group kernel of attn4.cu (60.0 against 70.3 us at 720p).  In the
   // e4m3 path it is the slower one (57.7 against 52.2 us): its per-chunk fixed work outweighs the extra warps.
   if (splits == 1 && !fp8 && attn4_enabled()) return launch_attn4(K_cache, Vt_cache, a, p->n_kv_heads, fp8, st);
   const bool forced = p->kv_splits > 0;
-  if (!fp8) return launch_attn<false, false>(tmK, tmV, a, Hq, splits, forced, st);
-  return g_attn_exact_exp ? launch_attn<true, false>(tmK, tmV, a, Hq, splits, forced, st) : launch_attn<true, true>(tmK, tmV, a, Hq, splits, forced, st);
+  if (!fp8) return launch_attn<false, false>(tmK, tmV, a, Hq, splits, forced, helped, st);
+  return g_attn_exact_exp ? launch_attn<true, false>(tmK, tmV, a, Hq, splits, forced, helped, st) : launch_attn<true, true>(tmK, tmV, a, Hq, splits, forced, helped, st);
 }

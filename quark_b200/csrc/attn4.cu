@@ -83,9 +83,151 @@ __device__ __forceinline__ uint64_t a4_desc(uint32_t addr) {
   return kFp8 ? umma_desc_k_sw64(addr) : umma_desc_k_sw128(addr);
 }
 
+// Chunks u = g + 3 i, i = 0, 1, ..., below `end`: those of softmax group g.
+__device__ __forceinline__ int group_chunks(int end, int g) { return (end - g + kA4Groups - 1) / kA4Groups; }
+
+// Q row -> RoPE -> shared memory (K-major, swizzled like a TMA tile).  Groups 0 and 1 rotate pairs 0..15 (spatial
+// angles) and 16..31 (temporal angles, which follow the abort flags behind q_ready); group 2 has nothing to do here.
 template <bool kFp8>
+__device__ __forceinline__ void stage_q4(const AttnArgs& a, uint8_t* smem, uint64_t* q_ready, int t, int qh, int r, int g, int lane) {
+  uint8_t* q_s = smem + A4Smem<kFp8>::kQOff;
+  const float* tm = reinterpret_cast<const float*>(q_ready + 1) + 3;
+  if (g < 2) {
+    float y0[16], y1[16];
+    if (t < a.tpf) {
+      float xy[16];
+      if (g == 0) {
+        const float4* rp = reinterpret_cast<const float4*>(a.rope_xy + static_cast<size_t>(t) * 16);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 v = __ldg(rp + i);
+          xy[4 * i] = v.x; xy[4 * i + 1] = v.y; xy[4 * i + 2] = v.z; xy[4 * i + 3] = v.w;
+        }
+      }
+      const uint4* src = reinterpret_cast<const uint4*>(after_wait(a.qkv) + static_cast<size_t>(t) * a.q_row + static_cast<size_t>(qh) * a.q_head + g * 32);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const uint4 x = src[v];
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int pl = v * 4 + j;
+          const int i = pl >> 1;
+          const float c = g == 0 ? xy[i] : tm[i];
+          const float s = g == 0 ? xy[8 + i] : tm[8 + i];
+          const float x0 = bf16lo(w[j]), x1 = bf16hi(w[j]);
+          y0[pl] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
+          y1[pl] = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s));
+        }
+      }
+    } else {
+#pragma unroll
+      for (int p = 0; p < 16; ++p) y0[p] = y1[p] = 0.f;
+    }
+    if (kFp8) {
+      // 64-byte rows; 16-byte chunk index XOR ((row >> 1) & 3); y0 of this group is chunk g, y1 chunk 2 + g
+      uint8_t* rowp = q_s + r * 64;
+      const int sw = (r >> 1) & 3;
+      *reinterpret_cast<uint4*>(rowp + ((g ^ sw) << 4)) =
+          make_uint4(pack_e4m3x4(y0[0], y0[1], y0[2], y0[3]), pack_e4m3x4(y0[4], y0[5], y0[6], y0[7]),
+                     pack_e4m3x4(y0[8], y0[9], y0[10], y0[11]), pack_e4m3x4(y0[12], y0[13], y0[14], y0[15]));
+      *reinterpret_cast<uint4*>(rowp + (((2 + g) ^ sw) << 4)) =
+          make_uint4(pack_e4m3x4(y1[0], y1[1], y1[2], y1[3]), pack_e4m3x4(y1[4], y1[5], y1[6], y1[7]),
+                     pack_e4m3x4(y1[8], y1[9], y1[10], y1[11]), pack_e4m3x4(y1[12], y1[13], y1[14], y1[15]));
+    } else {
+      // 128-byte rows; chunk XOR (row & 7); y0 of this group is chunks 2g, 2g+1, y1 chunks 4+2g, 5+2g
+      uint8_t* rowp = q_s + r * 128;
+      const int sw = r & 7;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        *reinterpret_cast<uint4*>(rowp + (((2 * g + c) ^ sw) << 4)) =
+            make_uint4(pack_bf16x2(y0[8 * c], y0[8 * c + 1]), pack_bf16x2(y0[8 * c + 2], y0[8 * c + 3]),
+                       pack_bf16x2(y0[8 * c + 4], y0[8 * c + 5]), pack_bf16x2(y0[8 * c + 6], y0[8 * c + 7]));
+        *reinterpret_cast<uint4*>(rowp + (((4 + 2 * g + c) ^ sw) << 4)) =
+            make_uint4(pack_bf16x2(y1[8 * c], y1[8 * c + 1]), pack_bf16x2(y1[8 * c + 2], y1[8 * c + 3]),
+                       pack_bf16x2(y1[8 * c + 4], y1[8 * c + 5]), pack_bf16x2(y1[8 * c + 6], y1[8 * c + 7]));
+      }
+    }
+    fence_proxy_async_smem();
+  }
+  warp_arrive(smem_u32(q_ready), lane);
+}
+
+// kHelped: the end of a piece, for the softmax warps.  Reads O, brings the groups' results together, stages the next piece's query rows
+// and hands the finished rows on.  A function of its own, because what it works with (addresses, the places of pieces) would
+// otherwise be kept in registers, or spilled, through the loop over the chunks (60.0 -> 64.7 us at 720p).
+template <bool kFp8>
+__device__ __noinline__ NextPiece end_piece4(const AttnArgs& a, uint8_t* smem, uint64_t* q_ready, uint32_t tmem_o, uint32_t o_final, int chunks, int item, int piece,
+                                             bool any, bool ok, float m_run) {
+  constexpr int G = kA4Groups;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(reinterpret_cast<uint32_t*>(q_ready + 1) + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = (warp - 4) >> 2, r = (warp & 3) * 32 + lane;
+  const KeyShares kr(a, chunks, kHelperCost4);
+  const Piece done = kr.at(item), next = kr.at(item + 1);
+  float o[64];
+  float l = 0.f;
+#pragma unroll
+  for (int d = 0; d < 64; ++d) o[d] = 0.f;
+  if (ok) {
+    ok = __all_sync(0xffffffffu, mbar_wait(o_final, piece & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
+    if (ok && any) {
+      tc_fence_after();
+      uint32_t oo[2][32];
+      tmem_ld32(tmem_o, oo[0]);
+      tmem_ld32(tmem_o + 32, oo[1]);
+      uint32_t lsum = tmem_ld1(tmem_o + 64);
+      tmem_wait_ld_into(oo[0]);
+      tmem_loaded(oo[1]);
+      tmem_loaded(lsum);
+#pragma unroll
+      for (int d = 0; d < 64; ++d) o[d] = __uint_as_float(oo[d >> 5][d & 31]);
+      l = __uint_as_float(lsum);
+    }
+  }
+  // The groups' results meet in the P area (every PV of the piece is finished; the next P is written after q_ready, for which
+  // group 0 arrives when it has read the others' rows).
+  float* comb = reinterpret_cast<float*>(smem + A4Smem<kFp8>::kPOff);  // [2][66][128]
+  asm volatile("bar.sync 2, 384;" ::: "memory");
+  if (g > 0) {
+    float* mine = comb + (g - 1) * kPartial + r;
+    mine[0] = m_run;
+    mine[128] = l;
+#pragma unroll
+    for (int d = 0; d < 64; ++d) mine[(2 + d) * 128] = o[d];
+  }
+  asm volatile("bar.sync 2, 384;" ::: "memory");
+  if (g == 0) {
+    float m = m_run;
+#pragma unroll
+    for (int j = 0; j < G - 1; ++j) m = fmaxf(m, comb[j * kPartial + r]);
+    const float a0 = ex2_approx(m_run - m);
+    l *= a0;
+    m_run = m;
+#pragma unroll
+    for (int d = 0; d < 64; ++d) o[d] *= a0;
+#pragma unroll 1
+    for (int j = 0; j < G - 1; ++j) {
+      const float* part = comb + j * kPartial + r;
+      const float aj = ex2_approx(part[0] - m);
+      l = fmaf(part[128], aj, l);
+#pragma unroll
+      for (int d = 0; d < 64; ++d) o[d] = fmaf(part[(2 + d) * 128], aj, o[d]);
+    }
+  }
+  const bool good = ok && *abort_flag == 0;
+  int q0 = 0, qh = 0, kvh = 0;
+  if (next.n > 0) {
+    next.place(a, q0, qh, kvh);
+    stage_q4<kFp8>(a, smem, q_ready, q0 + r, qh, r, g, lane);
+  }
+  if (g == 0) kr.finish(a, done, r, good, m_run, l, o, reinterpret_cast<int*>(q_ready + 1) + 19);
+  return NextPiece{next.item, next.n, next.tile0, (next.item - kr.first_item) * done.n + next.n, kvh};
+}
+
+// kHelped: a one-dimensional grid, one CTA per item and helpers (KeyShares); otherwise one CTA per item.
+template <bool kFp8, bool kHelped>
 __global__ void __launch_bounds__(kA4Threads, 1)
-owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const AttnArgs a) {
+owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnArgs a) {
   using L = A4Smem<kFp8>;
   constexpr int kStages = L::kStages;
   constexpr int G = kA4Groups;
@@ -116,9 +258,9 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int q0 = blockIdx.x * 128;
-  const int qh = blockIdx.y;
-  const int kvh = qh / a.gqa;
+  int q0 = blockIdx.x * 128;
+  int qh = blockIdx.y;
+  int kvh = qh / a.gqa;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmK);
@@ -183,6 +325,14 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     if (threadIdx.x == 0) atomicOr(a.status, QB_DEV_BAD_SEGMENT);
   }
 
+  KeyShares kr;
+  Piece pc;
+  if (kHelped) {
+    kr = KeyShares(a, n_chunks, kHelperCost4);
+    pc = kr.first();
+    pc.place(a, q0, qh, kvh);
+  }
+
   if (threadIdx.x < 8) temporal_cos_sin(*after_wait(a.frame_t), threadIdx.x, tm);
   __syncthreads();
 
@@ -192,12 +342,19 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
       // ---------------- TMA producer
       if (elect_one()) {
         int issued = 0;
-        for (int u = 0; u < n_chunks; ++u) {
+        int chunk = pc.tile0;  // within the item
+        if (kHelped) n_chunks = kr.all_tiles();
+        for (int u = 0; u < n_chunks; ++u, ++chunk) {
+          if (kHelped && chunk == pc.tile0 + pc.n) {  // on to the next item
+            kr.next(pc);
+            chunk = pc.tile0;
+            pc.place(a, q0, qh, kvh);
+          }
           const int s = u % kStages;
           const uint32_t ph = (u / kStages) & 1;
           if (!mbar_wait(smem_u32(&kv_empty[s]), ph ^ 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN)) break;
           int row, valid;
-          locate_chunk(seg, u, row, valid);
+          locate_chunk(seg, chunk, row, valid);
           const uint32_t fb = smem_u32(&kv_full[s]);
           mbar_arrive_expect_tx(fb, L::kKBytes + 64 * L::kRowBytes);
           uint8_t* st = smem + L::kStageOff + s * L::kStageBytes;
@@ -221,8 +378,10 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
       // (and rescaled O if a row maximum jumped), O += P(i) V(i) accumulates in the group's O columns.  S(i + 1) is issued
       // ahead of PV(i).
       const int g = warp - 1;
-      const int n_g = n_chunks > g ? (n_chunks - g + G - 1) / G : 0;
-      if (elect_one() && n_g > 0) {
+      // A piece of work is a run of chunks of one item: all that this CTA has, or (kHelped) one after the other.  Chunks are counted
+      // over the pieces, so stages and barrier phases run on; only O starts anew.
+      int i0 = 0, i1 = group_chunks(kHelped ? pc.n : n_chunks, g);  // the group's chunks of the piece
+      if (elect_one()) {
         const uint32_t q_addr = smem_u32(q_s);
         const uint32_t tmem_sg = tmem_base + g * 64;
         const uint32_t tmem_og = tmem_base + kOCol + g * kOStride;
@@ -240,14 +399,19 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
           }
           umma_commit(smem_u32(&s_full[g]));
         };
-        bool ok = mbar_wait(smem_u32(q_ready), 0, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
-        ok = ok && wait_chunk(0);
-        if (ok) {
-          tc_fence_after();
-          issue_s(0);
+        bool ok = true;
+        int end = pc.n;  // chunks of the CTA up to the end of the piece
+        for (int piece = 0; ok && (kHelped ? pc.n > 0 : piece == 0); ++piece) {
+        if (kHelped || i0 < i1) ok = mbar_wait(smem_u32(q_ready), piece & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
+        if (i0 < i1) {
+          ok = ok && wait_chunk(i0);
+          if (ok) {
+            tc_fence_after();
+            issue_s(i0);
+          }
         }
-        for (int i = 0; i < n_g && ok; ++i) {
-          if (i + 1 < n_g) {
+        for (int i = i0; i < i1 && ok; ++i) {
+          if (i + 1 < i1) {
             ok = wait_chunk(i + 1);
             ok = ok && mbar_wait(smem_u32(&s_free[g]), i & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
             if (!ok) break;
@@ -261,13 +425,20 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
           const uint64_t pd = a4_desc<kFp8>(p_addr), vd = a4_desc<kFp8>(stage_addr(i) + L::kKBytes);
 #pragma unroll
           for (int m = 0; m < kMmas; ++m) {
-            if (kFp8) umma_f8(tmem_og, pd + 2 * m, vd + 2 * m, kIdescPV, (i | m) > 0);
-            else umma_f16(tmem_og, pd + 2 * m, vd + 2 * m, kIdescPV, (i | m) > 0);
+            if (kFp8) umma_f8(tmem_og, pd + 2 * m, vd + 2 * m, kIdescPV, i > i0 || m > 0);
+            else umma_f16(tmem_og, pd + 2 * m, vd + 2 * m, kIdescPV, i > i0 || m > 0);
           }
           umma_commit(smem_u32(&pv_done[g]));
           umma_commit(smem_u32(&kv_empty[(g + G * i) % kStages]));
         }
-        if (ok) umma_commit(smem_u32(&o_final[g]));  // the end of the accumulation has a barrier of its own
+        if (ok && (kHelped || i0 < i1)) umma_commit(smem_u32(&o_final[g]));  // the end of the accumulation has a barrier of its own
+        if (kHelped) {
+          kr.next(pc);
+          i0 = i1;
+          end += pc.n;
+          i1 = group_chunks(end, g);
+        }
+        }
       }
     }
   } else {
@@ -281,81 +452,25 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     const uint32_t lane_addr = static_cast<uint32_t>(lane_grp * 32) << 16;
     uint8_t* p_g = smem + L::kPOff + g * L::kPBufs * L::kPBytes;
 
-    // Q row -> RoPE -> shared memory (K-major, swizzled like a TMA tile).  Groups 0 and 1 rotate pairs 0..15 (spatial
-    // angles) and 16..31 (temporal angles); group 2 has nothing to do here.
-    if (g < 2) {
-      float y0[16], y1[16];
-      if (row_ok) {
-        float xy[16];
-        if (g == 0) {
-          const float4* rp = reinterpret_cast<const float4*>(a.rope_xy + static_cast<size_t>(t) * 16);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float4 v = __ldg(rp + i);
-            xy[4 * i] = v.x; xy[4 * i + 1] = v.y; xy[4 * i + 2] = v.z; xy[4 * i + 3] = v.w;
-          }
-        }
-        const uint4* src = reinterpret_cast<const uint4*>(a.qkv + static_cast<size_t>(t) * a.q_row + static_cast<size_t>(qh) * a.q_head + g * 32);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const uint4 x = src[v];
-          const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int pl = v * 4 + j;
-            const int i = pl >> 1;
-            const float c = g == 0 ? xy[i] : tm[i];
-            const float s = g == 0 ? xy[8 + i] : tm[8 + i];
-            const float x0 = bf16lo(w[j]), x1 = bf16hi(w[j]);
-            y0[pl] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
-            y1[pl] = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s));
-          }
-        }
-      } else {
-#pragma unroll
-        for (int p = 0; p < 16; ++p) y0[p] = y1[p] = 0.f;
-      }
-      if (kFp8) {
-        // 64-byte rows; 16-byte chunk index XOR ((row >> 1) & 3); y0 of this group is chunk g, y1 chunk 2 + g
-        uint8_t* rowp = q_s + r * 64;
-        const int sw = (r >> 1) & 3;
-        *reinterpret_cast<uint4*>(rowp + ((g ^ sw) << 4)) =
-            make_uint4(pack_e4m3x4(y0[0], y0[1], y0[2], y0[3]), pack_e4m3x4(y0[4], y0[5], y0[6], y0[7]),
-                       pack_e4m3x4(y0[8], y0[9], y0[10], y0[11]), pack_e4m3x4(y0[12], y0[13], y0[14], y0[15]));
-        *reinterpret_cast<uint4*>(rowp + (((2 + g) ^ sw) << 4)) =
-            make_uint4(pack_e4m3x4(y1[0], y1[1], y1[2], y1[3]), pack_e4m3x4(y1[4], y1[5], y1[6], y1[7]),
-                       pack_e4m3x4(y1[8], y1[9], y1[10], y1[11]), pack_e4m3x4(y1[12], y1[13], y1[14], y1[15]));
-      } else {
-        // 128-byte rows; chunk XOR (row & 7); y0 of this group is chunks 2g, 2g+1, y1 chunks 4+2g, 5+2g
-        uint8_t* rowp = q_s + r * 128;
-        const int sw = r & 7;
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          *reinterpret_cast<uint4*>(rowp + (((2 * g + c) ^ sw) << 4)) =
-              make_uint4(pack_bf16x2(y0[8 * c], y0[8 * c + 1]), pack_bf16x2(y0[8 * c + 2], y0[8 * c + 3]),
-                         pack_bf16x2(y0[8 * c + 4], y0[8 * c + 5]), pack_bf16x2(y0[8 * c + 6], y0[8 * c + 7]));
-          *reinterpret_cast<uint4*>(rowp + (((4 + 2 * g + c) ^ sw) << 4)) =
-              make_uint4(pack_bf16x2(y1[8 * c], y1[8 * c + 1]), pack_bf16x2(y1[8 * c + 2], y1[8 * c + 3]),
-                         pack_bf16x2(y1[8 * c + 4], y1[8 * c + 5]), pack_bf16x2(y1[8 * c + 6], y1[8 * c + 7]));
-        }
-      }
-      fence_proxy_async_smem();
-    }
-    warp_arrive(smem_u32(q_ready), lane);
+    stage_q4<kFp8>(a, smem, q_ready, t, qh, r, g, lane);
 
-    const float ks = a.k_scale ? __ldg(a.k_scale + kvh) : 1.0f;
-    const float sl2 = ks * 0.125f * 1.4426950408889634f;  // scores -> log2 domain, 1/sqrt(64) folded in
     const uint32_t tmem_s = tmem_base + g * 64 + lane_addr;  // this thread's row of the group's S
     const uint32_t tmem_o = tmem_base + kOCol + g * kOStride + lane_addr;
-    float m_run = -1.0e30f;
     bool ok = true;
     // every segment a multiple of the chunk (the usual case): no chunk needs a mask, so none is looked up
     const bool whole = ((seg[1] | seg[3] | seg[5]) & (kA4Chunk - 1)) == 0;
-    const int my_chunks = n_chunks > g ? (n_chunks - g + G - 1) / G : 0;
+    int i0 = 0, i1 = group_chunks(kHelped ? pc.n : n_chunks, g);  // the group's chunks of the piece, as the MMA warp counts them
+    // What the end of a piece needs is worked out there from its item's number, so that it takes no registers in the loop.
+    int item = pc.item, chunk0 = pc.tile0;
+    bool more = !kHelped || pc.n > 0;
 
-    for (int i = 0; i < my_chunks && ok; ++i) {
+    for (int piece = 0; more; ++piece) {
+    const float ks = a.k_scale ? __ldg(a.k_scale + kvh) : 1.0f;
+    const float sl2 = ks * 0.125f * 1.4426950408889634f;  // scores -> log2 domain, 1/sqrt(64) folded in
+    float m_run = -1.0e30f;
+    for (int i = i0; i < i1 && ok; ++i) {
       int row, valid = kA4Chunk;
-      if (!whole) locate_chunk(seg, g + G * i, row, valid);
+      if (!whole) locate_chunk(seg, chunk0 + g + G * i, row, valid);
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[g]), i & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
       if (!ok) break;
       tc_fence_after();
@@ -385,7 +500,7 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         mx[c] = fmaxf(m0, m1);
       }
       const float m_tile = max3f(mx[0], mx[1], -1.0e30f) * sl2;
-      if (i == 0) {
+      if (i == i0) {
         m_run = m_tile;
       } else {
         const bool jump = m_tile > m_run + kSlack;
@@ -446,12 +561,23 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
       tc_fence_before();
       warp_arrive(smem_u32(&p_full[2 * g + (i & 1)]), lane);
     }
+    if constexpr (kHelped) {
+      const NextPiece next = end_piece4<kFp8>(a, smem, q_ready, tmem_o, smem_u32(&o_final[g]), kr.tiles, item, piece, i0 < i1, ok, m_run);
+      item = next.item;
+      kvh = next.kvh;
+      chunk0 = next.tile0 + next.n - next.done;
+      i0 = i1;
+      i1 = group_chunks(next.done, g);
+      more = next.n > 0;
+      continue;
+    }
+    more = kHelped;
     // the group's result: 64 outputs and the row sum, still scaled by 2^(kPShift - m_run)
     float o[64];
     float l_run = 0.f;
 #pragma unroll
     for (int d = 0; d < 64; ++d) o[d] = 0.f;
-    if (ok && my_chunks > 0) {
+    if (ok && i0 < i1) {
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&o_final[g]), 0, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
       if (ok) {
         tc_fence_after();
@@ -511,6 +637,8 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         }
       }
     }
+    }
+    if (kHelped && kr.tiles == 0) KeyShares::write_zeros(a, r, g, G);
   }
 
   tc_fence_before();
@@ -524,7 +652,9 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 int32_t make_tmap_2d_sw(CUtensorMap* tm, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint32_t box_rows,
                         uint32_t box_cols, int swizzle_bytes);
 
-// Launches the three-group kernel for one (query tile, head) per CTA (no key splits).
+int num_sms();
+
+// Launches the three-group kernel: with helpers where `a` has a workspace, otherwise one (query tile, head) per CTA.
 int32_t launch_attn4(const void* K_cache, const void* Vt_cache, const AttnArgs& a, int n_kv_heads, bool fp8, cudaStream_t st) {
   const int es = fp8 ? 1 : 2;
   CUtensorMap tmK, tmV;
@@ -532,13 +662,13 @@ int32_t launch_attn4(const void* K_cache, const void* Vt_cache, const AttnArgs& 
   if (rc != QB_OK) return rc;
   rc = make_tmap_2d_sw(&tmV, Vt_cache, es, static_cast<uint64_t>(n_kv_heads) * 64, a.capacity, 64, kA4Chunk, fp8 ? 64 : 128);
   if (rc != QB_OK) return rc;
-  dim3 grid((a.tpf + 127) / 128, a.n_q_heads, 1);
-  if (fp8) {
-    QB_CUDA_OK(cudaFuncSetAttribute(owl_attn4_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, A4Smem<true>::kTotal));
-    return launch_dep("owl_attn kernel (three groups)", owl_attn4_kernel<true>, grid, dim3(kA4Threads), A4Smem<true>::kTotal, st, tmK, tmV, a);
-  }
-  QB_CUDA_OK(cudaFuncSetAttribute(owl_attn4_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, A4Smem<false>::kTotal));
-  return launch_dep("owl_attn kernel (three groups)", owl_attn4_kernel<false>, grid, dim3(kA4Threads), A4Smem<false>::kTotal, st, tmK, tmV, a);
+  // helpers have a workspace
+  const dim3 grid = a.partials != nullptr ? dim3(num_sms()) : dim3((a.tpf + 127) / 128, a.n_q_heads);
+  auto kernel = fp8 ? (a.partials != nullptr ? owl_attn4_kernel<true, true> : owl_attn4_kernel<true, false>)
+                    : (a.partials != nullptr ? owl_attn4_kernel<false, true> : owl_attn4_kernel<false, false>);
+  const int smem = fp8 ? A4Smem<true>::kTotal : A4Smem<false>::kTotal;
+  QB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  return launch_dep("owl_attn kernel (three groups)", kernel, grid, dim3(kA4Threads), smem, st, tmK, tmV, a);
 }
 
 }  // namespace qb

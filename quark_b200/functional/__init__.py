@@ -543,7 +543,7 @@ def owl_attn(Q, K_cache, Vt_cache, segments, n_segments, B, n_kv_heads, gqa_rati
     p = _params(_lib.AttnParams, n_kv_heads, gqa_ratio, H_spatial, W_spatial, num_buckets, pinned_dilation, _lib.DTYPE_CODE[kvd], _lib.DTYPE_CODE[cd],
                 max_segments, 1 if packed_qkv else 0, quilt_factor, int(kv_splits), _p(k_scale), _p(v_scale))  # fmt: skip
     lib = _lib.load()
-    ws = _attn_workspace(_need(p, lib.qb_owl_attn_workspace_bytes))
+    ws = _attn_workspace(_need(p, lib.qb_owl_attn_scratch_bytes))
     _lib.check(
         lib.qb_owl_attn(
             Q.data_ptr(), K_cache.data_ptr(), Vt_cache.data_ptr(), segments.data_ptr(), n_segments.data_ptr(), frame_t.data_ptr(), out.data_ptr(), _p(out_q),

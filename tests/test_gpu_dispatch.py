@@ -30,6 +30,10 @@ def qb():
     (16, 16, 5, 2, 9, 100),
     (16, 8, 8, 4, 16, 100),
     (8, 18, 16, 2, 3, 9),  # more items than clusters fit at once
+    (16, 16, 24, 2, 64, 100),  # 96 items and 52 helpers of one or two items
+    (16, 16, 24, 2, 64, 2),  # the same before the ring has filled: whole items
+    (16, 9, 25, 2, 96, 200),  # keys and queries that end inside a tile
+    (20, 16, 43, 1, 100, 200),  # 129 items: helpers of six or seven
 ])  # fmt: skip
 def test_attention_key_shares_by_size(qb, kv_dt, H, W, Hk, gqa, nb, ft):
     r = util.rng([81, H, Hk])
