@@ -81,6 +81,10 @@ int32_t qb_memset_async(void* dst, int32_t byte_value, size_t bytes, void* strea
 int32_t qb_memset32_async(void* dst, uint32_t value, size_t count, void* stream);
 int32_t qb_stream_create(void** stream_host);
 int32_t qb_stream_destroy(void* stream);
+/* What `stream` receives from now on starts after `event` (recorded on another stream). */
+int32_t qb_stream_wait_event(void* stream, void* event);
+/* Fetches up to 8 ranges of device memory (16-byte aligned) into L2; nothing is read or written as far as the program can tell. */
+int32_t qb_prefetch_l2(const void* const* ptrs, const size_t* bytes, int32_t n, void* stream);
 int32_t qb_stream_sync(void* stream);
 int32_t qb_device_sync(void);
 int32_t qb_event_create(void** event_host);

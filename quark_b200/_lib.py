@@ -103,6 +103,8 @@ SIGNATURES = {
     "qb_stream_create": (_I, [C.POINTER(_P)]),
     "qb_stream_destroy": (_I, [_P]),
     "qb_stream_sync": (_I, [_P]),
+    "qb_stream_wait_event": (_I, [_P, _P]),
+    "qb_prefetch_l2": (_I, [C.POINTER(_P), C.POINTER(_Z), _I, _P]),
     "qb_device_sync": (_I, []),
     "qb_event_create": (_I, [C.POINTER(_P)]),
     "qb_event_destroy": (_I, [_P]),

@@ -43,6 +43,28 @@ int32_t fail(int32_t code, const char* fmt, ...) {
 
 using namespace qb;
 
+namespace qb {
+// Brings ranges of device memory (weights that the next kernels will read) into L2 and returns at once: the copy engine of each SM is
+// handed 8 KB pieces, neighbouring pieces to neighbouring threads.  For a stream beside kernels that leave DRAM idle: 512 threads keep
+// it busy (4 CTAs: a frame's time goes up by half, because the next such kernel waits its turn; 16 and 64 alike).
+constexpr int kPrefetchRanges = 8, kPrefetchCtas = 16;
+constexpr size_t kPrefetchPiece = 8192;
+struct PrefetchArgs {
+  const uint8_t* ptr[kPrefetchRanges];
+  size_t bytes[kPrefetchRanges];
+};
+static __global__ void __launch_bounds__(32) prefetch_l2_kernel(const PrefetchArgs a, int n) {
+  const size_t step = static_cast<size_t>(gridDim.x) * 32 * kPrefetchPiece;
+  for (int i = 0; i < n; ++i) {
+    const size_t bytes = a.bytes[i] & ~static_cast<size_t>(15);
+    for (size_t at = (static_cast<size_t>(blockIdx.x) * 32 + threadIdx.x) * kPrefetchPiece; at < bytes; at += step) {
+      const uint32_t size = static_cast<uint32_t>(bytes - at < kPrefetchPiece ? bytes - at : kPrefetchPiece);
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.ptr[i] + at), "r"(size) : "memory");
+    }
+  }
+}
+}  // namespace qb
+
 extern "C" {
 
 int32_t qb_version(void) { return 100; }
@@ -151,6 +173,21 @@ int32_t qb_stream_destroy(void* stream) {
 int32_t qb_stream_sync(void* stream) {
   QB_CUDA_OK(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
   return QB_OK;
+}
+int32_t qb_stream_wait_event(void* stream, void* event) {
+  QB_CUDA_OK(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), static_cast<cudaEvent_t>(event), 0));
+  return QB_OK;
+}
+int32_t qb_prefetch_l2(const void* const* ptrs, const size_t* bytes, int32_t n, void* stream) {
+  QB_REQUIRE(n >= 1 && n <= qb::kPrefetchRanges && ptrs != nullptr && bytes != nullptr, QB_ERR_INVALID_ARG, "prefetch_l2: %d ranges", n);
+  qb::PrefetchArgs a{};
+  for (int i = 0; i < n; ++i) {
+    QB_REQUIRE(ptrs[i] != nullptr && qb::aligned16(ptrs[i]), QB_ERR_ALIGN, "prefetch_l2: range %d must be 16-byte aligned", i);
+    a.ptr[i] = static_cast<const uint8_t*>(ptrs[i]);
+    a.bytes[i] = bytes[i];
+  }
+  qb::prefetch_l2_kernel<<<qb::kPrefetchCtas, 32, 0, static_cast<cudaStream_t>(stream)>>>(a, n);
+  return qb::check_launch("prefetch_l2");
 }
 int32_t qb_device_sync(void) {
   QB_CUDA_OK(cudaDeviceSynchronize());

@@ -251,6 +251,13 @@ def gemm_tp(A, B, arena, *, compute_dtype=None, b_constant=False):
     _lib.check(lib.qb_gemm_tp(_p(A), _p(B), gp[1], C.byref(tp), _p(ws), ws.nbytes if ws is not None else 0, _s()))
 
 
+def prefetch_l2(tensors, *, stream=None) -> None:
+    """Fetches up to eight tensors into L2 (a hint: no result depends on it), on ``stream`` or the active one."""
+    n = len(tensors)
+    ptrs, sizes = (C.c_void_p * n)(*(t.data_ptr() for t in tensors)), (C.c_size_t * n)(*(t.nbytes for t in tensors))
+    _lib.check(_lib.load().qb_prefetch_l2(ptrs, sizes, n, _s() if stream is None else stream))
+
+
 def quantize_e4m3(X, *, out=None):
     """bf16 / f32 -> e4m3, unscaled, RN-even, saturating (``src/quark/functional/quantize_e4m3.py:25-69``)."""
     if out is not None:

@@ -357,14 +357,14 @@ class TransformerBlock(nn.Module):
             self.mlp = nn.MLP(d, cfg.mlp_dim_local, d, out_dtype="bf16", fuse_silu=cfg.fuse_silu)
         self.mlp_gate = nn.AdaGateResidual()
 
-    def forward(self, x, sigma_idx: int, frame_t, *, qkv_first, ctrl_emb=None, frozen: bool = False, x_out=None, h_in=None, next_norm=None):
+    def forward(self, x, sigma_idx: int, frame_t, *, qkv_first, ctrl_emb=None, frozen: bool = False, x_out=None, h_in=None, next_norm=None, prefetch=None):
         """Returns ``(x, qkv)`` (``src/quark/models/waypoint_15.py:389-440``).
 
         Tensor-parallel ranks with a fused reduction (``comm.fused``): the sum over the ranks, gate + residual and the
         AdaRMSNorm that follows are one kernel, so the pre-MLP norm never runs as a launch of its own, and the norm that
         follows the block (``next_norm = (scale, bias, activation, emit_e4m3)``: the next block's pre-attention norm, or
         the output norm) is produced by this block's last reduction and left in ``self.h_next``; ``h_in`` is what the
-        previous block left there."""
+        previous block left there.  ``prefetch`` is called just before the attention is launched."""
         s0, b0, g0, s1, b1, g1 = self._cond_lut[sigma_idx]
         fp8 = self.qkv_proj.weight.data.dtype == "e4m3"
         tp = self._cfg.tp_world > 1
@@ -408,6 +408,8 @@ class TransformerBlock(nn.Module):
             if use_first:
                 qkv = self.v_residual(qkv, qkv_first)
             self.kv_cache(qkv, frame_t, frozen=frozen)
+        if prefetch is not None:
+            prefetch()
         attn_out = self.attn(qkv, self.kv_cache, frame_t, emit_e4m3=fp8, frozen=frozen)
         h = None
         if fuse:
@@ -464,6 +466,7 @@ class Waypoint15(nn.Module):
         # Two residual-stream buffers used alternately by consecutive blocks when the gate/residual
         # epilogue is fused: a GEMM must not write the tensor it reads its residual from.
         self._x_bufs = None
+        self._side = None  # the stream of _weights_ahead
 
     def load_params(self, params: dict) -> "Waypoint15":
         """Upload a ``make_params``-style dict (full-size weights; a tensor-parallel rank keeps its slices);
@@ -537,6 +540,7 @@ class Waypoint15(nn.Module):
         qkv_first = None
         fp8 = self.cfg.quant.linear == "fp8"
         h_in = None
+        ahead = self._weights_ahead() if _stream.capturing() else None
         for li, block in enumerate(self.blocks):
             # what follows this block's last reduction (used by tensor-parallel ranks with the fused reduction only)
             if li + 1 < len(self.blocks):
@@ -545,12 +549,34 @@ class Waypoint15(nn.Module):
             else:
                 next_norm = (s_on, b_on, "silu", False)
             x, qkv = block(x, sigma_idx, frame_t, qkv_first=qkv_first, ctrl_emb=ctrl_emb, frozen=frozen, x_out=self._x_bufs[li & 1], h_in=h_in,
-                           next_norm=next_norm)  # fmt: skip
+                           next_norm=next_norm, prefetch=ahead and ahead[li])  # fmt: skip
             h_in = block.h_next
             if li == 0 and self.cfg.value_residual:
                 qkv_first = qkv
+        if ahead is not None:
+            self._side.join()
         x = h_in if h_in is not None else self.out_norm(x, s_on, b_on, activation="silu")
         return self.unpatchify(x)
+
+    def _weights_ahead(self):
+        """Per block, a call that fetches the weights up to the next attention into L2 while this block's attention leaves DRAM
+        idle; None where that does not pay.  It does where the GEMMs wait for their weights: one 128-row tile of tokens (360p
+        bf16 7052 -> 6699 us a frame) and more weights than L2 holds from one pass to the next.  At 720p the GEMMs are bound by
+        their operands' way into the SMs, and the attention, longer than the fetch, loses more to it (bf16 16292 -> 16937)."""
+        if self.cfg.tpf > 128 or self.cfg.tp_world > 1 or not self.blocks:
+            return None
+        qkv = [b.qkv_proj.weight.data for b in self.blocks]
+        rest = [[b.out_proj.weight.data] + ([] if self.cfg.moe else [b.mlp.fc1.weight.data, b.mlp.fc2.weight.data]) for b in self.blocks]
+        if sum(w.nbytes for ws in [qkv] + rest for w in ws) < PREFETCH_MIN_BYTES:
+            return None
+        if self._side is None:
+            self._side = _stream.SideStream()
+        side = self._side
+        return [lambda ws=rest[i] + [qkv[(i + 1) % len(qkv)]]: qf.prefetch_l2(ws, stream=side.fork()) for i in range(len(qkv))]
+
+
+# Three quarters of the 126 MB L2 of a B200.
+PREFETCH_MIN_BYTES = 96 << 20
 
 
 class GenerateFrame(nn.Module):

@@ -59,6 +59,42 @@ class Event:
             pass
 
 
+class SideStream:
+    """A second stream for work beside the active one, joined again before what follows may be captured or timed as a whole."""
+
+    def __init__(self):
+        p = C.c_void_p()
+        _lib.check(_lib.load().qb_stream_create(C.byref(p)))
+        self.handle = int(p.value)
+        self._fork, self._join = Event(), Event()
+
+    def fork(self) -> int:
+        """The side stream, behind everything the active stream has been given so far."""
+        self._fork.record()
+        _lib.check(_lib.load().qb_stream_wait_event(C.c_void_p(self.handle), C.c_void_p(self._fork.handle)))
+        return self.handle
+
+    def join(self) -> None:
+        """What the active stream is given from now on comes after the side stream's work."""
+        lib = _lib.load()
+        _lib.check(lib.qb_event_record(C.c_void_p(self._join.handle), C.c_void_p(self.handle)))
+        _lib.check(lib.qb_stream_wait_event(C.c_void_p(active_stream()), C.c_void_p(self._join.handle)))
+
+    def __del__(self):
+        try:
+            _lib.load().qb_stream_destroy(C.c_void_p(self.handle))
+        except Exception:
+            pass
+
+
+_capturing = False
+
+
+def capturing() -> bool:
+    """Whether ``capture_graph`` is recording the active stream."""
+    return _capturing
+
+
 class Graph:
     """An instantiated CUDA graph; ``launch()`` replays it on the active stream."""
 
@@ -87,11 +123,15 @@ class capture_graph:
         self.graph: Graph | None = None
 
     def __enter__(self):
+        global _capturing
         synchronize()
         _lib.check(_lib.load().qb_graph_begin(C.c_void_p(active_stream())))
+        _capturing = True
         return self
 
     def __exit__(self, exc_type, exc, tb):
+        global _capturing
+        _capturing = False
         p = C.c_void_p()
         rc = _lib.load().qb_graph_end(C.c_void_p(active_stream()), C.byref(p))
         if exc_type is None:

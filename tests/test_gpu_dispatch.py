@@ -139,6 +139,26 @@ def test_append_pass_captured_equals_call_by_call(qb, quant):
                 np.testing.assert_array_equal(getattr(a.kv_cache, x).to_numpy(), getattr(b.kv_cache, x).to_numpy())
 
 
+@pytest.mark.parametrize("quant", ["bf16", "fp8"])
+def test_weights_fetched_ahead_change_no_bit(qb, quant, monkeypatch):
+    from quark_b200.models import QuantConfig, Waypoint15Config, make_params, waypoint_15
+
+    q = QuantConfig.all_fp8() if quant == "fp8" else QuantConfig.all_bf16()
+    cfg = Waypoint15Config(d_model=128, n_layers=3, n_heads=2, n_kv_heads=1, height=8, width=8, channels=4, local_window=2, global_window=4,
+                           global_pinned_dilation=2, quant=q)  # fmt: skip
+    params = make_params(cfg, seed=7, weight_std=0.08)
+    frames = []
+    for least in (1 << 62, 0):  # never, always
+        monkeypatch.setattr(waypoint_15, "PREFETCH_MIN_BYTES", least)
+        eng, r = qb.Engine(cfg=cfg, quant=q, params=params), util.rng(87)
+        for _ in range(3):
+            eng.append_frame(codec.f32_to_bf16(r.standard_normal((1, cfg.latent_numel)).astype(np.float32)))
+        frames.append([eng.gen_frame(noise=r.standard_normal((1, cfg.latent_numel)).astype(np.float32)) for _ in range(3)])
+        assert (eng.model._side is not None) == (least == 0)
+    for a, b in zip(*frames):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_calls_made_in_c_equal_the_python_path(qb, monkeypatch):
     """Same bytes with and without the extension, and the Python path's errors for what it does not take."""
     qf, r = qb.qf, util.rng(86)
