@@ -196,7 +196,7 @@ def load():
 
 # The entry points that csrc/fastcall.c calls by address.
 FASTCALL = ("qb_gemm", "qb_gemm_workspace_bytes", "qb_ada_rmsnorm", "qb_rmsnorm", "qb_head_rmsnorm", "qb_ada_gate_residual", "qb_silu", "qb_add",
-            "qb_euler_step", "qb_quantize_e4m3", "qb_dequantize_e4m3")  # fmt: skip
+            "qb_euler_step", "qb_quantize_e4m3", "qb_dequantize_e4m3", "qb_kv_cache_update", "qb_kv_cache_update_kv", "qb_owl_attn_scratch_bytes", "qb_owl_attn")  # fmt: skip
 
 
 class _NoFastcall:

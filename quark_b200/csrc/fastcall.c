@@ -26,6 +26,11 @@ typedef int32_t (*add_fn)(const void*, const void*, void*, size_t, void*);
 typedef int32_t (*euler_fn)(const void*, const void*, const float*, void*, size_t, void*);
 typedef int32_t (*quant_fn)(const void*, void*, size_t, int32_t, void*);
 typedef int32_t (*dequant_fn)(const void*, void*, size_t, void*);
+typedef int32_t (*append_fn)(const void*, const int32_t*, const int32_t*, void*, void*, int32_t*, int32_t*, const float*, const qb_kv_params*, void*);
+typedef int32_t (*append_kv_fn)(const void*, const void*, const int32_t*, const int32_t*, void*, void*, int32_t*, int32_t*, const float*, const qb_kv_params*, void*);
+typedef size_t (*attn_ws_fn)(const qb_attn_params*);
+typedef int32_t (*attn_fn)(const void*, const void*, const void*, const int32_t*, const int32_t*, const int32_t*, void*, void*, const float*, const qb_attn_params*, void*,
+                           size_t, void*);
 
 static struct {
   gemm_fn gemm;
@@ -39,6 +44,10 @@ static struct {
   euler_fn euler;
   quant_fn quant;
   dequant_fn dequant;
+  append_fn append;
+  append_kv_fn append_kv;
+  attn_ws_fn attn_ws;
+  attn_fn attn;
 } g_lib;
 
 typedef struct {
@@ -251,6 +260,86 @@ static PyObject* fast_dequantize(PyObject* self, PyObject* const* a, Py_ssize_t 
   RUN(g_lib.dequant(X.ptr, out.ptr, (size_t)X.numel, st));
 }
 
+/* The geometry that the append and the attention share, and the cache tensors' shapes against it. */
+typedef struct {
+  long long nk, H, W, nb, pd, segs, qf, qo, tpf;
+  int packed;
+} Geometry;
+static int geometry(Geometry* g, PyObject* B, PyObject* nk, PyObject* H, PyObject* W, PyObject* nb, PyObject* pd, PyObject* segs, PyObject* packed, PyObject* qf, PyObject* qo,
+                    const Tensor* K, const Tensor* Vt, const Tensor* seg, const Tensor* nseg) {
+  long long b;
+  if (!as_ll(B, &b) || b != 1 || !as_ll(nk, &g->nk) || !as_ll(H, &g->H) || !as_ll(W, &g->W) || !as_ll(nb, &g->nb) || !as_ll(pd, &g->pd) || !as_ll(segs, &g->segs) ||
+      !as_ll(qf, &g->qf) || !as_ll(qo, &g->qo) || (packed != Py_True && packed != Py_False))
+    return 0;
+  g->packed = packed == Py_True;
+  if (g->nk <= 0 || g->nk > 65536 || g->H <= 0 || g->H > 65536 || g->W <= 0 || g->W > 65536 || g->nb <= 0 || g->nb > (1 << 24) || !SMALL(g->pd) || g->segs <= 0 ||
+      g->segs > 65536 || g->qf < 1 || g->qf > 65536 || (g->qf & (g->qf - 1)) != 0 || g->qo < 0 || g->qo >= g->qf)
+    return 0;
+  g->tpf = g->H * g->W;
+  if (g->tpf % g->qf != 0) return 0;
+  const long long cap = (g->nb + 1) * (g->tpf / g->qf);
+  return PyTuple_GET_SIZE(K->shape) == 2 && dim(K, 0) == g->nk * cap && dim(K, 1) == 64 && PyTuple_GET_SIZE(Vt->shape) == 2 && dim(Vt, 0) == g->nk * 64 && dim(Vt, 1) == cap &&
+         dim(seg, 0) == g->segs * 2 && dim(nseg, 0) == 1 && K->dtype == Vt->dtype && (K->dtype == QB_BF16 || K->dtype == QB_E4M3);
+}
+/* per-head scales: None, or f32 of one value per KV head */
+static int head_scale(PyObject* o, long long nk, const float** p) {
+  Tensor t;
+  if (!tensor_or_none(o, &t) || (t.ptr != NULL && (t.dtype != QB_F32 || t.numel != nk))) return 0;
+  *p = (const float*)t.ptr;
+  return 1;
+}
+
+/* (K, V, frame_t, frozen, Vt_cache, segments, n_segments, K_cache, B, n_kv_heads, H, W, num_buckets, pinned_dilation, kv_dtype, max_segments, packed, n_q_heads,
+ *  quilt_factor, quilt_offset, k_scale, v_scale, rope table, stream) */
+static PyObject* fast_kv_cache_update(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  Tensor K, V, ft, fz, Vc, seg, nseg, Kc, rope;
+  Geometry g;
+  long long nq;
+  qb_kv_params p;
+  void* st;
+  if (n != 24 || g_lib.append == NULL || !tensor(a[0], &K) || !tensor(a[2], &ft) || !tensor(a[3], &fz) || !tensor(a[4], &Vc) || !tensor(a[5], &seg) || !tensor(a[6], &nseg) ||
+      !tensor(a[7], &Kc) || !tensor(a[22], &rope) || !as_ll(a[17], &nq) || !stream_of(a[23], &st) ||
+      !geometry(&g, a[8], a[9], a[10], a[11], a[12], a[13], a[15], a[16], a[18], a[19], &Kc, &Vc, &seg, &nseg) || !head_scale(a[20], g.nk, &p.k_scale) ||
+      !head_scale(a[21], g.nk, &p.v_scale))
+    Py_RETURN_NONE;
+  if (nq < 0 || nq > (1 << 20) || K.dtype != QB_BF16 || PyTuple_GET_SIZE(K.shape) != 2 || (a[14] != Py_None && dtype_code(a[14]) != Kc.dtype)) Py_RETURN_NONE;
+  if (g.packed ? dim(&K, 0) != g.tpf || dim(&K, 1) != (nq + 2 * g.nk) * 64 : dim(&K, 0) != g.nk * g.tpf || dim(&K, 1) != 64) Py_RETURN_NONE;
+  if (!g.packed && (!tensor(a[1], &V) || V.dtype != QB_BF16 || PyTuple_GET_SIZE(V.shape) != 2 || dim(&V, 0) != dim(&K, 0) || dim(&V, 1) != 64)) Py_RETURN_NONE;
+  p.n_q_heads = (int32_t)nq; p.n_kv_heads = (int32_t)g.nk; p.H_spatial = (int32_t)g.H; p.W_spatial = (int32_t)g.W;
+  p.num_buckets = (int32_t)g.nb; p.pinned_dilation = (int32_t)g.pd; p.kv_dtype = Kc.dtype; p.max_segments = (int32_t)g.segs;
+  p.quilt_factor = (int32_t)g.qf; p.packed_qkv = g.packed; p.quilt_offset = (int32_t)g.qo;
+  if (g.packed) RUN(g_lib.append(K.ptr, ft.ptr, fz.ptr, Kc.ptr, Vc.ptr, seg.ptr, nseg.ptr, rope.ptr, &p, st));
+  RUN(g_lib.append_kv(K.ptr, V.ptr, ft.ptr, fz.ptr, Kc.ptr, Vc.ptr, seg.ptr, nseg.ptr, rope.ptr, &p, st));
+}
+
+/* (Q, K_cache, Vt_cache, segments, n_segments, B, n_kv_heads, gqa_ratio, H, W, num_buckets, pinned_dilation, out_dtype, compute_dtype, max_segments, packed,
+ *  quilt_factor, quilt_offset, frame_t, out, out_q, k_scale, v_scale, kv_splits, rope table, workspace, stream) */
+static PyObject* fast_owl_attn(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  Tensor Q, Kc, Vc, seg, nseg, ft, out, oq, rope, ws;
+  Geometry g;
+  long long gqa, splits;
+  qb_attn_params p;
+  void* st;
+  if (n != 27 || g_lib.attn == NULL || !tensor(a[0], &Q) || !tensor(a[1], &Kc) || !tensor(a[2], &Vc) || !tensor(a[3], &seg) || !tensor(a[4], &nseg) || !tensor(a[18], &ft) ||
+      !tensor(a[19], &out) || !tensor_or_none(a[20], &oq) || !tensor(a[24], &rope) || !tensor_or_none(a[25], &ws) || !as_ll(a[7], &gqa) || !as_ll(a[23], &splits) ||
+      !stream_of(a[26], &st) || !geometry(&g, a[5], a[6], a[8], a[9], a[10], a[11], a[14], a[15], a[16], a[17], &Kc, &Vc, &seg, &nseg) ||
+      !head_scale(a[21], g.nk, &p.k_scale) || !head_scale(a[22], g.nk, &p.v_scale))
+    Py_RETURN_NONE;
+  /* a cache of another dtype than the compute dtype is cast first: Python's way */
+  if ((a[13] == Py_None ? QB_BF16 : dtype_code(a[13])) != Kc.dtype || (a[12] != Py_None && dtype_code(a[12]) != QB_BF16) || gqa <= 0 || gqa > 65536 || splits < 0 ||
+      splits > 16 || Q.dtype != QB_BF16 || out.dtype != QB_BF16 || PyTuple_GET_SIZE(Q.shape) != 2)
+    Py_RETURN_NONE;
+  const long long nq = g.nk * gqa;
+  if (g.packed ? dim(&Q, 0) != g.tpf || dim(&Q, 1) != (nq + 2 * g.nk) * 64 : dim(&Q, 0) != nq * g.tpf || dim(&Q, 1) != 64) Py_RETURN_NONE;
+  if (out.numel != g.tpf * nq * 64 || (oq.ptr != NULL && (oq.dtype != QB_E4M3 || oq.numel != out.numel))) Py_RETURN_NONE;
+  p.n_kv_heads = (int32_t)g.nk; p.gqa_ratio = (int32_t)gqa; p.H_spatial = (int32_t)g.H; p.W_spatial = (int32_t)g.W;
+  p.num_buckets = (int32_t)g.nb; p.pinned_dilation = (int32_t)g.pd; p.kv_dtype = p.compute_dtype = Kc.dtype; p.max_segments = (int32_t)g.segs;
+  p.packed_qkv = g.packed; p.quilt_factor = (int32_t)g.qf; p.kv_splits = (int32_t)splits;
+  const size_t need = g_lib.attn_ws(&p);
+  if (need > (size_t)ws.nbytes) Py_RETURN_NONE;
+  RUN(g_lib.attn(Q.ptr, Kc.ptr, Vc.ptr, seg.ptr, nseg.ptr, ft.ptr, out.ptr, oq.ptr, rope.ptr, &p, need > 0 ? ws.ptr : NULL, need > 0 ? (size_t)ws.nbytes : 0, st));
+}
+
 /* (tensor class, {entry point: address}) */
 static PyObject* fast_bind(PyObject* self, PyObject* args) {
   PyObject *cls, *table;
@@ -265,10 +354,11 @@ static PyObject* fast_bind(PyObject* self, PyObject* args) {
     }
     *at[i] = ((PyMemberDescrObject*)d)->d_member->offset;
   }
-  static const char* const names[11] = {"qb_gemm", "qb_gemm_workspace_bytes", "qb_ada_rmsnorm", "qb_rmsnorm", "qb_head_rmsnorm", "qb_ada_gate_residual",
-                                        "qb_silu", "qb_add", "qb_euler_step", "qb_quantize_e4m3", "qb_dequantize_e4m3"};
+  static const char* const names[15] = {"qb_gemm", "qb_gemm_workspace_bytes", "qb_ada_rmsnorm", "qb_rmsnorm", "qb_head_rmsnorm", "qb_ada_gate_residual",
+                                        "qb_silu", "qb_add", "qb_euler_step", "qb_quantize_e4m3", "qb_dequantize_e4m3", "qb_kv_cache_update",
+                                        "qb_kv_cache_update_kv", "qb_owl_attn_scratch_bytes", "qb_owl_attn"};
   void** const fn = (void**)&g_lib;
-  for (int i = 0; i < 11; ++i) {
+  for (int i = 0; i < 15; ++i) {
     PyObject* v = PyDict_GetItemString(table, names[i]);
     if (v == NULL) {
       PyErr_Format(PyExc_KeyError, "bind: %s", names[i]);
@@ -285,7 +375,7 @@ static PyObject* fast_bind(PyObject* self, PyObject* args) {
 
 #define F(name) {#name, (PyCFunction)(void (*)(void))fast_##name, METH_FASTCALL, NULL}
 static PyMethodDef methods[] = {{"bind", fast_bind, METH_VARARGS, NULL}, F(gemm), F(ada_rmsnorm), F(rmsnorm), F(head_rmsnorm), F(gate_residual), F(silu),
-                                F(add), F(euler_step), F(quantize), F(dequantize), {NULL, NULL, 0, NULL}};
+                                F(add), F(euler_step), F(quantize), F(dequantize), F(kv_cache_update), F(owl_attn), {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", NULL, -1, methods, NULL, NULL, NULL, NULL};
 
 PyMODINIT_FUNC PyInit__fastcall(void) {

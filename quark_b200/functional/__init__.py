@@ -349,6 +349,13 @@ def kv_cache_update(K, V, frame_t, frozen, Vt_cache, segments, n_segments, K_cac
     Returns ``(K_cache, Vt_cache, segments, n_segments)``, the very tensors that were passed in.
     """
     del rope_n_frames
+    rc = _fast.kv_cache_update(K, V, frame_t, frozen, Vt_cache, segments, n_segments, K_cache, B, n_kv_heads, H_spatial, W_spatial, num_buckets, pinned_dilation,
+                               kv_dtype, max_segments, packed_qkv, n_q_heads, quilt_factor, quilt_offset, k_scale, v_scale, _ROPE.get((H_spatial, W_spatial)),
+                               _s())  # fmt: skip
+    if rc is not None:
+        if rc:
+            _lib.check(rc)
+        return K_cache, Vt_cache, segments, n_segments
     tpf = int(H_spatial) * int(W_spatial)
     _quilt_checks("qf.kv_cache_update", tpf, quilt_factor, quilt_offset)
     if B != 1:
@@ -493,6 +500,14 @@ def owl_attn(Q, K_cache, Vt_cache, segments, n_segments, B, n_kv_heads, gqa_rati
              quilt_offset=0, frame_t=None, *, out=None, out_q=None, k_scale=None, v_scale=None, kv_splits=0):  # fmt: skip
     """Segment-sparse GQA attention with inline Q RoPE (``src/quark/functional/owl_attn.py:322-394``)."""
     global _DUMMY_FRAME_T
+    if out is not None:
+        rc = _fast.owl_attn(Q, K_cache, Vt_cache, segments, n_segments, B, n_kv_heads, gqa_ratio, H_spatial, W_spatial, num_buckets, pinned_dilation, out_dtype,
+                            compute_dtype, max_segments, packed_qkv, quilt_factor, quilt_offset, frame_t, out, out_q, k_scale, v_scale, kv_splits,
+                            _ROPE.get((H_spatial, W_spatial)), _ATTN_WS, _s())  # fmt: skip
+        if rc is not None:
+            if rc:
+                _lib.check(rc)
+            return out
     if Q.ndim != 2:
         raise ValueError(f"qf.owl_attn: Q must be rank-2 (flat), got {Q.shape}")
     tpf = int(H_spatial) * int(W_spatial)

@@ -183,7 +183,25 @@ def test_calls_made_in_c_equal_the_python_path(qb, monkeypatch):
         lambda: qf.quantize_e4m3(x, out=e(24, 256, dt="e4m3")),
         lambda: qf.dequantize_e4m3(wq, out=e(72, 256)),
     ]
+    geo = dict(B=1, n_kv_heads=2, H_spatial=8, W_spatial=8, num_buckets=3, pinned_dilation=1)
+    hk, hv, hq = (T(qb, bf16_randn(r, (n * 64, 64)), "bf16") for n in (2, 2, 4))
+    pk = T(qb, bf16_randn(r, (64, 8 * 64)), "bf16")
+    ft, fz = T(qb, np.array([5], np.int32)), T(qb, np.array([0], np.int32))
+
+    def attend(packed, dt, **kw):
+        Kc, Vc = T(qb, np.zeros((512, 64), np.uint16 if dt == "bf16" else np.uint8), dt), T(qb, np.zeros((128, 256), np.uint16 if dt == "bf16" else np.uint8), dt)
+        seg, nseg = T(qb, np.zeros(6, np.int32)), T(qb, np.zeros(1, np.int32))
+        for i in range(4):
+            ft.copy_from_numpy(np.array([i], np.int32))
+            qf.kv_cache_update(pk if packed else hk, None if packed else hv, ft, fz, Vc, seg, nseg, Kc, packed_qkv=packed, n_q_heads=4, **geo)
+        return qf.owl_attn(pk if packed else hq, Kc, Vc, seg, nseg, gqa_ratio=2, packed_qkv=packed, frame_t=ft,
+                           **{**geo, "compute_dtype": dt, "out": e(64 if packed else 256, 256 if packed else 64), **kw})  # fmt: skip
+
+    calls += [lambda: attend(False, "bf16"), lambda: attend(True, "e4m3"), lambda: attend(False, "e4m3", kv_splits=2, out_q=e(256, 64, dt="e4m3"))]
     wrong = [
+        (ValueError, lambda: attend(False, "bf16", quilt_factor=3)),
+        (ValueError, lambda: attend(False, "bf16", out=e(64, 64))),
+        (NotImplementedError, lambda: attend(True, "bf16", B=2)),
         (ValueError, lambda: qf.gemm(x, w, out=e(24, 64))),
         (ValueError, lambda: qf.gemm(x, w, out=e(24, 72), out_dtype="f32")),
         (ValueError, lambda: qf.gemm(x, w, out=e(24, 72), gate=g72)),
