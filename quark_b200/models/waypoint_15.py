@@ -357,14 +357,19 @@ class TransformerBlock(nn.Module):
             self.mlp = nn.MLP(d, cfg.mlp_dim_local, d, out_dtype="bf16", fuse_silu=cfg.fuse_silu)
         self.mlp_gate = nn.AdaGateResidual()
 
-    def forward(self, x, sigma_idx: int, frame_t, *, qkv_first, ctrl_emb=None, frozen: bool = False, x_out=None, h_in=None, next_norm=None, prefetch=None):
+    def ctrl_row(self, ctrl_emb):
+        return self.ctrl_fusion.cond_row(self.ctrl_emb_norm(ctrl_emb))
+
+    def forward(self, x, sigma_idx: int, frame_t, *, qkv_first, ctrl_emb=None, frozen: bool = False, x_out=None, h_in=None, next_norm=None, prefetch=None,
+                ctrl_row=None):  # fmt: skip
         """Returns ``(x, qkv)`` (``src/quark/models/waypoint_15.py:389-440``).
 
         Tensor-parallel ranks with a fused reduction (``comm.fused``): the sum over the ranks, gate + residual and the
         AdaRMSNorm that follows are one kernel, so the pre-MLP norm never runs as a launch of its own, and the norm that
         follows the block (``next_norm = (scale, bias, activation, emit_e4m3)``: the next block's pre-attention norm, or
         the output norm) is produced by this block's last reduction and left in ``self.h_next``; ``h_in`` is what the
-        previous block left there.  ``prefetch`` is called just before the attention is launched."""
+        previous block left there.  ``prefetch`` is called just before the attention is launched.  ``ctrl_row`` is what
+        ``Waypoint15.ctrl_rows`` made of the controller embedding for this block; without it the block works it out."""
         s0, b0, g0, s1, b1, g1 = self._cond_lut[sigma_idx]
         fp8 = self.qkv_proj.weight.data.dtype == "e4m3"
         tp = self._cfg.tp_world > 1
@@ -428,7 +433,8 @@ class TransformerBlock(nn.Module):
                 self._comm.all_reduce_sum(y)
             x = self.attn_gate(x, y, g0)
         if ctrl_emb is not None and hasattr(self, "ctrl_fusion"):
-            x = self.ctrl_residual(x, self.ctrl_fusion(self.ctrl_x_norm(x), self.ctrl_emb_norm(ctrl_emb)))
+            row = ctrl_row if ctrl_row is not None else self.ctrl_row(ctrl_emb)
+            x = self.ctrl_residual(x, self.ctrl_fusion(self.ctrl_x_norm(x), cond_row=row))
         moe = self._cfg.moe
         if h is None:
             h = self.pre_mlp_norm(x, s1, b1, emit_e4m3=fp8 and not moe)  # the router reads bf16; MoE narrows for its experts itself
@@ -521,6 +527,11 @@ class Waypoint15(nn.Module):
             raise TypeError(f"encode_ctrl: expected a bf16 [1, {self.cfg.ctrl_input_width}] row, got {ctrl_input.dtype} {ctrl_input.shape}")
         return self.ctrl_emb(ctrl_input)
 
+    def ctrl_rows(self, ctrl_emb):
+        """Per block, its projection of the controller embedding (None without one).  It is the same in every pass of a frame, so
+        a frame works it out once: two launches fewer per conditioned block and pass."""
+        return [blk.ctrl_row(ctrl_emb) if ctrl_emb is not None and hasattr(blk, "ctrl_fusion") else None for blk in self.blocks]
+
     def set_frame_t(self, value: int) -> None:
         for blk in self.blocks:
             blk.kv_cache.set_frame_t(value)
@@ -529,7 +540,7 @@ class Waypoint15(nn.Module):
         for blk in self.blocks:
             blk.kv_cache.reset()
 
-    def forward(self, latent, sigma_idx: int, frame_t=None, ctrl_emb=None, frozen: bool = False):
+    def forward(self, latent, sigma_idx: int, frame_t=None, ctrl_emb=None, frozen: bool = False, *, ctrl_rows=None):
         """One NFE on a ``[1, C*2H*2W]`` bf16 latent (``src/quark/models/waypoint_15.py:626-661``)."""
         if latent.dtype != "bf16" or latent.numel != self.cfg.latent_numel:
             raise TypeError(f"Waypoint15: latent must be bf16 with {self.cfg.latent_numel} elements, got {latent.dtype} {latent.shape}")
@@ -549,7 +560,7 @@ class Waypoint15(nn.Module):
             else:
                 next_norm = (s_on, b_on, "silu", False)
             x, qkv = block(x, sigma_idx, frame_t, qkv_first=qkv_first, ctrl_emb=ctrl_emb, frozen=frozen, x_out=self._x_bufs[li & 1], h_in=h_in,
-                           next_norm=next_norm, prefetch=ahead and ahead[li])  # fmt: skip
+                           next_norm=next_norm, prefetch=ahead and ahead[li], ctrl_row=ctrl_rows and ctrl_rows[li])  # fmt: skip
             h_in = block.h_next
             if li == 0 and self.cfg.value_residual:
                 qkv_first = qkv
@@ -611,10 +622,11 @@ class GenerateFrame(nn.Module):
         ft = self.frame_t
         x = latent
         ctrl_emb = self.model.encode_ctrl(ctrl_input)
+        rows = self.model.ctrl_rows(ctrl_emb)
         for si in range(self.n_denoise):
-            v = self.model(x, sigma_idx=si, frame_t=ft, ctrl_emb=ctrl_emb, frozen=True)
+            v = self.model(x, sigma_idx=si, frame_t=ft, ctrl_emb=ctrl_emb, frozen=True, ctrl_rows=rows)
             x = self.euler_steps[si](x, v, self.dsig_tensors[si])
-        self.model(x, sigma_idx=self.n_denoise, frame_t=ft, ctrl_emb=ctrl_emb)
+        self.model(x, sigma_idx=self.n_denoise, frame_t=ft, ctrl_emb=ctrl_emb, ctrl_rows=rows)
         qf.increment(ft)
         return x
 

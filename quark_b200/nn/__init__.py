@@ -309,8 +309,12 @@ class MLPFusion(Module):
         self.fc1_c = Linear(d_model, d_model, out_dtype=out_dtype)
         self.fc2 = Linear(d_model, d_model, out_dtype=out_dtype)
 
-    def forward(self, x, cond):
-        h_c = self.fc1_c(cond).reshape(-1)
+    def cond_row(self, cond):
+        """The cond projection, for callers that use it with several ``x``; its buffer is this module's own."""
+        return self.fc1_c(cond).reshape(-1)
+
+    def forward(self, x, cond=None, *, cond_row=None):
+        h_c = cond_row if cond_row is not None else self.cond_row(cond)
         return self.fc2(self.fc1_x(x, bias=h_c, activation="silu"))
 
 
