@@ -12,6 +12,7 @@ result back: those copies are the only host <-> device traffic per frame.
 from __future__ import annotations
 
 import ctypes as C
+import operator
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -48,30 +49,61 @@ class CtrlInput:
 
 
 class _AppendGraph:
-    """The commit pass of ``Engine.append_frame`` as a CUDA graph: issued call by call the pass is bound by the host.  It holds the
-    addresses it was captured with, so ``current()`` says whether the model still has the tensors it had then."""
+    """The commit pass of ``Engine.append_frame`` as a CUDA graph: issued call by call the pass is bound by the host.
 
-    def __init__(self, engine: "Engine", ctrl_dev):
-        self._settings = _lib.settings_version
-        self._blocks = list(engine.model.blocks)
-        self._params = [(p, p.data) for _, p in engine.model.named_parameters()]
-        self._caches = [(kc, kc.K_cache, kc.Vt_cache, kc.k_scale, kc.v_scale) for kc in (b.kv_cache for b in self._blocks)]
-        si = engine.gen.n_denoise
-        self._luts = [(b, si, b._cond_lut[si]) for b in self._blocks]
-        self._out_lut = (engine.model, si, engine.model._out_norm_luts[si])
+    The graph holds the addresses and choices of the pass it was captured from, so ``current()`` says whether a pass issued now
+    would make the same calls: every attribute of every module (tensors, scales, sub-modules, the configuration), the lists and dicts
+    among them by content, and the library's switches are what they were.  (Comparing them takes 26 us for 24 layers.)"""
+
+    def __init__(self, engine: "Engine", capture: bool):
+        self._graph = None
+        if capture:
+            self._capture(engine)
+        else:
+            self._watch(engine)
+
+    @staticmethod
+    def possible(engine: "Engine") -> bool:
+        """Whether a replay stands for the whole pass: the host side of a ``forward`` that is not this package's own has to run."""
+        package = __name__.partition(".")[0]
+        return engine.model.comm is None and all(
+            "forward" not in vars(m) and type(m).forward.__module__.partition(".")[0] == package for _, m in engine.model.named_modules()
+        )
+
+    def _capture(self, engine: "Engine") -> None:
         with _stream.capture_graph() as cap:
-            engine._append_pass(ctrl_dev)
+            engine._append_pass(engine._ctrl_dev)
         self._graph = cap.graph
+        self._watch(engine)
 
-    def current(self) -> bool:
-        model, si, rows = self._out_lut
-        return (self._settings == _lib.settings_version and model._out_norm_luts[si] is rows and all(p.data is d for p, d in self._params)
-                and all(b._cond_lut[i] is r for b, i, r in self._luts)
-                and all(kc.K_cache is K and kc.Vt_cache is V and kc.k_scale is ks and kc.v_scale is vs for kc, K, V, ks, vs in self._caches))  # fmt: skip
+    def _watch(self, engine: "Engine") -> None:
+        model, host_only = engine.model, ("_bufs", "_shadow_seen")  # filled as the host goes through a pass
+        modules = [m for _, m in model.named_modules()]
+        live = [vars(m) for m in modules]
+        live += [v for m in modules for k, v in vars(m).items() if isinstance(v, (list, dict)) and k not in host_only]
+        self._live, self._held = live, [v.copy() for v in live]
+        self._classes = [(t, t.forward) for t in {type(m) for m in modules}]
+        self._params = [p for _, p in model.named_parameters()]
+        self._data = [p.data for p in self._params]
+        self._around = self._surroundings(engine)
 
-    def launch(self) -> None:
-        for b in self._blocks:
+    @staticmethod
+    def _surroundings(engine: "Engine") -> tuple:
+        return engine.model, engine.gen, engine.gen.n_denoise, engine.gen.frame_t, engine._append_dev, engine._ctrl_dev, _lib.settings_version
+
+    def current(self, engine: "Engine") -> bool:
+        # (equal values are the same object or equal numbers: tensors and modules compare by identity)
+        try:
+            return (self._surroundings(engine) == self._around and [p.data for p in self._params] == self._data
+                    and all(map(operator.eq, self._live, self._held)) and all(t.forward is f for t, f in self._classes))  # fmt: skip
+        except ValueError:  # an array of the caller's among the attributes, replaced by another
+            return False
+
+    def launch(self, engine: "Engine") -> None:
+        for b in engine.model.blocks:
             b.kv_cache.sync_shadow()
+        if self._graph is None:
+            self._capture(engine)
         self._graph.launch()
 
 
@@ -233,13 +265,16 @@ class Engine:
         self._noise_host.array[:] = self._to_bf16(latent)
         self._h2d(self._append_dev, self._noise_host.ptr, self.cfg.latent_numel * 2)
         ctrl_dev = self._encode_ctrl(ctrl)
-        if self._append_graph is not None and self._append_graph.current():
-            self._append_graph.launch()
+        seen = self._append_graph
+        if seen is not None and seen.current(self):
+            seen.launch(self)
         else:
             self._append_graph = None
             self._append_pass(ctrl_dev)
-            if self._use_graph and self.model.comm is None:  # every buffer of the pass exists now
-                self._append_graph = _AppendGraph(self, ctrl_dev)
+            if self._use_graph and _AppendGraph.possible(self):
+                # Every buffer of the pass exists now.  A model that was changed is captured again once it has stayed as it is for
+                # a frame: one that changes with every frame would pay for a capture each time.
+                self._append_graph = _AppendGraph(self, capture=seen is None)
         _stream.synchronize()
         self._frame += 1
         return np.asarray(latent)

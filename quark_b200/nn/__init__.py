@@ -408,6 +408,8 @@ class KVCacheUpdate(Module):
         self._L, self._tpf = L, tpf
         # optional per-head quantisation scales (f32 [n_kv_heads]); None = the reference's scale-free caches
         self.k_scale = self.v_scale = None
+        self._shadow = None
+        self._shadow_seen = []  # host writes of the two caches that the shadow holds
         self._kw = dict(B=B, n_kv_heads=n_kv_heads, H_spatial=H_spatial, W_spatial=W_spatial, num_buckets=num_buckets,
                         pinned_dilation=pinned_dilation, packed_qkv=packed_qkv, n_q_heads=n_q_heads, quilt_factor=quilt_factor,
                         quilt_offset=quilt_offset)  # fmt: skip
@@ -425,32 +427,33 @@ class KVCacheUpdate(Module):
         attention loads (``src/quark/kernels/owl_attn/kernel.py:342-348``): same values."""
         if dtype == self.K_cache.dtype:
             return self.K_cache, self.Vt_cache
-        if getattr(self, "_shadow", None) is None or self._shadow[0].dtype != dtype:
+        if self._shadow is None or self._shadow[0].dtype != dtype:
             self._shadow = (QuarkTensor.empty(*self.K_cache.shape, dtype=dtype), QuarkTensor.empty(*self.Vt_cache.shape, dtype=dtype))
-            self._shadow_seen = None
-        seen = (self.K_cache._storage.host_writes, self.Vt_cache._storage.host_writes)
-        if self._shadow_seen != seen:
+            self._shadow_seen.clear()
+        if self._shadow_seen != self._host_writes():
             self.refresh_shadow()
         else:
             qf.kv_cast_appended(self.K_cache, self.Vt_cache, self._shadow[0], self._shadow[1], frame_t if frame_t is not None else self.frame_t,
                                 self._frozen[1 if frozen else 0], **self._kw)  # fmt: skip
         return self._shadow
 
+    def _host_writes(self) -> list:
+        return [self.K_cache._storage.host_writes, self.Vt_cache._storage.host_writes]
+
     def sync_shadow(self) -> None:
         """Converts both caches whole if they were written from the host since they were last (a captured pass only converts the
         rows its own append writes)."""
-        if getattr(self, "_shadow", None) is not None:
-            if self._shadow_seen != (self.K_cache._storage.host_writes, self.Vt_cache._storage.host_writes):
-                self.refresh_shadow()
+        if self._shadow is not None and self._shadow_seen != self._host_writes():
+            self.refresh_shadow()
 
     def refresh_shadow(self) -> None:
         """Converts both caches whole (after the caches were written by anything but the append)."""
-        if getattr(self, "_shadow", None) is None:
+        if self._shadow is None:
             return
         conv = qf.quantize_e4m3 if self._shadow[0].dtype == "e4m3" else qf.dequantize_e4m3
         conv(self.K_cache, out=self._shadow[0])
         conv(self.Vt_cache, out=self._shadow[1])
-        self._shadow_seen = (self.K_cache._storage.host_writes, self.Vt_cache._storage.host_writes)
+        self._shadow_seen[:] = self._host_writes()
 
     def set_scales(self, k_scale, v_scale) -> None:
         """Per-KV-head scales as host arrays (or None): the caches then hold ``K / k_scale[h]`` and ``V / v_scale[h]``."""

@@ -1,6 +1,8 @@
 """The branches that a call's sizes choose: key shares of the attention, expert runs of the routing and of the grouped GEMM, column
 remainders of the GEMM epilogues, the captured append pass, and the calls that are checked and made in C."""
 
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -137,6 +139,64 @@ def test_append_pass_captured_equals_call_by_call(qb, quant):
         for a, b in zip(engines[0].model.blocks, engines[1].model.blocks):
             for x in ("K_cache", "Vt_cache", "segments", "n_segments"):
                 np.testing.assert_array_equal(getattr(a.kv_cache, x).to_numpy(), getattr(b.kv_cache, x).to_numpy())
+
+
+def _new_caches(qb, e):
+    kc = e.model.blocks[1].kv_cache
+    new = qb.nn.KVCacheUpdate(rope_n_frames=1, Dh=64, dtype=kc.K_cache.dtype, **kc._kw)
+    for k in ("K_cache", "Vt_cache", "segments", "n_segments"):
+        getattr(new, k).copy_from(getattr(kc, k))
+    e.model.blocks[1].kv_cache = new
+
+
+def _host_side_of_its_own(qb, e):
+    blk, own = e.model.blocks[1], e.model.blocks[1].forward
+    e.seen = []
+    blk.forward = lambda *a, **kw: (e.seen.append(1), own(*a, **kw))[1]
+
+
+def _new_lut_row(qb, e):
+    lut = e.model.blocks[1]._cond_lut
+    lut[-1] = tuple(T(qb, np.zeros(t.shape, np.uint16), "bf16") for t in lut[-1])
+
+
+def _new_counter(qb, e):
+    e.gen.frame_t = T(qb, e.gen.frame_t.to_numpy() + 3)
+
+
+@pytest.mark.parametrize("change", [
+    _new_caches,
+    _host_side_of_its_own,
+    _new_lut_row,
+    _new_counter,
+    lambda qb, e: setattr(e.model.blocks[1].qkv_proj, "w_scale", T(qb, np.linspace(0.5, 2.0, e.cfg.qkv_dim, dtype=np.float32))),
+    lambda qb, e: e.model.blocks[1].kv_cache.set_scales(np.full(1, 2.0, np.float32), np.full(1, 0.5, np.float32)),
+    lambda qb, e: setattr(e.model.blocks[1], "mlp", e.model.blocks[2].mlp),
+    lambda qb, e: setattr(e.model.blocks[1], "_cfg", dataclasses.replace(e.cfg, fuse_gate_residual=False)),
+])  # fmt: skip
+def test_append_pass_captured_follows_a_changed_model(qb, change):
+    """Whatever a pass reads of the model and of the engine, changed after the capture, is seen by the next append."""
+    from quark_b200.models import QuantConfig, Waypoint15Config, make_params
+
+    q = QuantConfig(linear="fp8", kv_cache="fp8", attn_compute="bf16")  # the attention reads shadow caches
+    cfg = Waypoint15Config(d_model=128, n_layers=3, n_heads=2, n_kv_heads=1, height=8, width=8, channels=4, local_window=2, global_window=4,
+                           global_pinned_dilation=2, quant=q)  # fmt: skip
+    params = make_params(cfg, seed=9, weight_std=0.08)
+    r = util.rng(88)
+    engines = [qb.Engine(cfg=cfg, quant=q, params=params, use_graph=g) for g in (True, False)]
+    for i in range(7):
+        lat = codec.f32_to_bf16(r.standard_normal((1, cfg.latent_numel)).astype(np.float32))
+        for e in engines:
+            if i == 3:
+                change(qb, e)
+            e.append_frame(lat)
+        for a, b in zip(engines[0].model.blocks, engines[1].model.blocks):
+            for x in ("K_cache", "Vt_cache", "segments", "n_segments"):
+                np.testing.assert_array_equal(getattr(a.kv_cache, x).to_numpy(), getattr(b.kv_cache, x).to_numpy(), err_msg=f"append {i}")
+    if change is _host_side_of_its_own:
+        assert len(engines[0].seen) == len(engines[1].seen) == 4
+    else:
+        assert engines[0]._append_graph._graph is not None  # captured again
 
 
 @pytest.mark.parametrize("quant", ["bf16", "fp8"])
