@@ -67,7 +67,7 @@ class _AppendGraph:
         """Whether a replay stands for the whole pass: the host side of a ``forward`` that is not this package's own has to run."""
         package = __name__.partition(".")[0]
         return engine.model.comm is None and all(
-            "forward" not in vars(m) and type(m).forward.__module__.partition(".")[0] == package for _, m in engine.model.named_modules()
+            "forward" not in vars(m) and str(getattr(type(m).forward, "__module__", "")).partition(".")[0] == package for _, m in engine.model.named_modules()
         )
 
     def _capture(self, engine: "Engine") -> None:

@@ -409,7 +409,7 @@ class KVCacheUpdate(Module):
         # optional per-head quantisation scales (f32 [n_kv_heads]); None = the reference's scale-free caches
         self.k_scale = self.v_scale = None
         self._shadow = None
-        self._shadow_seen = []  # host writes of the two caches that the shadow holds
+        self._shadow_seen = []  # the memory of the caches that the shadow holds, and their host writes then
         self._kw = dict(B=B, n_kv_heads=n_kv_heads, H_spatial=H_spatial, W_spatial=W_spatial, num_buckets=num_buckets,
                         pinned_dilation=pinned_dilation, packed_qkv=packed_qkv, n_q_heads=n_q_heads, quilt_factor=quilt_factor,
                         quilt_offset=quilt_offset)  # fmt: skip
@@ -423,7 +423,7 @@ class KVCacheUpdate(Module):
     def shadow(self, dtype: str, frame_t=None, frozen: bool = False):
         """``(K, Vt)`` equal to ``cast(K_cache), cast(Vt_cache)`` in ``dtype``, to be called after the append of the step:
         the rows that append wrote are converted (``qf.kv_cast_appended``); if the caches were written from the host since
-        the last call (loaded, restored, reset) or this is the first call, everything is.  The reference casts as the
+        the last call (loaded, restored, reset), are other tensors than then or this is the first call, everything is.  The reference casts as the
         attention loads (``src/quark/kernels/owl_attn/kernel.py:342-348``): same values."""
         if dtype == self.K_cache.dtype:
             return self.K_cache, self.Vt_cache
@@ -438,7 +438,8 @@ class KVCacheUpdate(Module):
         return self._shadow
 
     def _host_writes(self) -> list:
-        return [self.K_cache._storage.host_writes, self.Vt_cache._storage.host_writes]
+        K, Vt = self.K_cache._storage, self.Vt_cache._storage
+        return [K, K.host_writes, Vt, Vt.host_writes]
 
     def sync_shadow(self) -> None:
         """Converts both caches whole if they were written from the host since they were last (a captured pass only converts the

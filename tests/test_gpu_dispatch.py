@@ -199,6 +199,28 @@ def test_append_pass_captured_follows_a_changed_model(qb, change):
         assert engines[0]._append_graph._graph is not None  # captured again
 
 
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_shadow_caches_follow_replaced_caches(qb, use_graph):
+    """Caches put in the place of others are brought over whole, however often either was written from the host."""
+    from quark_b200.models import QuantConfig, Waypoint15Config, make_params
+
+    q = QuantConfig(linear="fp8", kv_cache="fp8", attn_compute="bf16")
+    cfg = Waypoint15Config(d_model=128, n_layers=2, n_heads=2, n_kv_heads=1, height=8, width=8, channels=4, local_window=2, global_window=4,
+                           global_pinned_dilation=2, quant=q)  # fmt: skip
+    eng, r = qb.Engine(cfg=cfg, quant=q, params=make_params(cfg, seed=9, weight_std=0.08), use_graph=use_graph), util.rng(89)
+    kc = eng.model.blocks[0].kv_cache
+    for i in range(4):
+        if i == 2:
+            for name in ("K_cache", "Vt_cache"):
+                old = getattr(kc, name)
+                new = T(qb, e4m3_randn(r, old.shape), "e4m3")
+                new._storage.host_writes = old._storage.host_writes
+                setattr(kc, name, new)
+        eng.append_frame(codec.f32_to_bf16(r.standard_normal((1, cfg.latent_numel)).astype(np.float32)))
+        for cache, sh in zip((kc.K_cache, kc.Vt_cache), kc._shadow):
+            np.testing.assert_array_equal(f32(sh.to_numpy(), "bf16"), f32(cache.to_numpy(), "e4m3"), err_msg=f"append {i}")
+
+
 @pytest.mark.parametrize("quant", ["bf16", "fp8"])
 def test_weights_fetched_ahead_change_no_bit(qb, quant, monkeypatch):
     from quark_b200.models import QuantConfig, Waypoint15Config, make_params, waypoint_15
