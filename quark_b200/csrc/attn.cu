@@ -585,6 +585,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         umma_commit(smem_u32(&kv_empty[(2 * i + g) % kStages]));
         QB_TR(2 + g, i, 5);
       }
+      if (ok && late(g == 0 && blockIdx.x == gridDim.x - 1 && blockIdx.z == gridDim.z - 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN)) ok = false;
       // pv_done flips once per tile and the fp8 softmax warps rarely look at it, so its parity cannot tell
       // "all finished" from "two still in flight"; the end of the accumulation has a barrier of its own
       if (ok && (kSplit == kHelped || i0 < i1)) umma_commit(smem_u32(&o_final[g]));
@@ -765,6 +766,9 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       const int S = static_cast<int>(gridDim.z), rows = merge_rows(S);
       float* area = reinterpret_cast<float*>(smem + L::kStageOff);
       cluster_sync();  // the stages of every CTA are free (its tensor work and TMA traffic are finished)
+      // Nobody waits any more, so the flag now tells whether one of this CTA's waits ran out; if so, the rows that its results belong
+      // to are not written by any CTA of the cluster.
+      if (*abort_flag != 0 && threadIdx.x - 128 < S) st_dsmem(map_to_cta(smem_u32(const_cast<const int*>(abort_flag)), threadIdx.x - 128), 1);
       {
         const uint32_t base = map_to_cta(smem_u32(area), r / rows);
         const int part = 2 * static_cast<int>(blockIdx.z) + g, rl = r % rows;
@@ -776,7 +780,8 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
       }
       cluster_sync();
       const float vs = a.v_scale ? __ldg(a.v_scale + kvh) : 1.0f;
-      for (int i = threadIdx.x - 128; i < rows * 8; i += 256) {  // 8 outputs of a row per thread
+      const bool whole_cluster = *abort_flag == 0;
+      for (int i = threadIdx.x - 128; whole_cluster && i < rows * 8; i += 256) {  // 8 outputs of a row per thread
         const int rl = i >> 3, d0 = (i & 7) * 8, rr = static_cast<int>(blockIdx.z) * rows + rl;
         if (rr >= kQTile || q0 + rr >= a.tpf) continue;
         float m = -1.0e30f;
@@ -862,7 +867,12 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         __threadfence();
         asm volatile("bar.sync 3, 128;" ::: "memory");
         int* last = reinterpret_cast<int*>(comb);  // the group's exchange buffer is free again
-        if (r == 0) *last = atomicAdd(a.tickets + item, 1) == n_splits - 1;
+        if (r == 0) {
+          const int was = atomicAdd(a.tickets + item, *abort_flag == 0 ? 1 : kLostTicket + 1);
+          const bool mine_is_last = (was & (kLostTicket - 1)) == n_splits - 1;
+          if (mine_is_last) a.tickets[item] = 0;  // ready for the next launch
+          *last = mine_is_last && was < kLostTicket;
+        }
         asm volatile("bar.sync 3, 128;" ::: "memory");
         writer = *last != 0;
         if (writer) {
@@ -881,7 +891,6 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
 #pragma unroll
             for (int d = 0; d < 64; ++d) e[d] = fmaf(w, __ldcg(pz + (2 + d) * 128 + r), e[d]);
           }
-          if (r == 0) a.tickets[item] = 0;  // ready for the next launch
         }
       }
       if (writer && good && row_ok) {

@@ -431,6 +431,7 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
           umma_commit(smem_u32(&pv_done[g]));
           umma_commit(smem_u32(&kv_empty[(g + G * i) % kStages]));
         }
+        if (ok && late(g == 0 && blockIdx.x == gridDim.x - 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN)) ok = false;
         if (ok && (kHelped || i0 < i1)) umma_commit(smem_u32(&o_final[g]));  // the end of the accumulation has a barrier of its own
         if (kHelped) {
           kr.next(pc);

@@ -35,6 +35,10 @@ struct AttnArgs {
 
 __device__ __forceinline__ float ex2_approx(float x);
 
+// A ticket for a partial result that must not be used (a wait of its CTA ran out): the CTA that draws the last ticket, which counts
+// them in the lower bits, then writes no row of the item.
+constexpr int kLostTicket = 1 << 16;
+
 constexpr int kPartial = 66 * 128;  // floats of a partial result: m and row sum of 128 rows, then 64 x 128 outputs
 
 // What the softmax warps do next: `n` more tiles (0: nothing) of an item, the tile0-th first, `done` tiles into the CTA's work.
@@ -131,9 +135,10 @@ struct KeyShares {
     __threadfence();
     asm volatile("bar.sync 3, 128;" ::: "memory");
     if (r == 0) {
-      const bool last = atomicAdd(a.tickets + p.item, 1) == 1;
+      const int was = atomicAdd(a.tickets + p.item, good ? 1 : kLostTicket + 1);
+      const bool last = (was & (kLostTicket - 1)) == 1;
       if (last) a.tickets[p.item] = 0;  // ready for the next launch
-      *exchange = last;
+      *exchange = last && was < kLostTicket;
     }
     asm volatile("bar.sync 3, 128;" ::: "memory");
     if (*exchange == 0) return;

@@ -1,19 +1,26 @@
 #!/bin/bash
 # Builds libquark_b200.so (sm_100a only) next to the Python package.  Usage: build.sh [-v]
+# QB_BUILD_DIR puts objects and library there instead (and leaves the extension out), with QB_BUILD_FLAGS for the compiler.
 set -e
 HERE="$(cd "$(dirname "$0")" && pwd)"
 OUT="$HERE/../libquark_b200.so"
+OBJ="$HERE/build"
+if [ -n "$QB_BUILD_DIR" ]; then
+  OUT="$QB_BUILD_DIR/libquark_b200.so"
+  OBJ="$QB_BUILD_DIR"
+fi
 NVCC="${NVCC:-nvcc}"
-FLAGS="-gencode arch=compute_100a,code=sm_100a -lineinfo -O3 -std=c++17 -Xcompiler -fPIC"
+FLAGS="-gencode arch=compute_100a,code=sm_100a -lineinfo -O3 -std=c++17 -Xcompiler -fPIC $QB_BUILD_FLAGS"
 [ "$1" = "-v" ] && FLAGS="$FLAGS -Xptxas -v"
-mkdir -p "$HERE/build"
+mkdir -p "$OBJ"
 pids=()
 for f in runtime gemm gemm_pair gemm_grouped attn attn4 kv glue qkv_post tp; do
-  $NVCC $FLAGS -c "$HERE/$f.cu" -o "$HERE/build/$f.o" &
+  $NVCC $FLAGS -c "$HERE/$f.cu" -o "$OBJ/$f.o" &
   pids+=($!)
 done
 for p in "${pids[@]}"; do wait $p; done
-$NVCC -shared -o "$OUT" "$HERE"/build/{runtime,gemm,gemm_pair,gemm_grouped,attn,attn4,kv,glue,qkv_post,tp}.o -cudart static
+$NVCC -shared -o "$OUT" "$OBJ"/{runtime,gemm,gemm_pair,gemm_grouped,attn,attn4,kv,glue,qkv_post,tp}.o -cudart static
+[ -n "$QB_BUILD_DIR" ] && exit 0
 # The C side of the smallest calls (a CPython extension); without the interpreter's headers they stay in Python.
 PYTHON="${PYTHON:-python3}"
 PYINC="$($PYTHON -c 'import sysconfig; print(sysconfig.get_paths()["include"])')"

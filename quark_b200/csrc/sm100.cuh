@@ -98,6 +98,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// Whether the tensor work of a main loop is reported late.  Never, but in the library that the tests of a wait that ran out build for
+// themselves (QB_LATE_WAIT): there the chosen CTAs' MMA threads, all their work done, wait about half a millisecond for a flag that
+// nothing sets.
+__device__ __forceinline__ bool late(bool chosen, volatile int* abort_flag, unsigned int* status_word, unsigned status_bit) {
+#ifdef QB_LATE_WAIT
+  if (chosen) {
+    for (const long long t0 = clock64(); clock64() - t0 < (1ll << 20);) __nanosleep(1000);
+    *abort_flag = 1;
+    atomicOr(status_word, status_bit);
+    return true;
+  }
+#endif
+  return false;
+}
+
 // ---------------------------------------------------------------- TMA (every copy lands in the issuing CTA only)
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
@@ -122,6 +137,9 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t cta_
 }
 __device__ __forceinline__ void st_dsmem_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void st_dsmem(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
