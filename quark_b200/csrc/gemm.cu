@@ -62,6 +62,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* last_flag = abort_flag + 1;
   volatile int* drain_flag = abort_flag + 2;  // never set: lets the drain waits below run their own limit
+  volatile int* lost_flag = abort_flag + 3;   // set by a CTA of the cluster whose slice is missing
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -86,6 +87,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     *abort_flag = 0;
     *last_flag = 0;
     *drain_flag = 0;
+    *lost_flag = 0;
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -162,7 +164,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
         umma_commit(smem_u32(&empty_bar[s]));
       }
-      umma_commit(smem_u32(acc_bar));
+      if (ok && late(blockIdx.x == gridDim.x - 1 && blockIdx.z == gridDim.z - 1, abort_flag, g.status, QB_DEV_WAIT_TIMEOUT_GEMM)) ok = false;
+      if (ok) umma_commit(smem_u32(acc_bar));  // else the epilogue gives up as well
       QB_GT(4);
     }
   } else {
@@ -337,7 +340,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         uint16_t* vt = reinterpret_cast<uint16_t*>(smem);  // over the stage memory (this CTA's MMAs are done)
         if (clustered) {
           if (ok) push_slices<1, BN>(smem + L::kSliceOffset, taddr, split, 0, row, half, g.splits);
+          else if (threadIdx.x == 64) tell_lost<1>(lost_flag, 0, g.splits);
           cluster_sync();  // warps 0 and 1 join it below
+          ok = ok && *lost_flag == 0;
         } else if (ok) {  // scaled (acc * (a_scale * w_scale[n])) and rounded to bf16, as the plain epilogue would store it
           const bool has_scale = g.a_scale != nullptr || g.w_scale != nullptr;
 #pragma unroll 1
@@ -370,8 +375,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     } else if (clustered) {
       if constexpr (BN == 64 && !QKV) {
         if (ok) push_slices<1, BN>(smem + L::kSliceOffset, taddr, split, 0, row, half, g.splits);
+        else if (threadIdx.x == 64) tell_lost<1>(lost_flag, 0, g.splits);
         cluster_sync();  // every slice's share of this CTA's rows has arrived after this barrier (warps 0 and 1 join it below)
-        if (ok) finish_slices<BN>(g, reinterpret_cast<const float4*>(smem + L::kSliceOffset), reinterpret_cast<const float*>(smem + L::kColOffset), m0, n0,
+        if (ok && *lost_flag == 0) finish_slices<BN>(g, reinterpret_cast<const float4*>(smem + L::kSliceOffset), reinterpret_cast<const float*>(smem + L::kColOffset), m0, n0,
                                   slice_row0, slice_rows, one_gate, pre);
       }
     } else if (g.splits == 1) {
@@ -393,11 +399,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       }
     } else if (half == 1) {
       // K slices through the workspace are summed by the first four epilogue warps
-    } else if (ok) {
+    } else {
       // K slices through the global workspace: partial tile out, ticket, last CTA adds the slices in order
       float* part = g.partials + static_cast<size_t>(split) * g.M * g.N;
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = 0; ok && c < BN / 32; ++c) {
         uint32_t r[32];
         tmem_ld32(taddr + c * 32, r);
         tmem_wait_ld_into(r);
@@ -416,8 +422,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       asm volatile("bar.sync 1, 128;" ::: "memory");
       int* counter = g.counters + blockIdx.y * gridDim.x + blockIdx.x;
       if (threadIdx.x == 64) {
-        const int ticket = atomicAdd(counter, 1);
-        *last_flag = (ticket == g.splits - 1) ? 1 : 0;
+        const int ticket = atomicAdd(counter, ok ? 1 : kLostTicket + 1);
+        const bool last = (ticket & (kLostTicket - 1)) == g.splits - 1;
+        if (last) *counter = 0;  // ready for the next launch
+        *last_flag = last && ok && ticket < kLostTicket;
         __threadfence();
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -437,7 +445,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
           epilogue_store8(g, v, mm, n);
         }
-        if (threadIdx.x == 64) *counter = 0;  // ready for the next launch
       }
     }
   }

@@ -179,6 +179,15 @@ __device__ __forceinline__ void push_slices(uint8_t* scratch, uint32_t taddr, in
   }
 }
 
+// A CTA whose slice is missing (a wait ran out) tells the CTAs that would sum it, in front of the cluster barrier behind which they
+// do; they write no row of the tile then.
+template <int CG>
+__device__ __forceinline__ void tell_lost(volatile int* lost_flag, int rank, int splits) {
+  for (int s = 0; s < splits; ++s) st_dsmem(map_to_cta(smem_u32(const_cast<const int*>(lost_flag)), CG * s + rank), 1);
+}
+// The same for slices through the workspace: what such a CTA adds to the tile's counter, whose lower half counts the tickets.
+constexpr int kLostTicket = 1 << 16;
+
 // Whether `ok` holds for all 256 epilogue threads (a barrier of theirs).
 __device__ __forceinline__ bool all_of_epilogue(bool ok) {
   uint32_t r;

@@ -107,8 +107,10 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     if (elect_one()) {
       int s = 0;
       uint32_t ph = 0;
+      bool ok = true;
       for (int it = 0; it < n_iter; ++it) {
-        if (!mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag, g.status, QB_DEV_WAIT_TIMEOUT_GEMM)) break;
+        ok = mbar_wait(smem_u32(&full_bar[s]), ph, abort_flag, g.status, QB_DEV_WAIT_TIMEOUT_GEMM);
+        if (!ok) break;
         tc_fence_after();
         const uint32_t st = smem_u32(smem + s * L::kStageBytes);
         const uint64_t b_desc = umma_desc_k_sw128(st + 2 * L::kABytes);
@@ -124,7 +126,8 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         umma_commit(smem_u32(&empty_bar[s]));
         if (++s == kStages) { s = 0; ph ^= 1; }
       }
-      umma_commit(smem_u32(acc_bar));
+      if (ok && late(blockIdx.x == gridDim.x - 1, abort_flag, g.status, QB_DEV_WAIT_TIMEOUT_GEMM)) ok = false;
+      if (ok) umma_commit(smem_u32(acc_bar));  // else the epilogue gives up as well
     }
   } else {
     // epilogue: two warps share each TMEM lane quarter and split the row's columns

@@ -71,6 +71,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* acc_empty = acc_full + 2;           // [2] the epilogue warps (of both CTAs of a pair) have read it
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* lost_flag = abort_flag + 1;  // set by a CTA of the cluster whose slice is missing
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -93,6 +94,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       mbar_init(smem_u32(&acc_empty[b]), 16);
     }
     *abort_flag = 0;
+    *lost_flag = 0;
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -208,7 +210,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           commit(&empty_bar[s]);
           if (++s == stages) { s = 0; ph ^= 1; }
         }
-        commit(&acc_full[acc]);
+        if (ok && late(blockIdx.x / 2 == gridDim.x / 2 - 1 && blockIdx.z == gridDim.z - 1, abort_flag, g.status, QB_DEV_WAIT_TIMEOUT_GEMM)) ok = false;
+        if (ok) commit(&acc_full[acc]);  // else both CTAs' epilogues give up as well
         ++done;
       }
     }
@@ -301,8 +304,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       } else {
         wait_acc();
         if (ok) push_slices<2, BN>(scratch, taddr, split, rank, row, half, g.splits);
+        else if (threadIdx.x == 64) tell_lost<2>(lost_flag, rank, g.splits);
         cluster_sync();  // every slice's share of this CTA's rows has arrived after this barrier (warps 0 and 1 join it below)
-        if (ok) finish_slices<BN>(g, reinterpret_cast<const float4*>(scratch), col, m0, n0, slice_row0, slice_rows, one_gate, pre);
+        if (ok && *lost_flag == 0) finish_slices<BN>(g, reinterpret_cast<const float4*>(scratch), col, m0, n0, slice_row0, slice_rows, one_gate, pre);
       }
       tc_fence_before();
       __syncwarp();

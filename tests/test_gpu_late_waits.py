@@ -44,6 +44,48 @@ def attention(kv_dt, H, W, Hk, gqa, nb, splits):
     return run
 
 
+def product(fp8, M, N, K, **kw):
+    """The result; whether the tile counters were left at zero."""
+
+    def run(qb):
+        from tests import util
+        from tests.test_gpu_kernels import T
+
+        r, dt = util.rng([91, M, N]), "e4m3" if fp8 else "bf16"
+        make = util.e4m3_randn if fp8 else util.bf16_randn
+        out = T(qb, np.full((M, N), MARK, np.uint16), "bf16")
+        gate = dict(gate=T(qb, util.bf16_randn(r, (1, N)), "bf16"), residual=T(qb, util.bf16_randn(r, (M, N)), "bf16"))
+        qb.qf.gemm(T(qb, make(r, (M, K)), dt), T(qb, make(r, (N, K), 0.05), dt), out=out, **gate, **kw)
+        ws = qb.functional._WS
+        return out.to_numpy(), ws is None or not ws.to_numpy()[: 64 << 10].any()
+
+    return run
+
+
+def projection(qb):
+    """The QKV projection with its epilogue, four K slices a tile (2 Q heads, 1 KV head, 128 tokens)."""
+    from tests import util
+    from tests.test_gpu_kernels import T
+
+    r, i32 = util.rng(92), lambda *v: T(qb, np.array(v, np.int32))
+    out = T(qb, np.full((128, 256), MARK, np.uint16), "bf16")
+    qb.qf.gemm_qkv_post(T(qb, util.bf16_randn(r, (128, 2048)), "bf16"), T(qb, util.bf16_randn(r, (256, 2048), 0.05), "bf16"), None, None, i32(3), i32(0),
+                        T(qb, np.zeros((64, 640), np.uint16), "bf16"), i32(0, 0, 0, 0, 0, 0), i32(0), T(qb, np.zeros((640, 64), np.uint16), "bf16"),
+                        n_q_heads=2, n_kv_heads=1, H_spatial=16, W_spatial=8, num_buckets=4, pinned_dilation=1, out=out)  # fmt: skip
+    return out.to_numpy(), True
+
+
+def grouped(qb):
+    from tests import util
+    from tests.test_gpu_kernels import T
+
+    r = util.rng(93)
+    out = T(qb, np.full((512, 64), MARK, np.uint16), "bf16")
+    qb.qf.gemm_grouped(T(qb, util.bf16_randn(r, (512, 512)), "bf16"), T(qb, util.bf16_randn(r, (128, 512), 0.05), "bf16"), T(qb, np.array([0, 0, 0, 1], np.int32)),
+                       n_experts=2, out=out)  # fmt: skip
+    return out.to_numpy(), True
+
+
 # name -> (call, which part of its result is late)
 LAST_QUERY_TILE, LAST_HEAD = np.s_[128:], np.s_[:, 47:]
 CASES = {
@@ -57,6 +99,20 @@ CASES = {
         ("helpers", 24, 64, 0, LAST_HEAD),  # 96 items, 52 helpers: the last takes the two query tiles of head 47
     ]
 }
+CASES.update({
+    f"gemm {'e4m3' if fp8 else 'bf16'} {name}": (product(fp8, M, N, K, **kw), late)
+    for fp8 in (False, True)
+    for name, M, N, K, kw, late in [
+        ("one slice", 200, 192, 512, dict(split_k=1, tile_n=64), np.s_[:, 128:]),
+        ("one slice, column remainder", 200, 200, 512, dict(split_k=1, tile_n=128), np.s_[:, 128:]),
+        ("cluster of 4 slices", 200, 192, 2048, dict(split_k=4, tile_n=64), np.s_[:, 128:]),
+        ("3 slices through the workspace", 200, 192, 2048, dict(split_k=3, tile_n=64, slice_mode=1), np.s_[:, 128:]),
+        ("pairs", 1700, 1800, 4096 if fp8 else 2048, dict(), np.s_[1536:, 1792:]),
+        ("pairs, 2 slices", 300, 2048, 8192, dict(split_k=2, tile_n=128), np.s_[256:, 1920:]),
+    ]
+})
+CASES["qkv projection, cluster of 4 slices"] = projection, np.s_[:, 192:]
+CASES["grouped"] = grouped, np.s_[:]
 
 
 def run_all(qb):
