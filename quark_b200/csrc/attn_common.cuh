@@ -115,7 +115,7 @@ struct KeyShares {
   }
 
   // The 128 threads of group 0, one row each: writes the rows of a whole item; otherwise leaves them in the workspace and, as the
-  // second of the item's two CTAs, sums both parts, the owner's first.
+  // second of the item's two CTAs, sums both parts (the same bits whichever CTA is the second).
   __device__ __forceinline__ void finish(const AttnArgs& a, const Piece& p, int r, bool good, float m, float l, float (&o)[64], int* exchange) const {
     int q0, qh, kvh;
     p.place(a, q0, qh, kvh);
@@ -150,8 +150,7 @@ struct KeyShares {
     for (int d = 0; d < 64; ++d) o1[d] = __ldcg(theirs + (2 + d) * 128);
     const float top = fmaxf(m, m1);
     const float wm = ex2_approx(m - top), wt = ex2_approx(m1 - top);
-    const float lm = l * wm, lt = l1 * wt;
-    l = helper ? lt + lm : lm + lt;
+    l = __fadd_rn(__fmul_rn(l, wm), __fmul_rn(l1, wt));  // (contracted, it would depend on whose product is rounded)
 #pragma unroll
     for (int d = 0; d < 64; ++d) o[d] = __fadd_rn(__fmul_rn(o[d], wm), __fmul_rn(o1[d], wt));
     if (row) write_row(a, t, qh, kvh, l, o);

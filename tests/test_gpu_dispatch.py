@@ -54,6 +54,38 @@ def test_attention_key_shares_by_size(qb, kv_dt, H, W, Hk, gqa, nb, ft):
         np.testing.assert_array_equal(got, qb.qf.owl_attn(*args, kv_splits=splits, **kw).to_numpy())
 
 
+@pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
+def test_attention_with_helpers_does_not_depend_on_who_comes_last(qb, kv_dt):
+    """The two parts of an item are summed by the CTA that finishes second.  A product on another stream keeps 100 SMs for about 100 us,
+    so that the helpers, the last CTAs of the grid, start late: the same bits as alone."""
+    import ctypes as C
+
+    lib, stream, r = qb._lib.load(), qb.runtime.stream, util.rng(95)
+    make = bf16_randn if kv_dt == "bf16" else e4m3_randn
+    segs, n = ops.compute_segments(500, 64, 256, 1)
+    args = (T(qb, bf16_randn(r, (256, 96 * 64)), "bf16"), T(qb, make(r, (24 * 65 * 256, 64)), kv_dt), T(qb, make(r, (24 * 64, 65 * 256)), kv_dt),
+            T(qb, np.array(segs, np.int32)), T(qb, np.array([n], np.int32)), 1, 24, 2, 16, 16, 64, 1)  # fmt: skip
+    kw = dict(compute_dtype=kv_dt, packed_qkv=True, frame_t=T(qb, np.array([500], np.int32)))
+    want = qb.qf.owl_attn(*args, **kw).to_numpy()
+    outs = [T(qb, np.zeros(want.shape, np.uint16), "bf16") for _ in range(10)]
+    a, c = qb.QuarkTensor.zeros(1280, 32768, dtype="bf16"), qb.QuarkTensor.zeros(1280, 1280, dtype="bf16")
+    p, first = C.c_void_p(), qb.runtime.active_stream()
+    qb._lib.check(lib.qb_stream_create(C.byref(p)))
+    try:
+        for out in outs:
+            qb._lib.check(lib.qb_device_sync())
+            stream.set_stream(int(p.value))
+            qb.qf.gemm(a, a, out=c, split_k=1, tile_n=128)
+            stream.set_stream(first)
+            qb.qf.owl_attn(*args, out=out, **kw)
+    finally:
+        stream.set_stream(first)
+        qb._lib.check(lib.qb_device_sync())
+    for out in outs:
+        np.testing.assert_array_equal(out.to_numpy(), want)
+    qb._lib.check(lib.qb_stream_destroy(p))
+
+
 @pytest.mark.parametrize("M,E,K", [(1, 8, 2), (1025, 8, 4), (2500, 32, 3), (4096, 24, 2)])
 def test_routing_by_size(qb, M, E, K):
     r = util.rng([82, M])
