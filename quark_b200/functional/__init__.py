@@ -11,6 +11,7 @@ CUDA graph after one eager run.
 from __future__ import annotations
 
 import ctypes as C
+from collections import OrderedDict
 
 import numpy as np
 
@@ -83,12 +84,41 @@ def _need(params, entry) -> int:
 # workspace (K-slice partials, tile counters, e4m3 copies of bf16 activations)
 # ---------------------------------------------------------------------------
 
+# Of the active stream: calls on one stream never overlap.  Other streams have theirs in _OF_STREAM, and a captured graph takes the
+# workspaces it was captured with along, so that it may be replayed on any stream.
 _WS: QuarkTensor | None = None
 _ATTN_WS: QuarkTensor | None = None
-# Workspaces that were replaced by larger ones.  A CUDA graph captured while a smaller workspace was current
-# (an Engine's frame graph, say) still holds that buffer's device address, so a superseded workspace is never
+_OF_STREAM: OrderedDict = OrderedDict()
+_STREAMS_KEPT = 16
+# Workspaces that were replaced by larger ones.  A CUDA graph that the caller captured on the stream by other means than
+# ``capture_graph`` still holds that buffer's device address, so a superseded workspace is never
 # freed: it stays referenced here for the life of the process (a few MB each, and growth is rare).
 _RETIRED_WS: list = []
+
+
+def _change_stream(old: int | None, new: int) -> None:
+    global _WS, _ATTN_WS
+    if old == new:
+        return
+    if _WS is not None or _ATTN_WS is not None:
+        _OF_STREAM[old] = (_WS, _ATTN_WS)
+    kept = _OF_STREAM.pop(new, None)
+    if kept is None and len(_OF_STREAM) >= _STREAMS_KEPT and not _stream.capturing():
+        # the workspaces of the stream that was left first serve the new one, once nothing uses them any more
+        _lib.check(_lib.load().qb_device_sync())
+        kept = _OF_STREAM.popitem(last=False)[1]
+    _WS, _ATTN_WS = kept or (None, None)
+
+
+def _hand_over(graph) -> None:
+    """The workspaces go with the graph; the stream gets new ones at once, since a capture that follows may not allocate."""
+    global _WS, _ATTN_WS
+    graph.scratch = (_WS, _ATTN_WS)
+    _WS, _ATTN_WS = (None if t is None else QuarkTensor.zeros(t.nbytes, dtype="e4m3") for t in graph.scratch)
+
+
+_stream.on_stream_change.append(_change_stream)
+_stream.on_captured.append(_hand_over)
 
 
 def _grow(current: QuarkTensor | None, nbytes: int) -> QuarkTensor:
@@ -98,7 +128,7 @@ def _grow(current: QuarkTensor | None, nbytes: int) -> QuarkTensor:
 
 
 def _workspace(nbytes: int) -> QuarkTensor | None:
-    """One zero-initialised scratch buffer shared by every GEMM call (calls on one stream never overlap).  The
+    """One zero-initialised scratch buffer shared by every GEMM call of the active stream.  The
     library keeps the tile counters in a fixed area at its start, whatever the shape, so calls of different
     shapes can share it."""
     global _WS
@@ -110,7 +140,7 @@ def _workspace(nbytes: int) -> QuarkTensor | None:
 
 
 def _attn_workspace(nbytes: int) -> QuarkTensor | None:
-    """The attention kernel's own zero-initialised scratch (tickets first; never shared with the GEMM's)."""
+    """The attention kernel's own zero-initialised scratch, also of the active stream (tickets first; never shared with the GEMM's)."""
     global _ATTN_WS
     if nbytes <= 0:
         return None

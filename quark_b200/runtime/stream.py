@@ -24,10 +24,22 @@ def active_stream() -> int:
     return _stream
 
 
+# Called as (old, new) when the active stream changes, and as (graph,) when a capture has ended: the scratch memory of
+# ``functional`` belongs to a stream, or to the graph that was captured with it.
+on_stream_change: list = []
+on_captured: list = []
+
+
 def set_stream(handle: int) -> None:
-    """Run on a caller-owned ``cudaStream_t`` instead (must not be the legacy default stream when graphs are captured)."""
+    """Run on a caller-owned ``cudaStream_t`` instead (must not be the legacy default stream when graphs are captured).
+
+    The choice is the process's, for all its threads.  Work on different streams may overlap, with these exceptions: a module's
+    output buffers are its own whatever the stream, and ``patchify``, ``unpatchify`` and attention that casts its caches have one
+    intermediate buffer per shape."""
     global _stream
-    _stream = int(handle)
+    old, _stream = _stream, int(handle)
+    for f in on_stream_change:
+        f(old, _stream)
 
 
 def synchronize() -> None:
@@ -100,6 +112,7 @@ class Graph:
 
     def __init__(self, handle: int):
         self.handle = handle
+        self.scratch = None  # memory that the kernels of the graph use besides their arguments
 
     def launch(self) -> None:
         _lib.check(_lib.load().qb_graph_launch(C.c_void_p(self.handle), C.c_void_p(active_stream())))
@@ -137,4 +150,6 @@ class capture_graph:
         if exc_type is None:
             _lib.check(rc)
             self.graph = Graph(int(p.value))
+            for f in on_captured:
+                f(self.graph)
         return False

@@ -86,6 +86,50 @@ def test_attention_with_helpers_does_not_depend_on_who_comes_last(qb, kv_dt):
     qb._lib.check(lib.qb_stream_destroy(p))
 
 
+def test_attention_with_helpers_on_two_streams_and_in_a_graph(qb):
+    """The helpers' partial results and tickets lie in a workspace: calls that overlap, eager on two streams and replayed from a graph,
+    each have one, and every result is that of a call alone."""
+    import ctypes as C
+
+    lib, stream, r = qb._lib.load(), qb.runtime.stream, util.rng(94)
+    H = W = 16
+    Hk, nb = 24, 64
+    calls = []
+    for i in range(3):
+        args = (T(qb, bf16_randn(r, (256, 96 * 64)), "bf16"), T(qb, e4m3_randn(r, (Hk * 65 * 256, 64)), "e4m3"), T(qb, e4m3_randn(r, (Hk * 64, 65 * 256)), "e4m3"),
+                T(qb, np.array(ops.compute_segments(500, nb, 256, 1)[0], np.int32)), T(qb, np.array([ops.compute_segments(500, nb, 256, 1)[1]], np.int32)))  # fmt: skip
+        out, ft = T(qb, np.zeros((256, 48 * 64), np.uint16), "bf16"), T(qb, np.array([500], np.int32))
+        calls.append((lambda a=args, o=out, f=ft: qb.qf.owl_attn(*a, 1, Hk, 2, H, W, nb, 1, compute_dtype="e4m3", packed_qkv=True, frame_t=f, out=o), out))
+    want = []
+    for call, out in calls:
+        call()
+        want.append(out.to_numpy())
+        out.zero_()
+    cap = qb.runtime.capture_graph()
+    with cap:
+        calls[2][0]()
+    qb.runtime.synchronize()
+    first, handles = qb.runtime.active_stream(), []
+    for _ in range(2):
+        p = C.c_void_p()
+        qb._lib.check(lib.qb_stream_create(C.byref(p)))
+        handles.append(int(p.value))
+    try:
+        for _ in range(20):  # in turn, so that the streams' queues run side by side
+            for handle, run in zip([first, *handles], (calls[0][0], calls[1][0], cap.graph.launch)):
+                stream.set_stream(handle)
+                run()
+    finally:
+        stream.set_stream(first)
+        qb._lib.check(lib.qb_device_sync())
+    for (_, out), w in zip(calls, want):
+        np.testing.assert_array_equal(out.to_numpy(), w)
+    assert len({id(t) for t in (qb.functional._ATTN_WS, cap.graph.scratch[1], qb.functional._OF_STREAM[handles[0]][1])}) == 3
+    for handle in handles:
+        qb.functional._OF_STREAM.pop(handle, None)
+        qb._lib.check(lib.qb_stream_destroy(C.c_void_p(handle)))
+
+
 @pytest.mark.parametrize("M,E,K", [(1, 8, 2), (1025, 8, 4), (2500, 32, 3), (4096, 24, 2)])
 def test_routing_by_size(qb, M, E, K):
     r = util.rng([82, M])

@@ -39,6 +39,41 @@ def test_a_workspace_that_grows_is_retired_not_freed(monkeypatch):
     assert a2 is not a1 and any(t is a1 for t in qfm._RETIRED_WS) and qfm._attn_workspace(0) is None
 
 
+def test_streams_and_graphs_have_workspaces_of_their_own(monkeypatch):
+    """Tickets and partial results lie in the workspace, so calls that may overlap must not share one: calls on two streams, and a
+    captured graph and anything else."""
+    from quark_b200 import functional as qfm
+    from quark_b200.runtime import stream
+
+    monkeypatch.setattr(qfm, "QuarkTensor", _FakeTensor)
+    for name, value in (("_WS", None), ("_ATTN_WS", None), ("_RETIRED_WS", []), ("_OF_STREAM", type(qfm._OF_STREAM)())):
+        monkeypatch.setattr(qfm, name, value)
+    monkeypatch.setattr(stream, "_stream", 1)
+    both = lambda: (qfm._workspace(4096), qfm._attn_workspace(4096))  # noqa: E731
+    first = both()
+    stream.set_stream(2)
+    second = both()
+    assert not {t.data_ptr() for t in first} & {t.data_ptr() for t in second}
+    stream.set_stream(1)
+    assert both() == first
+    stream.set_stream(1)
+    assert both() == first and list(qfm._OF_STREAM) == [2]
+
+    graph = stream.Graph(0)
+    for f in stream.on_captured:
+        f(graph)
+    assert graph.scratch == first and not set(both()) & set(first)  # allocated already: the next capture may not
+
+    # bounded: the workspaces of the stream that was left first are taken over once the device is idle
+    synced = []
+    monkeypatch.setattr(qfm._lib, "load", lambda: type("Lib", (), {"qb_device_sync": staticmethod(lambda: synced.append(1) or 0)}))
+    seen = {both()[0]}
+    for s in range(10, 60):
+        stream.set_stream(s)
+        seen.add(both()[0])
+    assert synced and len(seen) <= qfm._STREAMS_KEPT + 2 and len(qfm._OF_STREAM) <= qfm._STREAMS_KEPT
+
+
 def test_counter_and_ticket_areas_do_not_depend_on_the_shape():
     """Calls of different shapes share one workspace, so the area that must stay zero between calls (tile
     counters of the GEMM, tickets of the attention key splits) has to end at the same offset for all of them."""
