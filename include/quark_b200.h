@@ -268,7 +268,7 @@ typedef struct {
   int32_t packed_qkv;    /* 1: qkv is the packed projection, out is [tpf, Hq * 64]; 0: qkv is Q alone, head-major
                           * [Hq * tpf, 64], and so is out (src/quark/kernels/owl_attn/reference.py:62-69, :106-110) */
   int32_t quilt_factor;  /* the caches keep H*W / quilt_factor tokens per frame (1: all): capacity = (nb + 1) * that */
-  int32_t kv_splits;     /* 0 = choose; > 1 splits the keys over CTAs (needs workspace) */
+  int32_t kv_splits;     /* 0 = choose; > 1 splits the keys over CTAs (needs a workspace) */
   const float* k_scale;
   const float* v_scale;
 } qb_attn_params;
@@ -281,15 +281,18 @@ typedef struct {
  * bf16 attention always uses ex2.approx. */
 int32_t qb_set_attn_exact_exp(int32_t on);
 
-/* Bytes of workspace qb_owl_attn needs for `p`: 0 unless the keys of one (query tile, head) are shared by
- * several CTAs, which is chosen when query tiles x heads would leave most SMs idle (360p; a tensor-parallel
- * rank with few heads) or forced with kv_splits.  The workspace starts with one ticket per (query tile,
- * head) in a fixed 16 KiB area (so calls of different geometries may share a workspace), which must be zero
- * before the first use (the kernel leaves it zero), followed by the CTAs' partial results; it must not be the workspace of qb_gemm.  Shares are summed in a fixed order. */
+/* Workspace of qb_owl_attn.  It starts with one ticket per (query tile, head) in a fixed 16 KiB area (so calls of different
+ * geometries may share a workspace), which must be zero before the first use (the kernel leaves it zero), followed by the CTAs'
+ * partial results; it must not be the workspace of qb_gemm, nor that of a call that may overlap.  Partial results are summed in a
+ * fixed order.
+ *
+ * The keys of one (query tile, head) are shared by several CTAs when query tiles x heads would leave most SMs idle (360p; a
+ * tensor-parallel rank with few heads) or when kv_splits forces it.  qb_owl_attn_workspace_bytes: what sharing through the workspace
+ * takes, which a forced number cannot do without; the kernel's own choice (kv_splits = 0) is a thread-block cluster, which needs none. */
 size_t qb_owl_attn_workspace_bytes(const qb_attn_params* p);
-/* Bytes of workspace with which qb_owl_attn can use every SM for `p` (not less than the above, which it cannot do without): where
- * the (query tile, head) items leave SMs idle and the history is long, CTAs on those SMs take a part of the items' keys and the partial
- * results meet in the workspace (tickets as above). */
+/* Bytes of workspace that a call can make use of: those above for a forced number; with kv_splits = 0, where the (query tile, head)
+ * items leave SMs idle and the history is long, those through which CTAs on the idle SMs take a part of the items' keys (a call
+ * without them has one CTA per item); otherwise 0. */
 size_t qb_owl_attn_scratch_bytes(const qb_attn_params* p);
 int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void* Vt_cache, const int32_t* segments,
                     const int32_t* n_segments, const int32_t* frame_t, void* out, void* out_q, const float* rope_xy,

@@ -1081,8 +1081,12 @@ static size_t attn_ticket_bytes(const qb_attn_params* p) {
   return need > (16u << 10) ? need : (16u << 10);
 }
 
+static bool attn_sizes_ok(const qb_attn_params* p) {
+  return p != nullptr && p->H_spatial > 0 && p->W_spatial > 0 && p->n_kv_heads > 0 && p->gqa_ratio > 0 && p->num_buckets > 0;
+}
+
 extern "C" size_t qb_owl_attn_workspace_bytes(const qb_attn_params* p) {
-  if (p == nullptr || p->H_spatial <= 0 || p->W_spatial <= 0 || p->n_kv_heads <= 0 || p->gqa_ratio <= 0 || p->num_buckets <= 0) return 0;
+  if (!attn_sizes_ok(p)) return 0;
   const int n = attn_key_splits(p);
   if (n <= 1) return 0;
   const int tpf = p->H_spatial * p->W_spatial;
@@ -1091,9 +1095,9 @@ extern "C" size_t qb_owl_attn_workspace_bytes(const qb_attn_params* p) {
 }
 
 extern "C" size_t qb_owl_attn_scratch_bytes(const qb_attn_params* p) {
-  const size_t need = qb_owl_attn_workspace_bytes(p);
-  if (p == nullptr || p->H_spatial <= 0 || p->W_spatial <= 0 || p->n_kv_heads <= 0 || p->gqa_ratio <= 0 || p->num_buckets <= 0) return 0;
-  if (!attn_helped(p, attn_key_splits(p))) return need;
+  if (!attn_sizes_ok(p)) return 0;
+  if (p->kv_splits > 0) return qb_owl_attn_workspace_bytes(p);  // splits of the kernel's own choice are clusters: no workspace
+  if (!attn_helped(p, attn_key_splits(p))) return 0;
   return attn_ticket_bytes(p) + static_cast<size_t>(2 * num_sms()) * kPartial * sizeof(float);
 }
 
@@ -1147,7 +1151,7 @@ extern "C" int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void*
 
   QB_REQUIRE(p->kv_splits >= 0 && p->kv_splits <= 16, QB_ERR_INVALID_ARG, "owl_attn: kv_splits %d", p->kv_splits);
   const int splits = attn_key_splits(p);
-  if (splits > 1) {
+  if (splits > 1 && p->kv_splits > 0) {
     const size_t need = qb_owl_attn_workspace_bytes(p);
     QB_REQUIRE(workspace != nullptr && workspace_bytes >= need, QB_ERR_WORKSPACE, "owl_attn: %d key splits need a workspace of %zu bytes, %zu given",
                splits, need, workspace_bytes);

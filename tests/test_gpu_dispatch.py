@@ -55,6 +55,26 @@ def test_attention_key_shares_by_size(qb, kv_dt, H, W, Hk, gqa, nb, ft):
 
 
 @pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
+@pytest.mark.parametrize("Hk,nb", [(1, 16), (24, 64)])  # key splits in clusters, one CTA per item (helpers want a workspace)
+def test_attention_call_without_a_workspace(qb, kv_dt, Hk, nb):
+    import ctypes as C
+
+    lib, r = qb._lib.load(), util.rng([96, Hk])
+    segs, n = ops.compute_segments(500, nb, 256, 1)
+    make = bf16_randn if kv_dt == "bf16" else e4m3_randn
+    qkv, K, V = T(qb, bf16_randn(r, (256, Hk * 4 * 64)), "bf16"), T(qb, make(r, (Hk * (nb + 1) * 256, 64)), kv_dt), T(qb, make(r, (Hk * 64, (nb + 1) * 256)), kv_dt)
+    seg, nseg, ft = T(qb, np.array(segs, np.int32)), T(qb, np.array([n], np.int32)), T(qb, np.array([500], np.int32))
+    want = qb.qf.owl_attn(qkv, K, V, seg, nseg, 1, Hk, 2, 16, 16, nb, 1, compute_dtype=kv_dt, packed_qkv=True, frame_t=ft, kv_splits=0 if Hk == 1 else 1).to_numpy()
+    out = T(qb, np.zeros(want.shape, np.uint16), "bf16")
+    dt = qb._lib.DTYPE_CODE[kv_dt]
+    p = qb._lib.AttnParams(n_kv_heads=Hk, gqa_ratio=2, H_spatial=16, W_spatial=16, num_buckets=nb, pinned_dilation=1, kv_dtype=dt, compute_dtype=dt, max_segments=3,
+                           packed_qkv=1, quilt_factor=1)  # fmt: skip
+    qb._lib.check(lib.qb_owl_attn(qkv.data_ptr(), K.data_ptr(), V.data_ptr(), seg.data_ptr(), nseg.data_ptr(), ft.data_ptr(), out.data_ptr(), None,
+                                  qb.qf.rope_table(16, 16).data_ptr(), C.byref(p), None, 0, qb.runtime.active_stream()))  # fmt: skip
+    np.testing.assert_array_equal(out.to_numpy(), want)
+
+
+@pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
 def test_attention_with_helpers_does_not_depend_on_who_comes_last(qb, kv_dt):
     """The two parts of an item are summed by the CTA that finishes second.  A product on another stream keeps 100 SMs for about 100 us,
     so that the helpers, the last CTAs of the grid, start late: the same bits as alone."""

@@ -91,3 +91,20 @@ def test_counter_and_ticket_areas_do_not_depend_on_the_shape():
     assert gemm_ws(128, 256, 512, 1, a_dtype=0) == counters + 128 * 512  # the e4m3 copy of a bf16 A follows the counters
     assert gemm_ws(512, 4096, 768, 3) == counters + 3 * 512 * 4096 * 4  # 256 tiles
     assert gemm_ws(1024, 4096, 768, 3) == counters + 3 * 1024 * 4096 * 4  # 512 tiles: same counter area
+
+
+def test_attention_asks_only_for_scratch_that_it_uses():
+    """Key splits of the kernel's own choice meet inside a cluster: no workspace.  Forced splits and the helpers of a long history use one."""
+    from quark_b200 import _lib
+
+    lib = _lib.load()
+
+    def scratch(H, W, Hk, nb=16, splits=0):
+        p = _lib.AttnParams(n_kv_heads=Hk, gqa_ratio=2, H_spatial=H, W_spatial=W, num_buckets=nb, pinned_dilation=1, kv_dtype=1, compute_dtype=1,
+                            max_segments=3, packed_qkv=1, quilt_factor=1, kv_splits=splits)  # fmt: skip
+        return int(lib.qb_owl_attn_scratch_bytes(C.byref(p)))
+
+    per = 66 * 128 * 4
+    assert scratch(16, 8, 16) == scratch(32, 16, 2) == scratch(32, 16, 16) == 0
+    assert scratch(16, 8, 16, splits=4) == 16384 + 32 * 4 * per
+    assert scratch(32, 16, 16, nb=128) == 16384 + 2 * 148 * per
