@@ -466,57 +466,54 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+typedef CUresult (*ReplaceAddressFn)(CUtensorMap*, void*);
 
-static EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
+static void* driver_entry(const char* name) {
+  void* p = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  return cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? p : nullptr;
 }
 
 // Tensor map of a contiguous row-major tensor [rows, cols] of 1- or 2-byte elements with a box of
 // [box_rows, box_cols] elements; box_cols * elem_bytes must equal the swizzle span (64 or 128).
 // Out-of-range parts of a box are filled with zeros.
 //
-// A map depends on its arguments alone, so each thread keeps the last few it made: a program calls with the same tensors again
-// and again, and the driver's encoder takes longer than the rest of a small call's host side.
+// The driver's encoder takes longer than the rest of a small call's host side, so each thread keeps the maps of the last geometries
+// and puts a call's own address into a copy: the layers of a model have a dozen geometries among hundreds of tensors.
 int32_t make_tmap_2d_sw(CUtensorMap* tm, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint32_t box_rows,
                         uint32_t box_cols, int swizzle_bytes) {
   struct Made {
     CUtensorMap map;
-    const void* base;  // NULL: empty
-    uint64_t rows, cols;
+    uint64_t rows, cols;  // 0: empty
     uint32_t box_rows, box_cols;
     int elem_bytes, swizzle_bytes;
   };
-  constexpr int kMade = 16;
+  constexpr int kMade = 64;
   static thread_local Made made[kMade];
-  const uint64_t h = (reinterpret_cast<uintptr_t>(base) >> 8) * 0x9E3779B97F4A7C15ull + box_rows;
-  Made& m = made[(h ^ (h >> 32)) % kMade];
-  if (m.base == base && base != nullptr && m.rows == rows && m.cols == cols && m.box_rows == box_rows && m.box_cols == box_cols && m.elem_bytes == elem_bytes &&
-      m.swizzle_bytes == swizzle_bytes) {
-    *tm = m.map;
-    return QB_OK;
-  }
-  EncodeTiledFn enc = encode_tiled_fn();
-  QB_REQUIRE(enc != nullptr, QB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  static const auto encode = reinterpret_cast<EncodeTiledFn>(driver_entry("cuTensorMapEncodeTiled"));
+  static const auto replace = reinterpret_cast<ReplaceAddressFn>(driver_entry("cuTensorMapReplaceAddress"));
+  QB_REQUIRE(encode != nullptr && replace != nullptr, QB_ERR_CUDA, "the driver has no tensor maps");
+  QB_REQUIRE(base != nullptr && aligned16(base), QB_ERR_ALIGN, "tensor map: address not 16-byte aligned");
   QB_REQUIRE((cols * elem_bytes) % 16 == 0, QB_ERR_ALIGN, "tensor map: row pitch of %llu bytes is not a multiple of 16",
              static_cast<unsigned long long>(cols * elem_bytes));
+  const uint64_t h = ((rows * 31 + cols) * 31 + box_rows) * 0x9E3779B97F4A7C15ull;
+  Made& m = made[(h >> 32) % kMade];
+  if (m.rows == rows && m.cols == cols && m.box_rows == box_rows && m.box_cols == box_cols && m.elem_bytes == elem_bytes && m.swizzle_bytes == swizzle_bytes) {
+    *tm = m.map;
+    const CUresult r = replace(tm, const_cast<void*>(base));
+    QB_REQUIRE(r == CUDA_SUCCESS, QB_ERR_CUDA, "cuTensorMapReplaceAddress failed with CUresult %d", static_cast<int>(r));
+    return QB_OK;
+  }
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {cols * elem_bytes};
   const cuuint32_t box[2] = {box_cols, box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUtensorMapDataType dt = elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
   const CUtensorMapSwizzle sw = swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
-  CUresult r = enc(tm, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = encode(tm, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   QB_REQUIRE(r == CUDA_SUCCESS, QB_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", static_cast<int>(r));
-  m = Made{*tm, base, rows, cols, box_rows, box_cols, elem_bytes, swizzle_bytes};
+  m = Made{*tm, rows, cols, box_rows, box_cols, elem_bytes, swizzle_bytes};
   return QB_OK;
 }
 

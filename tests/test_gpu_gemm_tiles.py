@@ -40,3 +40,19 @@ def test_gemm_tile_forms(qb, M, N, K, fp8, kw):
     _check_gemm(got, want, f"gemm {M}x{N}x{K} fp8={fp8} {kw}", fp8)
     again, _ = _gemm_case(qb, M, N, K, fp8=fp8, seed=M, **kw)
     np.testing.assert_array_equal(got.to_numpy(), again.to_numpy())
+
+
+def test_tensor_maps_of_many_geometries_and_addresses(qb):
+    """The maps kept are those of geometries: more of them than are kept, each with tensors at two addresses in turn."""
+    from oracle import ops
+    from tests import util
+    from tests.test_gpu_kernels import T
+
+    r = util.rng(97)
+    shapes = [(8 * i, 64 + 16 * (i % 7)) for i in range(1, 81)]
+    pairs = [[(util.bf16_randn(r, (5, K)), util.bf16_randn(r, (N, K))) for _ in range(2)] for N, K in shapes]
+    dev = [[(T(qb, a, "bf16"), T(qb, b, "bf16")) for a, b in two] for two in pairs]
+    for which in (0, 1, 0):
+        for two, d in zip(pairs, dev):
+            got = qb.qf.gemm(*d[which], out_dtype="f32", split_k=1)
+            _check_gemm(got, ops.gemm(*two[which], return_f32=True), f"{two[which][1].shape} {which}", False)
