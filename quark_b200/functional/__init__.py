@@ -57,12 +57,17 @@ def _name(dtype) -> str | None:
 
 
 # The parameter structs of calls already made, by their field values: filling one through ctypes takes longer than the rest of a
-# call.  Bounded; a struct is never written after it is made, so calls from several threads may share it.
+# call.  Bounded; a struct is never written after it is made, so calls from several threads may share it.  Only plain integers are
+# looked up (2.0 is equal to 2, but no size), and no struct that holds addresses is kept.
 _PARAMS: dict = {}
 
 
 def _params(cls, *values):
-    """``(struct, byref(struct), [])``; the list is for what a caller derives from the struct alone (a workspace size)."""
+    """``(struct, byref(struct), [])``; the last two fields are addresses, and the list is for what a caller derives from the struct
+    alone (a workspace size)."""
+    if values[-1] is not None or values[-2] is not None or {*map(type, values[:-2])} != {int}:
+        p = cls(*values)
+        return p, C.byref(p), []
     key = (cls, values)
     got = _PARAMS.get(key)
     if got is None:

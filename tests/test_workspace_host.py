@@ -2,6 +2,8 @@
 
 import ctypes as C
 
+import pytest
+
 
 class _FakeTensor:
     _next = 0x1000
@@ -108,3 +110,20 @@ def test_attention_asks_only_for_scratch_that_it_uses():
     assert scratch(16, 8, 16) == scratch(32, 16, 2) == scratch(32, 16, 16) == 0
     assert scratch(16, 8, 16, splits=4) == 16384 + 32 * 4 * per
     assert scratch(32, 16, 16, nb=128) == 16384 + 2 * 148 * per
+
+
+def test_parameter_structs_kept_do_not_loosen_a_check(monkeypatch):
+    """A struct is found again by its plain integers alone: a float that equals one of them is refused as it is without the lookup, and
+    a struct with addresses in it is not kept."""
+    from quark_b200 import _lib
+    from quark_b200 import functional as qfm
+
+    monkeypatch.setattr(qfm, "_PARAMS", {})
+    sizes = (4, 2, 8, 8, 16, 1, 1, 3, 1, 1, 0)
+    kept = qfm._params(_lib.KvParams, *sizes, None, None)
+    assert qfm._params(_lib.KvParams, *sizes, None, None) is kept and len(qfm._PARAMS) == 1
+    with pytest.raises(TypeError):
+        qfm._params(_lib.KvParams, 4, 2.0, *sizes[2:], None, None)
+    assert qfm._params(_lib.KvParams, *sizes, 4096, None)[0].k_scale == 4096
+    assert qfm._params(_lib.KvParams, True, *sizes[1:], None, None)[0].n_q_heads == 1
+    assert len(qfm._PARAMS) == 1
