@@ -184,7 +184,8 @@ class MoE(Module):
     padded to whole 128-row tiles), the tokens are gathered into slot order, the two expert projections are grouped
     GEMMs over ``M * top_k`` (+ padding) rows, and a reduction gathers each token's ``top_k`` partial rows.
     ``schedule="dense"`` keeps the earlier form (every expert over every token, routing weights zero outside a token's
-    top k: E / top_k times the flops, no data-dependent tables).  The capacity-bounded ``"balanced"`` and
+    top k: E / top_k times the flops, no data-dependent tables; the same bits as long as its products take one K slice, else another
+    order of the f32 sums).  The capacity-bounded ``"balanced"`` and
     ``"shared_experts"`` routings are rejected, as upstream's own ``forward`` does (``src/quark/nn/moe.py:340-347``)."""
 
     def __init__(self, M: int, d_model: int, d_intermediate: int, n_experts: int, top_k: int, *, routing: str = "correct", out_dtype: str = "bf16",
@@ -237,10 +238,11 @@ class MoE(Module):
         h = _cached(self, "h", (M, H), "bf16")
         partials = _cached(self, "partials", (E * M, D), "f32")
         for e in range(E):
-            # one K slice, as the grouped GEMMs have: both schedules give the same bits
-            qf.gemm(xq, self.expert_in.data.rows(e * H, (e + 1) * H), compute_dtype=cd, activation="silu", out=h, split_k=1, b_constant=True)
+            # K slices as the sizes ask for (the grouped GEMMs have one): with one slice 128 tokens of 8 experts, 2048 x 4096, took 180
+            # instead of 137 us in bf16 and 146 instead of 128 in e4m3
+            qf.gemm(xq, self.expert_in.data.rows(e * H, (e + 1) * H), compute_dtype=cd, activation="silu", out=h, b_constant=True)
             qf.gemm(h, self.expert_out.data.rows(e * D, (e + 1) * D), out_dtype="f32", compute_dtype=cd, out=partials.rows(e * M, (e + 1) * M),
-                    split_k=1, b_constant=True)  # fmt: skip
+                    b_constant=True)  # fmt: skip
         return qf.moe_combine(partials, weights, out=_cached(self, "out", (M, D), "bf16"))
 
 

@@ -175,6 +175,31 @@ def test_gather_narrows_as_quantize_does(qb, D):
     assert not out[90:].any()
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+def test_dense_experts_take_the_k_slices_of_their_products(qb, fp8):
+    """The dense schedule is one product after the other as ``qf.gemm`` plans them (a few slices each at this size)."""
+    from quark_b200 import nn as qnn
+
+    r, qf = util.rng([98, fp8]), qb.qf
+    M, D, H, E = 128, 1024, 2048, 8
+    layer = {s: qnn.MoE(M, D, H, E, 2, schedule=s) for s in ("dense", "sorted")}
+    weights = [T(qb, bf16_randn(r, shape, std), "bf16") for shape, std in (((E, D), 0.2), ((E * H, D), 0.05), ((E * D, H), 0.05))]
+    for m in layer.values():
+        m.router.weight.data, m.expert_in.data, m.expert_out.data = weights
+        m.prepare(fp8=fp8)
+    x = T(qb, bf16_randn(r, (M, D)), "bf16")
+    dense, w_in, w_out = layer["dense"], layer["dense"].expert_in.data, layer["dense"].expert_out.data
+    got = dense(x).to_numpy()
+    partials = T(qb, np.zeros((E * M, D), np.float32))
+    for e in range(E):
+        h = qf.gemm(qf.quantize_e4m3(x) if fp8 else x, w_in.rows(e * H, (e + 1) * H), activation="silu")
+        qf.gemm(h, w_out.rows(e * D, (e + 1) * D), out_dtype="f32", out=partials.rows(e * M, (e + 1) * M))
+    np.testing.assert_array_equal(qf.moe_combine(partials, qf.moe_route(dense.router(x), top_k=2)).to_numpy(), got)
+    # the sorted schedule's sums are in another order; a hidden value on the edge of two codes may take the other
+    g, s = f32(got, "bf16"), f32(layer["sorted"](x).to_numpy(), "bf16")
+    assert np.linalg.norm(g - s) <= (2e-2 if fp8 else 6e-3) * np.linalg.norm(g)
+
+
 @pytest.mark.parametrize("runs,N,K", [
     ([1, 0, 0], 64, 64),  # one tile of one expert
     ([3, 1, 2], 328, 192),  # odd numbers of tiles, columns that end inside a tile
