@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import warnings
 from pathlib import Path
 
 QB_BF16, QB_E4M3, QB_F32, QB_S32 = 0, 1, 2, 3
@@ -200,7 +201,7 @@ FASTCALL = ("qb_gemm", "qb_gemm_workspace_bytes", "qb_ada_rmsnorm", "qb_rmsnorm"
 
 
 class _NoFastcall:
-    """Stands in where the extension was not built (it needs the interpreter's headers): takes no call."""
+    """Stands in where the extension was not built for this interpreter (it needs its headers): takes no call."""
 
     def __getattr__(self, name):
         return lambda *args: None
@@ -218,6 +219,9 @@ def fastcall():
 def _bind_fastcall(lib) -> None:
     from .runtime.tensor import QuarkTensor
 
+    if isinstance(fastcall(), _NoFastcall):
+        warnings.warn("quark_b200._fastcall was not built for this interpreter (csrc/build.sh needs Python.h): every small call costs "
+                      "some microseconds more", RuntimeWarning, stacklevel=3)  # fmt: skip
     fastcall().bind(QuarkTensor, {name: C.cast(getattr(lib, name), C.c_void_p).value for name in FASTCALL})
 
 

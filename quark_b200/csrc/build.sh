@@ -24,9 +24,12 @@ $NVCC -shared -o "$OUT" "$OBJ"/{runtime,gemm,gemm_pair,gemm_grouped,attn,attn4,k
 # The C side of the smallest calls (a CPython extension); without the interpreter's headers they stay in Python.
 PYTHON="${PYTHON:-python3}"
 PYINC="$($PYTHON -c 'import sysconfig; print(sysconfig.get_paths()["include"])')"
+# (named for the interpreter it was built for: another one does not import it)
+EXT="$HERE/../_fastcall$($PYTHON -c 'import sysconfig; print(sysconfig.get_config_var("EXT_SUFFIX"))')"
+rm -f "$EXT" "$HERE/../_fastcall.so"
 if [ -f "$PYINC/Python.h" ]; then
-  ${CC:-gcc} -O2 -Wall -std=gnu11 -fPIC -shared -I"$PYINC" "$HERE/fastcall.c" -o "$HERE/../_fastcall.so"
+  ${CC:-gcc} -O2 -Wall -std=gnu11 -fPIC -shared -I"$PYINC" "$HERE/fastcall.c" -o "$EXT"
 else
-  echo "no Python.h under $PYINC: _fastcall.so not built"
+  echo "no Python.h under $PYINC: the C side of small calls is not built"
 fi
 echo "built $OUT"

@@ -39,6 +39,24 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
         _lib.load()
 
 
+def test_extension_is_named_for_its_interpreter_and_missed_aloud(monkeypatch):
+    """Another interpreter in the same tree must not import an extension that knows this one's object layout, and small calls that
+    stay in Python say so."""
+    import sys
+    import sysconfig
+
+    import quark_b200
+    from quark_b200 import _lib
+
+    lib = _lib.load()
+    assert _lib.fastcall().__file__.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+    assert not (ROOT / "quark_b200" / "_fastcall.so").exists()
+    monkeypatch.delattr(quark_b200, "_fastcall")
+    monkeypatch.setitem(sys.modules, "quark_b200._fastcall", None)
+    with pytest.warns(RuntimeWarning, match="_fastcall"):
+        _lib._bind_fastcall(lib)
+
+
 def test_argument_validation_needs_no_gpu():
     """Entry points reject bad arguments on the host, before touching the device."""
     import ctypes as C
