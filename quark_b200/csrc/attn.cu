@@ -934,7 +934,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
 }  // namespace qb
 
 namespace qb {
-int32_t launch_attn4(const void* K_cache, const void* Vt_cache, const AttnArgs& a, int n_kv_heads, bool fp8, cudaStream_t st);
+int32_t launch_attn4(const void* K_cache, const void* Vt_cache, const AttnArgs& a, int n_kv_heads, cudaStream_t st);
 // bf16 calls with one (query tile, head) per CTA go to the three-group kernel of attn4.cu; QB_ATTN4=0 in the environment
 // when the library is loaded keeps the two-group kernel of this file for everything (e4m3 and key splits always use it).
 // e4m3 probabilities: 0 = every second exponential on the FMA pipe (ex2_lin_from_biased), 1 = all on the special-function unit
@@ -1166,9 +1166,8 @@ extern "C" int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void*
     a.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + attn_ticket_bytes(p));
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // bf16, one CTA per (query tile, head): the three-group kernel of attn4.cu (60.0 against 70.3 us at 720p).  In the
-  // e4m3 path it is the slower one (57.7 against 52.2 us): its per-chunk fixed work outweighs the extra warps.
-  if (splits == 1 && !fp8 && attn4_enabled()) return launch_attn4(K_cache, Vt_cache, a, p->n_kv_heads, fp8, st);
+  // bf16, one CTA per (query tile, head): the three-group kernel of attn4.cu (60.0 against 70.3 us at 720p)
+  if (splits == 1 && !fp8 && attn4_enabled()) return launch_attn4(K_cache, Vt_cache, a, p->n_kv_heads, st);
   const bool forced = p->kv_splits > 0;
   if (!fp8) return launch_attn<false, false>(tmK, tmV, a, Hq, splits, forced, helped, st);
   return g_attn_exact_exp ? launch_attn<true, false>(tmK, tmV, a, Hq, splits, forced, helped, st) : launch_attn<true, true>(tmK, tmV, a, Hq, splits, forced, helped, st);

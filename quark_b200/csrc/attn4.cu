@@ -8,13 +8,13 @@
 // TMEM: per group one S chunk (64 columns) and the output accumulator O (80 columns: 64 outputs and, from the rows of
 // ones under every V^T chunk, the row sum of exactly the rounded P that is multiplied with V).
 // As in attn.cu: P = 2^(score - m) with m the maximum the row was last rescaled to (O is rescaled only when a chunk's
-// maximum exceeds m by more than kSlack), e4m3 P scaled by 2^5, two P buffers per group, every wait
+// maximum exceeds m by more than kSlack), two P buffers per group, every wait
 // bounded, a malformed segment table reported and treated as empty.  The three partial results are merged at the end.
 //
-// Measured on B200 at 720p (512 queries x 32 heads x 8320 keys, us per launch; attn.cu in brackets): bf16 60.0 (70.3),
-// e4m3 57.7 (52.2).  The extra warp per scheduler pays in the bf16 path, where attn.cu has one P tile per group and three
-// stages; in the e4m3 path the fixed work per chunk (barrier waits, TMEM loads, maxima: the same per 64 keys as attn.cu
-// spends per 128) outweighs it, so e4m3 calls stay with attn.cu.  A variant with four groups (16 softmax warps, 96
+// Measured on B200 at 720p (512 queries x 32 heads x 8320 keys, us per launch; attn.cu in brackets): bf16 60.0 (70.3).
+// The extra warp per scheduler pays in bf16, where attn.cu has one P tile per group.  An e4m3 form was slower than attn.cu
+// (57.7 against 52.2 us) and is gone: there the fixed work per chunk (barrier waits, TMEM loads, maxima: the same per 64 keys
+// as attn.cu spends per 128) outweighs it.  A variant with four groups (16 softmax warps, 96
 // registers per thread, row sums kept by the threads because four S chunks and four 80-column accumulators exceed the
 // 512 TMEM columns) was slower still: 60.7 us e4m3, with 3 % of its instructions spill traffic and 8.9 instructions per
 // exponential against 5.4 in attn.cu.  All three kernels issue about one instruction every second cycle per scheduler:
@@ -36,21 +36,19 @@ constexpr int kA4CtrlRegs = 40;
 constexpr int kA4SoftmaxRegs = 152;
 static_assert(128 * kA4CtrlRegs + 384 * kA4SoftmaxRegs <= kA4Threads * kA4LaunchRegs, "register budget of the CTA");
 
-template <bool kFp8>
 struct A4Smem {
-  static constexpr int kEs = kFp8 ? 1 : 2;
   // A group's MMA warp issues S one of its chunks (three chunks overall) ahead of the PV that frees a stage, after the
   // PV of its previous chunk in program order: chunk u + 3 may need the stage of chunk u - 3 at the earliest.
   static constexpr int kStages = 6;
-  static constexpr int kRowBytes = 64 * kEs;                 // one row of a K-major tile: 64 | 128 bytes
-  static constexpr int kQBytes = 128 * kRowBytes;            // 8 KB | 16 KB
-  static constexpr int kKBytes = kA4Chunk * kRowBytes;       // 4 KB | 8 KB: K chunk
-  static constexpr int kVBytes = kA4VRows * kRowBytes;       // 5 KB | 10 KB: V^T chunk and the rows of ones
-  static constexpr int kPBytes = 128 * kRowBytes;            // 8 KB | 16 KB
+  static constexpr int kRowBytes = 64 * 2;                   // one row of a K-major tile
+  static constexpr int kQBytes = 128 * kRowBytes;            // 16 KB
+  static constexpr int kKBytes = kA4Chunk * kRowBytes;       // 8 KB: K chunk
+  static constexpr int kVBytes = kA4VRows * kRowBytes;       // 10 KB: V^T chunk and the rows of ones
+  static constexpr int kPBytes = 128 * kRowBytes;            // 16 KB
   // Two P buffers per group: with one, P(i) waited for PV(i - 1), i.e. for the MMA warp to wake up and the tensor core to finish,
   // in every chunk (bf16, 720p: 67.5 -> 60.0 us; 128 buckets 466 -> 428 us).
   static constexpr int kPBufs = 2;
-  static constexpr int kStageBytes = kKBytes + kVBytes;      // 9 KB | 18 KB (a multiple of the swizzle atom: 512 | 1024)
+  static constexpr int kStageBytes = kKBytes + kVBytes;      // 18 KB (a multiple of the swizzle atom)
   static constexpr int kQOff = 0;
   static constexpr int kPOff = kQOff + kQBytes;
   static constexpr int kStageOff = kPOff + kA4Groups * kPBufs * kPBytes;
@@ -58,7 +56,7 @@ struct A4Smem {
   static constexpr int kTotal = kBarOff + 1024 + 1024;
   static constexpr int kMergeBytes = (kA4Groups - 1) * 66 * 128 * 4;  // groups 1, 2 hand (m, l, 64 outputs) per row to group 0
   static_assert(kBarOff - kPOff >= kMergeBytes, "merge buffer aliases the P and stage areas");
-  static_assert(kStageBytes % (kFp8 ? 512 : 1024) == 0, "stages keep the swizzle alignment");
+  static_assert(kStageBytes % 1024 == 0, "stages keep the swizzle alignment");
 };
 
 // j-th valid 64-key chunk of the segment table: first cache row and number of valid keys.
@@ -78,19 +76,13 @@ __device__ __forceinline__ void locate_chunk(const int (&seg)[6], int j, int& ro
   }
 }
 
-template <bool kFp8>
-__device__ __forceinline__ uint64_t a4_desc(uint32_t addr) {
-  return kFp8 ? umma_desc_k_sw64(addr) : umma_desc_k_sw128(addr);
-}
-
 // Chunks u = g + 3 i, i = 0, 1, ..., below `end`: those of softmax group g.
 __device__ __forceinline__ int group_chunks(int end, int g) { return (end - g + kA4Groups - 1) / kA4Groups; }
 
 // Q row -> RoPE -> shared memory (K-major, swizzled like a TMA tile).  Groups 0 and 1 rotate pairs 0..15 (spatial
 // angles) and 16..31 (temporal angles, which follow the abort flags behind q_ready); group 2 has nothing to do here.
-template <bool kFp8>
 __device__ __forceinline__ void stage_q4(const AttnArgs& a, uint8_t* smem, uint64_t* q_ready, int t, int qh, int r, int g, int lane) {
-  uint8_t* q_s = smem + A4Smem<kFp8>::kQOff;
+  uint8_t* q_s = smem + A4Smem::kQOff;
   const float* tm = reinterpret_cast<const float*>(q_ready + 1) + 3;
   if (g < 2) {
     float y0[16], y1[16];
@@ -124,29 +116,17 @@ __device__ __forceinline__ void stage_q4(const AttnArgs& a, uint8_t* smem, uint6
 #pragma unroll
       for (int p = 0; p < 16; ++p) y0[p] = y1[p] = 0.f;
     }
-    if (kFp8) {
-      // 64-byte rows; 16-byte chunk index XOR ((row >> 1) & 3); y0 of this group is chunk g, y1 chunk 2 + g
-      uint8_t* rowp = q_s + r * 64;
-      const int sw = (r >> 1) & 3;
-      *reinterpret_cast<uint4*>(rowp + ((g ^ sw) << 4)) =
-          make_uint4(pack_e4m3x4(y0[0], y0[1], y0[2], y0[3]), pack_e4m3x4(y0[4], y0[5], y0[6], y0[7]),
-                     pack_e4m3x4(y0[8], y0[9], y0[10], y0[11]), pack_e4m3x4(y0[12], y0[13], y0[14], y0[15]));
-      *reinterpret_cast<uint4*>(rowp + (((2 + g) ^ sw) << 4)) =
-          make_uint4(pack_e4m3x4(y1[0], y1[1], y1[2], y1[3]), pack_e4m3x4(y1[4], y1[5], y1[6], y1[7]),
-                     pack_e4m3x4(y1[8], y1[9], y1[10], y1[11]), pack_e4m3x4(y1[12], y1[13], y1[14], y1[15]));
-    } else {
-      // 128-byte rows; chunk XOR (row & 7); y0 of this group is chunks 2g, 2g+1, y1 chunks 4+2g, 5+2g
-      uint8_t* rowp = q_s + r * 128;
-      const int sw = r & 7;
+    // 128-byte rows; chunk XOR (row & 7); y0 of this group is chunks 2g, 2g+1, y1 chunks 4+2g, 5+2g
+    uint8_t* rowp = q_s + r * 128;
+    const int sw = r & 7;
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        *reinterpret_cast<uint4*>(rowp + (((2 * g + c) ^ sw) << 4)) =
-            make_uint4(pack_bf16x2(y0[8 * c], y0[8 * c + 1]), pack_bf16x2(y0[8 * c + 2], y0[8 * c + 3]),
-                       pack_bf16x2(y0[8 * c + 4], y0[8 * c + 5]), pack_bf16x2(y0[8 * c + 6], y0[8 * c + 7]));
-        *reinterpret_cast<uint4*>(rowp + (((4 + 2 * g + c) ^ sw) << 4)) =
-            make_uint4(pack_bf16x2(y1[8 * c], y1[8 * c + 1]), pack_bf16x2(y1[8 * c + 2], y1[8 * c + 3]),
-                       pack_bf16x2(y1[8 * c + 4], y1[8 * c + 5]), pack_bf16x2(y1[8 * c + 6], y1[8 * c + 7]));
-      }
+    for (int c = 0; c < 2; ++c) {
+      *reinterpret_cast<uint4*>(rowp + (((2 * g + c) ^ sw) << 4)) =
+          make_uint4(pack_bf16x2(y0[8 * c], y0[8 * c + 1]), pack_bf16x2(y0[8 * c + 2], y0[8 * c + 3]),
+                     pack_bf16x2(y0[8 * c + 4], y0[8 * c + 5]), pack_bf16x2(y0[8 * c + 6], y0[8 * c + 7]));
+      *reinterpret_cast<uint4*>(rowp + (((4 + 2 * g + c) ^ sw) << 4)) =
+          make_uint4(pack_bf16x2(y1[8 * c], y1[8 * c + 1]), pack_bf16x2(y1[8 * c + 2], y1[8 * c + 3]),
+                     pack_bf16x2(y1[8 * c + 4], y1[8 * c + 5]), pack_bf16x2(y1[8 * c + 6], y1[8 * c + 7]));
     }
     fence_proxy_async_smem();
   }
@@ -156,7 +136,6 @@ __device__ __forceinline__ void stage_q4(const AttnArgs& a, uint8_t* smem, uint6
 // kHelped: the end of a piece, for the softmax warps.  Reads O, brings the groups' results together, stages the next piece's query rows
 // and hands the finished rows on.  A function of its own, because what it works with (addresses, the places of pieces) would
 // otherwise be kept in registers, or spilled, through the loop over the chunks (60.0 -> 64.7 us at 720p).
-template <bool kFp8>
 __device__ __noinline__ NextPiece end_piece4(const AttnArgs& a, uint8_t* smem, uint64_t* q_ready, uint32_t tmem_o, uint32_t o_final, int chunks, int item, int piece,
                                              bool any, bool ok, float m_run) {
   constexpr int G = kA4Groups;
@@ -186,7 +165,7 @@ __device__ __noinline__ NextPiece end_piece4(const AttnArgs& a, uint8_t* smem, u
   }
   // The groups' results meet in the P area (every PV of the piece is finished; the next P is written after q_ready, for which
   // group 0 arrives when it has read the others' rows).
-  float* comb = reinterpret_cast<float*>(smem + A4Smem<kFp8>::kPOff);  // [2][66][128]
+  float* comb = reinterpret_cast<float*>(smem + A4Smem::kPOff);  // [2][66][128]
   asm volatile("bar.sync 2, 384;" ::: "memory");
   if (g > 0) {
     float* mine = comb + (g - 1) * kPartial + r;
@@ -218,25 +197,24 @@ __device__ __noinline__ NextPiece end_piece4(const AttnArgs& a, uint8_t* smem, u
   int q0 = 0, qh = 0, kvh = 0;
   if (next.n > 0) {
     next.place(a, q0, qh, kvh);
-    stage_q4<kFp8>(a, smem, q_ready, q0 + r, qh, r, g, lane);
+    stage_q4(a, smem, q_ready, q0 + r, qh, r, g, lane);
   }
   if (g == 0) kr.finish(a, done, r, good, m_run, l, o, reinterpret_cast<int*>(q_ready + 1) + 19);
   return NextPiece{next.item, next.n, next.tile0, (next.item - kr.first_item) * done.n + next.n, kvh};
 }
 
 // kHelped: a one-dimensional grid, one CTA per item and helpers (KeyShares); otherwise one CTA per item.
-template <bool kFp8, bool kHelped>
+template <bool kHelped>
 __global__ void __launch_bounds__(kA4Threads, 1)
 owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnArgs a) {
-  using L = A4Smem<kFp8>;
+  using L = A4Smem;
   constexpr int kStages = L::kStages;
   constexpr int G = kA4Groups;
   constexpr uint32_t kTmemCols = 512;
-  constexpr uint32_t kIdescS = kFp8 ? umma_idesc(0, 0, 128, 64) : umma_idesc(1, 1, 128, 64);
-  constexpr uint32_t kIdescPV = kFp8 ? umma_idesc(0, 0, 128, kA4VRows) : umma_idesc(1, 1, 128, kA4VRows);
-  constexpr int kMmas = kFp8 ? 2 : 4;  // 32 bytes of the contraction per instruction, rows of 64 | 128 bytes
-  constexpr float kPShift = kFp8 ? 5.0f : 0.0f;
-  constexpr float kSlack = kFp8 ? 3.0f : 8.0f;
+  constexpr uint32_t kIdescS = umma_idesc(1, 1, 128, 64);
+  constexpr uint32_t kIdescPV = umma_idesc(1, 1, 128, kA4VRows);
+  constexpr int kMmas = 4;  // 32 bytes of the contraction per instruction, rows of 128 bytes
+  constexpr float kSlack = 8.0f;
   constexpr uint32_t kOCol = 192, kOStride = 96;  // S of group g at columns 64 g, O (80 columns) at 192 + 96 g
 
   extern __shared__ uint8_t smem_raw[];
@@ -284,7 +262,7 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
   }
   // rows of ones under every V^T chunk (16 rows): the tensor core then returns the row sum of P in column 64 of O
   {
-    constexpr uint32_t kOnes = kFp8 ? 0x38383838u : 0x3F803F80u;
+    constexpr uint32_t kOnes = 0x3F803F80u;
     constexpr int kVecPerStage = 16 * L::kRowBytes / 16;  // 16-byte vectors of the ones rows of one stage
     for (int i = threadIdx.x; i < kStages * kVecPerStage; i += kA4Threads) {
       uint8_t* base = smem + L::kStageOff + (i / kVecPerStage) * L::kStageBytes + L::kKBytes + 64 * L::kRowBytes;
@@ -391,11 +369,10 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
           return mbar_wait(smem_u32(&kv_full[u % kStages]), (u / kStages) & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
         };
         auto issue_s = [&](int i) {
-          const uint64_t qd = a4_desc<kFp8>(q_addr), kd = a4_desc<kFp8>(stage_addr(i));
+          const uint64_t qd = umma_desc_k_sw128(q_addr), kd = umma_desc_k_sw128(stage_addr(i));
 #pragma unroll
           for (int m = 0; m < kMmas; ++m) {
-            if (kFp8) umma_f8(tmem_sg, qd + 2 * m, kd + 2 * m, kIdescS, m > 0);
-            else umma_f16(tmem_sg, qd + 2 * m, kd + 2 * m, kIdescS, m > 0);
+            umma_f16(tmem_sg, qd + 2 * m, kd + 2 * m, kIdescS, m > 0);
           }
           umma_commit(smem_u32(&s_full[g]));
         };
@@ -422,11 +399,10 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
           if (!ok) break;
           tc_fence_after();
           const uint32_t p_addr = smem_u32(smem + L::kPOff + (g * L::kPBufs + (i % L::kPBufs)) * L::kPBytes);
-          const uint64_t pd = a4_desc<kFp8>(p_addr), vd = a4_desc<kFp8>(stage_addr(i) + L::kKBytes);
+          const uint64_t pd = umma_desc_k_sw128(p_addr), vd = umma_desc_k_sw128(stage_addr(i) + L::kKBytes);
 #pragma unroll
           for (int m = 0; m < kMmas; ++m) {
-            if (kFp8) umma_f8(tmem_og, pd + 2 * m, vd + 2 * m, kIdescPV, i > i0 || m > 0);
-            else umma_f16(tmem_og, pd + 2 * m, vd + 2 * m, kIdescPV, i > i0 || m > 0);
+            umma_f16(tmem_og, pd + 2 * m, vd + 2 * m, kIdescPV, i > i0 || m > 0);
           }
           umma_commit(smem_u32(&pv_done[g]));
           umma_commit(smem_u32(&kv_empty[(g + G * i) % kStages]));
@@ -453,7 +429,7 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     const uint32_t lane_addr = static_cast<uint32_t>(lane_grp * 32) << 16;
     uint8_t* p_g = smem + L::kPOff + g * L::kPBufs * L::kPBytes;
 
-    stage_q4<kFp8>(a, smem, q_ready, t, qh, r, g, lane);
+    stage_q4(a, smem, q_ready, t, qh, r, g, lane);
 
     const uint32_t tmem_s = tmem_base + g * 64 + lane_addr;  // this thread's row of the group's S
     const uint32_t tmem_o = tmem_base + kOCol + g * kOStride + lane_addr;
@@ -533,29 +509,19 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
           tmem_wait_st();
         }
       }
-      const float nshift = kPShift - m_run;
+      const float nshift = -m_run;
       uint8_t* p_s = p_g + (i % L::kPBufs) * L::kPBytes;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         auto pr = [&](int q) { return ex2_approx(fmaf(__uint_as_float(sc[c][q]), sl2, nshift)); };
-        if (kFp8) {
-          uint32_t w[8];
+        uint8_t* rowp = p_s + r * 128;
+        const int sw = r & 7;
 #pragma unroll
-          for (int q = 0; q < 8; ++q) w[q] = pack_e4m3x4(pr(4 * q), pr(4 * q + 1), pr(4 * q + 2), pr(4 * q + 3));
-          uint8_t* rowp = p_s + r * 64;
-          const int sw = (r >> 1) & 3;
-          *reinterpret_cast<uint4*>(rowp + (((2 * c) ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-          *reinterpret_cast<uint4*>(rowp + (((2 * c + 1) ^ sw) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
-        } else {
-          uint8_t* rowp = p_s + r * 128;
-          const int sw = r & 7;
+        for (int h = 0; h < 4; ++h) {
+          uint32_t w[4];
 #pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            uint32_t w[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(pr(8 * h + 2 * q), pr(8 * h + 2 * q + 1));
-            *reinterpret_cast<uint4*>(rowp + (((4 * c + h) ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-          }
+          for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(pr(8 * h + 2 * q), pr(8 * h + 2 * q + 1));
+          *reinterpret_cast<uint4*>(rowp + (((4 * c + h) ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
       fence_proxy_async_smem();
@@ -563,7 +529,7 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
       warp_arrive(smem_u32(&p_full[2 * g + (i & 1)]), lane);
     }
     if constexpr (kHelped) {
-      const NextPiece next = end_piece4<kFp8>(a, smem, q_ready, tmem_o, smem_u32(&o_final[g]), kr.tiles, item, piece, i0 < i1, ok, m_run);
+      const NextPiece next = end_piece4(a, smem, q_ready, tmem_o, smem_u32(&o_final[g]), kr.tiles, item, piece, i0 < i1, ok, m_run);
       item = next.item;
       kvh = next.kvh;
       chunk0 = next.tile0 + next.n - next.done;
@@ -573,7 +539,7 @@ owl_attn4_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
       continue;
     }
     more = kHelped;
-    // the group's result: 64 outputs and the row sum, still scaled by 2^(kPShift - m_run)
+    // the group's result: 64 outputs and the row sum, still scaled by 2^-m_run
     float o[64];
     float l_run = 0.f;
 #pragma unroll
@@ -656,18 +622,16 @@ int32_t make_tmap_2d_sw(CUtensorMap* tm, const void* base, int elem_bytes, uint6
 int num_sms();
 
 // Launches the three-group kernel: with helpers where `a` has a workspace, otherwise one (query tile, head) per CTA.
-int32_t launch_attn4(const void* K_cache, const void* Vt_cache, const AttnArgs& a, int n_kv_heads, bool fp8, cudaStream_t st) {
-  const int es = fp8 ? 1 : 2;
+int32_t launch_attn4(const void* K_cache, const void* Vt_cache, const AttnArgs& a, int n_kv_heads, cudaStream_t st) {
   CUtensorMap tmK, tmV;
-  int32_t rc = make_tmap_2d_sw(&tmK, K_cache, es, static_cast<uint64_t>(n_kv_heads) * a.capacity, 64, kA4Chunk, 64, fp8 ? 64 : 128);
+  int32_t rc = make_tmap_2d_sw(&tmK, K_cache, 2, static_cast<uint64_t>(n_kv_heads) * a.capacity, 64, kA4Chunk, 64, 128);
   if (rc != QB_OK) return rc;
-  rc = make_tmap_2d_sw(&tmV, Vt_cache, es, static_cast<uint64_t>(n_kv_heads) * 64, a.capacity, 64, kA4Chunk, fp8 ? 64 : 128);
+  rc = make_tmap_2d_sw(&tmV, Vt_cache, 2, static_cast<uint64_t>(n_kv_heads) * 64, a.capacity, 64, kA4Chunk, 128);
   if (rc != QB_OK) return rc;
   // helpers have a workspace
   const dim3 grid = a.partials != nullptr ? dim3(num_sms()) : dim3((a.tpf + 127) / 128, a.n_q_heads);
-  auto kernel = fp8 ? (a.partials != nullptr ? owl_attn4_kernel<true, true> : owl_attn4_kernel<true, false>)
-                    : (a.partials != nullptr ? owl_attn4_kernel<false, true> : owl_attn4_kernel<false, false>);
-  const int smem = fp8 ? A4Smem<true>::kTotal : A4Smem<false>::kTotal;
+  auto kernel = a.partials != nullptr ? owl_attn4_kernel<true> : owl_attn4_kernel<false>;
+  const int smem = A4Smem::kTotal;
   QB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   return launch_dep("owl_attn kernel (three groups)", kernel, grid, dim3(kA4Threads), smem, st, tmK, tmV, a);
 }
