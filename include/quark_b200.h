@@ -119,8 +119,9 @@ typedef struct {
   int32_t gate_groups;               /* G: gate is [G, N], each row covers M/G rows */
   int32_t split_k;                   /* 0 = choose; >= 1 forces the number of K slices */
   int32_t tile_n;                    /* 0 = choose; 64, 128 or 256 */
-  int32_t reserved;                  /* flags.  bit 0, slice mode: 0 = sum K slices inside a thread-block cluster when there
-                                        are 2, 4 or 8 of them (no workspace traffic); 1 = always through the workspace.
+  int32_t reserved;                  /* flags.  bit 0, slice mode: 0 = sum K slices inside a thread-block cluster (no
+                                        workspace traffic) where they fit one: 2, 4 or 8 slices of 64-column tiles, 2 of
+                                        a pair's 128-column tiles; others, and with 1 all, go through the workspace.
                                         bit 1: B is constant (weights; no kernel in flight writes it), so its first tiles
                                         may be fetched before the kernels ahead of this one in the stream have finished.
                                         bit 2 (qb_gemm_grouped, e4m3 C): the result is rounded to bf16 before it is

@@ -8,7 +8,7 @@
 // kind::f16 (K = 16 per instruction), e4m3 operands kind::f8f6f4 (K = 32); both move 128 bytes of K per stage row, so the two
 // paths share every address computation.
 //
-// K can be split over `splits` CTAs per tile.  As the CTAs of one thread-block cluster they push the rows that other CTAs will
+// K can be split over `splits` CTAs per tile.  As the CTAs of one thread-block cluster (64-column tiles) they push the rows that other CTAs will
 // finish into those CTAs' shared memory; after one cluster barrier each CTA sums its 128 / splits rows in slice order and runs
 // the epilogue on them.  Through the workspace (any number of slices) each CTA writes its partial tile and takes a ticket, and
 // the CTA that draws the last ticket adds the partials in slice order.  Either way the sum does not depend on which CTA came
@@ -180,8 +180,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const bool fast = !QKV && g.splits == 1 && g.N % 32 == 0 && (reinterpret_cast<uintptr_t>(g.C) & 31u) == 0 &&
                       (g.gate == nullptr || m0 / g.rows_per_gate == m_last / g.rows_per_gate);
     // Two warps share each TMEM lane quarter (w and w + 4 see the same 32 rows): in the fast epilogue the
-    // first takes the even 32-column chunks of the row, the second the odd ones.  The other epilogue paths
-    // are run by the first four warps alone.
+    // first takes the even 32-column chunks of the row, the second the odd ones.  All eight warps run the other
+    // paths too, but for K slices through the workspace, which the first four sum alone.
     const int half = (warp - 2) >> 2;
     constexpr int kMyChunks = BN / 64;  // 32-column chunks per warp
     constexpr int kResInRegs = BN <= 128 ? 1 : 0;
@@ -565,6 +565,8 @@ static GemmPlan make_plan(const qb_gemm_params& p, int max_cg, double* cost_out)
         const bool cl = s > 1 && (p.reserved & 1) == 0 && cluster_slices(cg, bn, s);
         if (s > 1 && p.split_k == 0 && kbps < 4) continue;  // too little K to share
         if (s > 1 && !cl && (cg == 2 || static_cast<size_t>(tiles) * sizeof(int) > kCounterBytes)) continue;  // more tiles than counters
+        // Against every forced width and number of slices (60 shapes, M and N and K over the whole range, back to back with the
+        // operands in L2) the choice is the fastest or within 2.5 % of it for nine in ten, at worst 9.5 % (7954 x 144 x 80 e4m3).
         // Measured with 128 CTAs, e4m3 and bf16 alike: ns per 128 bytes of K, and the rest of a launch that waits for the one
         // before it.  Tiles run in rounds over the SMs; a pair's CTAs stay for all rounds and hide all epilogues but the last.
         // Slices add their exchange: through the cluster it grows with the CTAs that push at once (16 CTAs 0.4 us, 128 CTAs

@@ -5,7 +5,7 @@
 // issues for both, and each CTA's TMEM receives its own 128 rows.  An SM then takes (128 + BN / 2) instead of (128 + BN) rows of
 // operands per 128 bytes of K, and a 256 x 256 tile is bound by the tensor cores (512 clocks per 128 bytes of K) and no longer by
 // the way into shared memory.  Two TMEM accumulators: the epilogue warps read one while the next tile fills the other, so of all
-// epilogues only the last is seen.  8192^3 e4m3: 550 us in one-CTA tiles of one wave after the other, 424 us here (2.6 PFLOP/s,
+// epilogues only the last is seen.  8192^3 e4m3: 550 us in one-CTA tiles of one wave after the other, 413 - 424 us here (2.6 PFLOP/s,
 // at the power limit).  Small products stay with gemm.cu: a pair's barriers cost 1 us more per launch.
 //
 // K slices (tiles of 128 columns, for products with few tiles and a long K) are summed inside the cluster as in gemm.cu.

@@ -572,7 +572,7 @@ class Waypoint15(nn.Module):
     def _weights_ahead(self):
         """Per block, a call that fetches the weights up to the next attention into L2 while this block's attention leaves DRAM
         idle; None where that does not pay.  It does where the GEMMs wait for their weights: one or two 128-row tiles of tokens (24
-        layers of 128 tokens bf16 7052 -> 6699 us a frame; 12 layers of 192 and 256 tokens bf16 4359 -> 4271 and 4505 -> 4465, e4m3
+        layers of 128 tokens bf16 7052 -> 6645 us a frame; 12 layers of 192 and 256 tokens bf16 4359 -> 4271 and 4505 -> 4465, e4m3
         3239 -> 3182 and 3339 -> 3298) and more weights than L2 holds from one pass to the next.  At 720p the GEMMs are bound by
         their operands' way into the SMs, and the attention, longer than the fetch, loses more to it (bf16 16292 -> 16937)."""
         if self.cfg.tpf > 256 or self.cfg.tp_world > 1 or not self.blocks:
