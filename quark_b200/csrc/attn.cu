@@ -1,46 +1,35 @@
-// owl_attn: segment-sparse GQA flash attention with inline ortho-RoPE on Q, head_dim 64.
+// owl_attn: segment-sparse GQA flash attention with inline ortho-RoPE on Q, head_dim 64.  This file: the host side, and the kernel for
+// e4m3 caches and for key splits in either type; bf16 without key splits is in attn3.cu.
 //
-// One CTA owns 128 query tokens of one Q head and walks the valid keys in tiles of 128, enumerated
-// from the (start, length) segment table, so a masked bucket is never loaded.  384 threads:
-//   warp 0        TMA producer: K tile [128 keys x 64] and V^T tile [64 x 128 keys] per stage
+// One CTA owns 128 query tokens of one Q head and walks the valid keys in tiles of 128, enumerated from the (start, length)
+// segment table, so a masked bucket is never loaded.  384 threads:
+//   warp 0        TMA producer: a ring of K tiles [128 keys x 64] and one of V^T tiles [64 x 128 keys] (e4m3: + 16 rows of ones)
 //   warps 1, 2    one thread each issues tcgen05.mma for softmax group 0 / 1: S = Q K^T and O += P V
-//   warp 3        idle (keeps the softmax warps aligned to the TMEM lane quarters)
+//   warp 3        sines and cosines of the temporal angles
 //   warps 4-7     softmax group 0: even key tiles        warps 8-11  softmax group 1: odd key tiles
 // After set-up the control warps hand registers to the softmax warps (setmaxnreg), each of whose
-// threads keeps a whole score row of one query (128 values) in registers.
+// threads holds a whole score row of one query (128 values).
 //
-// Per group, TMEM holds one S tile (128 columns) and the output accumulator O (80 columns).  A softmax
-// thread copies its row of S(i) to registers (S(i + 1) may then be computed), takes the row maximum,
-// writes P(i) = 2^(score - m) to shared memory, and the MMA warp accumulates O += P(i) V(i) in TMEM.
-// m is the maximum the row was last rescaled to, not the running maximum: O (and the row sum) are
-// multiplied by 2^(m - m') only when a tile's maximum exceeds m by more than kSlack, which is rare after
-// the first tiles; P then stays below 2^(kPShift + kSlack), inside the range of e4m3 / bf16.  The two
-// partial results (m, row sum, 64 outputs) are merged once at the end.
+// Per group, TMEM holds one S tile (128 columns), the accumulator O and P (the A operand of O += P V).  A softmax
+// thread copies its row of S(i) to registers (S(i + 1) may then be computed), takes the row maximum, makes P(i) = 2^(score - m) and
+// stores it, packed, once PV(i - 1) has read the P before: long ago, since the exponentials of tile i come in between.
+// m is the maximum the row was last rescaled to, not the running maximum: O (and the row sum) are multiplied by 2^(m - m') only when
+// a tile's maximum exceeds m by more than kSlack, which is rare after the first tiles.
+// The two groups' results (m, row sum, 64 outputs) are merged once at the end.
 //
-// The exponentials bound this kernel (the special-function unit makes 16 per clock and SM; head_dim 64
-// gives it only 256 tensor-core flops per exponential to hide behind), so the two groups take turns on
-// them: while one group runs its exponentials the other loads its next row, finds the maximum and
-// synchronises with the MMA warp.  The turn passes when half of a tile's exponentials are issued, so the
-// unit always has two warps per scheduler to draw from.  Measured on B200 (720p, 8320 keys): free-running
-// groups fall into lock step and leave the unit idle half of the time (73 us); strict alternation 60 us;
-// alternation with the half-tile overlap 54 us.  A polynomial 2^x on the FMA pipe for part of the elements
-// (QB_POLY_OF8 > 0) is slower here, because the softmax warps are issue bound as well: 57 / 61 / 63 us for
-// 1 / 2 / 3 of every 8 elements.  Also measured and not kept (52 us as it stands): two threads per query row
-// (16 softmax warps of 64 keys each, row maxima exchanged through shared memory) 58 us; row maxima taken
-// during the exponentials instead of before them, with the rare row that outgrows its maximum written twice,
-// 57 us (the instructions moved into the exponential phase lengthen it by what the phase before it saves).
-// Every mbarrier wait on a softmax warp's path costs about 100 cycles per tile even when it succeeds at once
-// (2 us per launch), which is why each warp arrives once (lane 0, after __syncwarp) and waits as rarely as
-// the data flow allows.
+// The row sum is that of exactly the rounded P that is multiplied with V.  In e4m3 the tensor core makes it: 16 rows of ones follow the
+// 64 V^T rows of every stage, so PV has 80 columns and column 64 is sum_k P[q, k].  bf16 path: kind::f16 MMAs, P rounded to bf16.  fp8
+// path: Q (after RoPE), K, V and P are e4m3 (kind::f8f6f4); P is scaled by 2^kPShift so small probabilities keep mantissa bits (the
+// factor cancels in the division by the row sum).  exp2 is ex2.approx.f32 (ex2.approx.f16x2 issues at half the rate of the f32 form: no
+// gain per element), the chord of ex2_lin_from_biased for every second e4m3 probability, a polynomial for every fourth bf16 one.
 //
-// The row sum of P comes out of the tensor core: 16 rows of ones follow the 64 V^T rows of every
-// stage, so PV has 80 columns and column 64 is sum_k P[q, k] of exactly the rounded P that is
-// multiplied with V.  bf16 path: kind::f16 MMAs, P rounded to bf16.  fp8 path: Q (after RoPE), K, V
-// and P are e4m3 (kind::f8f6f4); P is scaled by 2^kPShift so small probabilities keep mantissa bits (the
-// factor cancels in the division by the row sum), and has two shared-memory tiles per group so that
-// writing P(i) never waits for PV(i - 1).  exp2 is ex2.approx.f32 in both paths: measured on B200,
-// ex2.approx.f16x2 issues at half the rate of the f32 form (no gain per element) and the f16x2 -> e4m3x2
-// conversion is four times slower than f32 -> e4m3x2.
+// What bounds it (e4m3, 720p, 8320 keys): instruction issue of the softmax warps, two per scheduler.  A loop with the same softmax
+// instructions and nothing else takes 726 cycles per tile, with one warp per scheduler 911; this kernel 1040, the waits, fences and
+// arrivals of a tile being what the other warp covers in part only.  Before (47.8 us at 16 buckets, 318 at 128, 168 at 64), a stage of
+// the one K / V ring was held from S to PV, so the MMA threads waited 850 to 1350 cycles per tile for K, and P went through shared
+// memory with the groups taking turns on the exponentials; now 41.8, 268 and 144 us.  Tried and dropped: the turns kept (46.0); a third
+// group of warps for the maxima (50.3: S, maximum, exponentials in a row take longer than the tile before covers); three groups over
+// 64-key tiles (46.9: the fixed work of a tile twice); the chord's integer multiply-add held on the FMA pipe (42.9).
 #include <atomic>
 
 #include <cuda.h>
@@ -50,231 +39,126 @@
 namespace qb {
 
 int num_sms();
+int32_t launch_attn3(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnArgs& a, int Hq, bool helped, cudaStream_t st);
 int32_t make_tmap_2d_sw(CUtensorMap* tm, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint32_t box_rows,
                         uint32_t box_cols, int swizzle_bytes);
 
-#ifdef QB_ATTN_TRACE
-__device__ long long g_attn_trace[5][80][8];  // [role: softmax g0, g1, mma g0, g1][tile][point]
-#define QB_TR(role, i, pt)                                                                    \
-  do {                                                                                        \
-    if (blockIdx.x == 1 && blockIdx.y == 5 && lane == 0 && (i) < 80) g_attn_trace[role][i][pt] = clock64(); \
-  } while (0)
-#else
-#define QB_TR(role, i, pt) do { } while (0)
-#endif
-
 constexpr int kAttnThreads = 384;
-#ifndef QB_HANDOFF
-#define QB_HANDOFF 2
-#endif
-constexpr int kHandoffChunk = QB_HANDOFF;  // the exponentials' turn passes to the other group before this 32-key chunk
-#ifndef QB_POLY_OF8
-#define QB_POLY_OF8 0
-#endif
-constexpr int kPolyOf8 = QB_POLY_OF8;      // exponentials out of every 8 that run as a polynomial on the FMA pipe
-constexpr int kCtrlRegs = 64;      // per thread, warps 0-3 (128 x 64 + 256 x 216 <= 64 K registers)
+// setmaxnreg moves registers inside the pool the CTA was given at launch (384 threads x 168 registers): an increase waits until
+// other warps of the CTA have released enough, so the budget must close or the softmax warps would wait for ever.
+constexpr int kLaunchRegs = 168;
+constexpr int kCtrlRegs = 72;      // per thread, warps 0-3
 constexpr int kSoftmaxRegs = 216;  // per thread, warps 4-11
-constexpr int kQTile = 128;
-constexpr int kKeyTile = 128;
-constexpr int kVRows = 80;  // 64 channels + 16 rows of ones (row sum of P)
+static_assert(128 * kCtrlRegs + 256 * kSoftmaxRegs <= kAttnThreads * kLaunchRegs, "register budget of the CTA");
 
 template <bool kFp8>
 struct AttnSmem {
   static constexpr int kEs = kFp8 ? 1 : 2;
-  // Even: tile j sits in stage j % kStages, so a stage then belongs to one group's tiles.  With three stages a group waited
-  // for a phase of a stage whose previous phase the other group watches: where that earlier copy was still on its way, the
-  // parity wait returned at once and the scores came from the stale tile (6 of 100 bf16 calls with key splits at 360p).
-  static constexpr int kStages = 4;
-  static constexpr int kQBytes = kQTile * 64 * kEs;          // 16 KB | 8 KB
-  static constexpr int kKBytes = kKeyTile * 64 * kEs;        // 16 KB | 8 KB
-  static constexpr int kVTile = kVRows * 128;                // one 128-byte-wide V^T tile incl. ones rows: 10 KB
-  static constexpr int kVBytes = kVTile * kEs;               // bf16: two tiles (keys 0-63, 64-127)
-  static constexpr int kPBytes = kQTile * kKeyTile * kEs;    // 32 KB | 16 KB, one P tile
-  static constexpr int kPBufs = kFp8 ? 2 : 1;                // P tiles per softmax group (bf16: no room for two)
-  static constexpr int kStageBytes = kKBytes + kVBytes;
+  // Of each ring.  A stage is given back when its MMAs are done, so the groups hold those of up to four tiles; with four stages the next
+  // tiles were only asked for when they were needed (e4m3, 720p: 47.8 -> 42.5 us with eight).  Even: a stage then belongs to one
+  // group's tiles.  (With three a group waited for a phase of a stage whose previous phase the other group watches: where that earlier
+  // copy was still on its way, the parity wait returned at once.)
+  static constexpr int kKStages = kFp8 ? 8 : 4, kVStages = kFp8 ? 8 : 6;
+  // e4m3: 16 rows of ones under the 64 V^T rows make the tensor core return the row sum of P in column 64 of O.  bf16 has no TMEM
+  // columns left for that (S 128, O 64, P 64 a group): the softmax threads add up the rounded probabilities.
+  static constexpr int kRows = kFp8 ? kVRows : 64;
+  static constexpr int kQBytes = kQTile * 64 * kEs;          // 8 KB | 16 KB
+  static constexpr int kKBytes = kKeyTile * 64 * kEs;        // 8 KB | 16 KB
+  static constexpr int kVTile = kRows * 128;                 // 128 bytes of keys a row: 10 KB | 8 KB
+  static constexpr int kVBytes = kVTile * kEs;               // bf16: two (keys 0-63, 64-127)
   static constexpr int kQOff = 0;
-  static constexpr int kPOff = kQOff + kQBytes;
-  static constexpr int kStageOff = kPOff + 2 * kPBufs * kPBytes;
-  static constexpr int kBarOff = kStageOff + kStages * kStageBytes;
-  static constexpr int kTotal = kBarOff + 512 + 1024;
-  static_assert(kStages * kStageBytes >= 266 * 68 * 4, "merge area of the cluster splits (7 CTAs need most) aliases the stage area");
-  static_assert(kStages * kStageBytes >= 66 * 128 * 4, "merge buffer aliases the stage area");
-  static_assert(kStages % 2 == 0 && kTotal <= 227 * 1024, "see kStages; shared memory of one CTA");
+  static constexpr int kKOff = kQOff + kQBytes;
+  static constexpr int kVOff = kKOff + kKStages * kKBytes;
+  static constexpr int kClusterOff = kKOff;                  // the rings are free when the CTAs of a cluster meet
+  static constexpr int kCombOff = kVOff + kVStages * kVBytes;  // where the groups meet
+  static constexpr int kBarOff = kCombOff + 2 * 34 * kQTile * 4;
+  static constexpr int kTotal = kBarOff + 640 + 1024;
+  static_assert(kCombOff - kClusterOff >= 266 * 68 * 4, "merge area of the cluster splits (7 CTAs need most) aliases the rings");
+  static_assert(kKStages % 2 == 0 && kVStages % 2 == 0 && kTotal <= 227 * 1024, "see kKStages; shared memory of one CTA");
 };
 
-// 2^x on the FMA and integer pipes, for the share of the exponentials that the special-function unit
-// has no time for: x = n + f with n = round(x) taken from the low mantissa bits of x + 1.5 * 2^23, a
-// minimax polynomial for 2^f on [-0.5, 0.5] (degree 2: 1.7e-3 relative error, below what an e4m3
-// probability resolves; degree 3: 7.5e-5, below a bf16 ulp), n added to the exponent field.
-template <int kDegree>
-__device__ __forceinline__ float ex2_poly(float x) {
-  x = fmaxf(x, -120.0f);
-  const float t = x + 12582912.0f;
-  const float f = x - (t - 12582912.0f);
-  float p;
-  if (kDegree == 2) {
-    p = fmaf(0.23842892f, f, 0.70344800f);
-    p = fmaf(p, f, 1.0004431f);
-  } else {
-    p = fmaf(0.055171669f, f, 0.24261113f);
-    p = fmaf(p, f, 0.69326097f);
-    p = fmaf(p, f, 0.99992806f);
-  }
-  return __uint_as_float(__float_as_uint(p) + (__float_as_uint(t) << 23));
-}
-// Element q of a chunk goes to the polynomial when (q mod 8) < kPolyOf8.
-template <bool kFp8, int kPolyOf8>
-__device__ __forceinline__ float p_exp(int q, float x) {
-  return (q & 7) < kPolyOf8 ? ex2_poly<kFp8 ? 2 : 3>(x) : ex2_approx(x);
-}
-
-// Which 128-key tile is the j-th valid one?  Returns its first cache row and how many of its
-// keys are valid.  Segments are (start, length) pairs; zero-length entries are legal.  Fully
-// unrolled so the table stays in registers.
-__device__ __forceinline__ void locate_tile(const int (&seg)[6], int j, int& row, int& valid) {
-  row = 0;
-  valid = 0;
-  bool found = false;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const int nt = (seg[2 * i + 1] + kKeyTile - 1) / kKeyTile;
-    if (!found && j < nt) {
-      row = seg[2 * i] + j * kKeyTile;
-      valid = min(kKeyTile, seg[2 * i + 1] - j * kKeyTile);
-      found = true;
-    }
-    j -= nt;
-  }
-}
-
-// 32 scores of one row (registers) -> probabilities -> the P tile in shared memory (layout of a TMA tile).
-template <bool kFp8, int kPolyOf8, bool kLin>
-__device__ __forceinline__ void p_chunk(const uint32_t (&sc)[32], int c, float sl2, float nshift, uint8_t* p_s, int r) {
-  const int sw = r & 7;
-  const float nshift_lin = nshift + kLinMagic;
-  auto pr = [&](int q) {
-    if (kFp8 && kLin && (q & 1)) return ex2_lin_from_biased(fmaf(__uint_as_float(sc[q]), sl2, nshift_lin));
-    return p_exp<kFp8, kPolyOf8>(q, fmaf(__uint_as_float(sc[q]), sl2, nshift));
-  };
-  if (kFp8) {
-    uint32_t w[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) w[q] = pack_e4m3x4(pr(4 * q), pr(4 * q + 1), pr(4 * q + 2), pr(4 * q + 3));
-    uint8_t* rowp = p_s + r * 128;
-    *reinterpret_cast<uint4*>(rowp + (((2 * c) ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-    *reinterpret_cast<uint4*>(rowp + (((2 * c + 1) ^ sw) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
-  } else {
-    // keys 0..63 in the first half of the P buffer, 64..127 in the second; 128-byte rows
-    uint8_t* rowp = p_s + (c >> 1) * (kQTile * kKeyTile) + r * 128;
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      uint32_t w[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(pr(8 * h + 2 * q), pr(8 * h + 2 * q + 1));
-      *reinterpret_cast<uint4*>(rowp + ((((c & 1) * 4 + h) ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-  }
-}
-
-// Whether the keys of a (query tile, head) are shared by gridDim.z CTAs, and how their results are brought together: through the
-// workspace (see AttnArgs::partials), or, the CTAs being one thread-block cluster, in shared memory.  The unsplit kernel is an
-// instantiation of its own so that none of this reaches its instruction stream.  kHelped: the CTAs that
-// the items leave over take a part of the keys of several items each (KeyShares).
-enum { kUnsplit = 0, kSplitWorkspace = 1, kSplitCluster = 2, kHelped = 3 };
+// What follows the rings in shared memory.
+struct AttnBars {
+  uint64_t k_full[8], k_empty[8], v_full[8], v_empty[8];
+  uint64_t s_full[2];       // [group] S(i) is in TMEM
+  uint64_t s_free[2];       // [group] the group holds S(i) in registers
+  uint64_t p_full[2];       // [group] P(i) is in TMEM
+  uint64_t pv_done[2];      // [group] O += P(i) V(i) has finished
+  uint64_t o_final[2];      // [group] every PV of a piece has finished
+  uint64_t q_ready;
+  uint32_t tmem_slot;
+  int abort_flag, drain_flag, exchange;
+  float tm[16];  // cosines and sines of the temporal angles
+  int seg[6];    // the segment table, for tiles that need a mask: tile j of the CTA is tile j + tile_shift of the table
+  int tiles, tile_shift;  // kHelped: tiles of an item
+};
+static_assert(sizeof(AttnBars) <= 640, "kBarOff + 640");
 
 // Cluster splits: 2 groups x S CTAs leave 64 outputs, m and the row sum of each query row with the CTA that writes the row
 // (128 / S rows each), [2 S][rows][kMergePitch] f32.
 constexpr int kMergePitch = 68;
+__host__ __device__ constexpr int merge_rows(int splits) { return (kQTile + splits - 1) / splits; }
 // Tiles j = 2 i + g, i = 0, 1, ..., below `end`: those of softmax group g.
 __device__ __forceinline__ int group_tiles(int end, int g) { return (end - g + 1) >> 1; }
-__host__ __device__ constexpr int merge_rows(int splits) { return (kQTile + splits - 1) / splits; }
 
-// The softmax threads' half of query row t of head qh and (group 0) its row of the RoPE table, on their way while something else
-// is done.
-__device__ __forceinline__ void load_q(const AttnArgs& a, int t, int qh, int g, uint4 (&q_pre)[4], float4 (&xy_pre)[4]) {
-  if (t >= a.tpf) return;
-  const uint4* src = reinterpret_cast<const uint4*>(after_wait(a.qkv) + static_cast<size_t>(t) * a.q_row + static_cast<size_t>(qh) * a.q_head + g * 32);
+// 32 scores of one row -> packed probabilities 2^(score * sl2 + nshift); bf16: `sum` grows by the rounded ones.  e4m3 makes every second
+// one by the chord of ex2_lin_from_biased (kLin); without the chord every fourth comes from the polynomial, since the special-function
+// unit would be the bound (e4m3, 720p: 56.6 -> 52.0 us; bf16, 360p: 14.2 -> 13.5).
+template <bool kFp8, bool kLin>
+__device__ __forceinline__ void p_chunk(const uint32_t (&s)[32], uint64_t sl2, uint64_t nshift, uint32_t* w, uint64_t (&sum)[2]) {
+  float e[32];
 #pragma unroll
-  for (int v = 0; v < 4; ++v) q_pre[v] = src[v];
-  if (g == 0) {
-    const float4* rp = reinterpret_cast<const float4*>(a.rope_xy + static_cast<size_t>(t) * 16);
+  for (int q = 0; q < 32; q += 2) {
+    fma_f32x2(e[q], e[q + 1], s[q], s[q + 1], sl2, nshift);
+    if (!kLin && (q & 7) == 6) {
+      ex2_poly_f32x2(e[q], e[q + 1]);
+      continue;
+    }
+    e[q] = ex2_approx(e[q]);
+    e[q + 1] = kLin ? ex2_lin_from_biased(e[q + 1]) : ex2_approx(e[q + 1]);
+  }
+  if (kFp8) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) xy_pre[i] = __ldg(rp + i);
+    for (int q = 0; q < 8; ++q) w[q] = merge_e4m3x4(e[4 * q], e[4 * q + 1], e[4 * q + 2], e[4 * q + 3]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      w[q] = pack_bf16x2(e[2 * q], e[2 * q + 1]);
+      add_f32x2(sum[q & 1], w[q] << 16, w[q] & 0xFFFF0000u);
+    }
   }
 }
 
-// Q row -> RoPE -> shared memory (K-major, swizzled like a TMA tile).  Group 0 rotates pairs 0..15 (spatial angles), group 1 pairs
-// 16..31 (temporal angles, which follow the abort flags behind q_ready).
-template <bool kFp8>
-__device__ __forceinline__ void stage_q(uint8_t* smem, uint64_t* q_ready, int r, int g, bool row_ok, const uint4 (&q_pre)[4], const float4 (&xy_pre)[4], int lane) {
-  uint8_t* q_s = smem + AttnSmem<kFp8>::kQOff;
-  const float* tm = reinterpret_cast<const float*>(q_ready + 1) + 3;
-  float y0[16], y1[16];
-  if (row_ok) {
-    float xy[16];
-    if (g == 0) {
+// Group 0's threads bring both groups' results for their row together (`comb`: [66][128], shared memory nobody else uses by then).
+__device__ __forceinline__ void merge_groups(float* comb, int g, int r, float& m, float& l, float (&o)[64]) {
+  asm volatile("bar.sync 2, 256;" ::: "memory");
+  if (g == 1) {
+    comb[r] = m;
+    comb[128 + r] = l;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 v = xy_pre[i];
-        xy[4 * i] = v.x; xy[4 * i + 1] = v.y; xy[4 * i + 2] = v.z; xy[4 * i + 3] = v.w;
-      }
-    }
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const uint4 x = q_pre[v];
-      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int pl = v * 4 + j;
-        const int i = pl >> 1;
-        const float c = g == 0 ? xy[i] : tm[i];
-        const float s = g == 0 ? xy[8 + i] : tm[8 + i];
-        const float x0 = bf16lo(w[j]), x1 = bf16hi(w[j]);
-        y0[pl] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
-        y1[pl] = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s));
-      }
-    }
-  } else {
-#pragma unroll
-    for (int p = 0; p < 16; ++p) y0[p] = y1[p] = 0.f;
+    for (int d = 0; d < 64; ++d) comb[(2 + d) * 128 + r] = o[d];
   }
-  if (kFp8) {
-    // 64-byte rows; 16-byte chunk index XOR ((row >> 1) & 3); y0 of this group is chunk g, y1 chunk 2 + g
-    uint8_t* rowp = q_s + r * 64;
-    const int sw = (r >> 1) & 3;
-    *reinterpret_cast<uint4*>(rowp + ((g ^ sw) << 4)) =
-        make_uint4(pack_e4m3x4(y0[0], y0[1], y0[2], y0[3]), pack_e4m3x4(y0[4], y0[5], y0[6], y0[7]),
-                   pack_e4m3x4(y0[8], y0[9], y0[10], y0[11]), pack_e4m3x4(y0[12], y0[13], y0[14], y0[15]));
-    *reinterpret_cast<uint4*>(rowp + (((2 + g) ^ sw) << 4)) =
-        make_uint4(pack_e4m3x4(y1[0], y1[1], y1[2], y1[3]), pack_e4m3x4(y1[4], y1[5], y1[6], y1[7]),
-                   pack_e4m3x4(y1[8], y1[9], y1[10], y1[11]), pack_e4m3x4(y1[12], y1[13], y1[14], y1[15]));
-  } else {
-    // 128-byte rows; chunk XOR (row & 7); y0 of this group is chunks 2g, 2g+1, y1 chunks 4+2g, 5+2g
-    uint8_t* rowp = q_s + r * 128;
-    const int sw = r & 7;
+  asm volatile("bar.sync 2, 256;" ::: "memory");
+  if (g == 0) {
+    const float m1 = comb[r], top = fmaxf(m, m1);
+    const float a0 = ex2_approx(m - top), a1 = ex2_approx(m1 - top);
+    l = l * a0 + comb[128 + r] * a1;
+    m = top;
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      *reinterpret_cast<uint4*>(rowp + (((2 * g + c) ^ sw) << 4)) =
-          make_uint4(pack_bf16x2(y0[8 * c], y0[8 * c + 1]), pack_bf16x2(y0[8 * c + 2], y0[8 * c + 3]),
-                     pack_bf16x2(y0[8 * c + 4], y0[8 * c + 5]), pack_bf16x2(y0[8 * c + 6], y0[8 * c + 7]));
-      *reinterpret_cast<uint4*>(rowp + (((4 + 2 * g + c) ^ sw) << 4)) =
-          make_uint4(pack_bf16x2(y1[8 * c], y1[8 * c + 1]), pack_bf16x2(y1[8 * c + 2], y1[8 * c + 3]),
-                     pack_bf16x2(y1[8 * c + 4], y1[8 * c + 5]), pack_bf16x2(y1[8 * c + 6], y1[8 * c + 7]));
-    }
+    for (int d = 0; d < 64; ++d) o[d] = o[d] * a0 + comb[(2 + d) * 128 + r] * a1;
   }
-  fence_proxy_async_smem();
-  warp_arrive(smem_u32(q_ready), lane);
 }
 
 // kHelped: the end of a piece, for the softmax warps.  Reads O, brings the groups' results together, asks for the next piece's
 // query rows and hands the finished rows on.  A function of its own, because what it works with (addresses, the places of pieces)
-// would otherwise be kept in registers, or spilled, through the loop over the tiles (46 -> 64 us at 720p).
-template <bool kFp8>
-__device__ __noinline__ NextPiece end_piece(const AttnArgs& a, uint8_t* smem, uint64_t* q_ready, uint32_t tmem_o, uint32_t o_final, int tiles, int item, int piece,
-                                            bool any, bool ok, float m_run) {
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(reinterpret_cast<uint32_t*>(q_ready + 1) + 1);
+// would otherwise be kept in registers, or spilled, through the loop over the tiles.
+__device__ __noinline__ int end_piece(const AttnArgs& a, uint8_t* smem, uint32_t tmem_o, int piece, bool any, float m) {
+  using L = AttnSmem<true>;
+  AttnBars* b = reinterpret_cast<AttnBars*>(smem + L::kBarOff);
+  volatile int* abort_flag = &b->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = (warp - 4) >> 2, r = (warp & 3) * 32 + lane;
-  const KeyShares kr(a, tiles, kHelperCost);
+  const KeyShares kr(a, *const_cast<volatile int*>(&b->tiles), kHelperCost);
+  const int item = kr.first_item + piece;
   const Piece done = kr.at(item), next = kr.at(item + 1);
   int q0 = 0, qh = 0, kvh = 0;
   uint4 q_pre[4];
@@ -287,88 +171,49 @@ __device__ __noinline__ NextPiece end_piece(const AttnArgs& a, uint8_t* smem, ui
   float l = 0.f;
 #pragma unroll
   for (int d = 0; d < 64; ++d) o[d] = 0.f;
-  if (ok) {
-    ok = __all_sync(0xffffffffu, mbar_wait(o_final, piece & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
-    if (ok && any) {
-      tc_fence_after();
-      uint32_t oo[2][32];
-      tmem_ld32(tmem_o, oo[0]);
-      tmem_ld32(tmem_o + 32, oo[1]);
-      uint32_t lsum = tmem_ld1(tmem_o + 64);
-      tmem_wait_ld_into(oo[0]);
-      tmem_loaded(oo[1]);
-      tmem_loaded(lsum);
-#pragma unroll
-      for (int d = 0; d < 64; ++d) o[d] = __uint_as_float(oo[d >> 5][d & 31]);
-      l = __uint_as_float(lsum);
-    }
+  mbar_wait_warp(smem_u32(&b->o_final[g]), piece & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
+  if (any) {
+    tc_fence_after();
+    read_o<true>(tmem_o, o, l);
   }
-  // The groups' results meet in the P area (every PV of the piece is finished; the next P is written after q_ready, for which
-  // group 0 arrives when it has read the other's rows).
-  float* comb = reinterpret_cast<float*>(smem + AttnSmem<kFp8>::kPOff);  // [66][128]
-  asm volatile("bar.sync 2, 256;" ::: "memory");
-  if (g == 1) {
-    comb[r] = m_run;
-    comb[128 + r] = l;
-#pragma unroll
-    for (int d = 0; d < 64; ++d) comb[(2 + d) * 128 + r] = o[d];
-  }
-  asm volatile("bar.sync 2, 256;" ::: "memory");
-  if (g == 0) {
-    const float m1 = comb[r], m = fmaxf(m_run, m1);
-    const float a0 = ex2_approx(m_run - m), a1 = ex2_approx(m1 - m);
-    l = l * a0 + comb[128 + r] * a1;
-    m_run = m;
-#pragma unroll
-    for (int d = 0; d < 64; ++d) o[d] = o[d] * a0 + comb[(2 + d) * 128 + r] * a1;
-  }
-  const bool good = ok && *abort_flag == 0;
-  if (next.n > 0) stage_q<kFp8>(smem, q_ready, r, g, q0 + r < a.tpf, q_pre, xy_pre, lane);
-  if (g == 0) kr.finish(a, done, r, good, m_run, l, o, reinterpret_cast<int*>(q_ready + 1) + 19);
-  return NextPiece{next.item, next.n, next.tile0, (next.item - kr.first_item) * done.n + next.n, kvh};
+  // The next piece's K and V are on their way into the rings, so the groups meet in memory of their own.
+  merge_groups(reinterpret_cast<float*>(smem + L::kCombOff), g, r, m, l, o);
+  const bool good = *abort_flag == 0;
+  if (g == 1 && r == 0) b->tile_shift = next.tile0 - (piece + 1) * done.n;  // (read again behind q_ready of the next piece)
+  if (next.n > 0) stage_q<true>(smem + L::kQOff, b->tm, &b->q_ready, r, g, q0 + r < a.tpf, q_pre, xy_pre, lane);
+  if (g == 0) kr.finish(a, done, r, good, m, l, o, &b->exchange);
+  return next.n;
 }
 
 template <bool kFp8, int kSplit, bool kLin>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnArgs a) {
   using L = AttnSmem<kFp8>;
-  constexpr int kStages = L::kStages;
+  constexpr int kKS = L::kKStages, kVS = L::kVStages;
   constexpr uint32_t kTmemCols = 512;
-  constexpr uint32_t kIdescS = kFp8 ? umma_idesc(0, 0, 128, 128) : umma_idesc(1, 1, 128, 128);
-  constexpr uint32_t kIdescPV = kFp8 ? umma_idesc(0, 0, 128, kVRows) : umma_idesc(1, 1, 128, kVRows);
-  // P = 2^(kPShift + score - m) with m the row maximum the group last rescaled to; m is raised (and O
+  constexpr uint32_t kIdescS = kFp8 ? umma_idesc(0, 0, 128, kKeyTile) : umma_idesc(1, 1, 128, kKeyTile);
+  constexpr uint32_t kIdescPV = kFp8 ? umma_idesc(0, 0, 128, L::kRows) : umma_idesc(1, 1, 128, L::kRows);
+  // P = 2^(kPShift + score - m) with m the maximum the row was last rescaled to; m is raised (and O
   // rescaled) only when a tile's maximum exceeds it by more than kSlack, so P <= 2^(kPShift + kSlack):
-  // 256 for e4m3 (largest finite value 448), 256 for bf16.
+  // 256, inside the range of e4m3 and bf16.  (Not rounded to a whole number: the key that m came from, often the one that counts
+  // most, then has a probability of exactly 2^kPShift.  A whole m doubled the e4m3 error of rows with few large scores.)
   constexpr float kPShift = kFp8 ? 5.0f : 0.0f;
   constexpr float kSlack = kFp8 ? 3.0f : 8.0f;
-  constexpr uint32_t kGroupCols = 256;  // TMEM columns per softmax group: S at 0..127, O (80 columns) at 128
-  constexpr uint32_t kOCol = 128;
+  constexpr uint32_t kGroupCols = 256;  // TMEM columns per softmax group: S at 0, O (80 | 64 columns) at 128, P (32 | 64) behind it
+  constexpr uint32_t kOCol = 128, kPCol = kOCol + L::kRows;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint8_t* q_s = smem + L::kQOff;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
-  uint64_t* kv_full = bars;                  // [stages]
-  uint64_t* kv_empty = bars + kStages;       // [stages]
-  uint64_t* s_full = bars + 2 * kStages;     // [group] S(i) is in TMEM
-  uint64_t* s_free = s_full + 2;             // [group] the group holds S(i) in registers
-  // p_full counts warps' arrivals, and a warp that had to rescale can be late: were there one barrier per group,
-  // an early warp's arrival for tile i + 1 could complete tile i's phase in the late warp's place.  Even and odd
-  // tiles therefore have barriers of their own (no warp can be two tiles ahead: S(i + 2) is not computed before
-  // all four have copied S(i + 1), which they do after finishing tile i).
-  uint64_t* p_full = s_free + 2;             // [group][tile parity] P(i) is in shared memory, O is rescaled
-  uint64_t* pv_done = p_full + 4;            // [group] O += P(i) V(i) has finished
-  uint64_t* turn = pv_done + 2;              // [group] the other group has issued its exponentials
-  uint64_t* o_final = turn + 2;              // [group] every PV of the group has finished
-  uint64_t* q_ready = o_final + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_ready + 1);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* drain_flag = abort_flag + 1;
-  float* tm = reinterpret_cast<float*>(const_cast<int*>(abort_flag + 2));  // 16 floats
+  AttnBars* bars = reinterpret_cast<AttnBars*>(smem + L::kBarOff);
+  volatile int* abort_flag = &bars->abort_flag;
+  volatile int* drain_flag = &bars->drain_flag;
+  // for single threads, which stop when a wait runs out
+  auto wait = [&](uint64_t& bar, uint32_t parity) { return mbar_wait(smem_u32(&bar), parity, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN); };
+  // for whole warps, which go on: what they work out then is not written (abort_flag)
+  auto wait_warp = [&](uint64_t& bar, uint32_t parity) { mbar_wait_warp(smem_u32(&bar), parity, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN); };
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp == 4) QB_TR(4, 0, 0);
   int q0 = blockIdx.x * kQTile;
   int qh = blockIdx.y;
   int kvh = qh / a.gqa;
@@ -376,74 +221,50 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(smem_u32(&kv_full[s]), 1);
-      mbar_init(smem_u32(&kv_empty[s]), 1);
+    for (int s = 0; s < 8; ++s) {
+      mbar_init(smem_u32(&bars->k_full[s]), 1);
+      mbar_init(smem_u32(&bars->k_empty[s]), 1);
+      mbar_init(smem_u32(&bars->v_full[s]), 1);
+      mbar_init(smem_u32(&bars->v_empty[s]), 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(smem_u32(&s_full[b]), 1);
-      mbar_init(smem_u32(&s_free[b]), 4);
-      mbar_init(smem_u32(&p_full[2 * b]), 4);
-      mbar_init(smem_u32(&p_full[2 * b + 1]), 4);
-      mbar_init(smem_u32(&pv_done[b]), 1);
-      mbar_init(smem_u32(&turn[b]), 4);
-      mbar_init(smem_u32(&o_final[b]), 1);
+    for (int g = 0; g < 2; ++g) {
+      mbar_init(smem_u32(&bars->s_full[g]), 1);
+      mbar_init(smem_u32(&bars->s_free[g]), 4);
+      mbar_init(smem_u32(&bars->p_full[g]), 4);
+      mbar_init(smem_u32(&bars->pv_done[g]), 1);
+      mbar_init(smem_u32(&bars->o_final[g]), 1);
     }
-    mbar_init(smem_u32(q_ready), 8);
+    mbar_init(smem_u32(&bars->q_ready), 8);
     *abort_flag = 0;
     *drain_flag = 0;
     fence_barrier_init();
   }
-  // rows of ones under every V^T tile (16 rows x 128 bytes each): the tensor core then returns the row sum of P
-  {
-    constexpr uint32_t kOnes = kFp8 ? 0x38383838u : 0x3F803F80u;
-    constexpr int kTilesPerStage = kFp8 ? 1 : 2;
-    for (int i = threadIdx.x; i < kStages * kTilesPerStage * 128; i += kAttnThreads) {  // 128 x 16 bytes per tile
-      const int tile = i >> 7, v = i & 127;
-      uint8_t* base = smem + L::kStageOff + (tile / kTilesPerStage) * L::kStageBytes + L::kKBytes + (tile % kTilesPerStage) * L::kVTile;
-      *reinterpret_cast<uint4*>(base + 64 * 128 + v * 16) = make_uint4(kOnes, kOnes, kOnes, kOnes);
-    }
+  if (kFp8) {  // rows of ones under every V^T tile (16 rows x 128 bytes each)
+    for (int i = threadIdx.x; i < kVS * 128; i += kAttnThreads)  // 128 x 16 bytes per tile
+      *reinterpret_cast<uint4*>(smem + L::kVOff + (i >> 7) * L::kVBytes + 64 * 128 + (i & 127) * 16) = make_uint4(0x38383838u, 0x38383838u, 0x38383838u, 0x38383838u);
     fence_proxy_async_smem();
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(tmem_slot), kTmemCols);
+    tmem_alloc(smem_u32(&bars->tmem_slot), kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  if (warp == 4) QB_TR(4, 0, 1);
+  const uint32_t tmem_base = bars->tmem_slot;
 
   // Everything above touched only this CTA's shared memory and TMEM, so it may run while the kernels
   // before this one in the stream are still at work; everything below reads what they wrote.
   grid_dep_launch();
   grid_dep_wait();
 
-  // segment table -> number of key tiles (same in every thread)
-  int seg[6] = {0, 0, 0, 0, 0, 0};
-  int nseg = min(*after_wait(a.n_segments), min(a.max_segments, 3));  // the table is the work of the kernel before: ordinary loads
-  bool seg_ok = true;
-  int n_tiles = 0;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    if (i < nseg) {
-      seg[2 * i] = after_wait(a.segments)[2 * i];
-      seg[2 * i + 1] = after_wait(a.segments)[2 * i + 1];
-      if (seg[2 * i] < 0 || seg[2 * i + 1] < 0 || (seg[2 * i] & 15) != 0 || seg[2 * i] + seg[2 * i + 1] > a.capacity) seg_ok = false;
-      n_tiles += (seg[2 * i + 1] + kKeyTile - 1) / kKeyTile;
-    }
-  }
-  if (!seg_ok) {
-#pragma unroll
-    for (int i = 0; i < 6; ++i) seg[i] = 0;
-  }
-  if (!seg_ok) {  // malformed table: report and attend to nothing (output rows become 0)
-    n_tiles = 0;
-    if (threadIdx.x == 0) atomicOr(a.status, QB_DEV_BAD_SEGMENT);
-  }
-  // this CTA's share of the key tiles: tiles tile0 .. tile0 + n_tiles - 1 of the list
-  const int n_splits = kSplit == kSplitWorkspace || kSplit == kSplitCluster ? static_cast<int>(gridDim.z) : 1;
+  // The table and the query rows are asked for at once, so that the first K tile is two trips to L2 away.
+  int seg[6];
+  const int nseg = request_table(a, seg);
+  uint4 q_pre[4];
+  float4 xy_pre[4];
+  if (kSplit != kHelped && warp >= 4) load_q(a, q0 + (warp & 3) * 32 + lane, qh, (warp - 4) >> 2, q_pre, xy_pre);
+  int n_tiles = load_table(a, nseg, seg);
   int tile0 = 0;
   KeyShares kr;
   Piece pc;
@@ -451,472 +272,377 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     kr = KeyShares(a, n_tiles, kHelperCost);
     pc = kr.first();
     pc.place(a, q0, qh, kvh);
+    tile0 = pc.tile0;
+    n_tiles = kr.all_tiles();
+    if (warp >= 4 && pc.n > 0) load_q(a, q0 + (warp & 3) * 32 + lane, qh, (warp - 4) >> 2, q_pre, xy_pre);
   }
+  // key splits: this CTA's share of the tiles
+  const int n_splits = kSplit == kSplitWorkspace || kSplit == kSplitCluster ? static_cast<int>(gridDim.z) : 1;
   if (kSplit == kSplitWorkspace || kSplit == kSplitCluster) {
     tile0 = static_cast<int>(blockIdx.z) * n_tiles / n_splits;
     n_tiles = static_cast<int>(blockIdx.z + 1) * n_tiles / n_splits - tile0;
   }
+  // every segment a multiple of the tile (720p: 512 keys a bucket): no tile needs a mask, so none is looked up
+  const bool whole = ((seg[1] | seg[3] | seg[5]) & (kKeyTile - 1)) == 0;
 
-  // The softmax threads ask for their half of the query row (and group 0 for the row of the RoPE table) now, so that the
-  // loads travel while the frame counter's sines and cosines are worked out and the CTA meets at the barrier below
-  // (46.5 -> 46.3 us at 720p).
-  uint4 q_pre[4];
-  float4 xy_pre[4];
-  if (warp >= 4) load_q(a, q0 + (warp & 3) * 32 + lane, qh, (warp - 4) >> 2, q_pre, xy_pre);
-  if (threadIdx.x >= 96 && threadIdx.x < 104) temporal_cos_sin(*after_wait(a.frame_t), threadIdx.x - 96, tm);
-  __syncthreads();
-
-
-  // Registers move from the four control warps to the softmax warps, which hold a whole score row each.
   if (warp < 4) {
-  setmaxnreg_dec<kCtrlRegs>();
-  if (warp == 0) {
-    // ---------------- TMA producer
-    if (elect_one()) {
-      int issued = 0;
-      int tile = tile0;  // within the item
-      if (kSplit == kHelped) {
-        n_tiles = kr.all_tiles();
-        tile = pc.tile0;
-      }
-      for (int j = 0; j < n_tiles; ++j, ++tile) {
-        if (kSplit == kHelped && tile == pc.tile0 + pc.n) {  // on to the next item
-          kr.next(pc);
-          tile = pc.tile0;
-          pc.place(a, q0, qh, kvh);
-        }
-        const int s = j % kStages;
-        const uint32_t ph = (j / kStages) & 1;
-        if (!mbar_wait(smem_u32(&kv_empty[s]), ph ^ 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN)) break;
-        int row, valid;
-        locate_tile(seg, tile, row, valid);
-        const uint32_t fb = smem_u32(&kv_full[s]);
-        mbar_arrive_expect_tx(fb, L::kKBytes + (kFp8 ? 1 : 2) * 64 * 128);
-        uint8_t* st = smem + L::kStageOff + s * L::kStageBytes;
-        tma_load_2d(smem_u32(st), &tmK, fb, 0, kvh * a.capacity + row);
-        tma_load_2d(smem_u32(st + L::kKBytes), &tmV, fb, row, kvh * 64);
-        if (!kFp8) tma_load_2d(smem_u32(st + L::kKBytes + L::kVTile), &tmV, fb, row + 64, kvh * 64);
-        issued = j + 1;
-      }
-      if (*abort_flag) {
-        // Giving up: let the copies already in flight land before this CTA's memory goes away.
-        for (int j = max(0, issued - kStages); j < issued; ++j)
-          mbar_wait(smem_u32(&kv_full[j % kStages]), (j / kStages) & 1, drain_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
-      } else {
-        // Tail: see the last stage releases land before the CTA can exit.
-        for (int j = max(0, n_tiles - kStages); j < n_tiles; ++j)
-          if (!mbar_wait(smem_u32(&kv_empty[j % kStages]), (j / kStages) & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN)) break;
-      }
-    }
-  } else if (warp == 1 || warp == 2) {
-    // ---------------- MMA issuers: warp 1 serves softmax group 0 (even tiles), warp 2 group 1 (odd tiles).
-    // Per group: S(i) goes to the group's S columns as soon as the group has copied S(i - 1) into its
-    // registers; once the group has written P(i) (and rescaled O if a row maximum jumped), O += P(i) V(i)
-    // accumulates in the group's O columns.  S(i + 1) is issued ahead of PV(i).
-    const int g = warp - 1;
-    // A piece of work is a run of tiles of one item: all that this CTA has, or (kHelped) one after the other.  Tiles are counted
-    // over the pieces, so stages, barrier phases and the turns of the two groups run on; only O starts anew.
-    int i0 = 0, i1 = n_tiles > g ? (n_tiles - g + 1) / 2 : 0;  // the group's tiles of the piece
-    if (kSplit == kHelped) i1 = group_tiles(pc.n, g);
-    if (elect_one()) {
-      const uint32_t q_addr = smem_u32(q_s);
-      const uint32_t p_base = smem_u32(smem + L::kPOff + g * L::kPBufs * L::kPBytes);
-      const uint32_t tmem_sg = tmem_base + g * kGroupCols;
-      const uint32_t tmem_og = tmem_sg + kOCol;
-      auto stage_addr = [&](int j) { return smem_u32(smem + L::kStageOff + (j % kStages) * L::kStageBytes); };
-      auto issue_s = [&](int i) {
-        const uint32_t k_addr = stage_addr(2 * i + g);
-        if (kFp8) {
-          const uint64_t qd = umma_desc_k_sw64(q_addr), kd = umma_desc_k_sw64(k_addr);
+    setmaxnreg_dec<kCtrlRegs>();
+    if (warp == 3) {
+      if (lane < 8) temporal_cos_sin(*after_wait(a.frame_t), lane, bars->tm);
+      if (lane == 8) {
 #pragma unroll
-          for (int k = 0; k < 2; ++k) umma_f8(tmem_sg, qd + 2 * k, kd + 2 * k, kIdescS, k > 0);
+        for (int i = 0; i < 6; ++i) bars->seg[i] = seg[i];
+        bars->tiles = kr.tiles;
+        bars->tile_shift = tile0;
+      }
+      __syncwarp();
+      asm volatile("bar.arrive 4, 160;" ::: "memory");  // group 1 waits for it
+    } else if (warp == 0) {
+      // ---------------- TMA producer: K(t), then V(t - 2), in the order in which they are used
+      if (elect_one()) {
+        int tile = tile0;  // within the item
+        int row[3] = {0, 0, 0}, head[3] = {0, 0, 0};  // of tiles t, t - 1, t - 2
+        int k_issued = 0, v_issued = 0;
+        for (int t = 0; t < n_tiles + 2; ++t) {
+          if (t < n_tiles) {
+            if (kSplit == kHelped && tile == pc.tile0 + pc.n) {  // on to the next item
+              kr.next(pc);
+              tile = pc.tile0;
+              pc.place(a, q0, qh, kvh);
+            }
+            int valid;
+            locate_tile(seg, tile, row[0], valid);
+            head[0] = kvh;
+            ++tile;
+            const int s = t % kKS;
+            if (!wait(bars->k_empty[s], ((t / kKS) & 1) ^ 1)) break;
+            const uint32_t fb = smem_u32(&bars->k_full[s]);
+            mbar_arrive_expect_tx(fb, L::kKBytes);
+            tma_load_2d(smem_u32(smem + L::kKOff + s * L::kKBytes), &tmK, fb, 0, kvh * a.capacity + row[0]);
+            k_issued = t + 1;
+          }
+          if (t >= 2) {
+            const int v = t - 2, s = v % kVS;
+            if (!wait(bars->v_empty[s], ((v / kVS) & 1) ^ 1)) break;
+            const uint32_t fb = smem_u32(&bars->v_full[s]);
+            mbar_arrive_expect_tx(fb, L::kEs * 64 * 128);
+            uint8_t* st = smem + L::kVOff + s * L::kVBytes;
+            tma_load_2d(smem_u32(st), &tmV, fb, row[2], head[2] * 64);
+            if (!kFp8) tma_load_2d(smem_u32(st + L::kVTile), &tmV, fb, row[2] + 64, head[2] * 64);
+            v_issued = v + 1;
+          }
+          row[2] = row[1]; row[1] = row[0];
+          head[2] = head[1]; head[1] = head[0];
+        }
+        if (*abort_flag) {
+          // Giving up: let the copies already in flight land before this CTA's memory goes away.
+          for (int j = max(0, k_issued - kKS); j < k_issued; ++j)
+            mbar_wait(smem_u32(&bars->k_full[j % kKS]), (j / kKS) & 1, drain_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
+          for (int j = max(0, v_issued - kVS); j < v_issued; ++j)
+            mbar_wait(smem_u32(&bars->v_full[j % kVS]), (j / kVS) & 1, drain_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
         } else {
-          const uint64_t qd = umma_desc_k_sw128(q_addr), kd = umma_desc_k_sw128(k_addr);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f16(tmem_sg, qd + 2 * k, kd + 2 * k, kIdescS, k > 0);
-        }
-        umma_commit(smem_u32(&s_full[g]));
-      };
-      auto wait_tile = [&](int j) {
-        return mbar_wait(smem_u32(&kv_full[j % kStages]), (j / kStages) & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
-      };
-      bool ok = true;
-      int end = pc.n;  // tiles of the CTA up to the end of the piece
-      for (int piece = 0; ok && (kSplit == kHelped ? pc.n > 0 : piece == 0); ++piece) {
-      if (kSplit == kHelped || i0 < i1) ok = mbar_wait(smem_u32(q_ready), piece & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
-      if (i0 < i1) {
-        ok = ok && wait_tile(2 * i0 + g);
-        if (ok) {
-          tc_fence_after();
-          issue_s(i0);
+          // Tail: see the last stage releases land before the CTA can exit.
+          for (int j = max(0, n_tiles - kKS); j < n_tiles; ++j)
+            if (!wait(bars->k_empty[j % kKS], (j / kKS) & 1)) break;
+          for (int j = max(0, n_tiles - kVS); j < n_tiles; ++j)
+            if (!wait(bars->v_empty[j % kVS], (j / kVS) & 1)) break;
         }
       }
-      for (int i = i0; i < i1 && ok; ++i) {
-        QB_TR(2 + g, i, 0);
-        if (i + 1 < i1) {
-          ok = wait_tile(2 * (i + 1) + g);
-          QB_TR(2 + g, i, 1);
-          ok = ok && mbar_wait(smem_u32(&s_free[g]), i & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
-          if (!ok) break;
-          QB_TR(2 + g, i, 2);
+    } else {
+      // ---------------- MMA issuers: warp 1 serves softmax group 0 (even tiles), warp 2 group 1 (odd tiles).
+      // Per group: S(i + 1) goes to the group's S columns as soon as the group has copied S(i) into its registers; once the group has
+      // written P(i), O += P(i) V(i) accumulates in the group's O columns.
+      const int g = warp - 1;
+      // A piece of work is a run of tiles of one item: all that this CTA has, or (kHelped) one after the other.  Tiles are counted
+      // over the pieces, so stages and barrier phases run on; only O starts anew.
+      if (elect_one()) {
+        const uint32_t q_addr = smem_u32(smem + L::kQOff), k0_addr = smem_u32(smem + L::kKOff), v0_addr = smem_u32(smem + L::kVOff);
+        const uint32_t tmem_sg = tmem_base + g * kGroupCols, tmem_og = tmem_sg + kOCol, tmem_pg = tmem_sg + kPCol;
+        bool ok = true;
+        auto issue_s = [&](int i) {
+          const int j = 2 * i + g, s = j % kKS;
+          if (!wait(bars->k_full[s], (j / kKS) & 1)) return false;
+          if (i > 0 && !wait(bars->s_free[g], (i - 1) & 1)) return false;
           tc_fence_after();
-          issue_s(i + 1);
-        }
-        QB_TR(2 + g, i, 3);
-        ok = mbar_wait(smem_u32(&p_full[2 * g + (i & 1)]), (i >> 1) & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN);
-        if (!ok) break;
-        QB_TR(2 + g, i, 4);
-        tc_fence_after();
-        const uint32_t v_addr = stage_addr(2 * i + g) + L::kKBytes;
-        const uint32_t p_addr = p_base + (i % L::kPBufs) * L::kPBytes;
-        if (kFp8) {
-          const uint64_t pd = umma_desc_k_sw128(p_addr), vd = umma_desc_k_sw128(v_addr);
+          const uint32_t k_addr = k0_addr + s * L::kKBytes;
+          if (kFp8) {
+            const uint64_t qd = umma_desc_k_sw64(q_addr), kd = umma_desc_k_sw64(k_addr);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f8(tmem_og, pd + 2 * k, vd + 2 * k, kIdescPV, i > i0 || k > 0);
-        } else {
+            for (int k = 0; k < 2; ++k) umma_f8(tmem_sg, qd + 2 * k, kd + 2 * k, kIdescS, k > 0);
+          } else {
+            const uint64_t qd = umma_desc_k_sw128(q_addr), kd = umma_desc_k_sw128(k_addr);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const uint64_t pd = umma_desc_k_sw128(p_addr + (k >> 2) * (L::kPBytes / 2));
-            const uint64_t vd = umma_desc_k_sw128(v_addr + (k >> 2) * L::kVTile);
-            umma_f16(tmem_og, pd + 2 * (k & 3), vd + 2 * (k & 3), kIdescPV, i > i0 || k > 0);
+            for (int k = 0; k < 4; ++k) umma_f16(tmem_sg, qd + 2 * k, kd + 2 * k, kIdescS, k > 0);
+          }
+          umma_commit(smem_u32(&bars->s_full[g]));
+          umma_commit(smem_u32(&bars->k_empty[s]));
+          return true;
+        };
+        int i0 = 0, end = kSplit == kHelped ? pc.n : n_tiles, i1 = group_tiles(end, g);  // the group's tiles of the piece
+        for (int piece = 0; ok && (kSplit == kHelped ? pc.n > 0 : piece == 0); ++piece) {
+          if (kSplit == kHelped || i0 < i1) ok = wait(bars->q_ready, piece & 1);
+          if (i0 < i1) ok = ok && issue_s(i0);
+          for (int i = i0; i < i1 && ok; ++i) {
+            if (i + 1 < i1) ok = issue_s(i + 1);
+            const int j = 2 * i + g, s = j % kVS;
+            ok = ok && wait(bars->v_full[s], (j / kVS) & 1) && wait(bars->p_full[g], i & 1);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t vd = umma_desc_k_sw128(v0_addr + s * L::kVBytes);
+            if (kFp8) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) umma_f8_ts(tmem_og, tmem_pg + 8 * k, vd + 2 * k, kIdescPV, i > i0 || k > 0);
+            } else {
+              const uint64_t vd1 = umma_desc_k_sw128(v0_addr + s * L::kVBytes + L::kVTile);
+#pragma unroll
+              for (int k = 0; k < 8; ++k) umma_f16_ts(tmem_og, tmem_pg + 8 * k, (k < 4 ? vd : vd1) + 2 * (k & 3), kIdescPV, i > i0 || k > 0);
+            }
+            umma_commit(smem_u32(&bars->pv_done[g]));
+            umma_commit(smem_u32(&bars->v_empty[s]));
+          }
+          if (ok && late(g == 0 && blockIdx.x == gridDim.x - 1 && blockIdx.z == gridDim.z - 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN)) ok = false;
+          // pv_done flips once per tile, so its parity cannot tell "all finished" from "two still in flight"; the end of the
+          // accumulation has a barrier of its own
+          if (ok && (kSplit == kHelped || i0 < i1)) umma_commit(smem_u32(&bars->o_final[g]));
+          if (kSplit == kHelped) {
+            kr.next(pc);
+            i0 = i1;
+            end += pc.n;
+            i1 = group_tiles(end, g);
           }
         }
-        umma_commit(smem_u32(&pv_done[g]));
-        umma_commit(smem_u32(&kv_empty[(2 * i + g) % kStages]));
-        QB_TR(2 + g, i, 5);
-      }
-      if (ok && late(g == 0 && blockIdx.x == gridDim.x - 1 && blockIdx.z == gridDim.z - 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN)) ok = false;
-      // pv_done flips once per tile and the fp8 softmax warps rarely look at it, so its parity cannot tell
-      // "all finished" from "two still in flight"; the end of the accumulation has a barrier of its own
-      if (ok && (kSplit == kHelped || i0 < i1)) umma_commit(smem_u32(&o_final[g]));
-      if (kSplit == kHelped) {
-        kr.next(pc);
-        i0 = i1;
-        end += pc.n;
-        i1 = group_tiles(end, g);
-      }
       }
     }
-  }
   } else {
     setmaxnreg_inc<kSoftmaxRegs>();
     // ---------------- softmax groups: one query row per thread, group g takes tiles j = 2 i + g
     const int g = (warp - 4) >> 2;
-    const int lane_grp = warp & 3;
-    const int r = lane_grp * 32 + lane;
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;
     const int t = q0 + r;
     const bool row_ok = t < a.tpf;
-    const uint32_t lane_addr = static_cast<uint32_t>(lane_grp * 32) << 16;
-    uint8_t* p_g = smem + L::kPOff + g * L::kPBufs * L::kPBytes;
+    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t tmem_s = tmem_base + g * kGroupCols + lane_addr;  // this thread's row of the group's S,
+    const uint32_t tmem_o = tmem_s + kOCol, tmem_p = tmem_s + kPCol;  // ... of its O and of its P
 
-    stage_q<kFp8>(smem, q_ready, r, g, row_ok, q_pre, xy_pre, lane);
-    if (warp == 4) QB_TR(4, 0, 2);
-    const uint32_t tmem_s = tmem_base + g * kGroupCols + lane_addr;  // this thread's row of the group's S
-    const uint32_t tmem_o = tmem_s + kOCol;                          // ... and of its O accumulator
-    bool ok = true;
-    // every segment a multiple of the tile (720p: 512 keys a bucket): no tile needs a mask, so none is looked up
-    const bool whole = ((seg[1] | seg[3] | seg[5]) & (kKeyTile - 1)) == 0;
-    int i0 = 0, i1 = n_tiles > g ? (n_tiles - g + 1) / 2 : 0;  // the group's tiles of the piece, as the MMA warp counts them
-    if (kSplit == kHelped) i1 = group_tiles(pc.n, g);
-    // What the end of a piece needs is worked out there from its item's number, so that it takes no registers in the loop.
-    int item = pc.item;
-    if (kSplit == kHelped) tile0 = pc.tile0;
+    if (g == 1) asm volatile("bar.sync 4, 160;" ::: "memory");  // the temporal angles
+    stage_q<kFp8>(smem + L::kQOff, bars->tm, &bars->q_ready, r, g, row_ok, q_pre, xy_pre, lane);
+    int i0 = 0, i1 = group_tiles(kSplit == kHelped ? pc.n : n_tiles, g);  // the group's tiles of the piece, as the MMA warp counts them
+    // What the end of a piece needs is worked out there from its number, so that it takes no registers in the loop.
+    int end = pc.n;
     bool more = kSplit != kHelped || pc.n > 0;
 
     for (int piece = 0; more; ++piece) {
-    const float ks = a.k_scale ? __ldg(a.k_scale + kvh) : 1.0f;
-    const float sl2 = ks * 0.125f * 1.4426950408889634f;  // scores -> log2 domain, 1/sqrt(64) folded in
-    float m_run = -1.0e30f;
-    for (int i = i0; i < i1 && ok; ++i) {
-      if (lane_grp == 0) QB_TR(g, i, 0);
-      int row, valid = kKeyTile;
-      if (!whole) locate_tile(seg, tile0 + 2 * i + g, row, valid);
-      if (lane_grp == 0) QB_TR(g, i, 1);
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[g]), i & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
-      if (!ok) break;
-      tc_fence_after();
-      if (lane_grp == 0) QB_TR(g, i, 2);
-      // the whole score row into registers; the S columns are then free for the next tile
-      uint32_t sc[4][32];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(tmem_s + c * 32, sc[c]);
-      // the wait names the loaded registers, so that nothing the compiler does with them (a move, a spill)
-      // can be placed between a load and the wait, where they do not hold the scores yet
-      tmem_wait_ld_into(sc[0]);
-      tmem_loaded(sc[1]);
-      tmem_loaded(sc[2]);
-      tmem_loaded(sc[3]);
-      if (lane_grp == 0) QB_TR(g, i, 3);
-      tc_fence_before();
-      warp_arrive(smem_u32(&s_free[g]), lane);
-      if (valid != kKeyTile) {  // last tile of a segment whose length is not a multiple of 128
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int q = 0; q < 32; ++q)
-            if (c * 32 + q >= valid) sc[c][q] = 0xff800000u;  // -inf
+      if (kSplit == kHelped && piece > 0) {
+        const KeyShares again(a, *const_cast<volatile int*>(&bars->tiles), kHelperCost);
+        again.at(again.first_item + piece).place(a, q0, qh, kvh);
       }
-      float mx[4];
+      const float ks = a.k_scale ? __ldg(a.k_scale + kvh) : 1.0f;
+      const float sl2 = ks * 0.125f * 1.4426950408889634f;  // scores -> log2 domain, 1/sqrt(64) folded in
+      const uint64_t sl2_2 = pack_f32x2(sl2, sl2);
+      float m_run = -1.0e30f, l_run = 0.f;  // bf16: the row sum, of the rounded probabilities
+      for (int i = i0; i < i1; ++i) {
+        wait_warp(bars->s_full[g], i & 1);
+        tc_fence_after();
+        int row, valid = kKeyTile;
+        if (!whole) locate_tile(bars->seg, 2 * i + g + bars->tile_shift, row, valid);  // (the table is there: Q was staged after it)
+        // the whole score row into registers; the S columns are then free for the next tile
+        uint32_t sc[kKeyTile / 32][32];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float m0 = __uint_as_float(sc[c][0]), m1 = __uint_as_float(sc[c][1]);
+        for (int c = 0; c < kKeyTile / 32; ++c) tmem_ld32(tmem_s + c * 32, sc[c]);
+        // the wait names the loaded registers, so that nothing the compiler does with them (a move, a spill)
+        // can be placed between a load and the wait, where they do not hold the scores yet
+        tmem_wait_ld_into(sc[0]);
 #pragma unroll
-        for (int q = 0; q < 15; ++q) {  // two chains of 3-input max
-          if (q & 1) m1 = max3f(m1, __uint_as_float(sc[c][2 + 2 * q]), __uint_as_float(sc[c][3 + 2 * q]));
-          else m0 = max3f(m0, __uint_as_float(sc[c][2 + 2 * q]), __uint_as_float(sc[c][3 + 2 * q]));
+        for (int c = 1; c < kKeyTile / 32; ++c) tmem_loaded(sc[c]);
+        tc_fence_before();
+        warp_arrive(smem_u32(&bars->s_free[g]), lane);
+        if (valid != kKeyTile) {  // last tile of a segment whose length is not a multiple of the tile
+#pragma unroll
+          for (int c = 0; c < kKeyTile / 32; ++c) mask_chunk(sc[c], c, valid);
         }
-        mx[c] = fmaxf(m0, m1);
-      }
-      const float m_tile = max3f(max3f(mx[0], mx[1], mx[2]), mx[3], -1.0e30f) * sl2;
-      if (lane_grp == 0) QB_TR(g, i, 4);
-      if (i == i0) {
-        m_run = m_tile;
-      } else {
-        const bool jump = m_tile > m_run + kSlack;
-        const bool any_jump = __any_sync(0xffffffffu, jump);
-        // O may be rescaled only when PV(i - 1) has finished.  The P tile written below was last read
-        // by PV(i - 1) when the group has one P tile; with two it was PV(i - 2), which finished before
-        // S(i) did (the MMA warp issued it earlier, and s_full covers everything issued before it).
-        if (L::kPBufs == 1 || any_jump) {
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&pv_done[g]), (i - 1) & 1, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
-          if (!ok) break;
-        }
-        if (any_jump) {
-          const float alpha = jump ? ex2_approx(m_run - m_tile) : 1.0f;
+        float mx[4] = {-1.0e30f, -1.0e30f, -1.0e30f, -1.0e30f};
+#pragma unroll
+        for (int q = 0; q < kKeyTile / 2; ++q) mx[q & 3] = max3f(mx[q & 3], __uint_as_float(sc[q >> 4][2 * (q & 15)]), __uint_as_float(sc[q >> 4][2 * (q & 15) + 1]));
+        const float m_tile = fmaxf(max3f(mx[0], mx[1], mx[2]), mx[3]) * sl2;
+        if (i == i0) {
+          m_run = m_tile;
+        } else if (const bool jump = m_tile > m_run + kSlack; __any_sync(0xffffffffu, jump)) {
+          wait_warp(bars->pv_done[g], (i - 1) & 1);  // O may be rescaled only when PV(i - 1) has finished
+          const float before = m_run;
           if (jump) m_run = m_tile;
+          const float alpha = ex2_approx(before - m_run);
           tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < 2; ++c) {
-            uint32_t oo[32];
-            tmem_ld32(tmem_o + c * 32, oo);
+          for (int c = 0; c < 4; ++c) {
+            uint32_t oo[16];
+            tmem_ld16(tmem_o + c * 16, oo);
             tmem_wait_ld_into(oo);
 #pragma unroll
-            for (int q = 0; q < 32; ++q) oo[q] = __float_as_uint(__uint_as_float(oo[q]) * alpha);
-            tmem_st32(tmem_o + c * 32, oo);
+            for (int q = 0; q < 16; ++q) oo[q] = __float_as_uint(__uint_as_float(oo[q]) * alpha);
+            tmem_st16(tmem_o + c * 16, oo);
           }
-          uint32_t lsum = tmem_ld1(tmem_o + 64);
-          tmem_wait_ld();
-          tmem_loaded(lsum);
-          tmem_st1(tmem_o + 64, __float_as_uint(__uint_as_float(lsum) * alpha));
+          if (kFp8) {
+            uint32_t lsum = tmem_ld1(tmem_o + 64);
+            tmem_wait_ld();
+            tmem_loaded(lsum);
+            tmem_st1(tmem_o + 64, __float_as_uint(__uint_as_float(lsum) * alpha));
+          } else {
+            l_run *= alpha;
+          }
           tmem_wait_st();
         }
-      }
-      const float nshift = kPShift - m_run;
-      if (lane_grp == 0) QB_TR(g, i, 5);
-      // The two groups take turns on the exponentials (the special-function unit is the scarcest
-      // resource of this kernel): order G0(0) G1(0) G0(1) G1(1) ...  While one group runs its
-      // exponentials the other loads its next score row, finds the maximum and talks to the MMA warps.
-      if (g == 0 ? i > 0 : true) {
-        const uint32_t par = g == 0 ? (i - 1) & 1 : i & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&turn[g]), par, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
-        if (!ok) break;
-      }
-      if (lane_grp == 0) QB_TR(g, i, 6);
-      uint8_t* p_s = p_g + (i % L::kPBufs) * L::kPBytes;
+        const float nshift = kPShift - m_run;
+        const uint64_t nshift_2 = pack_f32x2(nshift, kLin ? nshift + kLinMagic : nshift);
+        uint32_t pw[kFp8 ? 1 : 2][32];
+        uint64_t sum[2] = {0, 0};
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        // handed over before the last chunks: the other group needs a while to wake up, and two warps
-        // per scheduler keep the special-function unit busier than one
-        if (c == (kLin ? 0 : kHandoffChunk) && lane == 0) mbar_arrive(smem_u32(&turn[1 - g]));
-        p_chunk<kFp8, kPolyOf8, kLin>(sc[c], c, sl2, nshift, p_s, r);
-      }
-      fence_proxy_async_smem();
-      tc_fence_before();
-      warp_arrive(smem_u32(&p_full[2 * g + (i & 1)]), lane);
-      if (lane_grp == 0) QB_TR(g, i, 7);
-    }
-    if (warp == 4) QB_TR(4, 0, 3);
-    if constexpr (kSplit == kHelped) {
-      const NextPiece next = end_piece<kFp8>(a, smem, q_ready, tmem_o, smem_u32(&o_final[g]), kr.tiles, item, piece, i0 < i1, ok, m_run);
-      item = next.item;
-      kvh = next.kvh;
-      tile0 = next.tile0 + next.n - next.done;
-      i0 = i1;
-      i1 = group_tiles(next.done, g);
-      more = next.n > 0;
-      continue;
-    }
-    more = kSplit == kHelped;
-    // the group's result: 64 outputs and the row sum, still scaled by 2^(kPShift - m_run)
-    float o[64];
-    float l_run = 0.f;
+        for (int c = 0; c < kKeyTile / 32; ++c) p_chunk<kFp8, kLin>(sc[c], sl2_2, nshift_2, kFp8 ? pw[0] + c * 8 : pw[c >> 1] + (c & 1) * 16, sum);
+        if (!kFp8) l_run += sum_f32x2(sum[0], sum[1]);
+        if (!kFp8 && valid != kKeyTile) {  // the polynomial makes 2^-126 of -inf: a masked key counts exactly nothing
 #pragma unroll
-    for (int d = 0; d < 64; ++d) o[d] = 0.f;
-    if (ok && i0 < i1) {
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&o_final[g]), 0, abort_flag, a.status, QB_DEV_WAIT_TIMEOUT_ATTN));
-      if (ok) {
-        tc_fence_after();
-        uint32_t oo[2][32];
-        tmem_ld32(tmem_o, oo[0]);
-        tmem_ld32(tmem_o + 32, oo[1]);
-        uint32_t lsum = tmem_ld1(tmem_o + 64);
-        tmem_wait_ld_into(oo[0]);
-        tmem_loaded(oo[1]);
-        tmem_loaded(lsum);
-#pragma unroll
-        for (int d = 0; d < 64; ++d) o[d] = __uint_as_float(oo[d >> 5][d & 31]);
-        l_run = __uint_as_float(lsum);
+          for (int w = 0; w < 64; ++w)
+            if (2 * w + 1 >= valid) pw[kFp8 ? 0 : w >> 5][w & 31] &= 2 * w >= valid ? 0u : 0xFFFFu;
+        }
+        if (i > 0) wait_warp(bars->pv_done[g], (i - 1) & 1);  // PV(i - 1) has read the P before: long ago, as a rule
+        tmem_st32(tmem_p, pw[0]);
+        if constexpr (!kFp8) tmem_st32(tmem_p + 32, pw[1]);
+        tmem_wait_st();
+        tc_fence_before();
+        warp_arrive(smem_u32(&bars->p_full[g]), lane);
       }
-    }
+      if constexpr (kSplit == kHelped) {
+        const int n = end_piece(a, smem, tmem_o, piece, i0 < i1, m_run);
+        end += n;
+        i0 = i1;
+        i1 = group_tiles(end, g);
+        more = n > 0;
+        continue;
+      }
+      more = kSplit == kHelped;
 
-    if (warp == 4) QB_TR(4, 0, 4);
-    if constexpr (kSplit == kSplitCluster) {
-      // Both groups of every CTA of the cluster hand their rows to the CTA that writes them (against the merge of the groups and
-      // the trip through the workspace, 360p, 4 CTAs: e4m3 13.4 -> 12.1 us, bf16 16.0 -> 13.9 us).
-      const int S = static_cast<int>(gridDim.z), rows = merge_rows(S);
-      float* area = reinterpret_cast<float*>(smem + L::kStageOff);
-      cluster_sync();  // the stages of every CTA are free (its tensor work and TMA traffic are finished)
-      // Nobody waits any more, so the flag now tells whether one of this CTA's waits ran out; if so, the rows that its results belong
-      // to are not written by any CTA of the cluster.
-      if (*abort_flag != 0 && threadIdx.x - 128 < S) st_dsmem(map_to_cta(smem_u32(const_cast<const int*>(abort_flag)), threadIdx.x - 128), 1);
-      {
-        const uint32_t base = map_to_cta(smem_u32(area), r / rows);
-        const int part = 2 * static_cast<int>(blockIdx.z) + g, rl = r % rows;
-        const uint32_t row_at = base + static_cast<uint32_t>((part * rows + rl) * kMergePitch) * 4u;
+      float o[64];
 #pragma unroll
-        for (int d = 0; d < 64; d += 4)
-          st_dsmem_v4(row_at + d * 4u, __float_as_uint(o[d]), __float_as_uint(o[d + 1]), __float_as_uint(o[d + 2]), __float_as_uint(o[d + 3]));
-        st_dsmem_v4(row_at + 256u, __float_as_uint(m_run), __float_as_uint(l_run), 0u, 0u);
+      for (int d = 0; d < 64; ++d) o[d] = 0.f;
+      if (i0 < i1) {
+        wait_warp(bars->o_final[g], 0);
+        tc_fence_after();
+        read_o<kFp8>(tmem_o, o, l_run);
       }
-      cluster_sync();
-      const float vs = a.v_scale ? __ldg(a.v_scale + kvh) : 1.0f;
-      const bool whole_cluster = *abort_flag == 0;
-      for (int i = threadIdx.x - 128; whole_cluster && i < rows * 8; i += 256) {  // 8 outputs of a row per thread
-        const int rl = i >> 3, d0 = (i & 7) * 8, rr = static_cast<int>(blockIdx.z) * rows + rl;
-        if (rr >= kQTile || q0 + rr >= a.tpf) continue;
-        float m = -1.0e30f;
-        for (int q = 0; q < 2 * S; ++q) m = fmaxf(m, area[(q * rows + rl) * kMergePitch + 64]);
-        float l = 0.f, e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int q = 0; q < 2 * S; ++q) {
-          const float* part = area + (q * rows + rl) * kMergePitch;
-          const float w = ex2_approx(part[64] - m);
-          l = fmaf(w, part[65], l);
-          const float4 x = *reinterpret_cast<const float4*>(part + d0), y = *reinterpret_cast<const float4*>(part + d0 + 4);
-          e[0] = fmaf(w, x.x, e[0]); e[1] = fmaf(w, x.y, e[1]); e[2] = fmaf(w, x.z, e[2]); e[3] = fmaf(w, x.w, e[3]);
-          e[4] = fmaf(w, y.x, e[4]); e[5] = fmaf(w, y.y, e[5]); e[6] = fmaf(w, y.z, e[6]); e[7] = fmaf(w, y.w, e[7]);
+      if constexpr (kSplit == kSplitCluster) {
+        // Both groups of every CTA of the cluster hand their rows to the CTA that writes them (against the merge of the groups and
+        // the trip through the workspace, 360p, 4 CTAs, with an earlier form of the loop: e4m3 13.4 -> 12.1 us, bf16 16.0 -> 13.9 us).
+        const int S = static_cast<int>(gridDim.z), rows = merge_rows(S);
+        float* area = reinterpret_cast<float*>(smem + L::kClusterOff);
+        cluster_sync();  // the rings of every CTA are free (its tensor work and TMA traffic are finished)
+        // Nobody waits any more, so the flag now tells whether one of this CTA's waits ran out; if so, the rows that its results belong
+        // to are not written by any CTA of the cluster.
+        const int me = static_cast<int>(threadIdx.x) - 128;
+        if (*abort_flag != 0 && me < S) st_dsmem(map_to_cta(smem_u32(&bars->abort_flag), me), 1);
+        {
+          const uint32_t base = map_to_cta(smem_u32(area), r / rows);
+          const int part = 2 * static_cast<int>(blockIdx.z) + g, rl = r % rows;
+          const uint32_t row_at = base + static_cast<uint32_t>((part * rows + rl) * kMergePitch) * 4u;
+#pragma unroll
+          for (int d = 0; d < 64; d += 4)
+            st_dsmem_v4(row_at + d * 4u, __float_as_uint(o[d]), __float_as_uint(o[d + 1]), __float_as_uint(o[d + 2]), __float_as_uint(o[d + 3]));
+          st_dsmem_v4(row_at + 256u, __float_as_uint(m_run), __float_as_uint(l_run), 0u, 0u);
         }
-        const float inv = l > 0.f ? vs / l : 0.f;
-        const size_t at = static_cast<size_t>(q0 + rr) * a.o_row + static_cast<size_t>(qh) * a.o_head + d0;
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(e[2 * q] * inv, e[2 * q + 1] * inv);
-        *reinterpret_cast<uint4*>(a.out + at) = make_uint4(w[0], w[1], w[2], w[3]);
-        if (a.out_q != nullptr)  // narrowed from the bf16-rounded values: equals a separate bf16 -> e4m3 cast
-          *reinterpret_cast<uint2*>(a.out_q + at) = make_uint2(pack_e4m3x4(bf16lo(w[0]), bf16hi(w[0]), bf16lo(w[1]), bf16hi(w[1])),
-                                                               pack_e4m3x4(bf16lo(w[2]), bf16hi(w[2]), bf16lo(w[3]), bf16hi(w[3])));
-      }
-    } else {
-    // ---------------- merge the two groups (tensor work and TMA traffic are finished for both after the barrier)
-    asm volatile("bar.sync 2, 256;" ::: "memory");
-    if (warp == 4) QB_TR(4, 0, 5);
-    float* comb = reinterpret_cast<float*>(smem + L::kStageOff);  // [66][128]
-    if (g == 1) {
-      comb[0 * 128 + r] = m_run;
-      comb[1 * 128 + r] = l_run;
-#pragma unroll
-      for (int d = 0; d < 64; ++d) comb[(2 + d) * 128 + r] = o[d];
-    }
-    asm volatile("bar.sync 2, 256;" ::: "memory");
-    if (g == 0 && kSplit == kUnsplit) {
-      if (ok && row_ok && *abort_flag == 0) {
-        const float m1 = comb[r], l1 = comb[128 + r];
-        const float m = fmaxf(m_run, m1);
-        const float a0 = ex2_approx(m_run - m), a1 = ex2_approx(m1 - m);
-        const float l = l_run * a0 + l1 * a1;
+        cluster_sync();
         const float vs = a.v_scale ? __ldg(a.v_scale + kvh) : 1.0f;
-        const float inv = l > 0.f ? vs / l : 0.f;
-        const float s0 = a0 * inv, s1 = a1 * inv;
-        uint4* dst = reinterpret_cast<uint4*>(a.out + static_cast<size_t>(t) * a.o_row + static_cast<size_t>(qh) * a.o_head);
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          uint32_t w[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int d = 4 * v + q;
-            const float e0 = o[2 * d] * s0 + comb[(2 + 2 * d) * 128 + r] * s1;
-            const float e1 = o[2 * d + 1] * s0 + comb[(3 + 2 * d) * 128 + r] * s1;
-            w[q] = pack_bf16x2(e0, e1);
+        const bool whole_cluster = *abort_flag == 0;
+        for (int n = me; whole_cluster && n < rows * 8; n += 256) {  // 8 outputs of a row per thread
+          const int rl = n >> 3, d0 = (n & 7) * 8, rr = static_cast<int>(blockIdx.z) * rows + rl;
+          if (rr >= kQTile || q0 + rr >= a.tpf) continue;
+          float m = -1.0e30f;
+          for (int q = 0; q < 2 * S; ++q) m = fmaxf(m, area[(q * rows + rl) * kMergePitch + 64]);
+          float l = 0.f, e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          for (int q = 0; q < 2 * S; ++q) {
+            const float* part = area + (q * rows + rl) * kMergePitch;
+            const float w = ex2_approx(part[64] - m);
+            l = fmaf(w, part[65], l);
+            const float4 x = *reinterpret_cast<const float4*>(part + d0), y = *reinterpret_cast<const float4*>(part + d0 + 4);
+            e[0] = fmaf(w, x.x, e[0]); e[1] = fmaf(w, x.y, e[1]); e[2] = fmaf(w, x.z, e[2]); e[3] = fmaf(w, x.w, e[3]);
+            e[4] = fmaf(w, y.x, e[4]); e[5] = fmaf(w, y.y, e[5]); e[6] = fmaf(w, y.z, e[6]); e[7] = fmaf(w, y.w, e[7]);
           }
-          dst[v] = make_uint4(w[0], w[1], w[2], w[3]);
-          if (a.out_q != nullptr) {  // narrowed from the bf16-rounded values: equals a separate bf16 -> e4m3 cast
-            *reinterpret_cast<uint2*>(a.out_q + static_cast<size_t>(t) * a.o_row + static_cast<size_t>(qh) * a.o_head + v * 8) =
-                make_uint2(pack_e4m3x4(bf16lo(w[0]), bf16hi(w[0]), bf16lo(w[1]), bf16hi(w[1])),
-                           pack_e4m3x4(bf16lo(w[2]), bf16hi(w[2]), bf16lo(w[3]), bf16hi(w[3])));
-          }
-        }
-      }
-    } else if (kSplit == kSplitWorkspace && g == 0) {
-      // keys shared with other CTAs.  This CTA's result for the row: both groups brought to a common maximum,
-      // not yet divided by the row sum
-      const bool good = ok && *abort_flag == 0;
-      const float m1 = comb[r], l1 = comb[128 + r];
-      float m = fmaxf(m_run, m1);
-      const float a0 = ex2_approx(m_run - m), a1 = ex2_approx(m1 - m);
-      float l = l_run * a0 + l1 * a1;
-      float e[64];
+          const float inv = l > 0.f ? vs / l : 0.f;
 #pragma unroll
-      for (int d = 0; d < 64; ++d) e[d] = o[d] * a0 + comb[(2 + d) * 128 + r] * a1;
-      bool writer;  // does this CTA write the output rows?
-      {
-        const int item = qh * gridDim.x + blockIdx.x;  // (head, query tile)
-        float* mine = a.partials + (static_cast<size_t>(item) * n_splits + blockIdx.z) * (66 * 128);
-        mine[r] = m;
-        mine[128 + r] = l;
-#pragma unroll
-        for (int d = 0; d < 64; ++d) mine[(2 + d) * 128 + r] = e[d];
-        __threadfence();
-        asm volatile("bar.sync 3, 128;" ::: "memory");
-        int* last = reinterpret_cast<int*>(comb);  // the group's exchange buffer is free again
-        if (r == 0) {
-          const int was = atomicAdd(a.tickets + item, *abort_flag == 0 ? 1 : kLostTicket + 1);
-          const bool mine_is_last = (was & (kLostTicket - 1)) == n_splits - 1;
-          if (mine_is_last) a.tickets[item] = 0;  // ready for the next launch
-          *last = mine_is_last && was < kLostTicket;
+          for (int d = 0; d < 8; ++d) e[d] *= inv;
+          write_out(a, static_cast<size_t>(q0 + rr) * a.o_row + static_cast<size_t>(qh) * a.o_head + d0, e);
         }
-        asm volatile("bar.sync 3, 128;" ::: "memory");
-        writer = *last != 0;
-        if (writer) {
+      } else if constexpr (kSplit == kUnsplit) {
+        // The groups exchange halves: group g finishes outputs 32 g .. 32 g + 31 of the row.  (Tensor work and TMA traffic are finished
+        // for both behind the first barrier.)
+        float* comb = reinterpret_cast<float*>(smem + L::kCombOff);  // [group][34][128]
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        float* give = comb + g * (34 * 128) + r;
+        give[0] = m_run;
+        give[128] = l_run;
+        float h[32];
+#pragma unroll
+        for (int d = 0; d < 32; ++d) {
+          give[(2 + d) * 128] = g == 0 ? o[32 + d] : o[d];
+          h[d] = g == 0 ? o[d] : o[32 + d];
+        }
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        if (row_ok && *abort_flag == 0) {
+          const float* take = comb + (1 - g) * (34 * 128) + r;
+          const float m1 = take[0], l1 = take[128];
+          const float m = fmaxf(m_run, m1);
+          const float a0 = ex2_approx(m_run - m), a1 = ex2_approx(m1 - m);
+          const float l = __fadd_rn(__fmul_rn(l_run, a0), __fmul_rn(l1, a1));  // the same in both groups
+          const float vs = a.v_scale ? __ldg(a.v_scale + kvh) : 1.0f;
+          const float inv = l > 0.f ? vs / l : 0.f;
+          const float s0 = a0 * inv, s1 = a1 * inv;
+#pragma unroll
+          for (int d = 0; d < 32; ++d) h[d] = h[d] * s0 + take[(2 + d) * 128] * s1;
+          write_out(a, static_cast<size_t>(t) * a.o_row + static_cast<size_t>(qh) * a.o_head + g * 32, h);
+        }
+      } else if constexpr (kSplit == kSplitWorkspace) {
+        // Keys shared with other CTAs: the row's part, both groups brought to a common maximum and not yet divided by the row sum, goes
+        // to the workspace, and the CTA that draws the last ticket sums them.
+        merge_groups(reinterpret_cast<float*>(smem + L::kCombOff), g, r, m_run, l_run, o);
+        if (g == 0) {
+          const bool good = *abort_flag == 0;
+          const int it = qh * gridDim.x + blockIdx.x;  // (head, query tile)
+          float* mine = a.partials + (static_cast<size_t>(it) * n_splits + blockIdx.z) * kPartial;
+          mine[r] = m_run;
+          mine[128 + r] = l_run;
+#pragma unroll
+          for (int d = 0; d < 64; ++d) mine[(2 + d) * 128 + r] = o[d];
           __threadfence();
-          // sum the shares in order of z: the result does not depend on which CTA came last
-          const float* part = a.partials + static_cast<size_t>(item) * n_splits * (66 * 128);
-          m = -1.0e30f;
-          for (int z = 0; z < n_splits; ++z) m = fmaxf(m, __ldcg(part + z * (66 * 128) + r));
-          l = 0.f;
+          asm volatile("bar.sync 3, 128;" ::: "memory");
+          if (r == 0) {
+            const int was = atomicAdd(a.tickets + it, *abort_flag == 0 ? 1 : kLostTicket + 1);
+            const bool mine_is_last = (was & (kLostTicket - 1)) == n_splits - 1;
+            if (mine_is_last) a.tickets[it] = 0;  // ready for the next launch
+            *const_cast<volatile int*>(&bars->exchange) = mine_is_last && was < kLostTicket;
+          }
+          asm volatile("bar.sync 3, 128;" ::: "memory");
+          if (*const_cast<volatile int*>(&bars->exchange) != 0 && good && row_ok) {
+            __threadfence();
+            // sum the shares in order of z: the result does not depend on which CTA came last
+            const float* part = a.partials + static_cast<size_t>(it) * n_splits * kPartial;
+            float m = -1.0e30f;
+            for (int z = 0; z < n_splits; ++z) m = fmaxf(m, __ldcg(part + z * kPartial + r));
+            float l = 0.f;
 #pragma unroll
-          for (int d = 0; d < 64; ++d) e[d] = 0.f;
-          for (int z = 0; z < n_splits; ++z) {
-            const float* pz = part + z * (66 * 128);
-            const float w = ex2_approx(__ldcg(pz + r) - m);
-            l = fmaf(w, __ldcg(pz + 128 + r), l);
+            for (int d = 0; d < 64; ++d) o[d] = 0.f;
+            for (int z = 0; z < n_splits; ++z) {
+              const float* pz = part + z * kPartial;
+              const float w = ex2_approx(__ldcg(pz + r) - m);
+              l = fmaf(w, __ldcg(pz + 128 + r), l);
 #pragma unroll
-            for (int d = 0; d < 64; ++d) e[d] = fmaf(w, __ldcg(pz + (2 + d) * 128 + r), e[d]);
+              for (int d = 0; d < 64; ++d) o[d] = fmaf(w, __ldcg(pz + (2 + d) * 128 + r), o[d]);
+            }
+            KeyShares::write_row(a, t, qh, kvh, l, o);
           }
         }
       }
-      if (writer && good && row_ok) {
-        const float vs = a.v_scale ? __ldg(a.v_scale + kvh) : 1.0f;
-        const float inv = l > 0.f ? vs / l : 0.f;
-        uint4* dst = reinterpret_cast<uint4*>(a.out + static_cast<size_t>(t) * a.o_row + static_cast<size_t>(qh) * a.o_head);
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          uint32_t w[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(e[8 * v + 2 * q] * inv, e[8 * v + 2 * q + 1] * inv);
-          dst[v] = make_uint4(w[0], w[1], w[2], w[3]);
-          if (a.out_q != nullptr) {  // narrowed from the bf16-rounded values: equals a separate bf16 -> e4m3 cast
-            *reinterpret_cast<uint2*>(a.out_q + static_cast<size_t>(t) * a.o_row + static_cast<size_t>(qh) * a.o_head + v * 8) =
-                make_uint2(pack_e4m3x4(bf16lo(w[0]), bf16hi(w[0]), bf16lo(w[1]), bf16hi(w[1])),
-                           pack_e4m3x4(bf16lo(w[2]), bf16hi(w[2]), bf16lo(w[3]), bf16hi(w[3])));
-          }
-        }
-      }
-    }
-    }
     }
     if (kSplit == kHelped && kr.tiles == 0) KeyShares::write_zeros(a, r, g, 2);
   }
 
-  if (warp == 4) QB_TR(4, 0, 6);
   if (kSplit == kSplitCluster && warp < 4) {  // the softmax warps' two barriers
     __syncwarp();
     cluster_sync();
@@ -924,7 +650,6 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) QB_TR(4, 0, 7);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
@@ -934,21 +659,11 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
 }  // namespace qb
 
 namespace qb {
-int32_t launch_attn4(const void* K_cache, const void* Vt_cache, const AttnArgs& a, int n_kv_heads, cudaStream_t st);
-// bf16 calls with one (query tile, head) per CTA go to the three-group kernel of attn4.cu; QB_ATTN4=0 in the environment
-// when the library is loaded keeps the two-group kernel of this file for everything (e4m3 and key splits always use it).
 // e4m3 probabilities: 0 = every second exponential on the FMA pipe (ex2_lin_from_biased), 1 = all on the special-function unit
 static int g_attn_exact_exp = [] {
   const char* e = getenv("QB_ATTN_EXACT_EXP");
   return (e != nullptr && e[0] == '1') ? 1 : 0;
 }();
-static bool attn4_enabled() {
-  static const bool on = [] {
-    const char* e = getenv("QB_ATTN4");
-    return !(e != nullptr && e[0] == '0');
-  }();
-  return on;
-}
 }  // namespace qb
 
 using namespace qb;
@@ -958,12 +673,6 @@ extern "C" int32_t qb_set_attn_exact_exp(int32_t on) {
   g_attn_exact_exp = on ? 1 : 0;
   return was;
 }
-
-#ifdef QB_ATTN_TRACE
-extern "C" int32_t qb_debug_attn_trace(void* host_out) {
-  return cudaMemcpyFromSymbol(host_out, g_attn_trace, sizeof(g_attn_trace)) == cudaSuccess ? 0 : -1;
-}
-#endif
 
 // How many CTAs share the keys of one (query tile, head).  One when the grid already fills most of the GPU
 // (720p: 4 query tiles x 32 heads); otherwise as many as it takes to reach the SM count, while every
@@ -979,25 +688,14 @@ static int attn_key_splits(const qb_attn_params* p) {
   return n < 2 ? 1 : n;
 }
 
-template <typename K>
-static int32_t configure(K kernel, int smem_bytes, std::atomic<unsigned long long>& done) {  // once per device
-  int dev = 0;
-  QB_CUDA_OK(cudaGetDevice(&dev));
-  if (dev < 64 && (done.load(std::memory_order_relaxed) >> dev & 1) != 0) return QB_OK;
-  QB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-  if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_relaxed);
-  return QB_OK;
-}
-
 // Whether the CTAs that the items leave over help with their keys (owned_tiles, at the longest history; the kernel decides again for
 // the keys that are valid).
 static bool attn_helped(const qb_attn_params* p, int splits) {
-  if (p->kv_dtype != QB_E4M3 && !attn4_enabled()) return false;
   if (p->kv_splits != 0 || splits != 1) return false;
   const int tpf = p->H_spatial * p->W_spatial, sms = num_sms();
   const long long items = static_cast<long long>((tpf + kQTile - 1) / kQTile) * p->n_kv_heads * p->gqa_ratio;
   const long long tiles = (static_cast<long long>(p->num_buckets + 1) * (tpf / (p->quilt_factor > 0 ? p->quilt_factor : 1)) + kKeyTile - 1) / kKeyTile;  // at most
-  return 2 * items > sms && items < sms && tiles < (1 << 24) && owned_tiles(static_cast<int>(items), sms, static_cast<int>(tiles), p->kv_dtype == QB_E4M3 ? kHelperCost : kHelperCost4 / 2) < tiles;
+  return 2 * items > sms && items < sms && tiles < (1 << 24) && owned_tiles(static_cast<int>(items), sms, static_cast<int>(tiles), kHelperCost) < tiles;
 }
 
 static cudaLaunchConfig_t attn_config(dim3 grid, int smem_bytes, cudaStream_t st, cudaLaunchAttribute (&attr)[2]) {  // grid.z = CTAs of a cluster
@@ -1019,14 +717,13 @@ static cudaLaunchConfig_t attn_config(dim3 grid, int smem_bytes, cudaStream_t st
 
 // `splits` CTAs share the keys of each (query tile, head), as a cluster of up to 8 CTAs where the chip holds that many clusters at
 // once (B200: 15 of 8 CTAs, 33 of 4, 74 of 2); a wish for more is cut down to what it holds, a number that the caller forced goes
-// through the workspace instead.
+// through the workspace instead.  bf16 comes here for its key splits: where there are none, and with helpers, it goes to the three-group kernel.
 template <bool kFp8, bool kLin>
-static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnArgs& a, int Hq, int splits, bool forced, bool helped,
-                           cudaStream_t st) {
+static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnArgs& a, int Hq, int splits, bool forced, bool helped, cudaStream_t st) {
   constexpr int kSmem = AttnSmem<kFp8>::kTotal;
   if constexpr (kFp8) if (helped) {
     static std::atomic<unsigned long long> done{0};
-    const int32_t rc = configure(owl_attn_kernel<kFp8, kHelped, kLin>, kSmem, done);
+    const int32_t rc = configure_smem(owl_attn_kernel<kFp8, kHelped, kLin>, kSmem, done);
     if (rc != QB_OK) return rc;
     return launch_dep("owl_attn kernel", owl_attn_kernel<kFp8, kHelped, kLin>, dim3(num_sms()), dim3(kAttnThreads), kSmem, st, tmK, tmV, a);
   }
@@ -1036,7 +733,7 @@ static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const
   if (cluster > 1) {
     static std::atomic<unsigned long long> done{0};
     static std::atomic<int> held[9];  // clusters of this many CTAs that run at once (0 = not asked yet)
-    const int32_t rc = configure(owl_attn_kernel<kFp8, kSplitCluster, kLin>, kSmem, done);
+    const int32_t rc = configure_smem(owl_attn_kernel<kFp8, kSplitCluster, kLin>, kSmem, done);
     if (rc != QB_OK) return rc;
     cudaLaunchAttribute attr[2];
     while (cluster > 1) {
@@ -1062,14 +759,18 @@ static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const
   }
   if (splits > 1 && forced) {
     static std::atomic<unsigned long long> done{0};
-    const int32_t rc = configure(owl_attn_kernel<kFp8, kSplitWorkspace, kLin>, kSmem, done);
+    const int32_t rc = configure_smem(owl_attn_kernel<kFp8, kSplitWorkspace, kLin>, kSmem, done);
     if (rc != QB_OK) return rc;
     return launch_dep("owl_attn kernel", owl_attn_kernel<kFp8, kSplitWorkspace, kLin>, dim3(q_tiles, Hq, splits), dim3(kAttnThreads), kSmem, st, tmK, tmV, a);
   }
-  static std::atomic<unsigned long long> done{0};
-  const int32_t rc = configure(owl_attn_kernel<kFp8, kUnsplit, kLin>, kSmem, done);
-  if (rc != QB_OK) return rc;
-  return launch_dep("owl_attn kernel", owl_attn_kernel<kFp8, kUnsplit, kLin>, dim3(q_tiles, Hq), dim3(kAttnThreads), kSmem, st, tmK, tmV, a);
+  if constexpr (kFp8) {
+    static std::atomic<unsigned long long> done{0};
+    const int32_t rc = configure_smem(owl_attn_kernel<kFp8, kUnsplit, kLin>, kSmem, done);
+    if (rc != QB_OK) return rc;
+    return launch_dep("owl_attn kernel", owl_attn_kernel<kFp8, kUnsplit, kLin>, dim3(q_tiles, Hq), dim3(kAttnThreads), kSmem, st, tmK, tmV, a);
+  } else {
+    return launch_attn3(tmK, tmV, a, Hq, helped, st);
+  }
 }
 
 // The tickets take a fixed area at the start of the workspace (4096 (query tile, head) items; more only for a
@@ -1166,8 +867,6 @@ extern "C" int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void*
     a.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + attn_ticket_bytes(p));
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // bf16, one CTA per (query tile, head): the three-group kernel of attn4.cu (60.0 against 70.3 us at 720p)
-  if (splits == 1 && !fp8 && attn4_enabled()) return launch_attn4(K_cache, Vt_cache, a, p->n_kv_heads, st);
   const bool forced = p->kv_splits > 0;
   if (!fp8) return launch_attn<false, false>(tmK, tmV, a, Hq, splits, forced, helped, st);
   return g_attn_exact_exp ? launch_attn<true, false>(tmK, tmV, a, Hq, splits, forced, helped, st) : launch_attn<true, true>(tmK, tmV, a, Hq, splits, forced, helped, st);

@@ -1,6 +1,8 @@
-// Pieces shared by the two attention kernels (attn.cu: two softmax groups over 128-key tiles; attn4.cu: three groups
-// over 64-key chunks): the kernel arguments and a few instruction wrappers.
+// Pieces shared by the two attention kernels (attn.cu: two softmax groups, e4m3 and key splits; attn3.cu: three groups, bf16 without key
+// splits): the kernel arguments, the ways to share keys, the query tile, and a few instruction wrappers.
 #pragma once
+
+#include <atomic>
 
 #include <cuda.h>
 
@@ -41,11 +43,6 @@ constexpr int kLostTicket = 1 << 16;
 
 constexpr int kPartial = 66 * 128;  // floats of a partial result: m and row sum of 128 rows, then 64 x 128 outputs
 
-// What the softmax warps do next: `n` more tiles (0: nothing) of an item, the tile0-th first, `done` tiles into the CTA's work.
-struct NextPiece {
-  int item, n, tile0, done, kvh;
-};
-
 // A run of key tiles of one item, an item being one (query tile, head).
 struct Piece {
   int n = 0, tile0 = 0, item = 0;
@@ -61,8 +58,7 @@ struct Piece {
 // over are helpers that take the last tiles of up to `per` items each, one item after the other.  `cost` is what a piece costs a helper
 // on top of its tiles (the query tile, O, the trip of the partial result through the workspace), in tiles.  Where less than
 // the meeting of the two parts would be saved (a session's first frames, or 720p's ring of 16 buckets) the item stays whole.
-// 720p, 512 queries x 32 heads (20 helpers of up to 7 items), us per launch: 128 buckets e4m3 344 -> 319, bf16 427 -> 395; 64 buckets
-// 174 -> 169 and 221 -> 210; 96 items of 256 queries, 64 buckets 91 -> 73 and 120 -> 98.
+// 720p, 512 queries x 32 heads (20 helpers of up to 7 items), 128 buckets, e4m3: 268 us; cost 5 to 30 was tried.
 // The owners of the items that share a K / V head still walk its keys side by side, and so do the helpers, one after the other: equal
 // ranges of the row of all tiles (every CTA the end of one item and the start of the next) balance better but read each key from
 // DRAM once per query tile and head (720p, 128 buckets: 339 us against 344 unsplit).
@@ -71,7 +67,7 @@ __host__ __device__ inline int owned_tiles(int items, int sms, int tiles, int co
   const int keep = static_cast<int>((static_cast<long long>(per) * (tiles + cost) + per) / (per + 1));
   return keep + 2 * cost < tiles ? keep : tiles;
 }
-constexpr int kHelperCost = 7, kHelperCost4 = 18;  // tiles of 128 keys (attn.cu), chunks of 64 (attn4.cu); 5 to 12 and 10 to 24 were tried
+constexpr int kHelperCost = 9;
 
 struct KeyShares {
   int tiles = 0, keep = 0, items = 0, first_item = 0, last_item = 0;  // this CTA's items: [first_item, last_item)
@@ -192,6 +188,57 @@ __device__ __forceinline__ void warp_arrive(uint32_t bar, int lane) {
   __syncwarp();
   if (lane == 0) mbar_arrive(bar);
 }
+// Two multiply-adds in one instruction: x = a * s + t, s and t being pairs.
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void fma_f32x2(float& x0, float& x1, uint32_t a0, uint32_t a1, uint64_t s, uint64_t t) {
+  asm("{\n\t.reg .b64 A, D;\n\tmov.b64 A, {%2, %3};\n\tfma.rn.f32x2 D, A, %4, %5;\n\tmov.b64 {%0, %1}, D;\n\t}"
+      : "=f"(x0), "=f"(x1)
+      : "r"(a0), "r"(a1), "l"(s), "l"(t));
+}
+__device__ __forceinline__ void add_f32x2(uint64_t& acc, uint32_t a0, uint32_t a1) {
+  asm("{\n\t.reg .b64 A;\n\tmov.b64 A, {%1, %2};\n\tadd.rn.f32x2 %0, %0, A;\n\t}" : "+l"(acc) : "r"(a0), "r"(a1));
+}
+__device__ __forceinline__ float sum_f32x2(uint64_t a, uint64_t b) {
+  float a0, a1, b0, b1;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(b0), "=f"(b1) : "l"(b));
+  return (a0 + a1) + (b0 + b1);
+}
+// 2^x for two values on the FMA and integer pipes: x = n + f with n = round(x) in the low mantissa bits of x + 1.5 * 2^23, a
+// polynomial for 2^f on [-0.5, 0.5] (least squares, weighted until the relative error is level: 2.7e-6, a thousandth of what a bf16
+// probability resolves), n added to the exponent field.  x is clamped at -126: what underflows becomes 2^-126 instead of 0.
+__device__ __forceinline__ void ex2_poly_f32x2(float& x0, float& x1) {
+  x0 = fmaxf(x0, -126.0f);
+  x1 = fmaxf(x1, -126.0f);
+  const uint64_t x = pack_f32x2(x0, x1), magic = pack_f32x2(12582912.0f, 12582912.0f), nmagic = pack_f32x2(-12582912.0f, -12582912.0f),
+                 none = pack_f32x2(-1.0f, -1.0f);
+  uint64_t t, f, p;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(x), "l"(magic));
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(f) : "l"(t), "l"(nmagic));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(f) : "l"(f), "l"(none), "l"(x));
+  p = pack_f32x2(0.00957010034f, 0.00957010034f);
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.0559178591f, 0.0559178591f)));
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.240247443f, 0.240247443f)));
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.693121791f, 0.693121791f)));
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.999999285f, 0.999999285f)));
+  uint32_t t0, t1, p0, p1;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(t0), "=r"(t1) : "l"(t));
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(p0), "=r"(p1) : "l"(p));
+  x0 = __uint_as_float(p0 + (t0 << 23));
+  x1 = __uint_as_float(p1 + (t1 << 23));
+}
+// Four f32 -> four packed e4m3, joined by the conversions themselves.
+__device__ __forceinline__ uint32_t merge_e4m3x4(float a, float b, float c, float d) {
+  uint32_t r;
+  asm("{\n\t.reg .b16 l, h;\n\tcvt.rn.satfinite.e4m3x2.f32 l, %2, %1;\n\tcvt.rn.satfinite.e4m3x2.f32 h, %4, %3;\n\tmov.b32 %0, {l, h};\n\t}"
+      : "=r"(r)
+      : "f"(a), "f"(b), "f"(c), "f"(d));
+  return r;
+}
 __device__ __forceinline__ float max3f(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -215,11 +262,8 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw64(uint32_t smem_addr) {
 // that its mean error over the fraction is near zero (-5.2 % .. +2.3 %; an e4m3 code is 6.25 % wide; in a simulation of
 // 8192-key rows the output's 1 - cosine against exact arithmetic goes from 3.6e-4 to 4.3e-4 at worst).  x is clamped at -120 (the result then
 // narrows to zero).  Every second probability of a row is built this way in the kLin instantiations of the e4m3 kernel
-// (the default; qb_set_attn_exact_exp(1) or QB_ATTN_EXACT_EXP=1 selects the instantiations that use the special-function
-// unit for every element): the exponentials no longer queue behind one another there, at the same number of
-// instructions issued.  Measured at 720p, 8320 keys, us per launch: 52.0 exact; 49.5 with the turn passing at chunk 2 as
-// in the exact kernel; 46.5 with the turn passing before chunk 0 (the groups then overlap almost fully, which the exact
-// kernel cannot afford: 62.6); 47.9 without turns; 3 / 5 of every 8 elements instead of 4: 51.6 / 47.2; all: 56.0.
+// (the default; qb_set_attn_exact_exp(1) or QB_ATTN_EXACT_EXP=1 selects the instantiations without it): the exponentials no longer queue
+// behind one another at the special-function unit.  Measured at 720p, 8320 keys, us per launch: 41.8 against 51.6 without.
 constexpr float kLinMagic = 49152.0f;  // 1.5 * 2^15: floats in [2^15, 2^16) have an ulp of 2^-8
 // (The clamp is a maximum on the ALU pipe, the busiest one of the kernel at 58 %; moving it to the FMA pipe as a
 // saturating multiply-add followed by a second multiply-add costs one instruction more and measured 49.5 against 46.5 us:
@@ -228,6 +272,192 @@ __device__ __forceinline__ float ex2_lin_from_biased(float v) {
   v = fmaxf(v, kLinMagic - 120.0f);
   constexpr uint32_t kC = 0x3F800000u - 0x47400000u * 32768u - 436208u;  // 0x47400000 = bits of 49152.0f; 436208 = 0.052 * 2^23
   return __uint_as_float(__float_as_uint(v) * 32768u + kC);
+}
+
+constexpr int kQTile = 128;
+constexpr int kKeyTile = 128;
+constexpr int kVRows = 80;  // of a V^T tile: 64 channels + 16 rows of ones (row sum of P)
+
+// Which 128-key tile is the j-th valid one?  Returns its first cache row and how many of its
+// keys are valid.  Segments are (start, length) pairs; zero-length entries are legal.
+__device__ __forceinline__ void locate_tile(const int* seg, int j, int& row, int& valid) {
+  row = 0;
+  valid = 0;
+  bool found = false;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int nt = (seg[2 * i + 1] + kKeyTile - 1) / kKeyTile;
+    if (!found && j < nt) {
+      row = seg[2 * i] + j * kKeyTile;
+      valid = min(kKeyTile, seg[2 * i + 1] - j * kKeyTile);
+      found = true;
+    }
+    j -= nt;
+  }
+}
+
+// Whether the keys of a (query tile, head) are shared by gridDim.z CTAs, and how their results are brought together: through the
+// workspace (see AttnArgs::partials), or, the CTAs being one thread-block cluster, in shared memory.  The unsplit kernel is an
+// instantiation of its own so that none of this reaches its instruction stream.  kHelped: the CTAs that
+// the items leave over take a part of the keys of several items each (KeyShares).
+enum { kUnsplit = 0, kSplitWorkspace = 1, kSplitCluster = 2, kHelped = 3 };
+
+// The table on its way; returns n_segments.
+__device__ __forceinline__ int request_table(const AttnArgs& a, int (&seg)[6]) {
+  const int nseg = *after_wait(a.n_segments);
+  const int32_t* table = after_wait(a.segments);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    seg[2 * i] = i < a.max_segments ? table[2 * i] : 0;
+    seg[2 * i + 1] = i < a.max_segments ? table[2 * i + 1] : 0;
+  }
+  return nseg;
+}
+
+// What was requested, checked (ordinary loads: the table is the work of the kernel before).  Returns the number of key tiles, the same in
+// every thread; a malformed table is reported and counts as empty.
+__device__ __forceinline__ int load_table(const AttnArgs& a, int nseg, int (&seg)[6]) {
+  nseg = min(nseg, a.max_segments);
+  bool ok = true;
+  int n = 0;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    if (i >= nseg) seg[2 * i] = seg[2 * i + 1] = 0;
+    if (seg[2 * i] < 0 || seg[2 * i + 1] < 0 || (seg[2 * i] & 15) != 0 || seg[2 * i] + seg[2 * i + 1] > a.capacity) ok = false;
+    n += (seg[2 * i + 1] + kKeyTile - 1) / kKeyTile;
+  }
+  if (ok) return n;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) seg[i] = 0;
+  if (threadIdx.x == 0) atomicOr(a.status, QB_DEV_BAD_SEGMENT);
+  return 0;
+}
+
+// The half of query row t of head qh that group g (0, 1) rotates and, for group 0, its row of the RoPE table, on their way while
+// something else is done.
+__device__ __forceinline__ void load_q(const AttnArgs& a, int t, int qh, int g, uint4 (&q_pre)[4], float4 (&xy_pre)[4]) {
+  if (t >= a.tpf || g >= 2) return;
+  const uint4* src = reinterpret_cast<const uint4*>(after_wait(a.qkv) + static_cast<size_t>(t) * a.q_row + static_cast<size_t>(qh) * a.q_head + g * 32);
+#pragma unroll
+  for (int v = 0; v < 4; ++v) q_pre[v] = src[v];
+  if (g == 0) {
+    const float4* rp = reinterpret_cast<const float4*>(a.rope_xy + static_cast<size_t>(t) * 16);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xy_pre[i] = __ldg(rp + i);
+  }
+}
+
+// Q row -> RoPE -> shared memory (K-major, swizzled like a TMA tile).  Group 0 rotates pairs 0..15 (spatial angles), group 1 pairs
+// 16..31 (temporal angles `tm`).
+template <bool kFp8>
+__device__ __forceinline__ void stage_q(uint8_t* q_s, const float* tm, uint64_t* q_ready, int r, int g, bool row_ok, const uint4 (&q_pre)[4], const float4 (&xy_pre)[4],
+                                        int lane) {
+  if (g >= 2) return;
+  float y0[16], y1[16];
+  if (row_ok) {
+    float xy[16];
+    if (g == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 v = xy_pre[i];
+        xy[4 * i] = v.x; xy[4 * i + 1] = v.y; xy[4 * i + 2] = v.z; xy[4 * i + 3] = v.w;
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const uint4 x = q_pre[v];
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int pl = v * 4 + j;
+        const int i = pl >> 1;
+        const float c = g == 0 ? xy[i] : tm[i];
+        const float s = g == 0 ? xy[8 + i] : tm[8 + i];
+        const float x0 = bf16lo(w[j]), x1 = bf16hi(w[j]);
+        y0[pl] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
+        y1[pl] = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int p = 0; p < 16; ++p) y0[p] = y1[p] = 0.f;
+  }
+  if (kFp8) {
+    // 64-byte rows; 16-byte chunk index XOR ((row >> 1) & 3); y0 of this group is chunk g, y1 chunk 2 + g
+    uint8_t* rowp = q_s + r * 64;
+    const int sw = (r >> 1) & 3;
+    *reinterpret_cast<uint4*>(rowp + ((g ^ sw) << 4)) =
+        make_uint4(pack_e4m3x4(y0[0], y0[1], y0[2], y0[3]), pack_e4m3x4(y0[4], y0[5], y0[6], y0[7]),
+                   pack_e4m3x4(y0[8], y0[9], y0[10], y0[11]), pack_e4m3x4(y0[12], y0[13], y0[14], y0[15]));
+    *reinterpret_cast<uint4*>(rowp + (((2 + g) ^ sw) << 4)) =
+        make_uint4(pack_e4m3x4(y1[0], y1[1], y1[2], y1[3]), pack_e4m3x4(y1[4], y1[5], y1[6], y1[7]),
+                   pack_e4m3x4(y1[8], y1[9], y1[10], y1[11]), pack_e4m3x4(y1[12], y1[13], y1[14], y1[15]));
+  } else {
+    // 128-byte rows; chunk XOR (row & 7); y0 of this group is chunks 2g, 2g+1, y1 chunks 4+2g, 5+2g
+    uint8_t* rowp = q_s + r * 128;
+    const int sw = r & 7;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      *reinterpret_cast<uint4*>(rowp + (((2 * g + c) ^ sw) << 4)) =
+          make_uint4(pack_bf16x2(y0[8 * c], y0[8 * c + 1]), pack_bf16x2(y0[8 * c + 2], y0[8 * c + 3]),
+                     pack_bf16x2(y0[8 * c + 4], y0[8 * c + 5]), pack_bf16x2(y0[8 * c + 6], y0[8 * c + 7]));
+      *reinterpret_cast<uint4*>(rowp + (((4 + 2 * g + c) ^ sw) << 4)) =
+          make_uint4(pack_bf16x2(y1[8 * c], y1[8 * c + 1]), pack_bf16x2(y1[8 * c + 2], y1[8 * c + 3]),
+                     pack_bf16x2(y1[8 * c + 4], y1[8 * c + 5]), pack_bf16x2(y1[8 * c + 6], y1[8 * c + 7]));
+    }
+  }
+  fence_proxy_async_smem();
+  tc_fence_before();
+  warp_arrive(smem_u32(q_ready), lane);
+}
+
+// Keys from `valid` on of the 32 columns that start at c * 32 count nothing: -inf.
+__device__ __forceinline__ void mask_chunk(uint32_t (&s)[32], int c, int valid) {
+#pragma unroll
+  for (int q = 0; q < 32; ++q)
+    if (c * 32 + q >= valid) s[q] = 0xff800000u;
+}
+
+// A row's result: 64 outputs and, where the tensor core made it (kSum), the row sum, still scaled by 2^(kPShift - m).
+template <bool kSum>
+__device__ __forceinline__ void read_o(uint32_t tmem_o, float (&o)[64], float& l) {
+  uint32_t oo[2][32];
+  tmem_ld32(tmem_o, oo[0]);
+  tmem_ld32(tmem_o + 32, oo[1]);
+  uint32_t lsum = kSum ? tmem_ld1(tmem_o + 64) : 0;
+  tmem_wait_ld_into(oo[0]);
+  tmem_loaded(oo[1]);
+  tmem_loaded(lsum);
+#pragma unroll
+  for (int d = 0; d < 64; ++d) o[d] = __uint_as_float(oo[d >> 5][d & 31]);
+  if (kSum) l = __uint_as_float(lsum);
+}
+
+// 32 outputs of a query row (divided by the row sum already) and their e4m3 copy, narrowed from the bf16-rounded values: it equals a
+// separate cast.
+template <int kN>
+__device__ __forceinline__ void write_out(const AttnArgs& a, size_t at, const float (&o)[kN]) {
+#pragma unroll
+  for (int v = 0; v < kN / 8; ++v) {
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(o[8 * v + 2 * q], o[8 * v + 2 * q + 1]);
+    *reinterpret_cast<uint4*>(a.out + at + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (a.out_q != nullptr)
+      *reinterpret_cast<uint2*>(a.out_q + at + v * 8) = make_uint2(pack_e4m3x4(bf16lo(w[0]), bf16hi(w[0]), bf16lo(w[1]), bf16hi(w[1])),
+                                                                   pack_e4m3x4(bf16lo(w[2]), bf16hi(w[2]), bf16lo(w[3]), bf16hi(w[3])));
+  }
+}
+
+// The shared memory of a kernel, once per device (`done`: a bit per device).
+template <typename K>
+int32_t configure_smem(K kernel, int smem_bytes, std::atomic<unsigned long long>& done) {  // once per device
+  int dev = 0;
+  QB_CUDA_OK(cudaGetDevice(&dev));
+  if (dev < 64 && (done.load(std::memory_order_relaxed) >> dev & 1) != 0) return QB_OK;
+  QB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+  if (dev < 64) done.fetch_or(1ull << dev, std::memory_order_relaxed);
+  return QB_OK;
 }
 
 }  // namespace qb

@@ -14,12 +14,12 @@ FLAGS="-gencode arch=compute_100a,code=sm_100a -lineinfo -O3 -std=c++17 -Xcompil
 [ "$1" = "-v" ] && FLAGS="$FLAGS -Xptxas -v"
 mkdir -p "$OBJ"
 pids=()
-for f in runtime gemm gemm_pair gemm_grouped attn attn4 kv glue qkv_post tp; do
+for f in runtime gemm gemm_pair gemm_grouped attn attn3 kv glue qkv_post tp; do
   $NVCC $FLAGS -c "$HERE/$f.cu" -o "$OBJ/$f.o" &
   pids+=($!)
 done
 for p in "${pids[@]}"; do wait $p; done
-$NVCC -shared -o "$OUT" "$OBJ"/{runtime,gemm,gemm_pair,gemm_grouped,attn,attn4,kv,glue,qkv_post,tp}.o -cudart static
+$NVCC -shared -o "$OUT" "$OBJ"/{runtime,gemm,gemm_pair,gemm_grouped,attn,attn3,kv,glue,qkv_post,tp}.o -cudart static
 [ -n "$QB_BUILD_DIR" ] && exit 0
 # The C side of the smallest calls (a CPython extension); without the interpreter's headers they stay in Python.
 PYTHON="${PYTHON:-python3}"
