@@ -51,14 +51,19 @@ constexpr int kCtrlRegs = 72;      // per thread, warps 0-3
 constexpr int kSoftmaxRegs = 216;  // per thread, warps 4-11
 static_assert(128 * kCtrlRegs + 256 * kSoftmaxRegs <= kAttnThreads * kLaunchRegs, "register budget of the CTA");
 
-template <bool kFp8>
+// Cluster splits: 2 groups x S CTAs leave 64 outputs, m, the row sum and whether they are to be used of each query row with the CTA that
+// writes the row (128 / S rows each), [2 S][rows][kMergePitch] f32.
+constexpr int kMergePitch = 68;
+__host__ __device__ constexpr int merge_rows(int splits) { return (kQTile + splits - 1) / splits; }
+
+template <bool kFp8, bool kCluster = false>
 struct AttnSmem {
   static constexpr int kEs = kFp8 ? 1 : 2;
   // Of each ring.  A stage is given back when its MMAs are done, so the groups hold those of up to four tiles; with four stages the next
   // tiles were only asked for when they were needed (e4m3, 720p: 47.8 -> 42.5 us with eight).  Even: a stage then belongs to one
   // group's tiles.  (With three a group waited for a phase of a stage whose previous phase the other group watches: where that earlier
   // copy was still on its way, the parity wait returned at once.)
-  static constexpr int kKStages = kFp8 ? 8 : 4, kVStages = kFp8 ? 8 : 6;
+  static constexpr int kKStages = kFp8 ? (kCluster ? 6 : 8) : 4, kVStages = kFp8 ? (kCluster ? 6 : 8) : (kCluster ? 4 : 6);
   // e4m3: 16 rows of ones under the 64 V^T rows make the tensor core return the row sum of P in column 64 of O.  bf16 has no TMEM
   // columns left for that (S 128, O 64, P 64 a group): the softmax threads add up the rounded probabilities.
   static constexpr int kRows = kFp8 ? kVRows : 64;
@@ -69,11 +74,13 @@ struct AttnSmem {
   static constexpr int kQOff = 0;
   static constexpr int kKOff = kQOff + kQBytes;
   static constexpr int kVOff = kKOff + kKStages * kKBytes;
-  static constexpr int kClusterOff = kKOff;                  // the rings are free when the CTAs of a cluster meet
-  static constexpr int kCombOff = kVOff + kVStages * kVBytes;  // where the groups meet
-  static constexpr int kBarOff = kCombOff + 2 * 34 * kQTile * 4;
+  // A cluster's results: what this CTA has for each CTA's rows is laid out over its rings, what the others have for its rows arrives beside them.
+  static constexpr int kGiveOff = kKOff;
+  static constexpr int kMergeBytes = 266 * kMergePitch * 4;  // 2 groups, S CTAs, 128 / S rows each (7 CTAs need most)
+  static constexpr int kCombOff = kVOff + kVStages * kVBytes;  // where the groups meet | what the other CTAs have
+  static constexpr int kBarOff = kCombOff + (kCluster ? kMergeBytes : 2 * 34 * kQTile * 4);
   static constexpr int kTotal = kBarOff + 640 + 1024;
-  static_assert(kCombOff - kClusterOff >= 266 * 68 * 4, "merge area of the cluster splits (7 CTAs need most) aliases the rings");
+  static_assert(!kCluster || kCombOff - kGiveOff >= kMergeBytes, "results laid out over the rings");
   static_assert(kKStages % 2 == 0 && kVStages % 2 == 0 && kTotal <= 227 * 1024, "see kKStages; shared memory of one CTA");
 };
 
@@ -86,6 +93,7 @@ struct AttnBars {
   uint64_t pv_done[2];      // [group] O += P(i) V(i) has finished
   uint64_t o_final[2];      // [group] every PV of a piece has finished
   uint64_t q_ready;
+  uint64_t merge_full;      // the other CTAs' results for this CTA's rows are here
   uint32_t tmem_slot;
   int abort_flag, drain_flag, exchange;
   float tm[16];  // cosines and sines of the temporal angles
@@ -94,10 +102,6 @@ struct AttnBars {
 };
 static_assert(sizeof(AttnBars) <= 640, "kBarOff + 640");
 
-// Cluster splits: 2 groups x S CTAs leave 64 outputs, m and the row sum of each query row with the CTA that writes the row
-// (128 / S rows each), [2 S][rows][kMergePitch] f32.
-constexpr int kMergePitch = 68;
-__host__ __device__ constexpr int merge_rows(int splits) { return (kQTile + splits - 1) / splits; }
 // Tiles j = 2 i + g, i = 0, 1, ..., below `end`: those of softmax group g.
 __device__ __forceinline__ int group_tiles(int end, int g) { return (end - g + 1) >> 1; }
 
@@ -161,11 +165,11 @@ __device__ __noinline__ int end_piece(const AttnArgs& a, uint8_t* smem, uint32_t
   const int item = kr.first_item + piece;
   const Piece done = kr.at(item), next = kr.at(item + 1);
   int q0 = 0, qh = 0, kvh = 0;
-  uint4 q_pre[4];
-  float4 xy_pre[4];
+  QueryTile q;
   if (next.n > 0) {
     next.place(a, q0, qh, kvh);
-    load_q(a, q0 + r, qh, g, q_pre, xy_pre);
+    q.request_angles(a, q0);
+    q.request(a, q0, qh);
   }
   float o[64];
   float l = 0.f;
@@ -180,7 +184,7 @@ __device__ __noinline__ int end_piece(const AttnArgs& a, uint8_t* smem, uint32_t
   merge_groups(reinterpret_cast<float*>(smem + L::kCombOff), g, r, m, l, o);
   const bool good = *abort_flag == 0;
   if (g == 1 && r == 0) b->tile_shift = next.tile0 - (piece + 1) * done.n;  // (read again behind q_ready of the next piece)
-  if (next.n > 0) stage_q<true>(smem + L::kQOff, b->tm, &b->q_ready, r, g, q0 + r < a.tpf, q_pre, xy_pre, lane);
+  if (next.n > 0) q.stage<true>(smem + L::kQOff, b->tm, &b->q_ready);
   if (g == 0) kr.finish(a, done, r, good, m, l, o, &b->exchange);
   return next.n;
 }
@@ -188,7 +192,7 @@ __device__ __noinline__ int end_piece(const AttnArgs& a, uint8_t* smem, uint32_t
 template <bool kFp8, int kSplit, bool kLin>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnArgs a) {
-  using L = AttnSmem<kFp8>;
+  using L = AttnSmem<kFp8, kSplit == kSplitCluster>;
   constexpr int kKS = L::kKStages, kVS = L::kVStages;
   constexpr uint32_t kTmemCols = 512;
   constexpr uint32_t kIdescS = kFp8 ? umma_idesc(0, 0, 128, kKeyTile) : umma_idesc(1, 1, 128, kKeyTile);
@@ -218,26 +222,17 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   int qh = blockIdx.y;
   int kvh = qh / a.gqa;
 
-  if (threadIdx.x == 0) {
+  if (warp == 0) {  // (a barrier per lane: one thread took 700 cycles for all of them)
+    for (unsigned i = lane; i < offsetof(AttnBars, tmem_slot) / 8; i += 32)
+      mbar_init(smem_u32(reinterpret_cast<uint64_t*>(bars) + i), i >= offsetof(AttnBars, s_free) / 8 && i < offsetof(AttnBars, pv_done) / 8 ? 4 : i == offsetof(AttnBars, q_ready) / 8 ? 8 : 1);
+    if (lane == 0) {
+      *abort_flag = 0;
+      *drain_flag = 0;
+    }
+    fence_barrier_init();
+  } else if (threadIdx.x == 96) {
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
-    for (int s = 0; s < 8; ++s) {
-      mbar_init(smem_u32(&bars->k_full[s]), 1);
-      mbar_init(smem_u32(&bars->k_empty[s]), 1);
-      mbar_init(smem_u32(&bars->v_full[s]), 1);
-      mbar_init(smem_u32(&bars->v_empty[s]), 1);
-    }
-    for (int g = 0; g < 2; ++g) {
-      mbar_init(smem_u32(&bars->s_full[g]), 1);
-      mbar_init(smem_u32(&bars->s_free[g]), 4);
-      mbar_init(smem_u32(&bars->p_full[g]), 4);
-      mbar_init(smem_u32(&bars->pv_done[g]), 1);
-      mbar_init(smem_u32(&bars->o_final[g]), 1);
-    }
-    mbar_init(smem_u32(&bars->q_ready), 8);
-    *abort_flag = 0;
-    *drain_flag = 0;
-    fence_barrier_init();
   }
   if (kFp8) {  // rows of ones under every V^T tile (16 rows x 128 bytes each)
     for (int i = threadIdx.x; i < kVS * 128; i += kAttnThreads)  // 128 x 16 bytes per tile
@@ -252,18 +247,26 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_slot;
+  if (kSplit == kSplitCluster) {
+    // The bytes that will arrive are announced before the CTAs of the cluster tell one another that their barriers are there.
+    if (threadIdx.x == 0) mbar_arrive_expect_tx(smem_u32(&bars->merge_full), (gridDim.z - 1) * 2 * merge_rows(gridDim.z) * kMergePitch * 4);
+    __syncwarp();
+    cluster_arrive();
+  }
 
-  // Everything above touched only this CTA's shared memory and TMEM, so it may run while the kernels
+  QueryTile q;
+  if (kSplit != kHelped && warp >= 4) q.request_angles(a, q0);
+
+  // Everything above touched only this CTA's shared memory and TMEM, and a table that no kernel writes, so it may run while the kernels
   // before this one in the stream are still at work; everything below reads what they wrote.
   grid_dep_launch();
   grid_dep_wait();
 
-  // The table and the query rows are asked for at once, so that the first K tile is two trips to L2 away.
+  // The table, the query rows and the frame counter are asked for at once, so that the first K tile is two trips to L2 away.
+  if (kSplit != kHelped && warp >= 4) q.request(a, q0, qh);
   int seg[6];
   const int nseg = request_table(a, seg);
-  uint4 q_pre[4];
-  float4 xy_pre[4];
-  if (kSplit != kHelped && warp >= 4) load_q(a, q0 + (warp & 3) * 32 + lane, qh, (warp - 4) >> 2, q_pre, xy_pre);
+  const int frame_t = *after_wait(a.frame_t);
   int n_tiles = load_table(a, nseg, seg);
   int tile0 = 0;
   KeyShares kr;
@@ -274,7 +277,10 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     pc.place(a, q0, qh, kvh);
     tile0 = pc.tile0;
     n_tiles = kr.all_tiles();
-    if (warp >= 4 && pc.n > 0) load_q(a, q0 + (warp & 3) * 32 + lane, qh, (warp - 4) >> 2, q_pre, xy_pre);
+    if (warp >= 4 && pc.n > 0) {
+      q.request_angles(a, q0);
+      q.request(a, q0, qh);
+    }
   }
   // key splits: this CTA's share of the tiles
   const int n_splits = kSplit == kSplitWorkspace || kSplit == kSplitCluster ? static_cast<int>(gridDim.z) : 1;
@@ -288,7 +294,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   if (warp < 4) {
     setmaxnreg_dec<kCtrlRegs>();
     if (warp == 3) {
-      if (lane < 8) temporal_cos_sin(*after_wait(a.frame_t), lane, bars->tm);
+      if (lane < 8) temporal_cos_sin(frame_t, lane, bars->tm);
       if (lane == 8) {
 #pragma unroll
         for (int i = 0; i < 6; ++i) bars->seg[i] = seg[i];
@@ -296,7 +302,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         bars->tile_shift = tile0;
       }
       __syncwarp();
-      asm volatile("bar.arrive 4, 160;" ::: "memory");  // group 1 waits for it
+      asm volatile("bar.arrive 4, 288;" ::: "memory");  // groups 0 and 1 wait for it
     } else if (warp == 0) {
       // ---------------- TMA producer: K(t), then V(t - 2), in the order in which they are used
       if (elect_one()) {
@@ -425,8 +431,10 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     const uint32_t tmem_s = tmem_base + g * kGroupCols + lane_addr;  // this thread's row of the group's S,
     const uint32_t tmem_o = tmem_s + kOCol, tmem_p = tmem_s + kPCol;  // ... of its O and of its P
 
-    if (g == 1) asm volatile("bar.sync 4, 160;" ::: "memory");  // the temporal angles
-    stage_q<kFp8>(smem + L::kQOff, bars->tm, &bars->q_ready, r, g, row_ok, q_pre, xy_pre, lane);
+    if (g < 2) {
+      asm volatile("bar.sync 4, 288;" ::: "memory");  // the temporal angles
+      q.stage<kFp8>(smem + L::kQOff, bars->tm, &bars->q_ready);
+    }
     int i0 = 0, i1 = group_tiles(kSplit == kHelped ? pc.n : n_tiles, g);  // the group's tiles of the piece, as the MMA warp counts them
     // What the end of a piece needs is worked out there from its number, so that it takes no registers in the loop.
     int end = pc.n;
@@ -530,45 +538,71 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         read_o<kFp8>(tmem_o, o, l_run);
       }
       if constexpr (kSplit == kSplitCluster) {
-        // Both groups of every CTA of the cluster hand their rows to the CTA that writes them (against the merge of the groups and
-        // the trip through the workspace, 360p, 4 CTAs, with an earlier form of the loop: e4m3 13.4 -> 12.1 us, bf16 16.0 -> 13.9 us).
-        const int S = static_cast<int>(gridDim.z), rows = merge_rows(S);
-        float* area = reinterpret_cast<float*>(smem + L::kClusterOff);
-        cluster_sync();  // the rings of every CTA are free (its tensor work and TMA traffic are finished)
-        // Nobody waits any more, so the flag now tells whether one of this CTA's waits ran out; if so, the rows that its results belong
-        // to are not written by any CTA of the cluster.
+        // Both groups of every CTA of the cluster hand their rows to the CTA that writes them: laid out in shared memory, then one bulk copy
+        // per CTA and group, whose bytes the receiver's barrier counts.  (Pushed row by row between two cluster barriers the end took 10600
+        // of a launch's 23700 cycles at 360p; now 7900 of 21800, half of it the CTA with one tile more.)
+        const int S = static_cast<int>(gridDim.z), rows = merge_rows(S), cta = static_cast<int>(blockIdx.z);
         const int me = static_cast<int>(threadIdx.x) - 128;
-        if (*abort_flag != 0 && me < S) st_dsmem(map_to_cta(smem_u32(&bars->abort_flag), me), 1);
+        float* give = reinterpret_cast<float*>(smem + L::kGiveOff);  // [CTA][group][rows]
+        const float* take = reinterpret_cast<const float*>(smem + L::kCombOff);  // [CTA][group][rows]
+        asm volatile("bar.sync 2, 256;" ::: "memory");  // the rings are free: both groups' tensor work, and with it the TMA traffic, is finished
         {
-          const uint32_t base = map_to_cta(smem_u32(area), r / rows);
-          const int part = 2 * static_cast<int>(blockIdx.z) + g, rl = r % rows;
-          const uint32_t row_at = base + static_cast<uint32_t>((part * rows + rl) * kMergePitch) * 4u;
+          float* row = give + ((r / rows * 2 + g) * rows + r % rows) * kMergePitch;
 #pragma unroll
-          for (int d = 0; d < 64; d += 4)
-            st_dsmem_v4(row_at + d * 4u, __float_as_uint(o[d]), __float_as_uint(o[d + 1]), __float_as_uint(o[d + 2]), __float_as_uint(o[d + 3]));
-          st_dsmem_v4(row_at + 256u, __float_as_uint(m_run), __float_as_uint(l_run), 0u, 0u);
+          for (int d = 0; d < 64; d += 4) *reinterpret_cast<float4*>(row + d) = make_float4(o[d], o[d + 1], o[d + 2], o[d + 3]);
+          // where one of this CTA's waits ran out, the rows that its results belong to are not written by any CTA of the cluster
+          *reinterpret_cast<float4*>(row + 64) = make_float4(m_run, l_run, *abort_flag != 0 ? 1.0f : 0.0f, 0.0f);
         }
-        cluster_sync();
+        fence_proxy_async_smem();
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        cluster_wait();  // (long since: every CTA's barriers are there)
+        if (me < 2 * S && me >> 1 != cta) {
+          const uint32_t bytes = static_cast<uint32_t>(rows * kMergePitch * 4);
+          bulk_copy_cluster(map_to_cta(smem_u32(take) + static_cast<uint32_t>(2 * cta + (me & 1)) * bytes, me >> 1), smem_u32(give) + static_cast<uint32_t>(me) * bytes, bytes,
+                            map_to_cta(smem_u32(&bars->merge_full), me >> 1));
+        }
+        __syncwarp();
         const float vs = a.v_scale ? __ldg(a.v_scale + kvh) : 1.0f;
-        const bool whole_cluster = *abort_flag == 0;
-        for (int n = me; whole_cluster && n < rows * 8; n += 256) {  // 8 outputs of a row per thread
-          const int rl = n >> 3, d0 = (n & 7) * 8, rr = static_cast<int>(blockIdx.z) * rows + rl;
+        wait_warp(bars->merge_full, 0);
+        cluster_arrive();  // what the others copied here is here (see the end of the kernel)
+        const bool whole_cta = *abort_flag == 0;
+        for (int n = me; whole_cta && n < rows * 8; n += 256) {  // outputs d0 .. d0 + 3 and 32 more of a row per thread: no bank twice
+          const int rl = n >> 3, d0 = (n & 7) * 4, rr = cta * rows + rl;
           if (rr >= kQTile || q0 + rr >= a.tpf) continue;
-          float m = -1.0e30f;
-          for (int q = 0; q < 2 * S; ++q) m = fmaxf(m, area[(q * rows + rl) * kMergePitch + 64]);
+          auto part_of = [&](int q) { return (q >> 1 == cta ? give : take) + (q * rows + rl) * kMergePitch; };
+          float4 head[16];  // m, row sum, lost
+          float m = -1.0e30f, lost = 0.f;
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            if (q < 2 * S) head[q] = *reinterpret_cast<const float4*>(part_of(q) + 64);
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            if (q < 2 * S) {
+              m = fmaxf(m, head[q].x);
+              lost += head[q].z;
+            }
+          if (lost != 0.f) continue;
           float l = 0.f, e[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-          for (int q = 0; q < 2 * S; ++q) {
-            const float* part = area + (q * rows + rl) * kMergePitch;
-            const float w = ex2_approx(part[64] - m);
-            l = fmaf(w, part[65], l);
-            const float4 x = *reinterpret_cast<const float4*>(part + d0), y = *reinterpret_cast<const float4*>(part + d0 + 4);
-            e[0] = fmaf(w, x.x, e[0]); e[1] = fmaf(w, x.y, e[1]); e[2] = fmaf(w, x.z, e[2]); e[3] = fmaf(w, x.w, e[3]);
-            e[4] = fmaf(w, y.x, e[4]); e[5] = fmaf(w, y.y, e[5]); e[6] = fmaf(w, y.z, e[6]); e[7] = fmaf(w, y.w, e[7]);
-          }
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            if (q < 2 * S) {
+              const float* part = part_of(q) + d0;
+              const float w = ex2_approx(head[q].x - m);
+              l = fmaf(w, head[q].y, l);
+              const float4 x = *reinterpret_cast<const float4*>(part), y = *reinterpret_cast<const float4*>(part + 32);
+              e[0] = fmaf(w, x.x, e[0]); e[1] = fmaf(w, x.y, e[1]); e[2] = fmaf(w, x.z, e[2]); e[3] = fmaf(w, x.w, e[3]);
+              e[4] = fmaf(w, y.x, e[4]); e[5] = fmaf(w, y.y, e[5]); e[6] = fmaf(w, y.z, e[6]); e[7] = fmaf(w, y.w, e[7]);
+            }
           const float inv = l > 0.f ? vs / l : 0.f;
 #pragma unroll
           for (int d = 0; d < 8; ++d) e[d] *= inv;
-          write_out(a, static_cast<size_t>(q0 + rr) * a.o_row + static_cast<size_t>(qh) * a.o_head + d0, e);
+          const size_t at = static_cast<size_t>(q0 + rr) * a.o_row + static_cast<size_t>(qh) * a.o_head + d0;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t w0 = pack_bf16x2(e[4 * h], e[4 * h + 1]), w1 = pack_bf16x2(e[4 * h + 2], e[4 * h + 3]);
+            *reinterpret_cast<uint2*>(a.out + at + 32 * h) = make_uint2(w0, w1);
+            if (a.out_q != nullptr) *reinterpret_cast<uint32_t*>(a.out_q + at + 32 * h) = pack_e4m3x4(bf16lo(w0), bf16hi(w0), bf16lo(w1), bf16hi(w1));
+          }
         }
       } else if constexpr (kSplit == kUnsplit) {
         // The groups exchange halves: group g finishes outputs 32 g .. 32 g + 31 of the row.  (Tensor work and TMA traffic are finished
@@ -643,10 +677,14 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     if (kSplit == kHelped && kr.tiles == 0) KeyShares::write_zeros(a, r, g, 2);
   }
 
-  if (kSplit == kSplitCluster && warp < 4) {  // the softmax warps' two barriers
+  if (kSplit == kSplitCluster) {
+    // No CTA leaves while its results are still being copied: the softmax warps of all have seen theirs arrive.
     __syncwarp();
-    cluster_sync();
-    cluster_sync();
+    if (warp < 4) {
+      cluster_wait();
+      cluster_arrive();
+    }
+    cluster_wait();
   }
   tc_fence_before();
   __syncthreads();
@@ -720,7 +758,7 @@ static cudaLaunchConfig_t attn_config(dim3 grid, int smem_bytes, cudaStream_t st
 // through the workspace instead.  bf16 comes here for its key splits: where there are none, and with helpers, it goes to the three-group kernel.
 template <bool kFp8, bool kLin>
 static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnArgs& a, int Hq, int splits, bool forced, bool helped, cudaStream_t st) {
-  constexpr int kSmem = AttnSmem<kFp8>::kTotal;
+  constexpr int kSmem = AttnSmem<kFp8>::kTotal, kClusterSmem = AttnSmem<kFp8, true>::kTotal;
   if constexpr (kFp8) if (helped) {
     static std::atomic<unsigned long long> done{0};
     const int32_t rc = configure_smem(owl_attn_kernel<kFp8, kHelped, kLin>, kSmem, done);
@@ -733,13 +771,13 @@ static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const
   if (cluster > 1) {
     static std::atomic<unsigned long long> done{0};
     static std::atomic<int> held[9];  // clusters of this many CTAs that run at once (0 = not asked yet)
-    const int32_t rc = configure_smem(owl_attn_kernel<kFp8, kSplitCluster, kLin>, kSmem, done);
+    const int32_t rc = configure_smem(owl_attn_kernel<kFp8, kSplitCluster, kLin>, kClusterSmem, done);
     if (rc != QB_OK) return rc;
     cudaLaunchAttribute attr[2];
     while (cluster > 1) {
       int n = held[cluster].load(std::memory_order_relaxed);
       if (n == 0) {
-        const cudaLaunchConfig_t cfg = attn_config(dim3(q_tiles, Hq, cluster), kSmem, st, attr);
+        const cudaLaunchConfig_t cfg = attn_config(dim3(q_tiles, Hq, cluster), kClusterSmem, st, attr);
         if (cudaOccupancyMaxActiveClusters(&n, owl_attn_kernel<kFp8, kSplitCluster, kLin>, &cfg) != cudaSuccess || n <= 0) {
           cudaGetLastError();
           n = 1;
@@ -750,7 +788,7 @@ static int32_t launch_attn(const CUtensorMap& tmK, const CUtensorMap& tmV, const
       cluster = forced ? 1 : cluster - 1;
     }
     if (cluster > 1) {
-      const cudaLaunchConfig_t cfg = attn_config(dim3(q_tiles, Hq, cluster), kSmem, st, attr);
+      const cudaLaunchConfig_t cfg = attn_config(dim3(q_tiles, Hq, cluster), kClusterSmem, st, attr);
       const cudaError_t e = cudaLaunchKernelEx(&cfg, owl_attn_kernel<kFp8, kSplitCluster, kLin>, tmK, tmV, a);
       ++g_launch_count;
       if (e != cudaSuccess) return fail(QB_ERR_LAUNCH, "owl_attn kernel (cluster of %d): %s", cluster, cudaGetErrorString(e));

@@ -126,7 +126,7 @@ __device__ __forceinline__ void row_exp(uint32_t ts, int valid, float sl2, float
   }
 }
 
-// The softmax warps' tiles j0 .. j1 - 1 of one item, those of their group.  (Not inlined, the loop takes 55.3 instead of 52.5 us.)
+// The softmax warps' tiles j0 .. j1 - 1 of one item, those of their group.
 __device__ __forceinline__ void softmax_tiles(uint8_t* smem, uint32_t tmem_base, unsigned* status, float sl2, int j0, int j1, bool whole) {
   using L = Attn3Smem;
   // m is raised (and O rescaled) only when a tile's maximum exceeds it by more than kSlack, so P <= 2^kSlack.
@@ -196,6 +196,12 @@ __device__ __forceinline__ void softmax_tiles(uint8_t* smem, uint32_t tmem_base,
         }
 }
 
+// The same as a function of its own, for the kernel with helpers: inlined there, its registers and order changed with whatever surrounded
+// it (368 to 399 us at 128 buckets).  The kernel without is faster with it inlined (52.5 against 55.3 us at 16).
+__device__ __noinline__ void softmax_tiles_apart(uint8_t* smem, uint32_t tmem_base, unsigned* status, float sl2, int j0, int j1, bool whole) {
+  softmax_tiles(smem, tmem_base, status, sl2, j0, j1, whole);
+}
+
 // kHelped: the end of a piece, for the softmax warps.  Group 0 reads O and hands the finished rows on; groups 0 and 1 stage the
 // next piece's query rows.  A function of its own, because what it works with (addresses, the places of pieces)
 // would otherwise be kept in registers, or spilled, through the loop over the tiles.
@@ -208,11 +214,11 @@ __device__ __noinline__ int end_piece3(const AttnArgs& a, uint8_t* smem, uint32_
   const int item = kr.first_item + piece;
   const Piece done = kr.at(item), next = kr.at(item + 1);
   int q0 = 0, qh = 0, kvh = 0;
-  uint4 q_pre[4];
-  float4 xy_pre[4];
+  QueryTile q;
   if (next.n > 0) {
     next.place(a, q0, qh, kvh);
-    load_q(a, q0 + r, qh, g, q_pre, xy_pre);
+    q.request_angles(a, q0);
+    q.request(a, q0, qh);
   }
   float o[64];
   float l = 0.f;
@@ -225,7 +231,7 @@ __device__ __noinline__ int end_piece3(const AttnArgs& a, uint8_t* smem, uint32_
   const float m = reinterpret_cast<const float*>(smem + L::kRowOff)[r];
   const bool good = *abort_flag == 0;
   if (g == 1 && r == 0) b->tile_shift = next.tile0 - (piece + 1) * done.n;  // (read again behind q_ready of the next piece)
-  if (next.n > 0) stage_q<false>(smem + L::kQOff, b->tm, &b->q_ready, r, g, q0 + r < a.tpf, q_pre, xy_pre, lane);
+  if (next.n > 0) q.stage<false>(smem + L::kQOff, b->tm, &b->q_ready);
   if (g == 0) kr.finish(a, done, r, good, m, l, o, &b->exchange);
   return next.n;
 }
@@ -256,26 +262,17 @@ owl_attn3_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
   int qh = blockIdx.y;
   int kvh = qh / a.gqa;
 
-  if (threadIdx.x == 0) {
+  if (warp == 0) {  // (a barrier per lane: one thread took 700 cycles for all of them)
+    for (unsigned i = lane; i < offsetof(Attn3Bars, tmem_slot) / 8; i += 32)
+      mbar_init(smem_u32(reinterpret_cast<uint64_t*>(bars) + i), i >= offsetof(Attn3Bars, p_full) / 8 && i < offsetof(Attn3Bars, pv_done) / 8 ? 4 : i == offsetof(Attn3Bars, q_ready) / 8 ? 8 : 1);
+    if (lane == 0) {
+      *abort_flag = 0;
+      *drain_flag = 0;
+    }
+    fence_barrier_init();
+  } else if (threadIdx.x == 96) {
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(smem_u32(&bars->k_full[s]), 1);
-      mbar_init(smem_u32(&bars->k_empty[s]), 1);
-      mbar_init(smem_u32(&bars->v_full[s]), 1);
-      mbar_init(smem_u32(&bars->v_empty[s]), 1);
-    }
-    for (int g = 0; g < kGroups; ++g) {
-      mbar_init(smem_u32(&bars->s_full[g]), 1);
-      mbar_init(smem_u32(&bars->p_full[g]), 4);
-      mbar_init(smem_u32(&bars->pv_done[g]), 1);
-      for (int w = 0; w < 4; ++w) mbar_init(smem_u32(&bars->turn[g][w]), 1);
-    }
-    mbar_init(smem_u32(&bars->o_final), 1);
-    mbar_init(smem_u32(&bars->q_ready), 8);
-    *abort_flag = 0;
-    *drain_flag = 0;
-    fence_barrier_init();
   }
   // rows of ones under every V^T tile (16 rows x 128 bytes each): the tensor core then returns the row sum of P
   {
@@ -294,17 +291,19 @@ owl_attn3_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_slot;
 
-  // Everything above touched only this CTA's shared memory and TMEM, so it may run while the kernels
+  QueryTile q;
+  if (!kHelped && warp >= 4) q.request_angles(a, q0);
+
+  // Everything above touched only this CTA's shared memory and TMEM, and a table that no kernel writes, so it may run while the kernels
   // before this one in the stream are still at work; everything below reads what they wrote.
   grid_dep_launch();
   grid_dep_wait();
 
-  // The table and the query rows are asked for at once, so that the first K tile is two trips to L2 away.
+  // The table, the query rows and the frame counter are asked for at once, so that the first K tile is two trips to L2 away.
+  if (!kHelped && warp >= 4) q.request(a, q0, qh);
   int seg[6];
   const int nseg = request_table(a, seg);
-  uint4 q_pre[4];
-  float4 xy_pre[4];
-  if (!kHelped && warp >= 4) load_q(a, q0 + (warp & 3) * 32 + lane, qh, (warp - 4) >> 2, q_pre, xy_pre);
+  const int frame_t = *after_wait(a.frame_t);
   int n_tiles = load_table(a, nseg, seg);
   int tile0 = 0;
   KeyShares kr;
@@ -315,13 +314,16 @@ owl_attn3_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     pc.place(a, q0, qh, kvh);
     tile0 = pc.tile0;
     n_tiles = kr.all_tiles();
-    if (warp >= 4 && pc.n > 0) load_q(a, q0 + (warp & 3) * 32 + lane, qh, (warp - 4) >> 2, q_pre, xy_pre);
+    if (warp >= 4 && pc.n > 0) {
+      q.request_angles(a, q0);
+      q.request(a, q0, qh);
+    }
   }
   // Registers move from the four control warps to the softmax warps.
   if (warp < 4) {
     setmaxnreg_dec<kA3CtrlRegs>();
     if (warp == 3) {
-      if (lane < 8) temporal_cos_sin(*after_wait(a.frame_t), lane, bars->tm);
+      if (lane < 8) temporal_cos_sin(frame_t, lane, bars->tm);
       if (lane == 8) {
 #pragma unroll
         for (int i = 0; i < 6; ++i) bars->seg[i] = seg[i];
@@ -329,7 +331,7 @@ owl_attn3_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         bars->tile_shift = tile0;
       }
       __syncwarp();
-      asm volatile("bar.arrive 4, 160;" ::: "memory");  // group 1 waits for it
+      asm volatile("bar.arrive 4, 288;" ::: "memory");  // groups 0 and 1 wait for it
     } else if (warp == 0) {
       // ---------------- TMA producer: K(t), then V(t - 3), in the order in which they are used
       if (elect_one()) {
@@ -455,8 +457,10 @@ owl_attn3_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t tmem_o = tmem_base + kOCol + lane_addr;
 
-    if (g == 1) asm volatile("bar.sync 4, 160;" ::: "memory");  // the temporal angles
-    stage_q<false>(smem + L::kQOff, bars->tm, &bars->q_ready, r, g, row_ok, q_pre, xy_pre, lane);
+    if (g < 2) {
+      asm volatile("bar.sync 4, 288;" ::: "memory");  // the temporal angles
+      q.stage<false>(smem + L::kQOff, bars->tm, &bars->q_ready);
+    }
     // every segment a multiple of the tile (720p: 512 keys a bucket): no tile needs a mask, so none is looked up
     const bool whole = ((seg[1] | seg[3] | seg[5]) & (kKeyTile - 1)) == 0;
     int j0 = 0, j1 = kHelped ? pc.n : n_tiles;
@@ -470,7 +474,8 @@ owl_attn3_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
       }
       const float ks = a.k_scale ? __ldg(a.k_scale + kvh) : 1.0f;
       const float sl2 = ks * 0.125f * 1.4426950408889634f;  // scores -> log2 domain, 1/sqrt(64) folded in
-      softmax_tiles(smem, tmem_base, a.status, sl2, j0, j1, whole);
+      if (kHelped) softmax_tiles_apart(smem, tmem_base, a.status, sl2, j0, j1, whole);
+      else softmax_tiles(smem, tmem_base, a.status, sl2, j0, j1, whole);
       if constexpr (kHelped) {
         const int n = end_piece3(a, smem, tmem_o, piece);
         j0 = j1;

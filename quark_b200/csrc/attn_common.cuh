@@ -333,83 +333,81 @@ __device__ __forceinline__ int load_table(const AttnArgs& a, int nseg, int (&seg
   return 0;
 }
 
-// The half of query row t of head qh that group g (0, 1) rotates and, for group 0, its row of the RoPE table, on their way while
-// something else is done.
-__device__ __forceinline__ void load_q(const AttnArgs& a, int t, int qh, int g, uint4 (&q_pre)[4], float4 (&xy_pre)[4]) {
-  if (t >= a.tpf || g >= 2) return;
-  const uint4* src = reinterpret_cast<const uint4*>(after_wait(a.qkv) + static_cast<size_t>(t) * a.q_row + static_cast<size_t>(qh) * a.q_head + g * 32);
-#pragma unroll
-  for (int v = 0; v < 4; ++v) q_pre[v] = src[v];
-  if (g == 0) {
-    const float4* rp = reinterpret_cast<const float4*>(a.rope_xy + static_cast<size_t>(t) * 16);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) xy_pre[i] = __ldg(rp + i);
-  }
-}
+// The query tile: 128 rows of 8 units of 16 bytes, four units to a thread of groups 0 and 1 (256 threads): unit (n & 7) of row n >> 3, n =
+// the thread's number + 256 i.  (A row per thread and group, as the tensor core will want them, made every load touch 32 lines: 2500
+// cycles until the last one was here.)
+struct QueryTile {
+  uint4 x[4];      // 8 values: 4 pairs to rotate
+  float2 c[4], s[4];  // spatial units (0..3): cosines and sines of the two angles of the 4 pairs
 
-// Q row -> RoPE -> shared memory (K-major, swizzled like a TMA tile).  Group 0 rotates pairs 0..15 (spatial angles), group 1 pairs
-// 16..31 (temporal angles `tm`).
-template <bool kFp8>
-__device__ __forceinline__ void stage_q(uint8_t* q_s, const float* tm, uint64_t* q_ready, int r, int g, bool row_ok, const uint4 (&q_pre)[4], const float4 (&xy_pre)[4],
-                                        int lane) {
-  if (g >= 2) return;
-  float y0[16], y1[16];
-  if (row_ok) {
-    float xy[16];
-    if (g == 0) {
+  __device__ __forceinline__ static int number() { return static_cast<int>(threadIdx.x) - 128; }  // (the softmax warps start at thread 128)
+  // The rows' angles, from a table that no kernel writes.
+  __device__ __forceinline__ void request_angles(const AttnArgs& a, int q0) {
+    const int n = number(), u = n & 7;
+    if (n >= 256 || u >= 4) return;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 v = xy_pre[i];
-        xy[4 * i] = v.x; xy[4 * i + 1] = v.y; xy[4 * i + 2] = v.z; xy[4 * i + 3] = v.w;
-      }
+    for (int i = 0; i < 4; ++i) {
+      const int t = q0 + (n >> 3) + 32 * i;
+      if (t >= a.tpf) continue;
+      const float* xy = a.rope_xy + static_cast<size_t>(t) * 16 + 2 * u;
+      asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(c[i].x), "=f"(c[i].y) : "l"(xy) : "memory");
+      asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(s[i].x), "=f"(s[i].y) : "l"(xy + 8) : "memory");
+    }
+  }
+  // The rows.  (volatile: ordinary loads were moved down to where they are used, behind the segment table.)
+  __device__ __forceinline__ void request(const AttnArgs& a, int q0, int qh) {
+    const int n = number(), u = n & 7;
+    if (n >= 256) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = q0 + (n >> 3) + 32 * i;
+      x[i] = make_uint4(0, 0, 0, 0);
+      if (t >= a.tpf) continue;
+      const uint16_t* src = a.qkv + static_cast<size_t>(t) * a.q_row + static_cast<size_t>(qh) * a.q_head + 8 * u;
+      asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[i].x), "=r"(x[i].y), "=r"(x[i].z), "=r"(x[i].w) : "l"(src) : "memory");
+    }
+  }
+  // Rotated (RoPE; `tm`: cosines and sines of the temporal angles), narrowed and stored to shared memory, K-major and swizzled like a TMA
+  // tile: pair p = 4 u + j of a row becomes its values p and 32 + p.
+  template <bool kFp8>
+  __device__ __forceinline__ void stage(uint8_t* q_s, const float* tm, uint64_t* q_ready) {
+    const int n = number(), u = n & 7;
+    if (n >= 256) return;
+    float2 ct, st;
+    if (u >= 4) {
+      ct = make_float2(tm[2 * u - 8], tm[2 * u - 7]);
+      st = make_float2(tm[2 * u], tm[2 * u + 1]);
     }
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const uint4 x = q_pre[v];
-      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+    for (int i = 0; i < 4; ++i) {
+      const int r = (n >> 3) + 32 * i;
+      const float2 co = u < 4 ? c[i] : ct, si = u < 4 ? s[i] : st;
+      const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+      float y0[4], y1[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int pl = v * 4 + j;
-        const int i = pl >> 1;
-        const float c = g == 0 ? xy[i] : tm[i];
-        const float s = g == 0 ? xy[8 + i] : tm[8 + i];
+        const float cc = j < 2 ? co.x : co.y, ss = j < 2 ? si.x : si.y;
         const float x0 = bf16lo(w[j]), x1 = bf16hi(w[j]);
-        y0[pl] = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
-        y1[pl] = __fadd_rn(__fmul_rn(x1, c), __fmul_rn(x0, s));
+        y0[j] = __fsub_rn(__fmul_rn(x0, cc), __fmul_rn(x1, ss));
+        y1[j] = __fadd_rn(__fmul_rn(x1, cc), __fmul_rn(x0, ss));
+      }
+      if (kFp8) {  // 64-byte rows; 16-byte unit XOR ((row >> 1) & 3)
+        uint8_t* row = q_s + r * 64 + (u & 3) * 4;
+        const int sw = (r >> 1) & 3;
+        *reinterpret_cast<uint32_t*>(row + (((u >> 2) ^ sw) << 4)) = pack_e4m3x4(y0[0], y0[1], y0[2], y0[3]);
+        *reinterpret_cast<uint32_t*>(row + ((((u >> 2) + 2) ^ sw) << 4)) = pack_e4m3x4(y1[0], y1[1], y1[2], y1[3]);
+      } else {  // 128-byte rows; unit XOR (row & 7)
+        uint8_t* row = q_s + r * 128 + (u & 1) * 8;
+        const int sw = r & 7;
+        *reinterpret_cast<uint2*>(row + (((u >> 1) ^ sw) << 4)) = make_uint2(pack_bf16x2(y0[0], y0[1]), pack_bf16x2(y0[2], y0[3]));
+        *reinterpret_cast<uint2*>(row + ((((u >> 1) + 4) ^ sw) << 4)) = make_uint2(pack_bf16x2(y1[0], y1[1]), pack_bf16x2(y1[2], y1[3]));
       }
     }
-  } else {
-#pragma unroll
-    for (int p = 0; p < 16; ++p) y0[p] = y1[p] = 0.f;
+    fence_proxy_async_smem();
+    tc_fence_before();
+    warp_arrive(smem_u32(q_ready), threadIdx.x & 31);
   }
-  if (kFp8) {
-    // 64-byte rows; 16-byte chunk index XOR ((row >> 1) & 3); y0 of this group is chunk g, y1 chunk 2 + g
-    uint8_t* rowp = q_s + r * 64;
-    const int sw = (r >> 1) & 3;
-    *reinterpret_cast<uint4*>(rowp + ((g ^ sw) << 4)) =
-        make_uint4(pack_e4m3x4(y0[0], y0[1], y0[2], y0[3]), pack_e4m3x4(y0[4], y0[5], y0[6], y0[7]),
-                   pack_e4m3x4(y0[8], y0[9], y0[10], y0[11]), pack_e4m3x4(y0[12], y0[13], y0[14], y0[15]));
-    *reinterpret_cast<uint4*>(rowp + (((2 + g) ^ sw) << 4)) =
-        make_uint4(pack_e4m3x4(y1[0], y1[1], y1[2], y1[3]), pack_e4m3x4(y1[4], y1[5], y1[6], y1[7]),
-                   pack_e4m3x4(y1[8], y1[9], y1[10], y1[11]), pack_e4m3x4(y1[12], y1[13], y1[14], y1[15]));
-  } else {
-    // 128-byte rows; chunk XOR (row & 7); y0 of this group is chunks 2g, 2g+1, y1 chunks 4+2g, 5+2g
-    uint8_t* rowp = q_s + r * 128;
-    const int sw = r & 7;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      *reinterpret_cast<uint4*>(rowp + (((2 * g + c) ^ sw) << 4)) =
-          make_uint4(pack_bf16x2(y0[8 * c], y0[8 * c + 1]), pack_bf16x2(y0[8 * c + 2], y0[8 * c + 3]),
-                     pack_bf16x2(y0[8 * c + 4], y0[8 * c + 5]), pack_bf16x2(y0[8 * c + 6], y0[8 * c + 7]));
-      *reinterpret_cast<uint4*>(rowp + (((4 + 2 * g + c) ^ sw) << 4)) =
-          make_uint4(pack_bf16x2(y1[8 * c], y1[8 * c + 1]), pack_bf16x2(y1[8 * c + 2], y1[8 * c + 3]),
-                     pack_bf16x2(y1[8 * c + 4], y1[8 * c + 5]), pack_bf16x2(y1[8 * c + 6], y1[8 * c + 7]));
-    }
-  }
-  fence_proxy_async_smem();
-  tc_fence_before();
-  warp_arrive(smem_u32(q_ready), lane);
-}
+};
 
 // Keys from `valid` on of the 32 columns that start at c * 32 count nothing: -inf.
 __device__ __forceinline__ void mask_chunk(uint32_t (&s)[32], int c, int valid) {
