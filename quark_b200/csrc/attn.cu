@@ -52,9 +52,14 @@ constexpr int kSoftmaxRegs = 216;  // per thread, warps 4-11
 static_assert(128 * kCtrlRegs + 256 * kSoftmaxRegs <= kAttnThreads * kLaunchRegs, "register budget of the CTA");
 
 // Cluster splits: 2 groups x S CTAs leave 64 outputs, m, the row sum and whether they are to be used of each query row with the CTA that
-// writes the row (128 / S rows each), [2 S][rows][kMergePitch] f32.
-constexpr int kMergePitch = 68;
+// writes the row (128 / S rows each): 17 units of 16 bytes a row, [2 S][17][rows].  Neighbouring rows (the lanes of a pushing warp) are
+// neighbours, and each unit's rows are rotated so that the units of a row (the lanes that read them) lie in different banks.
+constexpr int kUnits = 17;
 __host__ __device__ constexpr int merge_rows(int splits) { return (kQTile + splits - 1) / splits; }
+__device__ __forceinline__ int merge_unit(int part, int u, int row, int rows) {
+  const int turned = row + u * (1 + (rows & 1));
+  return (part * kUnits + u) * rows + turned % rows;
+}
 
 template <bool kFp8, bool kCluster = false>
 struct AttnSmem {
@@ -74,13 +79,10 @@ struct AttnSmem {
   static constexpr int kQOff = 0;
   static constexpr int kKOff = kQOff + kQBytes;
   static constexpr int kVOff = kKOff + kKStages * kKBytes;
-  // A cluster's results: what this CTA has for each CTA's rows is laid out over its rings, what the others have for its rows arrives beside them.
-  static constexpr int kGiveOff = kKOff;
-  static constexpr int kMergeBytes = 266 * kMergePitch * 4;  // 2 groups, S CTAs, 128 / S rows each (7 CTAs need most)
-  static constexpr int kCombOff = kVOff + kVStages * kVBytes;  // where the groups meet | what the other CTAs have
+  static constexpr int kMergeBytes = 266 * kUnits * 16;        // 2 groups, S CTAs, 128 / S rows each (7 CTAs need most)
+  static constexpr int kCombOff = kVOff + kVStages * kVBytes;  // where the groups meet | the CTAs of a cluster (memory of its own, since others push early)
   static constexpr int kBarOff = kCombOff + (kCluster ? kMergeBytes : 2 * 34 * kQTile * 4);
   static constexpr int kTotal = kBarOff + 640 + 1024;
-  static_assert(!kCluster || kCombOff - kGiveOff >= kMergeBytes, "results laid out over the rings");
   static_assert(kKStages % 2 == 0 && kVStages % 2 == 0 && kTotal <= 227 * 1024, "see kKStages; shared memory of one CTA");
 };
 
@@ -93,7 +95,6 @@ struct AttnBars {
   uint64_t pv_done[2];      // [group] O += P(i) V(i) has finished
   uint64_t o_final[2];      // [group] every PV of a piece has finished
   uint64_t q_ready;
-  uint64_t merge_full;      // the other CTAs' results for this CTA's rows are here
   uint32_t tmem_slot;
   int abort_flag, drain_flag, exchange;
   float tm[16];  // cosines and sines of the temporal angles
@@ -247,12 +248,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_slot;
-  if (kSplit == kSplitCluster) {
-    // The bytes that will arrive are announced before the CTAs of the cluster tell one another that their barriers are there.
-    if (threadIdx.x == 0) mbar_arrive_expect_tx(smem_u32(&bars->merge_full), (gridDim.z - 1) * 2 * merge_rows(gridDim.z) * kMergePitch * 4);
-    __syncwarp();
-    cluster_arrive();
-  }
+  if (kSplit == kSplitCluster) cluster_arrive();  // this CTA is there (waited for before anyone pushes to it)
 
   QueryTile q;
   if (kSplit != kHelped && warp >= 4) q.request_angles(a, q0);
@@ -538,43 +534,34 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         read_o<kFp8>(tmem_o, o, l_run);
       }
       if constexpr (kSplit == kSplitCluster) {
-        // Both groups of every CTA of the cluster hand their rows to the CTA that writes them: laid out in shared memory, then one bulk copy
-        // per CTA and group, whose bytes the receiver's barrier counts.  (Pushed row by row between two cluster barriers the end took 10600
-        // of a launch's 23700 cycles at 360p; now 7900 of 21800, half of it the CTA with one tile more.)
+        // Both groups of every CTA of the cluster hand their rows to the CTA that writes them.  (Pushed with a row's 272 bytes together and
+        // between two cluster barriers, 32 rows an instruction, the end took 10600 of a launch's 23700 cycles at 360p; laid out per receiver
+        // and copied in bulk 7900.)
         const int S = static_cast<int>(gridDim.z), rows = merge_rows(S), cta = static_cast<int>(blockIdx.z);
         const int me = static_cast<int>(threadIdx.x) - 128;
-        float* give = reinterpret_cast<float*>(smem + L::kGiveOff);  // [CTA][group][rows]
-        const float* take = reinterpret_cast<const float*>(smem + L::kCombOff);  // [CTA][group][rows]
-        asm volatile("bar.sync 2, 256;" ::: "memory");  // the rings are free: both groups' tensor work, and with it the TMA traffic, is finished
+        const float4* parts = reinterpret_cast<const float4*>(smem + L::kCombOff);
+        cluster_wait();  // (long since)
         {
-          float* row = give + ((r / rows * 2 + g) * rows + r % rows) * kMergePitch;
+          const uint32_t base = map_to_cta(smem_u32(parts), r / rows);
+          auto push = [&](int u, float x, float y, float z, float w) {
+            st_dsmem_v4(base + 16u * merge_unit(2 * cta + g, u, r % rows, rows), __float_as_uint(x), __float_as_uint(y), __float_as_uint(z), __float_as_uint(w));
+          };
 #pragma unroll
-          for (int d = 0; d < 64; d += 4) *reinterpret_cast<float4*>(row + d) = make_float4(o[d], o[d + 1], o[d + 2], o[d + 3]);
+          for (int u = 0; u < 16; ++u) push(u, o[4 * u], o[4 * u + 1], o[4 * u + 2], o[4 * u + 3]);
           // where one of this CTA's waits ran out, the rows that its results belong to are not written by any CTA of the cluster
-          *reinterpret_cast<float4*>(row + 64) = make_float4(m_run, l_run, *abort_flag != 0 ? 1.0f : 0.0f, 0.0f);
+          push(16, m_run, l_run, *abort_flag != 0 ? 1.0f : 0.0f, 0.0f);
         }
-        fence_proxy_async_smem();
-        asm volatile("bar.sync 2, 256;" ::: "memory");
-        cluster_wait();  // (long since: every CTA's barriers are there)
-        if (me < 2 * S && me >> 1 != cta) {
-          const uint32_t bytes = static_cast<uint32_t>(rows * kMergePitch * 4);
-          bulk_copy_cluster(map_to_cta(smem_u32(take) + static_cast<uint32_t>(2 * cta + (me & 1)) * bytes, me >> 1), smem_u32(give) + static_cast<uint32_t>(me) * bytes, bytes,
-                            map_to_cta(smem_u32(&bars->merge_full), me >> 1));
-        }
-        __syncwarp();
+        cluster_arrive();
         const float vs = a.v_scale ? __ldg(a.v_scale + kvh) : 1.0f;
-        wait_warp(bars->merge_full, 0);
-        cluster_arrive();  // what the others copied here is here (see the end of the kernel)
-        const bool whole_cta = *abort_flag == 0;
-        for (int n = me; whole_cta && n < rows * 8; n += 256) {  // outputs d0 .. d0 + 3 and 32 more of a row per thread: no bank twice
-          const int rl = n >> 3, d0 = (n & 7) * 4, rr = cta * rows + rl;
+        cluster_wait();
+        for (int n = me; n < rows * 8; n += 256) {  // outputs d0 .. d0 + 3 and 32 more of a row per thread
+          const int rl = n >> 3, u = n & 7, d0 = 4 * u, rr = cta * rows + rl;
           if (rr >= kQTile || q0 + rr >= a.tpf) continue;
-          auto part_of = [&](int q) { return (q >> 1 == cta ? give : take) + (q * rows + rl) * kMergePitch; };
           float4 head[16];  // m, row sum, lost
           float m = -1.0e30f, lost = 0.f;
 #pragma unroll
           for (int q = 0; q < 16; ++q)
-            if (q < 2 * S) head[q] = *reinterpret_cast<const float4*>(part_of(q) + 64);
+            if (q < 2 * S) head[q] = parts[merge_unit(q, 16, rl, rows)];
 #pragma unroll
           for (int q = 0; q < 16; ++q)
             if (q < 2 * S) {
@@ -586,10 +573,9 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
 #pragma unroll
           for (int q = 0; q < 16; ++q)
             if (q < 2 * S) {
-              const float* part = part_of(q) + d0;
               const float w = ex2_approx(head[q].x - m);
               l = fmaf(w, head[q].y, l);
-              const float4 x = *reinterpret_cast<const float4*>(part), y = *reinterpret_cast<const float4*>(part + 32);
+              const float4 x = parts[merge_unit(q, u, rl, rows)], y = parts[merge_unit(q, u + 8, rl, rows)];
               e[0] = fmaf(w, x.x, e[0]); e[1] = fmaf(w, x.y, e[1]); e[2] = fmaf(w, x.z, e[2]); e[3] = fmaf(w, x.w, e[3]);
               e[4] = fmaf(w, y.x, e[4]); e[5] = fmaf(w, y.y, e[5]); e[6] = fmaf(w, y.z, e[6]); e[7] = fmaf(w, y.w, e[7]);
             }
@@ -677,13 +663,10 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     if (kSplit == kHelped && kr.tiles == 0) KeyShares::write_zeros(a, r, g, 2);
   }
 
-  if (kSplit == kSplitCluster) {
-    // No CTA leaves while its results are still being copied: the softmax warps of all have seen theirs arrive.
+  if (kSplit == kSplitCluster && warp < 4) {  // the softmax warps' barriers
     __syncwarp();
-    if (warp < 4) {
-      cluster_wait();
-      cluster_arrive();
-    }
+    cluster_wait();
+    cluster_arrive();
     cluster_wait();
   }
   tc_fence_before();

@@ -150,11 +150,6 @@ __device__ __forceinline__ void cluster_sync() {
 // Its two halves.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Shared memory of this CTA -> shared memory of another CTA of the cluster (`dst` and `bar`, of that CTA, in the cluster's shared window;
-// addresses and size multiples of 16 bytes); the barrier counts the bytes.
-__device__ __forceinline__ void bulk_copy_cluster(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
-}
 // Address in the cluster's shared window of what lies at `smem_addr` in the CTA of the given rank.
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t cta_rank) {
   uint32_t r;
