@@ -188,7 +188,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     uint32_t res[kResInRegs ? kMyChunks * 16 : 1];
     const int slice_rows = kBM / (clustered ? g.splits : 1), slice_row0 = clustered ? split * slice_rows : 0;  // rows this CTA finishes
     const bool one_gate = g.gate == nullptr || m0 / g.rows_per_gate == m_last / g.rows_per_gate;
-    uint4 pre[QKV || BN == 64 ? BN / 32 : 1][2];  // QKV: see qkv_prefetch; slices: the residuals of the 8-column groups this thread finishes
+    uint4 pre[QKV || BN == 64 ? 2 : 1][2];  // QKV: see qkv_fetch; slices: the residuals of the 8-column groups this thread finishes
+    QkvFrame fr{};  // QKV
     if (QKV || (clustered && one_gate)) {
       float* col = reinterpret_cast<float*>(smem + L::kColOffset);
       const int et = threadIdx.x - 64;
@@ -204,10 +205,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
       }
       if constexpr (QKV) {
-        const QkvFrame fr = qkv_frame(g.qkv);
-        if (et < 8) temporal_cos_sin(fr.ft, et, col + BN);
+        fr = qkv_frame(g.qkv);
+        qkv_share<BN>(g.qkv, fr, et, n0, reinterpret_cast<QkvShared*>(col + BN));
         if (blockIdx.x == 0 && blockIdx.y == 0 && split == 0 && et == 32) qkv_segments(g.qkv, fr);
-        qkv_prefetch<BN>(g, et, slice_row0, slice_rows, m0, n0, pre);
+        qkv_fetch<BN>(g, et, slice_row0, slice_rows, m0, n0, 0, pre[0]);
+        qkv_fetch<BN>(g, et, slice_row0, slice_rows, m0, n0, 1, pre[1]);
       } else if constexpr (BN == 64) {
         if (g.gate != nullptr) {
 #pragma unroll
@@ -368,8 +370,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
         if (ok) {
           const float4* parts = reinterpret_cast<const float4*>(smem + L::kSliceOffset);
-          if (g.qkv.kv_fp8) qkv_finish<BN, true>(g, parts, vt, col, col + BN, clustered ? g.splits : 1, slice_row0, slice_rows, m0, n0, pre);
-          else qkv_finish<BN, false>(g, parts, vt, col, col + BN, clustered ? g.splits : 1, slice_row0, slice_rows, m0, n0, pre);
+          if (g.qkv.kv_fp8) qkv_finish<BN, true>(g, parts, vt, col, reinterpret_cast<const QkvShared*>(col + BN), fr, clustered ? g.splits : 1, slice_row0, slice_rows, m0, n0, pre);
+          else qkv_finish<BN, false>(g, parts, vt, col, reinterpret_cast<const QkvShared*>(col + BN), fr, clustered ? g.splits : 1, slice_row0, slice_rows, m0, n0, pre);
         }
       }
     } else if (clustered) {

@@ -319,7 +319,12 @@ __device__ __forceinline__ void epilogue16(const GemmArgs& g, const uint32_t (&r
 // cosines and four sines.  Arithmetic, rounding points and summation order are those of qkv_post.cu (and through it of
 // head_rmsnorm, value_residual_packed and kv_cache_update), so the bytes written are the same.  V is transposed through
 // shared memory, two channels at a time.
-// With one thread per (token, head) and 64 elements each this epilogue took 3.7 us more than the plain one (720p, e4m3).
+// What bounds it is the chain of one round (about 0.4 us for a Q head: sum, shuffles, square root, reciprocal) and, before this
+// was a loop, fetching its instructions: they run once per launch, after other kernels have had the instruction caches.  In a
+// frame the rounds unrolled, with the divisions by run-time sizes and the loads of the cache scales in each of them, took 4.9 us
+// (Q heads 4.5, V heads 7.9) at 720p bf16 and 3.2 (V heads 5.2) at 360p; as a loop on shifts, with what the rounds share
+// prepared while the main loop runs, 2.4 (2.1, 3.8) and 2.5 (2.8).  Two rounds side by side were slower again (2.7): more
+// instructions.
 
 struct QkvFrame {  // where this frame's rows go
   int ft, slot, L, cap, tpf_c;
@@ -364,27 +369,41 @@ __device__ __forceinline__ int qkv_kind(const QkvTail& q, int col) {  // 0 Q, 1 
   return col < q.n_q_heads * 64 ? 0 : col < (q.n_q_heads + q.n_kv_heads) * 64 ? 1 : 2;
 }
 
-// While the main loop runs: what the rounds of qkv_finish need from global memory (cosines and sines of a K head's positions,
-// or the first block's V).
+__device__ __forceinline__ int log2i(int x) { return 31 - __clz(x); }  // x: a power of two
+
+// What the rounds of qkv_finish share, in shared memory before the main loop ends: the frame's temporal cosines and sines, the
+// reciprocals of the cache scales of the tile's heads (1 without scales: multiplying by it changes no bit) and the mix factor.
+struct QkvShared {
+  float tm[16], inv[2], lam;
+};
 template <int BN>
-__device__ __forceinline__ void qkv_prefetch(const GemmArgs& g, int et, int row0, int rows, int m0, int n0, uint4 (&pre)[BN / 32][2]) {
+__device__ __forceinline__ void qkv_share(const QkvTail& q, const QkvFrame& f, int et, int n0, QkvShared* sh) {
+  if (et < 8) temporal_cos_sin(f.ft, et, sh->tm);
+  if (et >= 32 && et < 32 + BN / 64) {
+    const int head = (n0 >> 6) + et - 32 - q.n_q_heads, vh = head - q.n_kv_heads;
+    const float* sc = vh >= 0 ? q.v_scale : q.k_scale;
+    sh->inv[et - 32] = sc != nullptr && head >= 0 && vh < q.n_kv_heads ? __fdiv_rn(1.0f, __ldg(sc + (vh >= 0 ? vh : head))) : 1.0f;
+  }
+  if (et == 64) sh->lam = q.qkv_first != nullptr ? *after_wait(q.lamb) : 0.f;
+}
+
+// What round k of qkv_finish needs from global memory: cosines and sines of a K head's positions, or the first block's V.
+template <int BN>
+__device__ __forceinline__ void qkv_fetch(const GemmArgs& g, int et, int row0, int rows, int m0, int n0, int k, uint4 (&pre)[2]) {
   const QkvTail& q = g.qkv;
-#pragma unroll
-  for (int k = 0; k < BN / 32; ++k) {
-    pre[k][0] = pre[k][1] = make_uint4(0u, 0u, 0u, 0u);
-    const int idx = et + 256 * k, l = idx & 3, rh = idx >> 2;
-    const int hd = rh / rows, t = m0 + row0 + rh % rows, col = n0 + hd * 64;
-    if (hd >= BN / 64 || t >= g.M || col >= g.N) continue;
-    const int kind = qkv_kind(q, col);
-    if (kind == 1 && l < 2) {
-      const uint4* rp = reinterpret_cast<const uint4*>(q.rope_xy + static_cast<size_t>(t) * 16);
-      pre[k][0] = __ldg(rp + l);
-      pre[k][1] = __ldg(rp + 2 + l);
-    } else if (kind == 2 && q.qkv_first != nullptr) {  // written earlier in this pass
-      const uint4* fp = reinterpret_cast<const uint4*>(after_wait(q.qkv_first) + static_cast<size_t>(t) * g.N + col + 16 * l);
-      pre[k][0] = fp[0];
-      pre[k][1] = fp[1];
-    }
+  pre[0] = pre[1] = make_uint4(0u, 0u, 0u, 0u);
+  const int idx = et + 256 * k, l = idx & 3, rh = idx >> 2;
+  const int hd = rh >> log2i(rows), t = m0 + row0 + (rh & (rows - 1)), col = n0 + hd * 64;
+  if (hd >= BN / 64 || t >= g.M || col >= g.N) return;
+  const int kind = qkv_kind(q, col);
+  if (kind == 1 && l < 2) {
+    const uint4* rp = reinterpret_cast<const uint4*>(q.rope_xy + static_cast<size_t>(t) * 16);
+    pre[0] = __ldg(rp + l);
+    pre[1] = __ldg(rp + 2 + l);
+  } else if (kind == 2 && q.qkv_first != nullptr) {  // written earlier in this pass
+    const uint4* fp = reinterpret_cast<const uint4*>(after_wait(q.qkv_first) + static_cast<size_t>(t) * g.N + col + 16 * l);
+    pre[0] = fp[0];
+    pre[1] = fp[1];
   }
 }
 
@@ -392,20 +411,24 @@ __device__ __forceinline__ void qkv_prefetch(const GemmArgs& g, int et, int row0
 // slices: the partial sums are in `partials` and `vt` (pitch 72) takes the V rows.  `col` holds the tile's per-column scales, `tm`
 // the frame's temporal cosines and sines.  Run by the 256 epilogue threads together.
 template <int BN, bool kCacheFp8>
-__device__ __forceinline__ void qkv_finish(const GemmArgs& g, const float4* partials, uint16_t* vt, const float* col, const float* tm, int splits, int row0, int rows, int m0,
-                                           int n0, const uint4 (&pre)[BN / 32][2]) {
+__device__ __forceinline__ void qkv_finish(const GemmArgs& g, const float4* partials, uint16_t* vt, const float* col, const QkvShared* sh, const QkvFrame& fr, int splits, int row0,
+                                           int rows, int m0, int n0, uint4 (&pre)[2][2]) {
   constexpr int kEs = kCacheFp8 ? 1 : 2;
   const QkvTail& q = g.qkv;
-  const QkvFrame fr = qkv_frame(q);
-  const int et = threadIdx.x - 64;
+  const int et = threadIdx.x - 64, lrows = log2i(rows), lquilt = log2i(q.quilt);
   const int k_off = q.n_q_heads * 64, v_off = (q.n_q_heads + q.n_kv_heads) * 64;
   const bool mix = q.qkv_first != nullptr;
-  const float lam = mix ? *after_wait(q.lamb) : 0.f;
+  const float lam = sh->lam;
   const int vpitch = splits == 1 ? BN + 8 : 72;
-#pragma unroll
-  for (int k = 0; k < BN / 32; ++k) {
+  const int rounds = max(rows * (BN / 64) / 64, 1);
+#pragma unroll 1
+  for (int k = 0; k < rounds; ++k) {
+    const uint4 p0 = pre[0][0], p1 = pre[0][1];
+    pre[0][0] = pre[1][0];
+    pre[0][1] = pre[1][1];
+    if (k + 2 < rounds) qkv_fetch<BN>(g, et, row0, rows, m0, n0, k + 2, pre[1]);
     const int idx = et + 256 * k, l = idx & 3, rh = idx >> 2;
-    const int hd = rh / rows, row = rh % rows, t = m0 + row0 + row, c0 = n0 + hd * 64;
+    const int hd = rh >> lrows, row = rh & (rows - 1), t = m0 + row0 + row, c0 = n0 + hd * 64;
     if (hd >= BN / 64 || c0 >= g.N) continue;  // uniform over the warp
     const int kind = qkv_kind(q, c0);
     uint16_t* staged = vt + row * vpitch + hd * 64 + 16 * l;
@@ -446,7 +469,7 @@ __device__ __forceinline__ void qkv_finish(const GemmArgs& g, const float4* part
 #pragma unroll
       for (int j = 0; j < 8; ++j) o[j] = pack_bf16x2(__fmul_rn(f[2 * j], inv), __fmul_rn(f[2 * j + 1], inv));
     } else if (mix) {
-      const uint32_t vf[8] = {pre[k][0].x, pre[k][0].y, pre[k][0].z, pre[k][0].w, pre[k][1].x, pre[k][1].y, pre[k][1].z, pre[k][1].w};
+      const uint32_t vf[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float a = f[2 * j], b = f[2 * j + 1];
@@ -463,20 +486,20 @@ __device__ __forceinline__ void qkv_finish(const GemmArgs& g, const float4* part
     if (t >= g.M) continue;
     st_global_v8(static_cast<uint16_t*>(g.C) + static_cast<size_t>(t) * g.N + c0 + 16 * l, o);
     const int tq = t - q.qoff;
-    if (kind == 1 && tq >= 0 && tq % q.quilt == 0) {  // this token is one of those the cache keeps
+    if (kind == 1 && tq >= 0 && (tq & (q.quilt - 1)) == 0) {  // this token is one of those the cache keeps
       // rotate what the stand-alone append would read back (the bf16-rounded normalised K): thread l holds pairs 8 l .. 8 l + 7,
       // whose angles are 4 (x, y, or half of the temporal ones); a cache row is the pairs' first outputs, then their second
-      const int head = (c0 - k_off) >> 6, tc = tq / q.quilt;
-      const float inv_k = q.k_scale != nullptr ? __fdiv_rn(1.0f, __ldg(q.k_scale + head)) : 1.0f;  // * 1 changes no bit
+      const int head = (c0 - k_off) >> 6, tc = tq >> lquilt;
+      const float inv_k = sh->inv[hd];
       float cs[4], sn[4];
       if (l < 2) {
-        cs[0] = __uint_as_float(pre[k][0].x); cs[1] = __uint_as_float(pre[k][0].y); cs[2] = __uint_as_float(pre[k][0].z); cs[3] = __uint_as_float(pre[k][0].w);
-        sn[0] = __uint_as_float(pre[k][1].x); sn[1] = __uint_as_float(pre[k][1].y); sn[2] = __uint_as_float(pre[k][1].z); sn[3] = __uint_as_float(pre[k][1].w);
+        cs[0] = __uint_as_float(p0.x); cs[1] = __uint_as_float(p0.y); cs[2] = __uint_as_float(p0.z); cs[3] = __uint_as_float(p0.w);
+        sn[0] = __uint_as_float(p1.x); sn[1] = __uint_as_float(p1.y); sn[2] = __uint_as_float(p1.z); sn[3] = __uint_as_float(p1.w);
       } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          cs[i] = tm[4 * (l - 2) + i];
-          sn[i] = tm[8 + 4 * (l - 2) + i];
+          cs[i] = sh->tm[4 * (l - 2) + i];
+          sn[i] = sh->tm[8 + 4 * (l - 2) + i];
         }
       }
       float y0[8], y1[8];
@@ -516,25 +539,25 @@ __device__ __forceinline__ void qkv_finish(const GemmArgs& g, const float4* part
   // neighbouring token vectors so that whole 32-byte sectors are written.  The tile's cached tokens are its rows qoff,
   // qoff + quilt, ... (m0 + row0 is a multiple of the quilt factor).
   constexpr int kTokPerVec = 16 / kEs;
-  const int vec_per_ch = rows / q.quilt / kTokPerVec;
-  const int jw = min(vec_per_ch, 2);
+  const int vec_per_ch = (rows >> lquilt) / kTokPerVec;
+  const int ljw = vec_per_ch > 1 ? 1 : 0;  // two vectors (a whole sector) side by side where there are two
   uint8_t* vc = static_cast<uint8_t*>(q.Vt_cache);
 #pragma unroll 1
   for (int hd = 0; hd < BN / 64; ++hd) {
     const int c0 = n0 + hd * 64;
     if (c0 < v_off || c0 >= g.N) continue;
     const int head = (c0 - v_off) >> 6;
-    const float inv_v = q.v_scale != nullptr ? __fdiv_rn(1.0f, __ldg(q.v_scale + head)) : 1.0f;
+    const float inv_v = sh->inv[hd];
     const uint16_t* src = vt + hd * 64;
 #pragma unroll 1
     for (int v = et; v < 32 * vec_per_ch; v += 256) {
-      const int d = v / jw % 32 * 2, j = v / (32 * jw) * jw + v % jw;
+      const int d = ((v >> ljw) & 31) * 2, j = ((v >> (5 + ljw)) << ljw) + (v & ljw);
       const int c1 = j * kTokPerVec;                      // first cached token of the vector, inside these rows
-      const int c_abs = (m0 + row0) / q.quilt + c1;       // ... and inside the frame's cached tokens
+      const int c_abs = ((m0 + row0) >> lquilt) + c1;       // ... and inside the frame's cached tokens
       if (c_abs + kTokPerVec > fr.tpf_c) continue;
       uint32_t x[kTokPerVec];
 #pragma unroll
-      for (int i = 0; i < kTokPerVec; ++i) x[i] = *reinterpret_cast<const uint32_t*>(src + (q.qoff + (c1 + i) * q.quilt) * vpitch + d);
+      for (int i = 0; i < kTokPerVec; ++i) x[i] = *reinterpret_cast<const uint32_t*>(src + (q.qoff + ((c1 + i) << lquilt)) * vpitch + d);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         uint32_t w[4];
