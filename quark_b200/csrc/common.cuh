@@ -33,6 +33,8 @@ unsigned int* status_word();
 // Kernels launched by this library since it was loaded (qb_kernel_launch_count).
 extern unsigned long long g_launch_count;
 
+int num_sms();  // of the current device (gemm.cu)
+
 inline int32_t check_launch(const char* what) {
   ++g_launch_count;
   cudaError_t e = cudaGetLastError();

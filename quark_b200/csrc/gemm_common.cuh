@@ -595,7 +595,6 @@ struct GemmPlan {
   size_t counters_bytes, aq_bytes, partial_bytes;
 };
 
-int num_sms();
 // Tensor maps and launch of the grouped kernel, and of the pair kernel for a plan with cg == 2.
 int32_t launch_gemm_grouped(int bn, const void* A, const void* B, int n_experts, const GemmArgs& g, bool fp8, cudaStream_t st);
 int32_t launch_gemm_pair(const GemmPlan& pl, const void* A, const void* B, const GemmArgs& g, bool fp8, cudaStream_t st);
