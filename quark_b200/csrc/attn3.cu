@@ -21,7 +21,7 @@
 // hence three groups.  A loop with the same softmax instructions and nothing else takes 965 cycles per tile with three warps per
 // scheduler (1180 with all exponentials on the special-function unit), this kernel 1330.  The K and V rings are separate and the loads
 // run ahead of the S that runs ahead of the PV: with one ring a stage was held from S to PV, and the next K tiles came too late.
-// 720p, us per launch: 60.4 -> 53.9 at 16 buckets, 210 -> 200 at 64, 394 -> 368 at 128.
+// 720p, us per launch: 60.4 -> 52.9 at 16 buckets, 211 -> 204 at 64, 394 -> 382 at 128.
 // Tried and dropped: a whole m (P's rounding is then the same for every m, but the key that m came from no longer has a probability of
 // exactly 1: 8 % more error); e4m3 in this form (44.5 against 42.0 us at 720p); key splits in this form (360p bf16 12.8 against 13.5 us,
 // but one m for all keys of a CTA makes 2 % more error than one per group); kSlack 8 (52.4 against 53.8 us at 720p, 3 % more error

@@ -55,6 +55,36 @@ def test_attention_key_shares_by_size(qb, kv_dt, H, W, Hk, gqa, nb, ft):
 
 
 @pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
+@pytest.mark.parametrize("H,W,ft", [
+    (8, 8, 0),  # half of one key tile: two of three groups have nothing
+    (8, 8, 1),  # two segments in one tile
+    (16, 8, 2),  # a tile for each of three groups, an odd number for two
+    (16, 8, 3),
+    (12, 20, 4),  # nine tiles and a remainder, a query tile of 112 rows
+    (17, 16, 5),
+])  # fmt: skip
+def test_attention_groups_over_tiles_whose_maximum_jumps(qb, kv_dt, H, W, ft):
+    """The groups of a CTA, and the CTAs that share an item (clusters of odd size among them), take key tiles in turn; the scores grow
+    and shrink from tile to tile by far more than the slack within which a maximum is kept.  Against the oracle fed the rotated
+    query as the kernel narrows it, as for scores that drift, with that test's tolerance."""
+    r = util.rng([97, H, ft])
+    Hk, gqa, nb = 2, 2, 6
+    tpf, cap = H * W, (nb + 1) * H * W
+    qkv = ops.head_rmsnorm(bf16_randn(r, (tpf, 8 * 64)), n_q_heads=4, n_kv_heads=2)
+    step = np.array([0.3, 6.0, 1.0, 14.0, 0.1, 9.0, 13.0], np.float32)[np.arange(cap) // 128 % 7]
+    to = codec.f32_to_bf16 if kv_dt == "bf16" else codec.f32_to_e4m3
+    Kc = to((r.standard_normal((Hk, cap, 64), dtype=np.float32) * step[None, :, None]).reshape(Hk * cap, 64))
+    Vc = to(r.standard_normal((Hk * 64, cap), dtype=np.float32))
+    segs, n = ops.compute_segments(ft, nb, tpf, 1)
+    with codec.bf16_rounding("rne"):
+        want = ops.owl_attn(qkv, Kc, Vc, segs, [n], ft, n_kv_heads=Hk, gqa_ratio=gqa, H_spatial=H, W_spatial=W, kv_dtype=kv_dt, q_quant=kv_dt)
+    args = (T(qb, qkv, "bf16"), T(qb, Kc, kv_dt), T(qb, Vc, kv_dt), T(qb, np.asarray(segs, np.int32)), T(qb, np.array([n], np.int32)), 1, Hk, gqa, H, W, nb, 1)
+    kw = dict(compute_dtype="e4m3" if kv_dt == "e4m3" else None, packed_qkv=True, frame_t=T(qb, np.array([ft], np.int32)))
+    for splits in (1, 2, 3, 5, 7):
+        _attn_check(qb.qf.owl_attn(*args, kv_splits=splits, **kw).to_numpy(), want, f"attn {H}x{W} ft={ft} splits={splits} {kv_dt}", kv_dt == "e4m3")
+
+
+@pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
 @pytest.mark.parametrize("Hk,nb", [(1, 16), (24, 64)])  # key splits in clusters, one CTA per item (helpers want a workspace)
 def test_attention_call_without_a_workspace(qb, kv_dt, Hk, nb):
     import ctypes as C
@@ -430,3 +460,20 @@ def test_calls_made_in_c_equal_the_python_path(qb, monkeypatch):
         with pytest.raises(kind):
             c()
     assert f32(first[0], "bf16").any()
+
+
+@pytest.mark.parametrize("rows", [1, 148, 149])  # up to a row per SM, and more
+@pytest.mark.parametrize("D", [8, 2048, 2056, 4104, 8192])  # one, two and four vectors a thread, rows that end inside one
+def test_ada_rmsnorm_rows_and_widths(qb, rows, D):
+    r = util.rng([98, rows, D])
+    X, s, b = bf16_randn(r, (rows, D)), bf16_randn(r, (1, D), 0.1), bf16_randn(r, (1, D), 0.1)
+    outq = qb.QuarkTensor.empty(rows, D, dtype="e4m3")
+    args = (T(qb, X, "bf16"), T(qb, s, "bf16"), T(qb, b, "bf16"))
+    first = qb.qf.ada_rmsnorm(*args, out_q=outq)
+    got, want = first.to_numpy(), ops.ada_rmsnorm(X, s, b)
+    # (the tolerance of the norm's own test: the sums differ in order only)
+    assert np.percentile(util.bf16_ulp_diff(got, want), 99.9) <= 1
+    np.testing.assert_array_equal(outq.to_numpy(), codec.f32_to_e4m3(codec.bf16_to_f32(got)))
+    # in a chain each call waits for the one before it
+    again = qb.qf.ada_rmsnorm(qb.qf.ada_rmsnorm(*args), *args[1:]).to_numpy()
+    assert np.percentile(util.bf16_ulp_diff(again, ops.ada_rmsnorm(got, s, b)), 99.9) <= 1
