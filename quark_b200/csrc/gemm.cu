@@ -262,14 +262,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const bool has_gate = g.gate != nullptr;
       const bool has_scale = g.a_scale != nullptr || g.w_scale != nullptr;
       const bool has_bias = g.bias != nullptr;
-      uint32_t rbuf[2][32];  // this warp's next chunk is on its way from TMEM while the current one is processed
-      tmem_ld32(taddr + half * 32, rbuf[0]);
-#pragma unroll
+      // One or two chunks to a warp: unrolled, the next one on its way from TMEM while the current one is processed.  The four of a
+      // 256-column tile: a loop, since its instructions, run once per launch, cost more to fetch than the loads from TMEM to wait for
+      // (512 x 8192 x 2048 e4m3 SiLU 9.27 -> 8.79 us, 512 x 4096 x 512 5.77 -> 5.60 e4m3, 8.72 -> 8.62 bf16).  Two as a loop: SiLU 6.04 ->
+      // 5.91 us (512 x 4096 x 2048, 128-column tiles), but with gate and residual, whose registers then move, 6.53 -> 6.60.
+      constexpr bool kRolled = kMyChunks > 2;
+      constexpr int kUnroll = kRolled ? 1 : kMyChunks;
+      uint32_t rbuf[kRolled ? 1 : 2][32];
+      if (!kRolled) tmem_ld32(taddr + half * 32, rbuf[0]);
+#pragma unroll kUnroll
       for (int lc = 0; lc < kMyChunks; ++lc) {
         const int c = 2 * lc + half;
-        tmem_wait_ld_into(rbuf[lc & 1]);
-        if (lc + 1 < kMyChunks) tmem_ld32(taddr + (c + 2) * 32, rbuf[(lc + 1) & 1]);
-        const uint32_t(&r)[32] = rbuf[lc & 1];
+        uint32_t(&r)[32] = rbuf[kRolled ? 0 : lc & 1];
+        if (kRolled) tmem_ld32(taddr + c * 32, r);
+        tmem_wait_ld_into(r);
+        if (!kRolled && lc + 1 < kMyChunks) tmem_ld32(taddr + (c + 2) * 32, rbuf[kRolled ? 0 : (lc + 1) & 1]);
         const int n = n0 + c * 32;
         if (m < g.M && n < g.N) {
           float v[32];
