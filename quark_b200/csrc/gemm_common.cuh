@@ -408,8 +408,8 @@ __device__ __forceinline__ void qkv_fetch(const GemmArgs& g, int et, int row0, i
 }
 
 // Rows [row0, row0 + rows) of the tile to the packed QKV and the caches.  One K slice: the tile is in `vt` (pitch BN + 8); S
-// slices: the partial sums are in `partials` and `vt` (pitch 72) takes the V rows.  `col` holds the tile's per-column scales, `tm`
-// the frame's temporal cosines and sines.  Run by the 256 epilogue threads together.
+// slices: the partial sums are in `partials` and `vt` (pitch 72) takes the V rows.  `col` holds the tile's per-column scales, `sh`
+// what qkv_share left there, `pre` the first two rounds' qkv_fetch.  Run by the 256 epilogue threads together.
 template <int BN, bool kCacheFp8>
 __device__ __forceinline__ void qkv_finish(const GemmArgs& g, const float4* partials, uint16_t* vt, const float* col, const QkvShared* sh, const QkvFrame& fr, int splits, int row0,
                                            int rows, int m0, int n0, uint4 (&pre)[2][2]) {
