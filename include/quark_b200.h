@@ -276,11 +276,11 @@ typedef struct {
 
 /* e4m3 probabilities: by default every second exponential of a score row is built on the FMA pipe as
  * 2^floor(x) * (1 + frac(x) - 0.052) (relative error -5.2 % .. +2.3 %, below the 6.25 % an e4m3 code spans) so that
- * the special-function unit is not the kernel's bottleneck; on = 1 computes three of four with ex2.approx, as the
- * reference kernel does (ref: src/quark/kernels/owl_attn/kernel.py:587-614), and every fourth with a polynomial of relative error
- * 2.7e-6, at about 24 % more time per call.
+ * the special-function unit is not the kernel's bottleneck; on = 1 computes every one with ex2.approx, as the
+ * reference kernel does (ref: src/quark/kernels/owl_attn/kernel.py:587-614), at up to 38 % more time per call.  NaN among the
+ * scores always reaches the output then; by default only at even positions (the chord's clamp takes it at odd ones).
  * Process-wide; returns the previous setting.  QB_ATTN_EXACT_EXP=1 in the environment sets it at load time.
- * bf16 attention always does the latter. */
+ * bf16 attention has no such setting: it takes every fourth from a polynomial of relative error 2.7e-6. */
 int32_t qb_set_attn_exact_exp(int32_t on);
 
 /* Workspace of qb_owl_attn.  It starts with one ticket per (query tile, head) in a fixed 16 KiB area (so calls of different

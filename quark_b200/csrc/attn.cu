@@ -107,15 +107,15 @@ static_assert(sizeof(AttnBars) <= 640, "kBarOff + 640");
 __device__ __forceinline__ int group_tiles(int end, int g) { return (end - g + 1) >> 1; }
 
 // 32 scores of one row -> packed probabilities 2^(score * sl2 + nshift); bf16: `sum` grows by the rounded ones.  e4m3 makes every second
-// one by the chord of ex2_lin_from_biased (kLin); without the chord every fourth comes from the polynomial, since the special-function
-// unit would be the bound (e4m3, 720p: 56.6 -> 52.0 us; bf16, 360p: 14.2 -> 13.5).
+// one by the chord of ex2_lin_from_biased (kLin), or none: the setting is there for ex2.approx throughout (720p: 57.0 us; every fourth by the
+// polynomial took 50.9).  bf16 takes every fourth from the polynomial, since the special-function unit would be the bound (360p: 14.2 -> 13.5).
 template <bool kFp8, bool kLin>
 __device__ __forceinline__ void p_chunk(const uint32_t (&s)[32], uint64_t sl2, uint64_t nshift, uint32_t* w, uint64_t (&sum)[2]) {
   float e[32];
 #pragma unroll
   for (int q = 0; q < 32; q += 2) {
     fma_f32x2(e[q], e[q + 1], s[q], s[q + 1], sl2, nshift);
-    if (!kLin && (q & 7) == 6) {
+    if (!kFp8 && (q & 7) == 6) {
       ex2_poly_f32x2(e[q], e[q + 1]);
       continue;
     }

@@ -1,0 +1,66 @@
+"""The exponentials of attention: e4m3 kernels set to ``ex2.approx`` lose no score that is not finite."""
+
+import numpy as np
+import pytest
+
+from oracle import codec, ops
+from tests import util
+from tests.test_gpu_kernels import T, f32, qb  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+# a cluster of key splits, one CTA per item, splits through the workspace, helpers
+FORMS = [(12, 12, 8, 2, 11, 0), (12, 12, 8, 2, 11, 1), (12, 12, 8, 2, 11, 16), (8, 8, 16, 5, 240, 0)]
+
+
+@pytest.mark.parametrize("kv_dt", ["e4m3"])
+@pytest.mark.parametrize("H,W,Hk,gqa,nb,splits", FORMS)
+def test_a_key_that_is_not_finite_is_seen_at_every_position(qb, kv_dt, H, W, Hk, gqa, nb, splits):  # noqa: F811
+    """A KV head holds one bad value in a key at position h of eight, somewhere or among the last keys (where tiles are masked).  NaN: all of the
+    head's outputs are NaN.  Infinity (bf16): NaN where the score is +inf, and where it is -inf the bits that any score far below gives.  The
+    other heads' bits do not change."""
+    r = util.rng([77, H, nb])
+    tpf, Hq, cap, ft = H * W, Hk * gqa, (nb + 1) * H * W, 1000
+    make = util.bf16_randn if kv_dt == "bf16" else util.e4m3_randn
+    qkv = util.bf16_randn(r, (tpf, (Hq + 2 * Hk) * 64))
+    Kc, Vc = make(r, (Hk * cap, 64)), make(r, (Hk * 64, cap))
+    segs, n = ops.compute_segments(ft, nb, tpf, 1)
+    keys = np.concatenate([np.arange(segs[2 * i], segs[2 * i] + segs[2 * i + 1]) for i in range(n)])
+    channel = 5
+    anywhere = [h * cap + int(r.choice(keys[keys % 8 == h % 8])) for h in range(Hk)]
+    at_the_end = [h * cap + int(keys[-8 + h % 8]) for h in range(Hk)]
+
+    def run(K):
+        return qb.qf.owl_attn(T(qb, qkv, "bf16"), T(qb, K, kv_dt), T(qb, Vc, kv_dt), T(qb, np.asarray(segs, np.int32)), T(qb, np.array([n], np.int32)), 1, Hk, gqa, H, W,
+                              nb, 1, compute_dtype=kv_dt, packed_qkv=True, frame_t=T(qb, np.array([ft], np.int32)), kv_splits=splits).to_numpy().reshape(tpf, Hk, gqa * 64)  # fmt: skip
+
+    def planted(value, rows, which):
+        K = Kc.copy()
+        for h in which:
+            K[rows[h], channel] = value
+        return run(K)
+
+    was = qb._lib.set_attn_exact_exp(True)
+    try:
+        clean = run(Kc)
+        for rows, which in ((anywhere, range(Hk)), (at_the_end, range(Hk)), (anywhere, range(0, Hk, 3))):
+            got = planted(0x7FC0 if kv_dt == "bf16" else 0x7F, rows, which)
+            for h in range(Hk):
+                if h in which:
+                    assert np.isnan(f32(got[:, h], "bf16")).all(), h
+                else:
+                    np.testing.assert_array_equal(got[:, h], clean[:, h])
+        if kv_dt == "e4m3":
+            return
+        q = f32(qkv[:, : Hq * 64], "bf16").reshape(tpf, Hq, 64).transpose(1, 0, 2)
+        cos, sin = ops.rope_tables(H, W, ft, 64)
+        y = ops.apply_rope(q, cos[None], sin[None])[..., channel].T.reshape(tpf, Hk, gqa)  # the sign of the score
+        low, high = y < -0.05, y > 0.01
+        assert low.any() and high.any()
+        for rows in (anywhere, at_the_end):
+            got = planted(0x7F80, rows, range(Hk)).reshape(tpf, Hk, gqa, 64)
+            far = planted(int(codec.f32_to_bf16(np.array([1e6], np.float32))[0]), rows, range(Hk)).reshape(got.shape)
+            assert np.isnan(f32(got, "bf16"))[high].all() and np.isfinite(f32(got, "bf16"))[low].all()
+            np.testing.assert_array_equal(got[low], far[low])
+    finally:
+        qb._lib.set_attn_exact_exp(was)
