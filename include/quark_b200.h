@@ -280,7 +280,7 @@ typedef struct {
  * reference kernel does (ref: src/quark/kernels/owl_attn/kernel.py:587-614), at up to 38 % more time per call.  NaN among the
  * scores always reaches the output then; by default only at even positions (the chord's clamp takes it at odd ones).
  * Process-wide; returns the previous setting.  QB_ATTN_EXACT_EXP=1 in the environment sets it at load time.
- * bf16 attention has no such setting: it takes every fourth from a polynomial of relative error 2.7e-6. */
+ * bf16 attention has no such setting: it takes every fourth from a polynomial of relative error 1.7e-7 (ex2.approx: 2^-22). */
 int32_t qb_set_attn_exact_exp(int32_t on);
 
 /* Workspace of qb_owl_attn.  It starts with one ticket per (query tile, head) in a fixed 16 KiB area (so calls of different

@@ -209,8 +209,9 @@ __device__ __forceinline__ float sum_f32x2(uint64_t a, uint64_t b) {
   return (a0 + a1) + (b0 + b1);
 }
 // 2^x for two values on the FMA and integer pipes: x = n + f with n = round(x) in the low mantissa bits of x + 1.5 * 2^23, a
-// polynomial for 2^f on [-0.5, 0.5] (least squares, weighted until the relative error is level: 2.7e-6, a thousandth of what a bf16
-// probability resolves), n added to the exponent field.  x is clamped at -126: what underflows becomes 2^-126 instead of 0.
+// polynomial for 2^f on [-0.5, 0.5] (least squares with 2^0 = 1 held, weighted until the relative error is level: 9.1e-8, evaluated in f32
+// 1.7e-7, below the 2^-22 of ex2.approx; a degree less made 2.7e-6 of it), n added to the exponent field.  x is clamped at -126: what
+// underflows becomes 2^-126 instead of 0.
 __device__ __forceinline__ void ex2_poly_f32x2(float& x0, float& x1) {
   x0 = fmaxf(x0, -126.0f);
   x1 = fmaxf(x1, -126.0f);
@@ -220,11 +221,12 @@ __device__ __forceinline__ void ex2_poly_f32x2(float& x0, float& x1) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(x), "l"(magic));
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(f) : "l"(t), "l"(nmagic));
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(f) : "l"(f), "l"(none), "l"(x));
-  p = pack_f32x2(0.00957010034f, 0.00957010034f);
-  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.0559178591f, 0.0559178591f)));
-  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.240247443f, 0.240247443f)));
-  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.693121791f, 0.693121791f)));
-  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.999999285f, 0.999999285f)));
+  p = pack_f32x2(0.0013264727f, 0.0013264727f);
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.009671513f, 0.009671513f)));
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.055507336f, 0.055507336f)));
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.24022242f, 0.24022242f)));
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.693147f, 0.693147f)));
+  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(1.0f, 1.0f)));
   uint32_t t0, t1, p0, p1;
   asm("mov.b64 {%0, %1}, %2;" : "=r"(t0), "=r"(t1) : "l"(t));
   asm("mov.b64 {%0, %1}, %2;" : "=r"(p0), "=r"(p1) : "l"(p));

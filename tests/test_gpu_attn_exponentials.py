@@ -1,4 +1,10 @@
-"""The exponentials of attention: e4m3 kernels set to ``ex2.approx`` lose no score that is not finite."""
+"""The exponentials of attention: the polynomial is as close as ``ex2.approx``, and e4m3 kernels set to ``ex2.approx`` lose no score that is
+not finite."""
+
+import ctypes
+import shutil
+import subprocess
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -8,6 +14,58 @@ from tests import util
 from tests.test_gpu_kernels import T, f32, qb  # noqa: F401
 
 pytestmark = pytest.mark.gpu
+
+CSRC = Path(__file__).resolve().parent.parent / "quark_b200" / "csrc"
+# a thread takes a pair of x[0 .. n): both functions of attn_common.cuh on the same values
+HARNESS = """
+#include "attn_common.cuh"
+__global__ void pairs(const float* x, float* poly, float* approx, int n) {
+  const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (i + 1 >= n) return;
+  float a = x[i], b = x[i + 1];
+  qb::ex2_poly_f32x2(a, b);
+  poly[i] = a;
+  poly[i + 1] = b;
+  approx[i] = qb::ex2_approx(x[i]);
+  approx[i + 1] = qb::ex2_approx(x[i + 1]);
+}
+extern "C" int run(const float* x, float* poly, float* approx, int n) {
+  pairs<<<(n / 2 + 255) / 256, 256>>>(x, poly, approx, n);
+  return cudaDeviceSynchronize();
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def exponentials(qb, tmp_path_factory):  # noqa: F811
+    """x (f32) -> the polynomial's and ex2.approx's 2^x, by the kernels' own source."""
+    tmp = tmp_path_factory.mktemp("exponentials")
+    (tmp / "pairs.cu").write_text(HARNESS)
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-I", str(CSRC), "-shared", "-Xcompiler", "-fPIC", str(tmp / "pairs.cu"),
+                    "-o", str(tmp / "pairs.so")], check=True, timeout=600)  # fmt: skip
+    lib = ctypes.CDLL(str(tmp / "pairs.so"))
+    lib.run.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int]
+
+    def run(x):
+        assert x.size % 2 == 0
+        xd, poly, approx = T(qb, x, "f32"), qb.QuarkTensor.empty(x.size, dtype="f32"), qb.QuarkTensor.empty(x.size, dtype="f32")
+        qb.runtime.synchronize()
+        assert lib.run(xd.data_ptr(), poly.data_ptr(), approx.data_ptr(), x.size) == 0
+        return poly.to_numpy(), approx.to_numpy()
+
+    return run
+
+
+def test_the_polynomial_is_as_close_as_ex2_approx(exponentials):
+    """Against 64 bits, within the 2^-22 that ex2.approx.f32 is documented to keep, over what scores are narrowed from: up to 2^8, and down to
+    where the result is no longer a normal number."""
+    x = np.concatenate([np.linspace(-125, 8, 1 << 18, dtype=np.float32), np.linspace(-2, 2, 1 << 16, dtype=np.float32), np.arange(-125, 9, 0.5, dtype=np.float32)])
+    poly, _ = exponentials(x)
+    want = np.exp2(x.astype(np.float64))
+    assert np.abs(poly / want - 1).max() <= 2.0**-22
+    np.testing.assert_array_equal(poly[x == np.rint(x)], want[x == np.rint(x)])  # the key that the maximum came from counts exactly 1
+
 
 # a cluster of key splits, one CTA per item, splits through the workspace, helpers
 FORMS = [(12, 12, 8, 2, 11, 0), (12, 12, 8, 2, 11, 1), (12, 12, 8, 2, 11, 16), (8, 8, 16, 5, 240, 0)]
