@@ -503,11 +503,6 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
 #pragma unroll
         for (int c = 0; c < kKeyTile / 32; ++c) p_chunk<kFp8, kLin>(sc[c], sl2_2, nshift_2, kFp8 ? pw[0] + c * 8 : pw[c >> 1] + (c & 1) * 16, sum);
         if (!kFp8) l_run += sum_f32x2(sum[0], sum[1]);
-        if (!kFp8 && valid != kKeyTile) {  // the polynomial makes 2^-126 of -inf: a masked key counts exactly nothing
-#pragma unroll
-          for (int w = 0; w < 64; ++w)
-            if (2 * w + 1 >= valid) pw[kFp8 ? 0 : w >> 5][w & 31] &= 2 * w >= valid ? 0u : 0xFFFFu;
-        }
         if (i > 0) wait_warp(bars->pv_done[g], (i - 1) & 1);  // PV(i - 1) has read the P before: long ago, as a rule
         tmem_st32(tmem_p, pw[0]);
         if constexpr (!kFp8) tmem_st32(tmem_p + 32, pw[1]);

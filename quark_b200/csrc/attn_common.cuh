@@ -210,11 +210,11 @@ __device__ __forceinline__ float sum_f32x2(uint64_t a, uint64_t b) {
 }
 // 2^x for two values on the FMA and integer pipes: x = n + f with n = round(x) in the low mantissa bits of x + 1.5 * 2^23, a
 // polynomial for 2^f on [-0.5, 0.5] (least squares with 2^0 = 1 held, weighted until the relative error is level: 9.1e-8, evaluated in f32
-// 1.7e-7, below the 2^-22 of ex2.approx; a degree less made 2.7e-6 of it), n added to the exponent field.  x is clamped at -126: what
-// underflows becomes 2^-126 instead of 0.
+// 1.7e-7, below the 2^-22 of ex2.approx; a degree less made 2.7e-6 of it), times 2^n.  As with ex2.approx.ftz, NaN stays NaN and what would be
+// below 2^-126, -inf among it, is 0: x is clamped at -127 by a maximum that keeps NaN, and the bits of 2^-127 come out as those of 0.
 __device__ __forceinline__ void ex2_poly_f32x2(float& x0, float& x1) {
-  x0 = fmaxf(x0, -126.0f);
-  x1 = fmaxf(x1, -126.0f);
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(-127.0f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(-127.0f));
   const uint64_t x = pack_f32x2(x0, x1), magic = pack_f32x2(12582912.0f, 12582912.0f), nmagic = pack_f32x2(-12582912.0f, -12582912.0f),
                  none = pack_f32x2(-1.0f, -1.0f);
   uint64_t t, f, p;
@@ -227,11 +227,11 @@ __device__ __forceinline__ void ex2_poly_f32x2(float& x0, float& x1) {
   asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.24022242f, 0.24022242f)));
   asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(0.693147f, 0.693147f)));
   asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(p) : "l"(f), "l"(pack_f32x2(1.0f, 1.0f)));
-  uint32_t t0, t1, p0, p1;
+  uint32_t t0, t1;
   asm("mov.b64 {%0, %1}, %2;" : "=r"(t0), "=r"(t1) : "l"(t));
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(p0), "=r"(p1) : "l"(p));
-  x0 = __uint_as_float(p0 + (t0 << 23));
-  x1 = __uint_as_float(p1 + (t1 << 23));
+  const uint64_t s = pack_f32x2(__uint_as_float((t0 << 23) + 0x3F800000u), __uint_as_float((t1 << 23) + 0x3F800000u));
+  asm("mul.rn.ftz.f32x2 %0, %0, %1;" : "+l"(p) : "l"(s));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(p));
 }
 // Four f32 -> four packed e4m3, joined by the conversions themselves.
 __device__ __forceinline__ uint32_t merge_e4m3x4(float a, float b, float c, float d) {

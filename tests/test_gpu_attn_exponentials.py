@@ -1,5 +1,5 @@
-"""The exponentials of attention: the polynomial is as close as ``ex2.approx``, and e4m3 kernels set to ``ex2.approx`` lose no score that is
-not finite."""
+"""The exponentials of attention: the polynomial is as close as ``ex2.approx``, and neither bf16 kernels nor e4m3 kernels set to ``ex2.approx``
+lose a score that is not finite."""
 
 import ctypes
 import shutil
@@ -67,11 +67,22 @@ def test_the_polynomial_is_as_close_as_ex2_approx(exponentials):
     np.testing.assert_array_equal(poly[x == np.rint(x)], want[x == np.rint(x)])  # the key that the maximum came from counts exactly 1
 
 
+def test_the_polynomial_keeps_nan_and_underflow(exponentials):
+    """What ex2.approx.ftz makes of NaN, of -inf and of what is too small for a normal number, in either place of a pair."""
+    x = np.array([np.nan, -np.inf, -1e30, -127.4, -126.75, -126.5, -126.25, -126.01], np.float32)
+    for at in (0, 1):
+        pairs = np.zeros((x.size, 2), np.float32)
+        pairs[:, at] = x
+        poly, approx = exponentials(pairs.ravel())
+        np.testing.assert_array_equal(poly, approx)
+        assert np.isnan(poly[at]) and (poly.reshape(-1, 2)[1:, at] == 0).all() and (poly.reshape(-1, 2)[:, 1 - at] == 1).all()
+
+
 # a cluster of key splits, one CTA per item, splits through the workspace, helpers
 FORMS = [(12, 12, 8, 2, 11, 0), (12, 12, 8, 2, 11, 1), (12, 12, 8, 2, 11, 16), (8, 8, 16, 5, 240, 0)]
 
 
-@pytest.mark.parametrize("kv_dt", ["e4m3"])
+@pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
 @pytest.mark.parametrize("H,W,Hk,gqa,nb,splits", FORMS)
 def test_a_key_that_is_not_finite_is_seen_at_every_position(qb, kv_dt, H, W, Hk, gqa, nb, splits):  # noqa: F811
     """A KV head holds one bad value in a key at position h of eight, somewhere or among the last keys (where tiles are masked).  NaN: all of the
