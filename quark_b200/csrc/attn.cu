@@ -250,16 +250,18 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
   const uint32_t tmem_base = bars->tmem_slot;
   if (kSplit == kSplitCluster) cluster_arrive();  // this CTA is there (waited for before anyone pushes to it)
 
-  QueryTile q;
-  if (kSplit != kHelped && warp >= 4) q.request_angles(a, q0);
-
-  // Everything above touched only this CTA's shared memory and TMEM, and a table that no kernel writes, so it may run while the kernels
-  // before this one in the stream are still at work; everything below reads what they wrote.
+  // Everything above touched only this CTA's shared memory and TMEM, so it may run while the kernels before this one in the stream are
+  // still at work; everything below reads what they wrote.
   grid_dep_launch();
   grid_dep_wait();
 
-  // The table, the query rows and the frame counter are asked for at once, so that the first K tile is two trips to L2 away.
-  if (kSplit != kHelped && warp >= 4) q.request(a, q0, qh);
+  // The table, the query rows with their angles and the frame counter are asked for at once, so that the first K tile is two trips to L2
+  // away.
+  QueryTile q;
+  if (kSplit != kHelped && warp >= 4) {
+    q.request(a, q0, qh);
+    q.request_angles(a, q0);
+  }
   int seg[6];
   const int nseg = request_table(a, seg);
   const int frame_t = *after_wait(a.frame_t);

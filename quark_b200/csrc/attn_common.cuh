@@ -343,7 +343,7 @@ struct QueryTile {
   float2 c[4], s[4];  // spatial units (0..3): cosines and sines of the two angles of the 4 pairs
 
   __device__ __forceinline__ static int number() { return static_cast<int>(threadIdx.x) - 128; }  // (the softmax warps start at thread 128)
-  // The rows' angles, from a table that no kernel writes.
+  // The rows' angles.  Behind grid_dep_wait like the rows: the table may be the work of a kernel before (qb_rope_table_build).
   __device__ __forceinline__ void request_angles(const AttnArgs& a, int q0) {
     const int n = number(), u = n & 7;
     if (n >= 256 || u >= 4) return;

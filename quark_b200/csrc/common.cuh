@@ -73,8 +73,8 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 // What an earlier kernel of the stream may have written is read with ordinary loads through a pointer that has passed
 // through after_wait(): a read-only load (ld.global.nc: __ldg, or what the compiler makes of a const __restrict__
 // parameter) counts as invariant for the whole kernel, so the compiler may issue it before griddepcontrol.wait, i.e.
-// while the earlier kernel is still writing.  __ldg stays for tables nothing on the device ever writes (RoPE table,
-// weights and their scales).
+// while the earlier kernel is still writing.  __ldg stays for what nothing on the device writes while kernels that read it may be in
+// flight (weights and their scales); the RoPE table is not of these, since qb_rope_table_build writes it.
 template <class T>
 __device__ __forceinline__ T* after_wait(T* p) {
   asm volatile("" : "+l"(p)::"memory");

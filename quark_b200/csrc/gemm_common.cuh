@@ -397,9 +397,9 @@ __device__ __forceinline__ void qkv_fetch(const GemmArgs& g, int et, int row0, i
   if (hd >= BN / 64 || t >= g.M || col >= g.N) return;
   const int kind = qkv_kind(q, col);
   if (kind == 1 && l < 2) {
-    const uint4* rp = reinterpret_cast<const uint4*>(q.rope_xy + static_cast<size_t>(t) * 16);
-    pre[0] = __ldg(rp + l);
-    pre[1] = __ldg(rp + 2 + l);
+    const uint4* rp = reinterpret_cast<const uint4*>(after_wait(q.rope_xy) + static_cast<size_t>(t) * 16);
+    pre[0] = rp[l];
+    pre[1] = rp[2 + l];
   } else if (kind == 2 && q.qkv_first != nullptr) {  // written earlier in this pass
     const uint4* fp = reinterpret_cast<const uint4*>(after_wait(q.qkv_first) + static_cast<size_t>(t) * g.N + col + 16 * l);
     pre[0] = fp[0];

@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(kKvThreads) kv_append_kernel(const KvArgs a) {
     const uint16_t* src = a.k_src + static_cast<size_t>(ts) * a.row_stride + head * a.head_stride + q * kPairs * 2;
     float xy[16];
     {
-      const float4* r = reinterpret_cast<const float4*>(a.rope_xy + static_cast<size_t>(ts) * 16);
-      const float4 r0 = __ldg(r), r1 = __ldg(r + 1), r2 = __ldg(r + 2), r3 = __ldg(r + 3);
+      const float4* r = reinterpret_cast<const float4*>(after_wait(a.rope_xy) + static_cast<size_t>(ts) * 16);
+      const float4 r0 = r[0], r1 = r[1], r2 = r[2], r3 = r[3];
       xy[0] = r0.x; xy[1] = r0.y; xy[2] = r0.z; xy[3] = r0.w; xy[4] = r1.x; xy[5] = r1.y; xy[6] = r1.z; xy[7] = r1.w;
       xy[8] = r2.x; xy[9] = r2.y; xy[10] = r2.z; xy[11] = r2.w; xy[12] = r3.x; xy[13] = r3.y; xy[14] = r3.z; xy[15] = r3.w;
     }

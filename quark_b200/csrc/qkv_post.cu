@@ -125,10 +125,10 @@ __global__ void __launch_bounds__(kPostThreads) qkv_post_kernel(const QkvPostArg
   const uint4 kb = *reinterpret_cast<const uint4*>(a.qkv_in + koff + 8);
   float xy[16];
   {
-    const float4* rp = reinterpret_cast<const float4*>(a.rope_xy + static_cast<size_t>(t) * 16);
+    const float4* rp = reinterpret_cast<const float4*>(after_wait(a.rope_xy) + static_cast<size_t>(t) * 16);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float4 v = __ldg(rp + i);
+      const float4 v = rp[i];
       xy[4 * i] = v.x; xy[4 * i + 1] = v.y; xy[4 * i + 2] = v.z; xy[4 * i + 3] = v.w;
     }
   }

@@ -105,6 +105,47 @@ def test_attention_call_without_a_workspace(qb, kv_dt, Hk, nb):
 
 
 @pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
+@pytest.mark.parametrize("Hk,nb", [(1, 16), (24, 64)])  # key splits in clusters, one CTA per item
+def test_attention_reads_the_table_that_the_kernel_before_it_builds(qb, kv_dt, Hk, nb):
+    """A caller's table made on the device by the call just before, where another grid's table stood: the angles of the finished one."""
+    import ctypes as C
+
+    lib, r, stream = qb._lib.load(), util.rng([94, Hk]), qb.runtime.active_stream()
+    H, W = 8, 32
+    segs, n = ops.compute_segments(500, nb, 256, 1)
+    make = bf16_randn if kv_dt == "bf16" else e4m3_randn
+    qkv, K, V = T(qb, bf16_randn(r, (256, Hk * 4 * 64)), "bf16"), T(qb, make(r, (Hk * (nb + 1) * 256, 64)), kv_dt), T(qb, make(r, (Hk * 64, (nb + 1) * 256)), kv_dt)
+    seg, nseg, ft = T(qb, np.array(segs, np.int32)), T(qb, np.array([n], np.int32)), T(qb, np.array([500], np.int32))
+    table = qb.QuarkTensor.empty(256, 16, dtype="f32")
+    dt = qb._lib.DTYPE_CODE[kv_dt]
+    p = qb._lib.AttnParams(n_kv_heads=Hk, gqa_ratio=2, H_spatial=H, W_spatial=W, num_buckets=nb, pinned_dilation=1, kv_dtype=dt, compute_dtype=dt, max_segments=3,
+                           packed_qkv=1, quilt_factor=1)  # fmt: skip
+
+    def attend(out):
+        qb._lib.check(lib.qb_owl_attn(qkv.data_ptr(), K.data_ptr(), V.data_ptr(), seg.data_ptr(), nseg.data_ptr(), ft.data_ptr(), out.data_ptr(), None,
+                                      table.data_ptr(), C.byref(p), None, 0, stream))  # fmt: skip
+
+    def build(h, w):
+        qb._lib.check(lib.qb_rope_table_build(table.data_ptr(), h, w, stream))
+
+    outs = [T(qb, np.zeros((256, Hk * 2 * 64), np.uint16), "bf16") for _ in range(12)]
+    build(H, W)
+    qb.runtime.synchronize()
+    attend(outs[0])
+    build(W, H)
+    qb.runtime.synchronize()
+    attend(outs[1])
+    for out in outs[2:]:
+        build(W, H)
+        build(H, W)
+        attend(out)
+    got = [o.to_numpy() for o in outs]
+    assert (got[0] != got[1]).any()
+    for g in got[2:]:
+        np.testing.assert_array_equal(g, got[0])
+
+
+@pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
 def test_attention_with_helpers_does_not_depend_on_who_comes_last(qb, kv_dt):
     """The two parts of an item are summed by the CTA that finishes second.  A product on another stream keeps 100 SMs for about 100 us,
     so that the helpers, the last CTAs of the grid, start late: the same bits as alone."""
