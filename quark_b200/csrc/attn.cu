@@ -429,10 +429,8 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
     const uint32_t tmem_s = tmem_base + g * kGroupCols + lane_addr;  // this thread's row of the group's S,
     const uint32_t tmem_o = tmem_s + kOCol, tmem_p = tmem_s + kPCol;  // ... of its O and of its P
 
-    if (g < 2) {
-      asm volatile("bar.sync 4, 288;" ::: "memory");  // the temporal angles
-      q.stage<kFp8>(smem + L::kQOff, bars->tm, &bars->q_ready);
-    }
+    asm volatile("bar.sync 4, 288;" ::: "memory");  // the temporal angles
+    if (kSplit != kHelped || pc.n > 0) q.stage<kFp8>(smem + L::kQOff, bars->tm, &bars->q_ready);  // (else nothing was requested)
     int i0 = 0, i1 = group_tiles(kSplit == kHelped ? pc.n : n_tiles, g);  // the group's tiles of the piece, as the MMA warp counts them
     // What the end of a piece needs is worked out there from its number, so that it takes no registers in the loop.
     int end = pc.n;

@@ -461,7 +461,7 @@ owl_attn3_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
 
     if (g < 2) {
       asm volatile("bar.sync 4, 288;" ::: "memory");  // the temporal angles
-      q.stage<false>(smem + L::kQOff, bars->tm, &bars->q_ready);
+      if (!kHelped || pc.n > 0) q.stage<false>(smem + L::kQOff, bars->tm, &bars->q_ready);  // (else nothing was requested)
     }
     // every segment a multiple of the tile (720p: 512 keys a bucket): no tile needs a mask, so none is looked up
     const bool whole = ((seg[1] | seg[3] | seg[5]) & (kKeyTile - 1)) == 0;

@@ -350,6 +350,7 @@ struct QueryTile {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int t = q0 + (n >> 3) + 32 * i;
+      c[i] = s[i] = make_float2(0.f, 0.f);
       if (t >= a.tpf) continue;
       const float* xy = a.rope_xy + static_cast<size_t>(t) * 16 + 2 * u;
       asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(c[i].x), "=f"(c[i].y) : "l"(xy) : "memory");
