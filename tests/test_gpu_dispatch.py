@@ -85,6 +85,34 @@ def test_attention_groups_over_tiles_whose_maximum_jumps(qb, kv_dt, H, W, ft):
 
 
 @pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
+@pytest.mark.parametrize("H,W,Hk,gqa,nb,ft", [
+    (16, 16, 24, 2, 65, 900),  # 96 items on 148 SMs: owners walk 93 tiles, helpers two pieces of 37
+    (17, 16, 43, 1, 101, 300),  # 129 items: up to seven pieces of 19 a helper, partial tiles of three segments, a query tile of 16 rows
+])  # fmt: skip
+def test_attention_with_helpers_over_tiles_whose_maximum_jumps(qb, kv_dt, H, W, Hk, gqa, nb, ft):
+    """The same keys for CTAs that work on one piece of an item after the other, so that a maximum, a barrier phase or a place in the table
+    left over from the piece before would show.  The oracle, fed and compared as above, computes the heads of three KV heads."""
+    r = util.rng([99, H, Hk])
+    tpf, cap, Hq = H * W, (nb + 1) * H * W, Hk * gqa
+    qkv = ops.head_rmsnorm(bf16_randn(r, (tpf, (Hq + 2 * Hk) * 64)), n_q_heads=Hq, n_kv_heads=Hk)
+    step = np.array([0.3, 6.0, 1.0, 14.0, 0.1, 9.0, 13.0], np.float32)[np.arange(cap) // 128 % 7]
+    to = codec.f32_to_bf16 if kv_dt == "bf16" else codec.f32_to_e4m3
+    one = to(r.standard_normal((cap, 64), dtype=np.float32) * step[:, None]), to(r.standard_normal((64, cap), dtype=np.float32))
+    turn = [int(t) * 16 for t in r.integers(0, cap // 16, Hk)]  # every head another order of the same keys
+    Kc, Vc = np.concatenate([np.roll(one[0], t, 0) for t in turn]), np.concatenate([np.roll(one[1], t, 1) for t in turn])
+    segs, n = ops.compute_segments(ft, nb, tpf, 1)
+    got = qb.qf.owl_attn(T(qb, qkv, "bf16"), T(qb, Kc, kv_dt), T(qb, Vc, kv_dt), T(qb, np.asarray(segs, np.int32)), T(qb, np.array([n], np.int32)), 1, Hk, gqa, H, W, nb, 1,
+                         compute_dtype=kv_dt, packed_qkv=True, frame_t=T(qb, np.array([ft], np.int32))).to_numpy().reshape(tpf, Hq, 64)  # fmt: skip
+    heads = qkv.reshape(tpf, Hq + 2 * Hk, 64)
+    for h in (0, Hk // 2, Hk - 1):
+        mine = np.concatenate([heads[:, h * gqa : (h + 1) * gqa], heads[:, Hq + h : Hq + h + 1], heads[:, Hq + Hk + h : Hq + Hk + h + 1]], 1).reshape(tpf, -1)
+        with codec.bf16_rounding("rne"):
+            want = ops.owl_attn(mine, Kc[h * cap : (h + 1) * cap], Vc[h * 64 : (h + 1) * 64], segs, [n], ft, n_kv_heads=1, gqa_ratio=gqa, H_spatial=H, W_spatial=W,
+                                kv_dtype=kv_dt, q_quant=kv_dt)  # fmt: skip
+        _attn_check(np.ascontiguousarray(got[:, h * gqa : (h + 1) * gqa]).reshape(tpf, -1), want, f"helpers {H}x{W} head {h} {kv_dt}", kv_dt == "e4m3")
+
+
+@pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
 @pytest.mark.parametrize("Hk,nb", [(1, 16), (24, 64)])  # key splits in clusters, one CTA per item (helpers want a workspace)
 def test_attention_call_without_a_workspace(qb, kv_dt, Hk, nb):
     import ctypes as C
