@@ -310,6 +310,11 @@ int32_t qb_owl_attn(const void* qkv, const void* K_cache, const void* Vt_cache, 
  * src/quark/kernels/ada_rmsnorm/reference.py:10-29. */
 int32_t qb_ada_rmsnorm(const void* X, const void* scale, const void* bias, void* out, void* out_q, int32_t rows, int32_t D,
                        int32_t groups, float eps, int32_t activation, void* stream);
+/* The same bytes, for a norm that stands between kernels of another kind in its stream, as in a block's forward pass: with at most
+ * a row per SM it goes through its code once on zeros while it waits for the kernel before it, and the kernel after it may begin its
+ * set-up (constant weights among it) before that one has ended.  Called back to back with itself it is slower than the plain one. */
+int32_t qb_ada_rmsnorm_chained(const void* X, const void* scale, const void* bias, void* out, void* out_q, int32_t rows, int32_t D,
+                               int32_t groups, float eps, int32_t activation, void* stream);
 /* RMS norm of each 64-wide Q and K head of packed qkv [rows, (Hq + 2 Hk) * Dh]; V copied.
  * ref: src/quark/kernels/head_rmsnorm/reference.py:10-26. */
 int32_t qb_head_rmsnorm(const void* X, void* out, int32_t rows, int32_t n_q_heads, int32_t n_kv_heads, int32_t Dh, float eps,

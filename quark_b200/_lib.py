@@ -132,6 +132,7 @@ SIGNATURES = {
     "qb_owl_attn_scratch_bytes": (_Z, [C.POINTER(AttnParams)]),
     "qb_owl_attn": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _P, C.POINTER(AttnParams), _P, _Z, _P]),
     "qb_ada_rmsnorm": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P]),
+    "qb_ada_rmsnorm_chained": (_I, [_P, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P]),
     "qb_rmsnorm": (_I, [_P, _P, _I, _I, _F, _P]),
     "qb_add": (_I, [_P, _P, _P, _Z, _P]),
     "qb_head_rmsnorm": (_I, [_P, _P, _I, _I, _I, _I, _F, _P]),
@@ -196,7 +197,7 @@ def load():
 
 
 # The entry points that csrc/fastcall.c calls by address.
-FASTCALL = ("qb_gemm", "qb_gemm_workspace_bytes", "qb_ada_rmsnorm", "qb_rmsnorm", "qb_head_rmsnorm", "qb_ada_gate_residual", "qb_silu", "qb_add",
+FASTCALL = ("qb_gemm", "qb_gemm_workspace_bytes", "qb_ada_rmsnorm", "qb_ada_rmsnorm_chained", "qb_rmsnorm", "qb_head_rmsnorm", "qb_ada_gate_residual", "qb_silu", "qb_add",
             "qb_euler_step", "qb_quantize_e4m3", "qb_dequantize_e4m3", "qb_kv_cache_update", "qb_kv_cache_update_kv", "qb_owl_attn_scratch_bytes", "qb_owl_attn")  # fmt: skip
 
 

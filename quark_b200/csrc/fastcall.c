@@ -36,6 +36,7 @@ static struct {
   gemm_fn gemm;
   gemm_ws_fn gemm_ws;
   ada_fn ada;
+  ada_fn ada_chained;
   rms_fn rms;
   head_fn head;
   gate_fn gate;
@@ -158,16 +159,16 @@ static PyObject* fast_gemm(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   RUN(g_lib.gemm(A.ptr, B.ptr, C.ptr, bias.ptr, gate.ptr, res.ptr, &p, ws.ptr, (size_t)ws.nbytes, st));
 }
 
-/* (X, scale, bias, eps, activation, out, out_q, only_q, stream) */
+/* (X, scale, bias, eps, activation, out, out_q, only_q, chained, stream) */
 static PyObject* fast_ada_rmsnorm(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   Tensor X, sc, bi, out, oq;
   float eps;
   void* st;
-  if (n != 9 || g_lib.ada == NULL || !tensor(a[0], &X) || !tensor(a[1], &sc) || !tensor(a[2], &bi) || !as_float(a[3], &eps) || !tensor_or_none(a[5], &out) ||
-      !tensor_or_none(a[6], &oq) || !stream_of(a[8], &st))
+  if (n != 10 || g_lib.ada == NULL || !tensor(a[0], &X) || !tensor(a[1], &sc) || !tensor(a[2], &bi) || !as_float(a[3], &eps) || !tensor_or_none(a[5], &out) ||
+      !tensor_or_none(a[6], &oq) || !stream_of(a[9], &st))
     Py_RETURN_NONE;
   const int act = activation_of(a[4]), only_q = a[7] == Py_True;
-  if (a[7] != Py_True && a[7] != Py_False) Py_RETURN_NONE;
+  if ((a[7] != Py_True && a[7] != Py_False) || (a[8] != Py_True && a[8] != Py_False)) Py_RETURN_NONE;
   if (only_q) out.ptr = NULL;
   if (act < 0 || (only_q ? oq.ptr == NULL : out.ptr == NULL) || X.dtype != QB_BF16 || sc.dtype != QB_BF16 || bi.dtype != QB_BF16) Py_RETURN_NONE;
   const long long D = dim(&X, -1);
@@ -176,7 +177,8 @@ static PyObject* fast_ada_rmsnorm(PyObject* self, PyObject* const* a, Py_ssize_t
   if (!SMALL(rows) || !SMALL(G) || sc.numel != G * D || bi.numel != G * D || rows % G != 0) Py_RETURN_NONE;
   if (out.ptr != NULL && (out.numel != X.numel || out.dtype != X.dtype)) Py_RETURN_NONE;
   if (oq.ptr != NULL && (oq.numel != X.numel || oq.dtype != QB_E4M3)) Py_RETURN_NONE;
-  RUN(g_lib.ada(X.ptr, sc.ptr, bi.ptr, out.ptr, oq.ptr, (int32_t)rows, (int32_t)D, (int32_t)G, eps, act, st));
+  const ada_fn call = a[8] == Py_True ? g_lib.ada_chained : g_lib.ada;
+  RUN(call(X.ptr, sc.ptr, bi.ptr, out.ptr, oq.ptr, (int32_t)rows, (int32_t)D, (int32_t)G, eps, act, st));
 }
 
 /* (X, eps, out, stream) */
@@ -354,11 +356,11 @@ static PyObject* fast_bind(PyObject* self, PyObject* args) {
     }
     *at[i] = ((PyMemberDescrObject*)d)->d_member->offset;
   }
-  static const char* const names[15] = {"qb_gemm", "qb_gemm_workspace_bytes", "qb_ada_rmsnorm", "qb_rmsnorm", "qb_head_rmsnorm", "qb_ada_gate_residual",
+  static const char* const names[16] = {"qb_gemm", "qb_gemm_workspace_bytes", "qb_ada_rmsnorm", "qb_ada_rmsnorm_chained", "qb_rmsnorm", "qb_head_rmsnorm", "qb_ada_gate_residual",
                                         "qb_silu", "qb_add", "qb_euler_step", "qb_quantize_e4m3", "qb_dequantize_e4m3", "qb_kv_cache_update",
                                         "qb_kv_cache_update_kv", "qb_owl_attn_scratch_bytes", "qb_owl_attn"};
   void** const fn = (void**)&g_lib;
-  for (int i = 0; i < 15; ++i) {
+  for (int i = 0; i < 16; ++i) {
     PyObject* v = PyDict_GetItemString(table, names[i]);
     if (v == NULL) {
       PyErr_Format(PyExc_KeyError, "bind: %s", names[i]);

@@ -39,9 +39,10 @@ __device__ __forceinline__ void round_through_bf16(float (&f)[8]) {
 // Latency bounds it (0.5 MB in and out at 128 rows): the wait for the kernel before, one trip to L2, a reduction.  A part of it
 // was fetching the instructions behind the wait, which run once per launch after other kernels have had the caches.  With
 // kRehearse a CTA therefore goes through them once on zeros, storing nothing, while it waits for the kernel before it, and lets the
-// next kernel begin its set-up before that.  Taken where there is at most a row per SM: a frame of 128 tokens, d 2048, bf16
-// 6.08 -> 5.93 ms, 100 x 8192 back to back 3.1 -> 2.95 us; with more rows the CTAs of an SM share one fetch and most start late,
-// so that the rehearsal holds them up (512 tokens bf16 14.81 -> 14.89 ms).  A warp of its own for the rehearsal instead: 6.01 ms,
+// next kernel begin its set-up before that.  Taken where the caller says that the call stands between kernels of another kind
+// (qb_ada_rmsnorm_chained: behind a kernel of its own kind there is nothing to fetch, and it only makes the call longer, 128 x 2048
+// 2.81 -> 2.96 us) and there is at most a row per SM: a frame of 128 tokens, d 2048, bf16 6.08 -> 5.93 ms; with more rows the CTAs of
+// an SM share one fetch and most start late, so that the rehearsal holds them up (512 tokens bf16 14.81 -> 14.89 ms).  A warp of its own for the rehearsal instead: 6.01 ms,
 // four 5.96; the early set-up without it 6.02.
 template <int kThreads, int kMaxVec, bool kRehearse>
 __global__ void __launch_bounds__(kThreads, kMaxVec == 1 ? 4 : 2) ada_rmsnorm_kernel(const uint16_t* X, const uint16_t* scale,
@@ -871,8 +872,8 @@ int32_t qb_quantize_e4m3_rows(const void* X, void* out, float* scale_out, int32_
   return check_launch("quantize_e4m3_rows");
 }
 
-int32_t qb_ada_rmsnorm(const void* X, const void* scale, const void* bias, void* out, void* out_q, int32_t rows, int32_t D,
-                       int32_t groups, float eps, int32_t activation, void* stream) {
+static int32_t ada_rmsnorm(const void* X, const void* scale, const void* bias, void* out, void* out_q, int32_t rows, int32_t D, int32_t groups, float eps, int32_t activation,
+                           bool chained, void* stream) {
   QB_REQUIRE(X && scale && bias && (out || out_q), QB_ERR_INVALID_ARG, "ada_rmsnorm: NULL pointer (out may be NULL only when out_q is given)");
   QB_REQUIRE(rows > 0 && D > 0 && groups > 0 && rows % groups == 0, QB_ERR_INVALID_ARG, "ada_rmsnorm: rows %d, D %d, groups %d", rows, D,
              groups);
@@ -880,13 +881,23 @@ int32_t qb_ada_rmsnorm(const void* X, const void* scale, const void* bias, void*
   QB_REQUIRE(activation == 0 || activation == 1, QB_ERR_INVALID_ARG, "ada_rmsnorm: activation %d", activation);
   QB_REQUIRE(aligned16(X) && aligned16(scale) && aligned16(bias) && aligned16(out) && aligned16(out_q), QB_ERR_ALIGN,
              "ada_rmsnorm: pointers must be 16-byte aligned");
-  const bool rehearse = rows <= num_sms();  // see the kernel
+  const bool rehearse = chained && rows <= num_sms();  // see the kernel
   auto kernel = D <= 2048   ? (rehearse ? ada_rmsnorm_kernel<256, 1, true> : ada_rmsnorm_kernel<256, 1, false>)
                 : D <= 4096 ? (rehearse ? ada_rmsnorm_kernel<256, 2, true> : ada_rmsnorm_kernel<256, 2, false>)
                             : (rehearse ? ada_rmsnorm_kernel<256, 4, true> : ada_rmsnorm_kernel<256, 4, false>);
   return launch_dep("ada_rmsnorm", kernel, dim3(rows), dim3(256), 0, static_cast<cudaStream_t>(stream),
                     static_cast<const uint16_t*>(X), static_cast<const uint16_t*>(scale), static_cast<const uint16_t*>(bias),
                     static_cast<uint16_t*>(out), static_cast<uint8_t*>(out_q), D, rows / groups, eps, activation);
+}
+
+int32_t qb_ada_rmsnorm(const void* X, const void* scale, const void* bias, void* out, void* out_q, int32_t rows, int32_t D,
+                       int32_t groups, float eps, int32_t activation, void* stream) {
+  return ada_rmsnorm(X, scale, bias, out, out_q, rows, D, groups, eps, activation, false, stream);
+}
+
+int32_t qb_ada_rmsnorm_chained(const void* X, const void* scale, const void* bias, void* out, void* out_q, int32_t rows, int32_t D,
+                               int32_t groups, float eps, int32_t activation, void* stream) {
+  return ada_rmsnorm(X, scale, bias, out, out_q, rows, D, groups, eps, activation, true, stream);
 }
 
 int32_t qb_head_rmsnorm(const void* X, void* out, int32_t rows, int32_t n_q_heads, int32_t n_kv_heads, int32_t Dh, float eps,

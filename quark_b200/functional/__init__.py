@@ -629,14 +629,15 @@ def _bf16_only(who, *ts):
             raise TypeError(f"{who}: dtype {_dt(t)!r} (expected bf16)")
 
 
-def ada_rmsnorm(X, scale, bias, eps: float = 1e-6, activation: str | None = None, *, out=None, out_q=None, only_q: bool = False):
+def ada_rmsnorm(X, scale, bias, eps: float = 1e-6, activation: str | None = None, *, out=None, out_q=None, only_q: bool = False, chained: bool = False):
     """``rmsnorm(x) * (1 + scale) + bias`` (+ SiLU) (``src/quark/functional/ada_rmsnorm.py:61``).
 
     ``out_q`` (extension): an e4m3 tensor that also receives the result, for a following fp8 GEMM; with ``only_q`` the
-    bf16 result is not written at all (``out_q`` is returned).
+    bf16 result is not written at all (``out_q`` is returned).  ``chained=True`` (extension) says that the call stands between
+    kernels of another kind, as in a block; the result is the same (``qb_ada_rmsnorm_chained``).
     """
     if out is not None or only_q:
-        rc = _fast.ada_rmsnorm(X, scale, bias, eps, activation, out, out_q, only_q, _s())
+        rc = _fast.ada_rmsnorm(X, scale, bias, eps, activation, out, out_q, only_q, chained, _s())
         if rc is not None:
             if rc:
                 _lib.check(rc)
@@ -654,9 +655,8 @@ def ada_rmsnorm(X, scale, bias, eps: float = 1e-6, activation: str | None = None
     out = None if only_q else _like(X, out, "qf.ada_rmsnorm")
     if out_q is not None and (out_q.dtype != "e4m3" or out_q.numel != X.numel):
         raise ValueError("qf.ada_rmsnorm: out_q must be an e4m3 tensor of the same size")
-    _lib.check(
-        _lib.load().qb_ada_rmsnorm(_p(X), _p(scale), _p(bias), _p(out), _p(out_q), rows, D, G, float(eps), 1 if activation == "silu" else 0, _s())
-    )
+    call = _lib.load().qb_ada_rmsnorm_chained if chained else _lib.load().qb_ada_rmsnorm
+    _lib.check(call(_p(X), _p(scale), _p(bias), _p(out), _p(out_q), rows, D, G, float(eps), 1 if activation == "silu" else 0, _s()))
     return out_q if only_q else out
 
 

@@ -326,7 +326,7 @@ class TransformerBlock(nn.Module):
             raise ValueError("TransformerBlock: tp_world > 1 needs a communicator of that size and rank")
         self._cond_lut: list[tuple] = []
         nq, nk = cfg.n_heads_local, cfg.n_kv_heads_local  # heads of this rank
-        self.pre_attn_norm = nn.AdaRMSNorm()
+        self.pre_attn_norm = nn.AdaRMSNorm(chained=True)
         self.qkv_proj = nn.Linear(d, cfg.qkv_dim_local, out_dtype="bf16")
         self.head_norm = nn.HeadRMSNorm(nq, nk, cfg.Dh)
         if cfg.value_residual:
@@ -350,7 +350,7 @@ class TransformerBlock(nn.Module):
             self.ctrl_x_norm = nn.RMSNorm()
             self.ctrl_emb_norm = nn.RMSNorm()
             self.ctrl_residual = nn.Add()
-        self.pre_mlp_norm = nn.AdaRMSNorm()
+        self.pre_mlp_norm = nn.AdaRMSNorm(chained=True)
         if cfg.moe:
             self.mlp = nn.MoE(cfg.tpf, d, cfg.mlp_dim // cfg.moe_top_k, cfg.moe_n_experts, cfg.moe_top_k, routing=cfg.moe_routing)
         else:
@@ -464,7 +464,7 @@ class Waypoint15(nn.Module):
         ph, pw = cfg.patch
         self.patchify = nn.Patchify(cfg.channels, cfg.d_model, cfg.height * ph, cfg.width * pw, ph, pw)
         self.blocks = nn.ModuleList([TransformerBlock(cfg, i, comm) for i in range(cfg.n_layers)])
-        self.out_norm = nn.AdaRMSNorm()
+        self.out_norm = nn.AdaRMSNorm(chained=True)
         self.unpatchify = nn.Unpatchify(cfg.d_model, cfg.channels, cfg.height * ph, cfg.width * pw, ph, pw)
         if cfg.ctrl_conditioning:
             self.ctrl_emb = nn.ControllerInputEmbedding(cfg.n_buttons, cfg.d_model, cfg.mlp_ratio, out_dtype="bf16")

@@ -280,12 +280,16 @@ class MLP(Module):
 
 
 class AdaRMSNorm(Module):
-    """Stateless ``rmsnorm(x) * (1 + scale) + bias`` (``layers.py:609-619``)."""
+    """Stateless ``rmsnorm(x) * (1 + scale) + bias`` (``layers.py:609-619``).  ``chained``: the layer runs between others of a model (see
+    ``qf.ada_rmsnorm``)."""
+
+    def __init__(self, chained: bool = False):
+        self.chained = chained
 
     def forward(self, x, scale, bias, *, activation=None, emit_e4m3: bool = False):
         if emit_e4m3:  # the bf16 copy has no reader: only the e4m3 result is written
-            return qf.ada_rmsnorm(x, scale, bias, activation=activation, out_q=_cached(self, "out_q", x.shape, "e4m3"), only_q=True)
-        return qf.ada_rmsnorm(x, scale, bias, activation=activation, out=_cached(self, "out", x.shape, x.dtype))
+            return qf.ada_rmsnorm(x, scale, bias, activation=activation, out_q=_cached(self, "out_q", x.shape, "e4m3"), only_q=True, chained=self.chained)
+        return qf.ada_rmsnorm(x, scale, bias, activation=activation, out=_cached(self, "out", x.shape, x.dtype), chained=self.chained)
 
 
 class RMSNorm(Module):

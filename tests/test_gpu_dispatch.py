@@ -546,3 +546,22 @@ def test_ada_rmsnorm_rows_and_widths(qb, rows, D):
     # in a chain each call waits for the one before it
     again = qb.qf.ada_rmsnorm(qb.qf.ada_rmsnorm(*args), *args[1:]).to_numpy()
     assert np.percentile(util.bf16_ulp_diff(again, ops.ada_rmsnorm(got, s, b)), 99.9) <= 1
+
+
+@pytest.mark.parametrize("rows", [1, 148, 149])  # a chained call rehearses with up to a row per SM
+@pytest.mark.parametrize("D", [8, 2056, 8192])
+def test_ada_rmsnorm_between_other_kernels_gives_the_same_bytes(qb, rows, D):
+    r = util.rng([93, rows, D])
+    args = T(qb, bf16_randn(r, (rows, D)), "bf16"), T(qb, bf16_randn(r, (1, D), 0.1), "bf16"), T(qb, bf16_randn(r, (1, D), 0.1), "bf16")
+    for kw in ({}, dict(activation="silu")):
+        want, want_q = qb.qf.ada_rmsnorm(*args, **kw).to_numpy(), qb.QuarkTensor.empty(rows, D, dtype="e4m3")
+        qb.qf.ada_rmsnorm(*args, out_q=want_q, only_q=True, **kw)
+        # made by Python (an output to be allocated) and in C, behind a kernel that writes its input
+        x, q = qb.QuarkTensor.zeros(rows, D, dtype="bf16"), qb.QuarkTensor.empty(rows, D, dtype="e4m3")
+        zero = qb.QuarkTensor.zeros(rows, D, dtype="bf16")
+        qb.qf.add(args[0], zero, out=x)
+        got = qb.qf.ada_rmsnorm(x, *args[1:], chained=True, **kw)
+        qb.qf.add(args[0], zero, out=x)
+        qb.qf.ada_rmsnorm(x, *args[1:], out_q=q, only_q=True, chained=True, **kw)
+        np.testing.assert_array_equal(got.to_numpy(), want)
+        np.testing.assert_array_equal(q.to_numpy(), want_q.to_numpy())
