@@ -518,7 +518,7 @@ owl_attn_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__
         more = n > 0;
         continue;
       }
-      more = kSplit == kHelped;
+      more = false;
 
       float o[64];
 #pragma unroll

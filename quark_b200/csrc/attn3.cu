@@ -143,57 +143,57 @@ __device__ __forceinline__ void softmax_tiles(uint8_t* smem, uint32_t tmem_base,
   uint64_t* next_turn = &bars->turn[g == kGroups - 1 ? 0 : g + 1][quarter];
   int i = (j0 - g + kGroups - 1) / kGroups;  // the group's tiles are j = 3 i + g
   for (int j = kGroups * i + g; j < j1; j += kGroups, ++i) {
-          wait_warp(bars->s_full[g], i & 1);
-          tc_fence_after();
-          int row, valid = kKeyTile;
-          if (!whole) locate_tile(bars->seg, j + bars->tile_shift, row, valid);  // (the table is there: Q was staged after it)
-          uint32_t s0[32];
-          const float m_tile = (valid == kKeyTile ? row_max<false>(ts, valid, s0) : row_max<true>(ts, valid, s0)) * sl2;
-          // m is settled tile by tile: after the turn it is what the tiles before this one left
-          if (j > 0) {
-            wait_warp(*my_turn, g == 0 ? (i - 1) & 1 : i & 1);
-          }
-          float m = *my_m;
-          if (j == j0) {
-            m = m_tile;
-            *my_m = m;
-          } else {
-            const bool jump = m_tile > m + kSlack;
-            if (__any_sync(0xffffffffu, jump)) {
-              // O may be rescaled only when PV(j - 1) has finished.  (S(j - 1) was issued after PV(j - 4), so the barrier is in the
-              // phase of tile j - 1 or has finished it.)
-              const int gp = g == 0 ? kGroups - 1 : g - 1, ip = g == 0 ? i - 1 : i;
-              wait_warp(bars->pv_done[gp], ip & 1);
-              const float old = m;
-              if (jump) m = m_tile;
-              const float alpha = ex2_approx(old - m);
-              tc_fence_after();
+    wait_warp(bars->s_full[g], i & 1);
+    tc_fence_after();
+    int row, valid = kKeyTile;
+    if (!whole) locate_tile(bars->seg, j + bars->tile_shift, row, valid);  // (the table is there: Q was staged after it)
+    uint32_t s0[32];
+    const float m_tile = (valid == kKeyTile ? row_max<false>(ts, valid, s0) : row_max<true>(ts, valid, s0)) * sl2;
+    // m is settled tile by tile: after the turn it is what the tiles before this one left
+    if (j > 0) {
+      wait_warp(*my_turn, g == 0 ? (i - 1) & 1 : i & 1);
+    }
+    float m = *my_m;
+    if (j == j0) {
+      m = m_tile;
+      *my_m = m;
+    } else {
+      const bool jump = m_tile > m + kSlack;
+      if (__any_sync(0xffffffffu, jump)) {
+        // O may be rescaled only when PV(j - 1) has finished.  (S(j - 1) was issued after PV(j - 4), so the barrier is in the
+        // phase of tile j - 1 or has finished it.)
+        const int gp = g == 0 ? kGroups - 1 : g - 1, ip = g == 0 ? i - 1 : i;
+        wait_warp(bars->pv_done[gp], ip & 1);
+        const float old = m;
+        if (jump) m = m_tile;
+        const float alpha = ex2_approx(old - m);
+        tc_fence_after();
 #pragma unroll 1
-              for (int c = 0; c < 4; ++c) {
-                uint32_t oo[16];
-                tmem_ld16(tmem_o + c * 16, oo);
-                tmem_wait_ld_into(oo);
+        for (int c = 0; c < 4; ++c) {
+          uint32_t oo[16];
+          tmem_ld16(tmem_o + c * 16, oo);
+          tmem_wait_ld_into(oo);
 #pragma unroll
-                for (int q = 0; q < 16; ++q) oo[q] = __float_as_uint(__uint_as_float(oo[q]) * alpha);
-                tmem_st16(tmem_o + c * 16, oo);
-              }
-              uint32_t lsum = tmem_ld1(tmem_o + 64);
-              tmem_wait_ld();
-              tmem_loaded(lsum);
-              tmem_st1(tmem_o + 64, __float_as_uint(__uint_as_float(lsum) * alpha));
-              tmem_wait_st();
-              tc_fence_before();
-              if (jump) *my_m = m;
-            }
-          }
-          warp_arrive(smem_u32(next_turn), lane);
-          const float nshift = -m;
-          if (valid == kKeyTile) row_exp<false>(ts, valid, sl2, nshift, s0);
-          else row_exp<true>(ts, valid, sl2, nshift, s0);
-          tmem_wait_st();
-          tc_fence_before();
-          warp_arrive(smem_u32(&bars->p_full[g]), lane);
+          for (int q = 0; q < 16; ++q) oo[q] = __float_as_uint(__uint_as_float(oo[q]) * alpha);
+          tmem_st16(tmem_o + c * 16, oo);
         }
+        uint32_t lsum = tmem_ld1(tmem_o + 64);
+        tmem_wait_ld();
+        tmem_loaded(lsum);
+        tmem_st1(tmem_o + 64, __float_as_uint(__uint_as_float(lsum) * alpha));
+        tmem_wait_st();
+        tc_fence_before();
+        if (jump) *my_m = m;
+      }
+    }
+    warp_arrive(smem_u32(next_turn), lane);
+    const float nshift = -m;
+    if (valid == kKeyTile) row_exp<false>(ts, valid, sl2, nshift, s0);
+    else row_exp<true>(ts, valid, sl2, nshift, s0);
+    tmem_wait_st();
+    tc_fence_before();
+    warp_arrive(smem_u32(&bars->p_full[g]), lane);
+  }
 }
 
 // The same as a function of its own, for the kernel with helpers: inlined there, its registers and order changed with whatever surrounded
@@ -485,7 +485,7 @@ owl_attn3_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant_
         more = n > 0;
         continue;
       }
-      more = kHelped;
+      more = false;
 
       // ---------------- the CTA's result: 64 outputs, still scaled by 2^-m, and the row sum in column 64
       if (g < 2) {  // 32 of the outputs each

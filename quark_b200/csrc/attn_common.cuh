@@ -69,6 +69,22 @@ __host__ __device__ inline int owned_tiles(int items, int sms, int tiles, int co
 }
 constexpr int kHelperCost = 9;
 
+// Outputs of a query row (divided by the row sum already) and their e4m3 copy, narrowed from the bf16-rounded values: it equals a
+// separate cast.
+template <int kN>
+__device__ __forceinline__ void write_out(const AttnArgs& a, size_t at, const float (&o)[kN]) {
+#pragma unroll
+  for (int v = 0; v < kN / 8; ++v) {
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(o[8 * v + 2 * q], o[8 * v + 2 * q + 1]);
+    *reinterpret_cast<uint4*>(a.out + at + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+    if (a.out_q != nullptr)
+      *reinterpret_cast<uint2*>(a.out_q + at + v * 8) = make_uint2(pack_e4m3x4(bf16lo(w[0]), bf16hi(w[0]), bf16lo(w[1]), bf16hi(w[1])),
+                                                                   pack_e4m3x4(bf16lo(w[2]), bf16hi(w[2]), bf16lo(w[3]), bf16hi(w[3])));
+  }
+}
+
 struct KeyShares {
   int tiles = 0, keep = 0, items = 0, first_item = 0, last_item = 0;  // this CTA's items: [first_item, last_item)
   bool helper = false;
@@ -98,16 +114,10 @@ struct KeyShares {
     const float vs = a.v_scale ? __ldg(a.v_scale + kvh) : 1.0f;
     const float inv = l > 0.f ? vs / l : 0.f;
     const size_t at = static_cast<size_t>(t) * a.o_row + static_cast<size_t>(qh) * a.o_head;
+    float y[64];
 #pragma unroll
-    for (int v = 0; v < 8; ++v) {
-      uint32_t w[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(o[8 * v + 2 * q] * inv, o[8 * v + 2 * q + 1] * inv);
-      *reinterpret_cast<uint4*>(a.out + at + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-      if (a.out_q != nullptr)  // narrowed from the bf16-rounded values: equals a separate bf16 -> e4m3 cast
-        *reinterpret_cast<uint2*>(a.out_q + at + v * 8) = make_uint2(pack_e4m3x4(bf16lo(w[0]), bf16hi(w[0]), bf16lo(w[1]), bf16hi(w[1])),
-                                                                     pack_e4m3x4(bf16lo(w[2]), bf16hi(w[2]), bf16lo(w[3]), bf16hi(w[3])));
-    }
+    for (int d = 0; d < 64; ++d) y[d] = o[d] * inv;
+    write_out(a, at, y);
   }
 
   // The 128 threads of group 0, one row each: writes the rows of a whole item; otherwise leaves them in the workspace and, as the
@@ -432,22 +442,6 @@ __device__ __forceinline__ void read_o(uint32_t tmem_o, float (&o)[64], float& l
 #pragma unroll
   for (int d = 0; d < 64; ++d) o[d] = __uint_as_float(oo[d >> 5][d & 31]);
   if (kSum) l = __uint_as_float(lsum);
-}
-
-// 32 outputs of a query row (divided by the row sum already) and their e4m3 copy, narrowed from the bf16-rounded values: it equals a
-// separate cast.
-template <int kN>
-__device__ __forceinline__ void write_out(const AttnArgs& a, size_t at, const float (&o)[kN]) {
-#pragma unroll
-  for (int v = 0; v < kN / 8; ++v) {
-    uint32_t w[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) w[q] = pack_bf16x2(o[8 * v + 2 * q], o[8 * v + 2 * q + 1]);
-    *reinterpret_cast<uint4*>(a.out + at + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-    if (a.out_q != nullptr)
-      *reinterpret_cast<uint2*>(a.out_q + at + v * 8) = make_uint2(pack_e4m3x4(bf16lo(w[0]), bf16hi(w[0]), bf16lo(w[1]), bf16hi(w[1])),
-                                                                   pack_e4m3x4(bf16lo(w[2]), bf16hi(w[2]), bf16lo(w[3]), bf16hi(w[3])));
-  }
 }
 
 // The shared memory of a kernel, once per device (`done`: a bit per device).
