@@ -390,6 +390,12 @@ SFU_EXP_PER_CLK_PER_SM = 16  # ex2.approx.f32: one warp instruction per 8 cycles
 N_SMS = 148
 
 
+def sfu_share(kv_dtype):
+    """Which share of attention's exponentials the special-function unit makes: the others come from the FMA pipe (every second one in
+    e4m3, none with exact exponentials; every fourth in bf16)."""
+    return 0.75 if kv_dtype == "bf16" else 1.0 if os.environ.get("QB_ATTN_EXACT_EXP", "")[:1] == "1" else 0.5
+
+
 def max_over_ranks(values, dist, device="cpu"):
     """Element-wise maximum of a list of floats over all ranks (identity without a process group)."""
     if dist is None:
@@ -608,12 +614,13 @@ def run_ours(args):
         dom = max(("owl_attn", "gemm_qkv", "gemm_out", "gemm_fc1", "gemm_fc2"), key=lambda k: kernels[k]["us_per_launch"])
         gemm_us = sum(kernels[k]["us_per_launch"] for k in ("gemm_qkv", "gemm_out", "gemm_fc1", "gemm_fc2"))
         dk = kernels[dom]
-        # head_dim 64 leaves 256 tensor flops per exponential: the attention kernel is bound by the
-        # special-function unit long before the tensor pipe; report that roofline beside the contract's one
+        # head_dim 64 leaves 256 tensor flops per exponential: the special-function unit is a roofline of the attention
+        # kernel long before the tensor pipe; report the time of the exponentials that go there beside the contract's one
         exps = cfg.tpf * cfg.n_heads * kernels["owl_attn"]["keys_attended_mean"]
+        sfu_exps = exps * sfu_share("e4m3")
         sm_hz = (clocks.summary().get("sm_mhz") or 1965.0) * 1e6
-        floor_us = exps / (SFU_EXP_PER_CLK_PER_SM * N_SMS * sm_hz) * 1e6
-        sfu = {"exponentials_per_launch": int(exps), "floor_us": round(floor_us, 2),
+        floor_us = sfu_exps / (SFU_EXP_PER_CLK_PER_SM * N_SMS * sm_hz) * 1e6
+        sfu = {"exponentials_per_launch": int(exps), "of_these_on_the_unit": int(sfu_exps), "floor_us": round(floor_us, 2),
                "frac": round(floor_us / kernels["owl_attn"]["us_per_launch"], 3)}
         traffic, traffic_src = dram_traffic_from_profiles()
         line = {
@@ -783,7 +790,7 @@ def run_attn_sweep(args):
                 rows.append({"kv": kv_dt, "buckets": nb, "frame_t": ft, "segments": int(n), "keys": S, "us": round(us, 1),
                              "tflops": round(flops / us / 1e6, 1), "tensor_frac": round(flops / us / 1e6 / tensor_peak, 3),
                              "gbs": round(byts / us / 1e3, 1), "hbm_frac": round(byts / us / 1e3 / peaks["hbm_gbs"], 3),
-                             "sfu_frac": round(tpf * 32 * S / (SFU_EXP_PER_CLK_PER_SM * N_SMS * 1.965e9) * 1e6 / us, 3)})  # fmt: skip
+                             "sfu_frac": round(sfu_share(kv_dt) * tpf * 32 * S / (SFU_EXP_PER_CLK_PER_SM * N_SMS * 1.965e9) * 1e6 / us, 3)})  # fmt: skip
             del Kc, Vc
     print(json.dumps({"attn_sweep_720p": rows, "device_status": qb._lib.device_status(), "peaks": peaks}), flush=True)
 
