@@ -27,7 +27,7 @@
 // instructions and nothing else takes 726 cycles per tile, with one warp per scheduler 911; this kernel 1040, the waits, fences and
 // arrivals of a tile being what the other warp covers in part only.  Before (47.8 us at 16 buckets, 318 at 128, 168 at 64), a stage of
 // the one K / V ring was held from S to PV, so the MMA threads waited 850 to 1350 cycles per tile for K, and P went through shared
-// memory with the groups taking turns on the exponentials; now 41.4, 264 and 142 us.  Tried and dropped: the turns kept (46.0); a third
+// memory with the groups taking turns on the exponentials; now 41.4, 272 and 143 us.  Tried and dropped: the turns kept (46.0); a third
 // group of warps for the maxima (50.3: S, maximum, exponentials in a row take longer than the tile before covers); three groups over
 // 64-key tiles (46.9: the fixed work of a tile twice); the chord's integer multiply-add held on the FMA pipe (42.9).
 #include <atomic>

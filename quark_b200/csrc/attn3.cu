@@ -21,11 +21,13 @@
 // hence three groups.  A loop with the same softmax instructions and nothing else takes 965 cycles per tile with three warps per
 // scheduler (1180 with all exponentials on the special-function unit), this kernel 1330.  The K and V rings are separate and the loads
 // run ahead of the S that runs ahead of the PV: with one ring a stage was held from S to PV, and the next K tiles came too late.
-// 720p, us per launch: 60.4 -> 52.9 at 16 buckets, 211 -> 204 at 64, 394 -> 382 at 128.
+// 720p, us per launch: 56.8 -> 53.6 at 16 buckets, 211 -> 208 at 64, 404 -> 393 at 128, 792 -> 745 at 256.
 // Tried and dropped: a whole m (P's rounding is then the same for every m, but the key that m came from no longer has a probability of
 // exactly 1: 8 % more error); e4m3 in this form (44.5 against 42.0 us at 720p); key splits in this form (360p bf16 12.8 against 13.5 us,
 // but one m for all keys of a CTA makes 2 % more error than one per group); kSlack 8 (52.4 against 53.8 us at 720p, 3 % more error
-// where few keys count).
+// where few keys count); kSlack 2, 1, 0 (84, 91, 100 us against 54 on rows that drift: a rescale waits for the PV before it).
+// Error against 64 bits, this kernel over three accumulators with an m each (161fee8): keys N(0, 1) 1.000 (16 buckets) to 1.003 (128, one
+// accumulator taking the rounding of all additions), rows where few keys count 0.997 to 1.007.
 #include <atomic>
 
 #include <cuda.h>
@@ -197,7 +199,7 @@ __device__ __forceinline__ void softmax_tiles(uint8_t* smem, uint32_t tmem_base,
 }
 
 // The same as a function of its own, for the kernel with helpers: inlined there, its registers and order changed with whatever surrounded
-// it (368 to 399 us at 128 buckets).  The kernel without is faster with it inlined (52.5 against 55.3 us at 16).
+// it (368 to 399 us at 128 buckets).  A tile takes a fifth longer in it (owned_tiles).  The kernel without is faster with it inlined (52.5 against 55.3 us at 16).
 __device__ __noinline__ void softmax_tiles_apart(uint8_t* smem, uint32_t tmem_base, unsigned* status, float sl2, int j0, int j1, bool whole) {
   softmax_tiles(smem, tmem_base, status, sl2, j0, j1, whole);
 }

@@ -58,7 +58,10 @@ struct Piece {
 // over are helpers that take the last tiles of up to `per` items each, one item after the other.  `cost` is what a piece costs a helper
 // on top of its tiles (the query tile, O, the trip of the partial result through the workspace), in tiles.  Where less than
 // the meeting of the two parts would be saved (a session's first frames, or 720p's ring of 16 buckets) the item stays whole.
-// 720p, 512 queries x 32 heads (20 helpers of up to 7 items), 128 buckets, e4m3: 264 us; cost 5 to 30 was tried.
+// 720p, 512 queries x 32 heads (20 helpers of up to 7 items), 64 / 128 / 256 buckets, e4m3: 143, 272, 517 us,
+// with the items whole 150, 295, 577; cost 12 149 at 64, the rest alike; cost 16 and more loses up to 9 %.  bf16: 208, 392, 745 us and whole
+// 192, 372, 721, since a tile takes a fifth longer in its kernel with helpers; kept, because two accumulators share the
+// additions (error at 128 buckets over that of three accumulators, keys N(0, 1): 0.3 against 0.4 % more, few keys that count: 0.4 against 0.8).
 // The owners of the items that share a K / V head still walk its keys side by side, and so do the helpers, one after the other: equal
 // ranges of the row of all tiles (every CTA the end of one item and the start of the next) balance better but read each key from
 // DRAM once per query tile and head (720p, 128 buckets: 339 us against 344 unsplit).

@@ -87,13 +87,20 @@ def test_attention_groups_over_tiles_whose_maximum_jumps(qb, kv_dt, H, W, ft):
 @pytest.mark.parametrize("kv_dt", ["bf16", "e4m3"])
 @pytest.mark.parametrize("H,W,Hk,gqa,nb,ft", [
     (16, 16, 24, 2, 65, 900),  # 96 items on 148 SMs: owners walk 93 tiles, helpers two pieces of 37
-    (17, 16, 43, 1, 101, 300),  # 129 items: up to seven pieces of 19 a helper, partial tiles of three segments, a query tile of 16 rows
+    (17, 16, 39, 1, 127, 300),  # 117 items: up to four pieces of 47 a helper, partial tiles of three segments, a query tile of 16 rows
+    (17, 16, 43, 1, 101, 300),  # 129 items: up to seven pieces of 19 a helper
 ])  # fmt: skip
 def test_attention_with_helpers_over_tiles_whose_maximum_jumps(qb, kv_dt, H, W, Hk, gqa, nb, ft):
     """The same keys for CTAs that work on one piece of an item after the other, so that a maximum, a barrier phase or a place in the table
     left over from the piece before would show.  The oracle, fed and compared as above, computes the heads of three KV heads."""
+    import ctypes as C
+
     r = util.rng([99, H, Hk])
     tpf, cap, Hq = H * W, (nb + 1) * H * W, Hk * gqa
+    dt = qb._lib.DTYPE_CODE[kv_dt]
+    p = qb._lib.AttnParams(n_kv_heads=Hk, gqa_ratio=gqa, H_spatial=H, W_spatial=W, num_buckets=nb, pinned_dilation=1, kv_dtype=dt, compute_dtype=dt, max_segments=3,
+                           packed_qkv=1, quilt_factor=1)  # fmt: skip
+    assert qb._lib.load().qb_owl_attn_scratch_bytes(C.byref(p)) > 0  # there are helpers
     qkv = ops.head_rmsnorm(bf16_randn(r, (tpf, (Hq + 2 * Hk) * 64)), n_q_heads=Hq, n_kv_heads=Hk)
     step = np.array([0.3, 6.0, 1.0, 14.0, 0.1, 9.0, 13.0], np.float32)[np.arange(cap) // 128 % 7]
     to = codec.f32_to_bf16 if kv_dt == "bf16" else codec.f32_to_e4m3
