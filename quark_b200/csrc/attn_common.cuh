@@ -278,7 +278,7 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw64(uint32_t smem_addr) {
 // 8192-key rows the output's 1 - cosine against exact arithmetic goes from 3.6e-4 to 4.3e-4 at worst).  x is clamped at -120 (the result then
 // narrows to zero).  Every second probability of a row is built this way in the kLin instantiations of the e4m3 kernel
 // (the default; qb_set_attn_exact_exp(1) or QB_ATTN_EXACT_EXP=1 selects the instantiations without it): the exponentials no longer queue
-// behind one another at the special-function unit.  Measured at 720p, 8320 keys, us per launch: 41.4 against 51.6 without.
+// behind one another at the special-function unit.  Measured at 720p, 8320 keys, us per launch: 41.4 against 57.0 without.
 constexpr float kLinMagic = 49152.0f;  // 1.5 * 2^15: floats in [2^15, 2^16) have an ulp of 2^-8
 // (The clamp is a maximum on the ALU pipe, the busiest one of the kernel at 58 %; moving it to the FMA pipe as a
 // saturating multiply-add followed by a second multiply-add costs one instruction more and measured 49.5 against 46.5 us:
